@@ -16,6 +16,8 @@ _DTYPES = {"fp32": torch.float32, "bf16": torch.bfloat16, "fp16": torch.float16}
 # and the multiply-adds of a step, no more than the largest listed cases of either kind.
 _MAX_TENSOR = (1 << 23, 1.2e12)
 _MAX_OTHER = (1 << 20, 1.2e10)
+# Multiply-adds of one contraction above which ``exact`` gives no value (about 20 seconds).
+_MAX_EXACT = 1 << 38
 
 
 def _case(op, B, N, H, W, C, ks, dtype, packed=False, scaled=True):
@@ -152,6 +154,63 @@ def work(case):
     if case["op"].startswith("forward"):
         return {"bytes": 4 * t + stat, "flops": 2 * mac}
     return {"bytes": 12 * t + 2 * stat, "flops": 7 * mac}
+
+
+def _window_index(n, ks):
+    """(n, ks) indices of each position's window on an axis of n, shifted inwards at the borders."""
+    start = (torch.arange(n) - ks // 2).clamp(0, n - ks)
+    return (start[:, None] + torch.arange(ks)).cuda()
+
+
+def _exact_units(q, k, v, d_o, rows, cols, scale):
+    """(o, dQ, dK, dV) in 64 bits for (units, H, W, C) operands; the gradients are None without d_o."""
+    U, H, W, C = q.shape
+    q, k, v = q.double(), k.double(), v.double()
+    offsets = [(a, b) for a in range(rows.shape[1]) for b in range(cols.shape[1])]
+    flat = [(rows[:, a, None] * W + cols[None, :, b]).flatten() for a, b in offsets]
+    k_flat, v_flat = k.reshape(U, H * W, C), v.reshape(U, H * W, C)
+    q_flat = q.reshape(U, H * W, C)
+    scores = torch.stack([(q_flat * k_flat[:, i]).sum(-1) for i in flat], -1)
+    p = torch.softmax(scores.mul_(scale), -1)
+    o = torch.zeros_like(q_flat)
+    for j, i in enumerate(flat):
+        o += p[..., j, None] * v_flat[:, i]
+    if d_o is None:
+        return o.view(U, H, W, C), None, None, None
+    g = d_o.double().reshape(U, H * W, C)
+    ds = torch.stack([(g * v_flat[:, i]).sum(-1) for i in flat], -1)
+    ds = p * (ds - (p * ds).sum(-1, keepdim=True)) * scale
+    d_q, d_k, d_v = torch.zeros_like(o), torch.zeros_like(o), torch.zeros_like(o)
+    for j, i in enumerate(flat):
+        d_q += ds[..., j, None] * k_flat[:, i]
+        d_k.index_add_(1, i, ds[..., j, None] * q_flat)
+        d_v.index_add_(1, i, p[..., j, None] * g)
+    return tuple(t.view(U, H, W, C) for t in (o, d_q, d_k, d_v))
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits by plain torch; the unfused pair and the fused
+    operator have the same value.  None for the few cases that would take too long."""
+    B, N, H, W, C, ks = (case[n] for n in ("B", "N", "H", "W", "C", "ks"))
+    if _pixels(case) * _taps(case) * C > _MAX_EXACT:
+        return None
+    state = prepare(case, seed)
+    qkv, d_o = state["qkv"], state.get("d_o")
+    q, k, v = (qkv.permute(3, 0, 4, 1, 2, 5).unbind(0) if case["packed"] else qkv)
+    out_shape = q.shape
+    units = [None if t is None else t.detach().reshape(B * N, H, W, C) for t in (q, k, v, d_o)]
+    rows = _window_index(H, 1 if case["op"].endswith("1d") else ks)
+    cols = _window_index(W, ks)
+    scale = C ** -0.5 if case["scaled"] else 1.0
+    step = max(1, (1 << 26) // (H * W * C))
+    parts = [_exact_units(*(None if t is None else t[u:u + step] for t in units), rows, cols, scale)
+             for u in range(0, B * N, step)]
+    o, *grads = (None if t[0] is None else torch.cat(t).view(out_shape) for t in zip(*parts))
+    if d_o is None:
+        return {"o": o}
+    if case["packed"]:
+        grads = [torch.stack(grads).permute(1, 3, 4, 0, 2, 5)]
+    return {"o": o, **{f"grad{i}": g for i, g in enumerate(grads)}}
 
 
 def tolerance(case):
