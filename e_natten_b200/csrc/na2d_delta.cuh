@@ -4,7 +4,7 @@
 // and o was rounded when stored), a few 1e-2 at most.  That is too coarse to form dS from directly
 // - the error would enter every dS of the row - but it is all the dQ kernel of the larger windows
 // needs to walk its key box once instead of twice: it forms dS from the estimate and corrects
-// the result exactly at the end (see na2d_tc_bwd.cuh).
+// the result exactly at the end (see na2d_tc_dq2.cuh).
 //
 // C / 8 lanes per query pixel, each lane one 16-byte piece of the two rows; a block covers
 // 256 / (C / 8) consecutive pixels of one (batch, head) image, so a warp's loads are whole rows

@@ -8,18 +8,11 @@
 //     dS = p (dP - delta)  -> tensor memory, 16 bit        (head + residual on the bf16 path)
 //     dQ += dS K_c                                         (dS read from tensor memory; the softmax
 //                                                           scale is applied to the finished dQ)
-// delta needs every chunk of the tile before any dS can be formed exactly.  With one chunk (kernel
-// sizes up to 5: at most 256 keys) a tile is a single unit and dQ reuses the S columns.  With
-// several chunks there are two ways:
-//   * one walk with a correction.  The caller hands in an estimate d~ of delta (dO . o from the
-//     stored output, see na2d_delta.cuh; off by the rounding of o, a few 1e-2 at most).  Every
-//     unit forms dS~ = p (dP - d~), adds dS~ K_c to dQ and, with one more MMA, p K_c to a
-//     second accumulator B, while the exact delta = sum_j p dP builds up in registers.  Since
-//     sum_j p (dP - delta) k = sum_j p (dP - d~) k - (delta - d~) sum_j p k, the epilogue stores
-//     scale (dQ - (delta - d~) B).  B only meets the small factor (delta - d~), so a single 16-bit
-//     p is enough for it.  The exact delta is what the kernel writes out for the dK/dV kernel.
-//   * two walks (no estimate given): units 0..NCH-1 only add up delta, units NCH..2NCH-1 repeat
-//     the two score MMAs and accumulate dQ.
+// delta needs every chunk of the tile before any dS can be formed.  With one chunk (kernel sizes up to 5: at most
+// 256 keys) a tile is a single unit and dQ reuses the S columns.  With several chunks this kernel walks them
+// twice: units 0..NCH-1 only add up delta, units NCH..2NCH-1 repeat the two score MMAs and accumulate dQ.
+// The calls it is left with are those without the forward's output (na2d_tc_dq2.cuh walks once with it) and
+// those that want delta alone.
 // Twelve warps: 0-7 softmax (warps w and w+4 share 32 queries and split the 16-column blocks),
 // 8 TMA producer, 9 MMA issue, 10-11 idle (register donors).
 #pragma once
@@ -40,10 +33,8 @@ struct DqCfg : Cfg<D, KS, dq_nmax(D, KS)> {
     static constexpr int TMEM_S = 0;
     static constexpr int TMEM_DP = NMAX;
     static constexpr int TMEM_DQ = ONE ? 0 : 2 * NMAX;                 // one chunk: dQ reuses the S columns
-    static constexpr int TMEM_BK = ONE ? 0 : 2 * NMAX + D;             // sum_j p k (several chunks only)
     static constexpr int TMEM_DSH = TMEM_DP;                           // dS (head) over dP
     static constexpr int TMEM_RES = ONE ? 384 : 0;                     // dS residual: upper dP half / lower half of S
-    static constexpr int TMEM_PH = B::NKP / 2;                         // p (head): upper half of S (several chunks only)
     static constexpr int OUT_BYTES = 8 * OutStage<D / 2>::BYTES;       // output staging of the 8 softmax warps
     static constexpr int FIXED = 2 * B::Q_BYTES + OUT_BYTES + 2 * 2 * 128 * 4 /*delta exchange*/ + 256 + 1024;
     // K and V chunk rings: two stages each where they fit, so that a chunk's loads run under the
@@ -53,7 +44,7 @@ struct DqCfg : Cfg<D, KS, dq_nmax(D, KS)> {
     static constexpr int NB16 = (B::NKP + 15) / 16;
     static_assert(SMEM <= kSmemLimit, "dQ kernel shared memory");
     static_assert(B::NKP <= NMAX, "tensor memory layout");
-    static_assert(ONE || TMEM_BK + D <= 512, "tensor memory layout");
+    static_assert(ONE || TMEM_DQ + D <= 512, "tensor memory layout");
     static_assert(!SPLIT || !ONE || B::NKP / 2 <= 128, "residual operand does not fit");
     static_assert((B::NKP / 2) % 8 == 0, "operand halves start on a block boundary");
 };
@@ -63,7 +54,7 @@ __global__ void __launch_bounds__(384, 1)
 dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
           const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* __restrict__ delta,
-          const float* __restrict__ delta_in, const int want_dq_arg, unsigned int* __restrict__ err_word,
+          const int want_dq_arg, unsigned int* __restrict__ err_word,
           const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = DqCfg<D, KS, SPLIT>;
@@ -149,10 +140,8 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
         bn = t / tiles_r;
     };
     // A unit u of a tile works on chunk u % NCH.  Units from first_ds on form dS and add to dQ; the
-    // units before it (a first walk, only when no estimate of delta is given) add up delta.
-    // Without a dQ output only the delta units run.
-    const bool given = !C::ONE && want_dq && delta_in != nullptr;      // one walk with the correction
-    const int first_ds = (C::ONE || given) ? 0 : NCH;
+    // units before it (the first walk) add up delta.  Without a dQ output only the delta units run.
+    constexpr int first_ds = C::ONE ? 0 : NCH;
     const int units_run = want_dq ? first_ds + NCH : NCH;
 
     if (warp == 8) {
@@ -267,12 +256,6 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                             umma_ts(tmem_base + C::TMEM_DQ, tmem_base + C::TMEM_RES + 8 * kk,
                                     desc64(hi, km_lo + ((kk * 16 * C::ROWB) >> 4)), idesc_o, 1u);
                     }
-                    if (given) {                                 // B (+)= p K_c
-#pragma unroll
-                        for (int kk = 0; kk < C::NKP / 16; ++kk)
-                            umma_ts(tmem_base + C::TMEM_BK, tmem_base + C::TMEM_PH + 8 * kk,
-                                    desc64(hi, km_lo + ((kk * 16 * C::ROWB) >> 4)), idesc_o, acc | (kk > 0));
-                    }
                     umma_commit(k_empty + st);
                     if (u == units_run - 1) umma_commit(dq_full);
                     NA2D_TR(2, 4, n);
@@ -311,15 +294,11 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
             const float lse2 = lse[qi] * kLog2e;
             float dl_part = 0.f;                             // this half's part of delta
             float dl = 0.f;                                  // delta, once every chunk has been seen
-            // The estimate is read before this tile's first partner barrier and the exact value
-            // written (by the partner warp of half 0, to the same address when delta_in == delta)
-            // after its last one, so the read never sees the new value.
-            const float d_est = given ? delta_in[qi] : 0.f;
 
             for (int u = 0; u < units_run; ++u, ++n) {
                 const int ch = u % NCH;
                 const bool forms_ds = want_dq && u >= first_ds;
-                const bool adds_delta = C::ONE || given || u < NCH;
+                const bool adds_delta = u < NCH;
                 const int row_off = ch * C::RC;
                 const int j_lo = max(wr_lo - row_off, 0) * C::HW;
                 const int j_hi = min(min(wr_hi + KS - row_off, C::RC) * C::HW, C::NK);       // exclusive
@@ -392,9 +371,7 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                     continue;
                 }
 
-                // dS = p (dP - delta) as packed 16-bit pairs (head, and residual on the bf16 path);
-                // with the one-walk scheme delta is the estimate, and p goes along as a third operand
-                const float dlu = given ? d_est : dl;
+                // dS = p (dP - delta) as packed 16-bit pairs (head, and residual on the bf16 path)
 #pragma unroll
                 for (int a = 0; a < NACT; ++a) {
                     const int blk = half + 2 * (bi_lo + a);
@@ -403,20 +380,14 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
 #pragma unroll
                         for (int e2 = 0; e2 < 8; ++e2) {
                             const float ds0 = ((vmask[a] >> (2 * e2)) & 1u)
-                                ? __uint_as_float(s[a][2 * e2]) * (__uint_as_float(dp[a][2 * e2]) - dlu) : 0.f;
+                                ? __uint_as_float(s[a][2 * e2]) * (__uint_as_float(dp[a][2 * e2]) - dl) : 0.f;
                             const float ds1 = ((vmask[a] >> (2 * e2 + 1)) & 1u)
-                                ? __uint_as_float(s[a][2 * e2 + 1]) * (__uint_as_float(dp[a][2 * e2 + 1]) - dlu) : 0.f;
+                                ? __uint_as_float(s[a][2 * e2 + 1]) * (__uint_as_float(dp[a][2 * e2 + 1]) - dl) : 0.f;
                             wd[e2] = pack2<DT>(ds0, ds1);
                             wr2[e2] = SPLIT ? pack2_residual_bf16(ds0, ds1, wd[e2]) : 0u;
                         }
                         tmem_st_32x8(tmem_lane + C::TMEM_DSH + 8 * blk, wd);
                         if (SPLIT) tmem_st_32x8(tmem_lane + C::TMEM_RES + 8 * blk, wr2);
-                        if (given) {                             // p of masked columns is an exact zero
-#pragma unroll
-                            for (int e2 = 0; e2 < 8; ++e2)
-                                wd[e2] = pack2<DT>(__uint_as_float(s[a][2 * e2]), __uint_as_float(s[a][2 * e2 + 1]));
-                            tmem_st_32x8(tmem_lane + C::TMEM_PH + 8 * blk, wd);
-                        }
                     }
                 }
                 {   // own blocks outside the range hold zeros
@@ -427,7 +398,6 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                         if (!in_range && 16 * blk < C::NKP) {
                             tmem_st_32x8(tmem_lane + C::TMEM_DSH + 8 * blk, z);
                             if (SPLIT) tmem_st_32x8(tmem_lane + C::TMEM_RES + 8 * blk, z);
-                            if (given) tmem_st_32x8(tmem_lane + C::TMEM_PH + 8 * blk, z);
                         }
                     }
                 }
@@ -448,19 +418,6 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
                 for (int piece = 0; piece < DH / 16; ++piece)
                     tmem_ld_32x16(tmem_lane + C::TMEM_DQ + half * DH + 16 * piece,
                                   *reinterpret_cast<uint32_t(*)[16]>(&acc[16 * piece]));
-                if (given) {
-                    // dQ - (delta - estimate) B, piece by piece
-                    const float corr = dl - d_est;
-#pragma unroll
-                    for (int piece = 0; piece < DH / 16; ++piece) {
-                        uint32_t bk[16];
-                        tmem_ld_32x16(tmem_lane + C::TMEM_BK + half * DH + 16 * piece, bk);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            acc[16 * piece + e] = __float_as_uint(fmaf(-corr, __uint_as_float(bk[e]), __uint_as_float(acc[16 * piece + e])));
-                    }
-                }
                 tmem_ld_wait();
                 tc_fence_before();
                 __syncwarp();
@@ -488,10 +445,13 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
 template <typename DT, int D, int KS>
 int launch_dq(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
               const TensorArg& d_o, const TensorArg& d_q, float* delta, const float* delta_in) {
-    // kernel sizes 3 and 5 with a dQ output go to the strip kernel; this one keeps the larger
-    // windows and the delta-only call
+    // kernel sizes 3 and 5 with a dQ output go to the strip kernel, larger ones with an estimate of delta to the
+    // pipelined kernel; this one keeps two walks and the delta-only call
     if constexpr (KS <= 5) {
         if (d_q.ptr != nullptr) return launch_dq1<DT, D, KS>(lc, q, k, v, lse, d_o, d_q, delta);
+    } else {
+        if (d_q.ptr != nullptr && delta_in != nullptr)
+            return launch_dq2<DT, D, KS>(lc, q, k, v, lse, d_o, d_q, delta, delta_in);
     }
     using C = DqCfg<D, KS, IsBf16<DT>::value>;
     const Na2dGeom& g = lc.g;
@@ -510,7 +470,7 @@ int launch_dq(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, delta_in, d_q.ptr != nullptr, lc.err_word, g,
+    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, d_q.ptr != nullptr, lc.err_word, g,
                                         tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
