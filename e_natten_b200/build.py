@@ -3,9 +3,9 @@
     python e_natten_b200/build.py [--force] [--verbose]
 
 The library is plain CUDA C++ behind a C ABI (include/na2d.h); it needs no framework headers.
-Its kernels are compiled as seven translation units in parallel (the API with the SIMT kernels,
-and each of the three tcgen05 kernel families once per 16-bit element type) and linked into one
-shared object.
+Its kernels are compiled as ten translation units in parallel (the API with the SIMT kernels, the
+tiled CUDA-core kernels once per element type, and each of the three tcgen05 kernel families once per
+16-bit element type) and linked into one shared object.
 """
 from __future__ import annotations
 
@@ -22,6 +22,9 @@ LIB_PATH = os.path.join(PKG_DIR, "libna2d.so")
 # (source, extra defines, object name)
 UNITS = [
     ("na2d_api.cu", [], "na2d_api.o"),
+    ("na2d_tile.cu", ["-DNA2D_TILE_DT=0"], "na2d_tile_f32.o"),
+    ("na2d_tile.cu", ["-DNA2D_TILE_DT=1"], "na2d_tile_bf16.o"),
+    ("na2d_tile.cu", ["-DNA2D_TILE_DT=2"], "na2d_tile_f16.o"),
     ("na2d_tc_fwd.cu", ["-DNA2D_TC_DT=1"], "na2d_tc_fwd_bf16.o"),
     ("na2d_tc_fwd.cu", ["-DNA2D_TC_DT=2"], "na2d_tc_fwd_f16.o"),
     ("na2d_tc_dq.cu", ["-DNA2D_TC_DT=1"], "na2d_tc_dq_bf16.o"),

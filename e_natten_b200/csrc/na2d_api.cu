@@ -14,6 +14,7 @@
 #include "na2d_index.cuh"
 #include "na2d_simt.cuh"
 #include "na2d_tc_entry.h"
+#include "na2d_tile_entry.h"
 
 namespace {
 
@@ -287,6 +288,15 @@ int after_launch() {
     return NA2D_OK;
 }
 
+na2d_tile::Tensor tile(const Tensor& t) { return na2d_tile::Tensor{t.ptr, t.st}; }
+
+// Status of a tiled-kernel launcher that makes `launches` launches.
+int after_tile(int rc, int launches) {
+    if (rc == NA2D_OK) g_launches.fetch_add(launches);
+    if (rc == NA2D_ERR_CUDA) return cuda_fail(cudaGetLastError(), "tiled kernel launch");
+    return rc;
+}
+
 na2d_tc::TensorArg targ(const Tensor& t) { return na2d_tc::TensorArg{t.ptr, t.st}; }
 
 int launch_ctx(const Problem& p, int* launched, na2d_tc::LaunchCtx* lc) {
@@ -310,6 +320,11 @@ int run_forward(const Problem& p) {
         g_launches.fetch_add(launched);
         if (rc == NA2D_ERR_CUDA) return tc_fail("tcgen05 forward launch");
         return rc;
+    }
+    if (na2d_tile::supported(g.ks)) {
+        const auto run = p.dtype == NA2D_F32 ? na2d_tile::forward_f32
+                         : p.dtype == NA2D_BF16 ? na2d_tile::forward_bf16 : na2d_tile::forward_f16;
+        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.o), p.lse), 1);
     }
     unsigned grid = 0;
     int rc = grid_for(g.BN, g.Hq, g.W, g.patch, &grid);

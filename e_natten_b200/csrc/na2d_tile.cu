@@ -1,0 +1,80 @@
+// Launchers of the tiled CUDA-core kernels for one element type.
+#include "na2d_tile_entry.h"
+
+#include <type_traits>
+
+#include "../../include/na2d.h"
+#include "na2d_tile.cuh"
+
+#if NA2D_TILE_DT == 0
+using Elem = float;
+#define NA2D_NAME(f) f##_f32
+#elif NA2D_TILE_DT == 1
+using Elem = __nv_bfloat16;
+#define NA2D_NAME(f) f##_bf16
+#else
+using Elem = __half;
+#define NA2D_NAME(f) f##_f16
+#endif
+
+namespace na2d_tile {
+namespace {
+
+template <int V> using IntTag = std::integral_constant<int, V>;
+template <bool V> using BoolTag = std::integral_constant<bool, V>;
+
+// Four neighbouring channels can be moved at once: rows start on a boundary of four elements and hold a
+// multiple of four.
+Operand operand(const Tensor& t, int C) {
+    const size_t quad = 4 * sizeof(Elem);
+    const bool vec = reinterpret_cast<uintptr_t>(t.ptr) % quad == 0 && C % 4 == 0 && t.st.b % 4 == 0 && t.st.n % 4 == 0 &&
+                     t.st.h % 4 == 0 && t.st.w % 4 == 0;
+    return Operand{t.ptr, t.st, vec ? 1 : 0};
+}
+
+// Calls f(kernel size tag, one-row tag).
+template <typename F>
+int by_window(const Na2dGeom& g, F&& f) {
+    auto with = [&](auto ks) -> int { return g.kh == 1 ? f(ks, BoolTag<true>{}) : f(ks, BoolTag<false>{}); };
+    switch (g.ks) {
+        case 3: return with(IntTag<3>{});
+        case 5: return with(IntTag<5>{});
+        case 7: return with(IntTag<7>{});
+        case 9: return with(IntTag<9>{});
+        case 11: return with(IntTag<11>{});
+        case 13: return with(IntTag<13>{});
+        default: return NA2D_ERR_UNSUPPORTED;
+    }
+}
+
+template <typename S>
+int tiles(const Na2dGeom& g, int H, unsigned* n) {
+    const long long t = (long long)g.BN * ((H + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw);
+    if (t > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
+    *n = (unsigned)t;
+    return NA2D_OK;
+}
+
+template <typename... P, typename... A>
+int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return NA2D_ERR_CUDA;
+    kernel<<<grid, threads, smem, st>>>(static_cast<P>(args)...);
+    return cudaPeekAtLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
+}
+
+}  // namespace
+
+int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+                       const Tensor& o, float* lse) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        unsigned n = 0;
+        if (int rc = tiles<S>(g, g.Hq, &n)) return rc;
+        return launch(fwd_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+                      operand(v, g.C), operand(o, g.C), lse, g);
+    });
+}
+
+}  // namespace na2d_tile

@@ -1,0 +1,29 @@
+// Host entry points of the tiled CUDA-core kernels, compiled in one translation unit per element type
+// (na2d_tile.cu with -DNA2D_TILE_DT=0 fp32, 1 bf16, 2 fp16).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "na2d_index.cuh"
+
+namespace na2d_tile {
+
+// A tensor as the caller describes it, strides resolved.
+struct Tensor {
+    void* ptr;
+    Na2dStride st;
+};
+
+// Kernel sizes the tiled kernels are built for.
+inline bool supported(int ks) { return ks == 3 || ks == 5 || ks == 7 || ks == 9 || ks == 11 || ks == 13; }
+
+// Status: 0, NA2D_ERR_TOO_LARGE (grid), or NA2D_ERR_CUDA (the launch's error is left for cudaGetLastError).
+#define NA2D_TILE_ENTRIES(suffix)                                                                                     \
+    int forward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,       \
+                         const Tensor& o, float* lse);
+NA2D_TILE_ENTRIES(f32)
+NA2D_TILE_ENTRIES(bf16)
+NA2D_TILE_ENTRIES(f16)
+#undef NA2D_TILE_ENTRIES
+
+}  // namespace na2d_tile
