@@ -39,7 +39,8 @@ class Args(C.Structure):
                 ("flags", C.c_int), ("scale", C.c_float), ("stream", C.c_void_p), ("rows", C.POINTER(Rows)),
                 ("q", TensorDesc), ("k", TensorDesc), ("v", TensorDesc), ("o", TensorDesc),
                 ("d_o", TensorDesc), ("d_q", TensorDesc), ("d_k", TensorDesc), ("d_v", TensorDesc),
-                ("lse", C.c_void_p), ("delta", C.c_void_p)]
+                ("lse", C.c_void_p), ("delta", C.c_void_p),
+                ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)]
 
 
 OP_2D, OP_1D = 0, 1
@@ -69,6 +70,7 @@ SIGNATURES = {
     "na2d_backward_dq_ex": (C.c_int, [C.POINTER(Args)]),
     "na2d_backward_dkdv_ex": (C.c_int, [C.POINTER(Args)]),
     "na2d_backward_ex": (C.c_int, [C.POINTER(Args)]),
+    "na2d_backward_workspace": (C.c_size_t, [C.POINTER(Args)]),
     "na1d_forward": (C.c_int, [C.c_void_p] * 5 + [C.c_int] * 6 + [C.c_int, C.c_void_p]),
     "na1d_backward": (C.c_int, [C.c_void_p] * 10 + [C.c_int] * 6 + [C.c_int, C.c_void_p]),
     "na2d_qk_forward": (C.c_int, [C.c_void_p] * 3 + _PAIR),

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -175,11 +176,14 @@ int simt_patch(long long BN, int H, int W) {
     return na2d_simt::patch_count(BN, H, W, na2d_simt::kPatch) < 2 * 148 ? na2d_simt::kPatchSmall : na2d_simt::kPatch;
 }
 
+// na2d_args without the workspace fields, which callers built against an earlier header do not have.
+constexpr size_t kArgsBase = offsetof(na2d_args, workspace);
+
 // `key_side`: the call is the key half of the backward, whose key band may be any part of the image
 // (each key sums over whichever local queries see it); the other calls need a key band that holds
 // every window of the query band.
 int make_problem(const na2d_args* a, Problem* out, bool key_side = false) {
-    if (!a || a->struct_size < sizeof(na2d_args)) return NA2D_ERR_BAD_ARG;
+    if (!a || a->struct_size < kArgsBase) return NA2D_ERR_BAD_ARG;
     const int B = a->B, N = a->N, H = a->H, W = a->W, C = a->C, ks = a->kernel_size, dtype = a->dtype, path = a->path;
     if (B <= 0 || N <= 0 || H <= 0 || W <= 0 || C <= 0) return NA2D_ERR_BAD_ARG;
     if (ks <= 0 || (ks & 1) == 0) return NA2D_ERR_BAD_ARG;
@@ -290,6 +294,10 @@ int after_launch() {
 
 na2d_tile::Tensor tile(const Tensor& t) { return na2d_tile::Tensor{t.ptr, t.st}; }
 
+// The launcher of the element type.
+#define NA2D_TILE_PICK(dtype, name) \
+    ((dtype) == NA2D_F32 ? na2d_tile::name##_f32 : (dtype) == NA2D_BF16 ? na2d_tile::name##_bf16 : na2d_tile::name##_f16)
+
 // Status of a tiled-kernel launcher that makes `launches` launches.
 int after_tile(int rc, int launches) {
     if (rc == NA2D_OK) g_launches.fetch_add(launches);
@@ -322,8 +330,7 @@ int run_forward(const Problem& p) {
         return rc;
     }
     if (na2d_tile::supported(g.ks)) {
-        const auto run = p.dtype == NA2D_F32 ? na2d_tile::forward_f32
-                         : p.dtype == NA2D_BF16 ? na2d_tile::forward_bf16 : na2d_tile::forward_f16;
+        const auto run = NA2D_TILE_PICK(p.dtype, forward);
         return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.o), p.lse), 1);
     }
     unsigned grid = 0;
@@ -385,6 +392,10 @@ int run_backward_dq(const Problem& p) {
         if (rc == NA2D_ERR_CUDA) return tc_fail("tcgen05 dQ launch");
         return rc;
     }
+    if (na2d_tile::supported(g.ks)) {
+        const auto run = NA2D_TILE_PICK(p.dtype, backward_dq);
+        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), p.lse, p.delta), 1);
+    }
     unsigned grid = 0;
     int rc = grid_for(g.BN, g.Hq, g.W, g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -422,6 +433,28 @@ int run_backward_dkdv(const Problem& p) {
             p.d_k.ptr, p.d_v.ptr, p.dkdv_f32 ? 1 : 0, p.q.st, p.k.st, p.v.st, p.d_o.st, p.d_k.st, p.d_v.st, g);
         return after_launch();
     });
+}
+
+// What na2d_backward_workspace asks for at most, unless a single unit needs more: a launch over that many
+// weights (2 x 64 M) fills the GPU many times over, so taking the units in several turns costs nothing.
+constexpr long long kWorkspaceBytes = 512ll << 20;
+
+// Bytes of workspace with which the backward keeps P and dS of one (batch, head) unit for its key half, or 0
+// where it has no use for one: the tensor-core kernels form them again, faster than they could be read, and row
+// views and fp32 partial sums stay with the kernels that take them.
+long long workspace_per_unit(const Problem& p, const na2d_args* a) {
+    if (p.tensor || a->rows || p.dkdv_f32 || !na2d_tile::supported(p.g.ks)) return 0;
+    return na2d_tile::workspace_floats(p.g) * (long long)sizeof(float);
+}
+
+// Both halves of the backward where they share a workspace of `units` units.
+int run_backward_shared(const Problem& p, void* workspace, int units) {
+    const auto run = NA2D_TILE_PICK(p.dtype, backward);
+    int launches = 0;
+    const int rc = run(p.g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), tile(p.d_k), tile(p.d_v), p.lse,
+                       p.delta, (float*)workspace, units, &launches);
+    g_launches.fetch_add(launches);
+    return after_tile(rc, 0);
 }
 
 // Validate, select the device, check it; then run `step`.
@@ -622,10 +655,33 @@ int na2d_backward_dkdv_ex(const na2d_args* a) {
     return enter(a, [](const Problem& p) { return run_backward_dkdv(p); }, /*key_side=*/true);
 }
 
+size_t na2d_backward_workspace(const na2d_args* a) {
+    Problem p;
+    if (make_problem(a, &p) != NA2D_OK) return 0;
+    const long long per_unit = workspace_per_unit(p, a);
+    if (per_unit == 0) return 0;
+    long long units = kWorkspaceBytes / per_unit;
+    if (units < 1) units = 1;
+    return (size_t)(per_unit * (units < p.g.BN ? units : p.g.BN));
+}
+
 int na2d_backward_ex(const na2d_args* a) {
     if (!a) return NA2D_ERR_BAD_ARG;
     if ((a->d_k.ptr == nullptr) != (a->d_v.ptr == nullptr)) return NA2D_ERR_BAD_ARG;
     if (!a->d_q.ptr && !a->d_k.ptr) return NA2D_ERR_BAD_ARG;
+    if (a->d_k.ptr && a->struct_size >= sizeof(na2d_args) && a->workspace) {
+        if (!a->q.ptr || !a->k.ptr || !a->v.ptr || !a->lse || !a->d_o.ptr || !a->delta) return NA2D_ERR_BAD_ARG;
+        if (reinterpret_cast<uintptr_t>(a->workspace) % 16) return NA2D_ERR_BAD_ARG;
+        bool shared = false;
+        const int rc = enter(a, [&](const Problem& p) -> int {
+            const long long per_unit = workspace_per_unit(p, a);
+            const long long units = per_unit ? (long long)(a->workspace_bytes / per_unit) : 0;
+            if (units < 1) return NA2D_OK;
+            shared = true;
+            return run_backward_shared(p, a->workspace, (int)(units < p.g.BN ? units : p.g.BN));
+        });
+        if (rc != NA2D_OK || shared) return rc;
+    }
     // the query half always runs: it produces delta, which the key half needs
     int rc = na2d_backward_dq_ex(a);
     if (rc != NA2D_OK || a->d_k.ptr == nullptr) return rc;

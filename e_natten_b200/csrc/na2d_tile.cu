@@ -5,6 +5,7 @@
 
 #include "../../include/na2d.h"
 #include "na2d_tile.cuh"
+#include "na2d_tile_bwd.cuh"
 
 #if NA2D_TILE_DT == 0
 using Elem = float;
@@ -48,8 +49,8 @@ int by_window(const Na2dGeom& g, F&& f) {
 }
 
 template <typename S>
-int tiles(const Na2dGeom& g, int H, unsigned* n) {
-    const long long t = (long long)g.BN * ((H + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw);
+int tiles(const Na2dGeom& g, int units, int H, unsigned* n) {
+    const long long t = (long long)units * ((H + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw);
     if (t > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
     *n = (unsigned)t;
     return NA2D_OK;
@@ -66,14 +67,64 @@ int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream
 
 }  // namespace
 
+#if NA2D_TILE_DT == 0
+long long workspace_floats(const Na2dGeom& g) {
+    long long floats = 0;
+    by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        floats = 2ll * ((g.Hq + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw) * S::kWeights * kR;
+        return NA2D_OK;
+    });
+    return floats;
+}
+#endif
+
 int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
                        const Tensor& o, float* lse) {
     return by_window(g, [&](auto ks, auto one_d) -> int {
         using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
         unsigned n = 0;
-        if (int rc = tiles<S>(g, g.Hq, &n)) return rc;
+        if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
         return launch(fwd_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(o, g.C), lse, g);
+    });
+}
+
+int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+                           const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        unsigned n = 0;
+        if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
+        return launch(dq_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+                      operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float4*)nullptr,
+                      (float4*)nullptr, 0, g);
+    });
+}
+
+int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+                        const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v, const float* lse,
+                        float* delta, float* workspace, int units, int* launches) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        using K = KeyShape<S>;
+        for (int unit0 = 0; unit0 < g.BN; unit0 += units) {
+            const int here = g.BN - unit0 < units ? g.BN - unit0 : units;
+            float4 *p = reinterpret_cast<float4*>(workspace), *ds = p + workspace_floats(g) / 8 * here;
+            unsigned n = 0;
+            if (int rc = tiles<S>(g, here, g.Hq, &n)) return rc;
+            if (int rc = launch(dq_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C),
+                                operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, p, ds,
+                                unit0, g))
+                return rc;
+            ++*launches;
+            const KeySum for_dk{ds, operand(q, g.C), operand(d_k, g.C)}, for_dv{p, operand(d_o, g.C), operand(d_v, g.C)};
+            if (int rc = launch(key_sum_kernel<Elem, float, true, S::kKs, S::kOneD>, dim3(n, 2), K::kThreads, K::kSmem, st, for_dk,
+                                for_dv, unit0, g))
+                return rc;
+            ++*launches;
+        }
+        return NA2D_OK;
     });
 }
 

@@ -17,10 +17,20 @@ struct Tensor {
 // Kernel sizes the tiled kernels are built for.
 inline bool supported(int ks) { return ks == 3 || ks == 5 || ks == 7 || ks == 9 || ks == 11 || ks == 13; }
 
+// fp32 values of P and dS that the backward of one unit hands from its query half to its key half.
+long long workspace_floats(const Na2dGeom& g);
+
+// backward: both halves, for whole images; the workspace holds workspace_floats() of `units` units, which
+// are taken that many at a time.
 // Status: 0, NA2D_ERR_TOO_LARGE (grid), or NA2D_ERR_CUDA (the launch's error is left for cudaGetLastError).
 #define NA2D_TILE_ENTRIES(suffix)                                                                                     \
     int forward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,       \
-                         const Tensor& o, float* lse);
+                         const Tensor& o, float* lse);                                                                \
+    int backward_dq_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,   \
+                             const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta);                   \
+    int backward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,      \
+                          const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v,                 \
+                          const float* lse, float* delta, float* workspace, int units, int* launches);
 NA2D_TILE_ENTRIES(f32)
 NA2D_TILE_ENTRIES(bf16)
 NA2D_TILE_ENTRIES(f16)

@@ -173,6 +173,21 @@ def backward_dkdv_into(q, k, v, lse, d_o, delta, d_k, d_v, kernel_size: int, row
     _lib.check(_lib.lib.na2d_backward_dkdv_ex(C.byref(a)))
 
 
+def _launch_backward(a: _lib.Args, device) -> None:
+    """Both halves of the backward, with the scratch the library asks for; where the allocator has no room
+    for that the key half forms the window weights again."""
+    nbytes = _lib.lib.na2d_backward_workspace(C.byref(a))
+    scratch = None
+    if nbytes:
+        try:
+            scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            pass
+        else:
+            a.workspace, a.workspace_bytes = scratch.data_ptr(), nbytes
+    _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
+
+
 # ---- 2D operator ----------------------------------------------------------------------------------------
 def natten2d_forward(q, k, v, kernel_size: int, rows: Optional[_lib.Rows] = None, path: str = "auto",
                      scale: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -208,6 +223,10 @@ def natten2d_backward(q, k, v, o, lse, d_o, kernel_size: int, rows: Optional[_li
     if q.numel() == 0 or not (need_dq or need_dkdv):
         return d_q, d_k, d_v
     delta = torch.empty((B, N, H, W), dtype=torch.float32, device=q.device)
+    if need_dkdv and rows is None and d_k.dtype == q.dtype:
+        _launch_backward(_args(q, kernel_size, None, path, scale, q=q, k=k, v=v, o=o, lse=lse, d_o=d_o, d_q=d_q, d_k=d_k,
+                               d_v=d_v, delta=delta), q.device)
+        return d_q, d_k, d_v
     # the query half always runs: it produces delta = rowsum(dO * o) for the key half
     backward_dq_into(q, k, v, o, lse, d_o, d_q, delta, kernel_size, rows, path, scale)
     if need_dkdv:
@@ -307,7 +326,7 @@ def natten1d_backward(q, k, v, o, lse, d_o, kernel_size: int, need_dq: bool = Tr
     delta = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
     a = _args(q, kernel_size, None, "auto", scale, q=q, k=k, v=v, lse=lse, d_o=d_o, d_q=d_q, d_k=d_k, d_v=d_v,
               delta=delta)
-    _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
+    _launch_backward(a, q.device)
     return d_q, d_k, d_v
 
 

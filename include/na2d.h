@@ -159,6 +159,8 @@ int na2d_backward(const void* q, const void* k, const void* v, const void* o, co
  *             costs accuracy.  NA2D_FLAG_SM_MARGIN(n): leave n SMs to a concurrent kernel.
  *   lse       fp32 (B, N, Hq, W), dense: written by the forward, read by the backward.
  *   delta     fp32 (B, N, Hq, W), dense scratch of the backward.
+ *   workspace, workspace_bytes: further, optional scratch of na2d_backward_ex.  A struct_size that ends before
+ *             these two fields is accepted: a caller built without them has no workspace.
  */
 typedef struct na2d_tensor {
     void* ptr;
@@ -189,6 +191,8 @@ typedef struct na2d_args {
     na2d_tensor q, k, v, o, d_o, d_q, d_k, d_v;
     float* lse;
     float* delta;
+    void* workspace;          /* optional scratch of na2d_backward_ex, 16-byte aligned; see na2d_backward_workspace */
+    size_t workspace_bytes;
 } na2d_args;
 
 /* As na2d_forward; writes a->o and a->lse.
@@ -201,6 +205,12 @@ int na2d_backward_dkdv_ex(const na2d_args* a);
 /* As na2d_backward: both halves.  Replaces Natten2d.backward (e_natten/triton.py:521-548) and
  * Natten1d.backward (454-483). */
 int na2d_backward_ex(const na2d_args* a);
+/* Bytes of scratch that na2d_backward_ex can use for this problem as a->workspace / a->workspace_bytes, 0 where it
+ * has no use for any.  Problems that run on CUDA cores (fp32, the 1D operator, head dims without tensor-core
+ * kernels) keep their window weights P and dS there, in fp32, instead of forming them again in the key half;
+ * without a workspace, or with one smaller than a single (batch, head) image needs, they form them again.  The
+ * contents are of no use after the call.  No reference counterpart. */
+size_t na2d_backward_workspace(const na2d_args* a);
 
 /* ---- 1D operator, dense tensors (B, N, T, C) ------------------------------------------------
  * natten1d of the reference: e_natten/triton.py:425-485 (autograd wrapper), 65-141 and 143-222

@@ -1,0 +1,128 @@
+"""GPU tests of the tiled CUDA-core kernels (fp32, the 1D operator, head dims without tensor-core kernels)
+at the sizes where they can go wrong: image sides around the tile and strip sizes, sides equal to the
+window, head dims that leave a channel chunk part empty or rule out 16-byte loads, backwards that take
+the units in several turns or have no workspace, and values that must not leave their windows."""
+import ctypes as C
+
+import pytest
+import torch
+
+import e_natten_b200 as na
+from e_natten_b200 import _lib
+from e_natten_b200 import functional as F
+from oracle import na2d_oracle as orc
+from helpers import assert_close, make_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# (kernel size, H, W, C): sides one below, at and above the 8-row, 4-column and 8- / 16-column tile edges,
+# whole-window images, and images whose every tile meets two borders
+CASES = [(3, 3, 3, 4), (3, 8, 15, 32), (3, 17, 33, 70), (5, 5, 9, 2), (5, 16, 16, 128), (5, 19, 37, 40),
+         (7, 7, 16, 33), (7, 21, 22, 96), (9, 9, 9, 48), (9, 25, 24, 36), (11, 11, 43, 64), (11, 26, 26, 20),
+         (13, 13, 13, 256), (13, 14, 14, 64), (13, 26, 33, 96)]
+
+
+def _device(*ts):
+    return tuple(t.to(DEV) for t in ts)
+
+
+@pytest.mark.parametrize("ks,H,W,Cd", CASES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_2d_against_oracle(ks, H, W, Cd, dtype):
+    scale = Cd ** -0.5
+    q, k, v, d_o = make_inputs((1, 2, H, W, Cd), dtype, 900 + ks + H)
+    ro, rlse = orc.natten2d_fwd(q, k, v, ks, scale=scale)
+    rdq, rdk, rdv = orc.natten2d_bwd(q, k, v, d_o, ks, scale=scale)
+    qd, kd, vd, gd = _device(q, k, v, d_o)
+    o, lse = na.natten2d_forward(qd, kd, vd, ks, path="simt", scale=scale)
+    dq, dk, dv = na.natten2d_backward(qd, kd, vd, o, lse, gd, ks, path="simt", scale=scale)
+    for got, want, what in ((o, ro, "o"), (lse, rlse, "lse"), (dq, rdq, "dq"), (dk, rdk, "dk"), (dv, rdv, "dv")):
+        assert_close(got, want, torch.float32 if what == "lse" else dtype, f"{what} ks={ks} {H}x{W}x{Cd} {dtype}")
+
+
+@pytest.mark.parametrize("ks,T,Cd", [(3, 3, 8), (5, 127, 40), (7, 128, 32), (9, 129, 48), (11, 11, 6), (13, 300, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_1d_against_oracle(ks, T, Cd, dtype):
+    g = torch.Generator().manual_seed(ks + T)
+    q, k, v, d_o = (torch.randn((2, 3, T, Cd), generator=g).to(dtype) for _ in range(4))
+    ro, rlse = orc.natten1d_fwd(q, k, v, ks, scale=0.3)
+    rdq, rdk, rdv = orc.natten1d_bwd(q, k, v, d_o, ks, scale=0.3)
+    qd, kd, vd, gd = _device(q, k, v, d_o)
+    o, lse = F.natten1d_forward(qd, kd, vd, ks, 0.3)
+    dq, dk, dv = F.natten1d_backward(qd, kd, vd, o, lse, gd, ks, scale=0.3)
+    for got, want, what in ((o, ro, "o"), (dq, rdq, "dq"), (dk, rdk, "dk"), (dv, rdv, "dv")):
+        assert_close(got, want, dtype, f"{what} ks={ks} T={T} C={Cd} {dtype}")
+
+
+@pytest.mark.parametrize("ks,H,W,Cd", [(5, 19, 37, 40), (13, 14, 30, 64), (3, 9, 9, 30)])
+def test_packed_views_equal_dense(ks, H, W, Cd):
+    """Strided operands, vector loads or not, give what dense ones give, bit for bit."""
+    g = torch.Generator().manual_seed(3)
+    qkv = torch.randn((2, H, W, 3, 2, Cd), generator=g).to(DEV)
+    d_o = torch.randn((2, H, W, 2, Cd), generator=g).to(DEV).permute(0, 3, 1, 2, 4)
+    views = qkv.permute(3, 0, 4, 1, 2, 5).unbind(0)
+    dense = tuple(t.contiguous() for t in views)
+    o1, l1 = na.natten2d_forward(*views, ks, scale=0.2)
+    o2, l2 = na.natten2d_forward(*dense, ks, scale=0.2)
+    assert torch.equal(o1, o2) and torch.equal(l1, l2)
+    for a, b in zip(na.natten2d_backward(*views, o1, l1, d_o, ks, scale=0.2),
+                    na.natten2d_backward(*dense, o2, l2, d_o.contiguous(), ks, scale=0.2)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ks,H,W", [(5, 20, 21), (9, 12, 33)])
+def test_workspace_of_any_size(ks, H, W):
+    """All units at once, one unit at a time, and no workspace (the key half forms the weights again)."""
+    B, N, Cd = 1, 3, 64
+    q, k, v, d_o = _device(*make_inputs((B, N, H, W, Cd), torch.float32, 77))
+    o, lse = na.natten2d_forward(q, k, v, ks, scale=0.125)
+    want = orc.natten2d_bwd(q.cpu(), k.cpu(), v.cpu(), d_o.cpu(), ks, scale=0.125)
+    delta = torch.empty_like(lse)
+
+    def run(units):
+        grads = [torch.full_like(q, float("nan")) for _ in range(3)]
+        a = F._args(q, ks, None, "auto", 0.125, q=q, k=k, v=v, o=o, lse=lse, d_o=d_o, d_q=grads[0], d_k=grads[1],
+                    d_v=grads[2], delta=delta)
+        per_unit = _lib.lib.na2d_backward_workspace(C.byref(a)) // (B * N)
+        assert per_unit >= 2 * H * W * ks * ks * 4 and per_unit % 16 == 0
+        scratch = torch.full((units * per_unit // 4 + 4,), -1.0, device=DEV)
+        a.workspace, a.workspace_bytes = (scratch.data_ptr(), units * per_unit) if units else (None, 0)
+        _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
+        assert bool((scratch[units * per_unit // 4:] == -1.0).all())            # nothing beyond what was given
+        return grads
+
+    whole = run(3)
+    for g, w, what in zip(whole, want, ("dq", "dk", "dv")):
+        assert_close(g, w, torch.float32, what)
+    for units in (1, 2):
+        assert all(torch.equal(x, y) for x, y in zip(run(units), whole))
+    for g, w, what in zip(run(0), want, ("dq", "dk", "dv")):
+        assert_close(g, w, torch.float32, what + " without workspace")
+
+
+@pytest.mark.parametrize("ks", [3, 5, 9])
+@pytest.mark.parametrize("at", [(0, 0), (7, 7), (8, 16), (23, 30)])
+def test_infinities_stay_in_their_windows(ks, at):
+    """An infinite value (and an infinite gradient) reaches the pixels whose windows hold it and no others."""
+    H, W = 24, 31
+    q, k, v, d_o = _device(*make_inputs((1, 1, H, W, 32), torch.float32, 5, q_scale=0.2))
+    v2, g2 = v.clone(), d_o.clone()
+    v2[0, 0, at[0], at[1]] = float("inf")
+    g2[0, 0, at[0], at[1]] = float("inf")
+    o, lse = na.natten2d_forward(q, k, v, ks)
+    o2, lse2 = na.natten2d_forward(q, k, v2, ks)
+    rows = torch.tensor([na.get_window_start(y, H, ks) <= at[0] < na.get_window_start(y, H, ks) + ks for y in range(H)])
+    cols = torch.tensor([na.get_window_start(x, W, ks) <= at[1] < na.get_window_start(x, W, ks) + ks for x in range(W)])
+    reached = (rows[:, None] & cols[None, :]).to(DEV)
+    assert torch.equal(torch.isinf(o2[0, 0]).all(-1), reached) and torch.equal(lse, lse2)
+    assert torch.equal(o2[0, 0][~reached], o[0, 0][~reached])
+    _, _, dv = na.natten2d_backward(q, k, v, o, lse, d_o, ks)
+    dq2, dk2, dv2 = na.natten2d_backward(q, k, v, o, lse, g2, ks)
+    ys = slice(na.get_window_start(at[0], H, ks), na.get_window_start(at[0], H, ks) + ks)
+    xs = slice(na.get_window_start(at[1], W, ks), na.get_window_start(at[1], W, ks) + ks)
+    held = torch.zeros(H, W, dtype=torch.bool, device=DEV)
+    held[ys, xs] = True
+    assert torch.equal(~torch.isfinite(dv2[0, 0]).all(-1), held)
+    assert torch.equal(dv2[0, 0][~held], dv[0, 0][~held])
+    assert torch.isfinite(dk2[0, 0][~held]).all()
