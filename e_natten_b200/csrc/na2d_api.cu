@@ -550,8 +550,11 @@ int enter_pair(int B, int N, int H, int W, int C, int ks, int dtype, int device,
     return step(p);
 }
 
+na2d_tile::Tensor tile_dense(const PairProblem& p, const void* ptr) { return na2d_tile::Tensor{const_cast<void*>(ptr), p.st}; }
+
 // x . y over the window -> attn
 int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
+    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_dot)(p.g, p.stream, tile_dense(p, x), tile_dense(p, y), attn), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -564,6 +567,7 @@ int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
 }
 // sum_j attn_j y_j -> out
 int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out) {
+    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_apply)(p.g, p.stream, attn, tile_dense(p, y), tile_dense(p, out)), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -577,6 +581,7 @@ int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out)
 }
 // key-side sum over the inverse neighbourhood of attn x -> out
 int pair_inverse(const PairProblem& p, const void* attn, const void* x, void* out) {
+    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_inverse)(p.g, p.stream, attn, tile_dense(p, x), tile_dense(p, out)), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hkv, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;

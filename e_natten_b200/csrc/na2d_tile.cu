@@ -6,6 +6,7 @@
 #include "../../include/na2d.h"
 #include "na2d_tile.cuh"
 #include "na2d_tile_bwd.cuh"
+#include "na2d_tile_pair.cuh"
 
 #if NA2D_TILE_DT == 0
 using Elem = float;
@@ -125,6 +126,37 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
             ++*launches;
         }
         return NA2D_OK;
+    });
+}
+
+int NA2D_NAME(pair_dot)(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        unsigned n = 0;
+        if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
+        return launch(window_dot_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(x, g.C),
+                      operand(y, g.C), (Elem*)attn, g);
+    });
+}
+
+int NA2D_NAME(pair_apply)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        unsigned n = 0;
+        if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
+        return launch(window_apply_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, (const Elem*)attn,
+                      operand(y, g.C), operand(out, g.C), g);
+    });
+}
+
+int NA2D_NAME(pair_inverse)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out) {
+    return by_window(g, [&](auto ks, auto one_d) -> int {
+        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+        using K = KeyShape<S>;
+        unsigned n = 0;
+        if (int rc = tiles<S>(g, g.BN, g.Hkv, &n)) return rc;
+        const KeySum sum{attn, operand(x, g.C), operand(out, g.C)};
+        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, S::kOneD>, n, K::kThreads, K::kSmem, st, sum, sum, 0, g);
     });
 }
 

@@ -30,7 +30,10 @@ long long workspace_floats(const Na2dGeom& g);
                              const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta);                   \
     int backward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,      \
                           const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v,                 \
-                          const float* lse, float* delta, float* workspace, int units, int* launches);
+                          const float* lse, float* delta, float* workspace, int units, int* launches);                \
+    int pair_dot_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn);          \
+    int pair_apply_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out); \
+    int pair_inverse_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out);
 NA2D_TILE_ENTRIES(f32)
 NA2D_TILE_ENTRIES(bf16)
 NA2D_TILE_ENTRIES(f16)
