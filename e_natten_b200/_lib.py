@@ -8,6 +8,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch  # noqa: F401  (the extension module needs its libraries loaded)
+
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("NA2D_LIB", os.path.join(_PKG_DIR, "libna2d.so"))
 
@@ -101,7 +103,19 @@ def _load() -> C.CDLL:
     return lib
 
 
+def _load_torch_ext():
+    """The native host path between tensors and the C ABI, calling the functions of ``lib``."""
+    path = os.path.join(_PKG_DIR, "_na2d_torch.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: run `python e_natten_b200/build.py`")
+    from . import _na2d_torch
+    _na2d_torch.bind_abi(*(C.cast(fn, C.c_void_p).value
+                           for fn in (lib.na2d_forward_ex, lib.na2d_backward_ex, lib.na2d_backward_workspace)))
+    return _na2d_torch
+
+
 lib = _load()
+torch_ext = _load_torch_ext()
 
 
 class Na2dError(RuntimeError):

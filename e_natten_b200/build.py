@@ -14,11 +14,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libna2d.so")
+EXT_PATH = os.path.join(PKG_DIR, "_na2d_torch.so")
 # (source, extra defines, object name)
 UNITS = [
     ("na2d_api.cu", [], "na2d_api.o"),
@@ -49,9 +51,9 @@ def _deps():
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(EXT_PATH):
         return True
-    built = os.path.getmtime(LIB_PATH)
+    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(EXT_PATH))
     return any(os.path.getmtime(d) > built for d in _deps())
 
 
@@ -63,6 +65,20 @@ def _compile(unit, verbose: bool, extra, obj_dir):
     return obj, proc.returncode, proc.stdout + proc.stderr, " ".join(cmd)
 
 
+def _compile_torch_ext():
+    """The Python extension module over PyTorch's C++ API (host code only)."""
+    import torch
+    from torch.utils import cpp_extension
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{p}" for p in (*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"])],
+           os.path.join(CSRC, "na2d_torch.cpp"), "-o", EXT_PATH,
+           *[f"-L{p}" for p in cpp_extension.library_paths("cuda")],
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    return os.path.basename(EXT_PATH), proc.returncode, proc.stdout + proc.stderr, " ".join(cmd)
+
+
 def build(force: bool = False, verbose: bool = False, extra_flags=(), lib_path: str = LIB_PATH) -> str:
     """Compile the library if it is missing or older than its sources; return its path."""
     if not force and lib_path == LIB_PATH and not _stale():
@@ -72,7 +88,10 @@ def build(force: bool = False, verbose: bool = False, extra_flags=(), lib_path: 
     os.makedirs(obj_dir, exist_ok=True)
     workers = max(1, min(len(UNITS), os.cpu_count() or 1))
     with concurrent.futures.ThreadPoolExecutor(workers) as pool:
+        ext = pool.submit(_compile_torch_ext) if lib_path == LIB_PATH else None
         results = list(pool.map(lambda u: _compile(u, verbose, list(extra_flags), obj_dir), UNITS))
+        if ext is not None:
+            results.append(ext.result())
     for obj, rc, out, cmd in results:
         if verbose or rc != 0:
             sys.stderr.write(f"--- {obj}\n{out}")

@@ -1,0 +1,141 @@
+// The per-call host path between PyTorch tensors and the C ABI: layout tests, output allocation, the
+// argument struct and the call itself, in one native step per direction.  In Python the same steps take
+// longer than the kernels of a small call.  Semantics live in functional.py; this file must not decide
+// anything that differs from it.
+#include <torch/csrc/utils/pybind.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cstring>
+#include <optional>
+#include <tuple>
+
+#include "../../include/na2d.h"
+
+namespace {
+
+using at::Tensor;
+using MaybeTensor = std::optional<Tensor>;
+
+// The library functions, as loaded by _lib.py (which may have been pointed at another build of them).
+struct Abi {
+    int (*forward)(const na2d_args*) = nullptr;
+    int (*backward)(const na2d_args*) = nullptr;
+    size_t (*backward_workspace)(const na2d_args*) = nullptr;
+} abi;
+
+void bind_abi(uintptr_t forward, uintptr_t backward, uintptr_t backward_workspace) {
+    abi.forward = reinterpret_cast<int (*)(const na2d_args*)>(forward);
+    abi.backward = reinterpret_cast<int (*)(const na2d_args*)>(backward);
+    abi.backward_workspace = reinterpret_cast<size_t (*)(const na2d_args*)>(backward_workspace);
+}
+
+// Whether the kernels can read t in place: contiguous channels, no broadcast or reversed dimension, and for
+// 16-bit types rows on 16-byte boundaries.
+bool kernel_ready(const Tensor& t) {
+    if (t.numel() == 0) return true;
+    const auto sizes = t.sizes();
+    const auto strides = t.strides();
+    const int64_t last = t.dim() - 1;
+    if (strides[last] != 1 && sizes[last] != 1) return false;
+    const bool half = t.element_size() == 2;
+    if (half && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
+    for (int64_t i = 0; i < last; ++i) {
+        if (sizes[i] <= 1) continue;
+        if (strides[i] <= 0 || (half && strides[i] % 8)) return false;
+    }
+    return true;
+}
+Tensor in_place_or_copy(const Tensor& t) { return kernel_ready(t) ? t : t.contiguous(); }
+
+// A dimension of extent 1 may report any stride; the library ignores it, but all-zero means dense.
+int64_t at_least_one(int64_t stride) { return stride < 1 ? 1 : stride; }
+na2d_tensor describe(const Tensor& t) {
+    const auto s = t.strides();
+    if (t.dim() == 5)
+        return {t.data_ptr(), at_least_one(s[0]), at_least_one(s[1]), at_least_one(s[2]), at_least_one(s[3])};
+    return {t.data_ptr(), at_least_one(s[0]), at_least_one(s[1]), 0, at_least_one(s[2])};
+}
+
+na2d_args arguments(const Tensor& q, int64_t kernel_size, int path, double scale) {
+    na2d_args a;
+    std::memset(&a, 0, sizeof(a));
+    a.struct_size = sizeof(a);
+    const bool one_d = q.dim() == 4;
+    a.op = one_d ? NA2D_OP_1D : NA2D_OP_2D;
+    a.B = (int)q.size(0);
+    a.N = (int)q.size(1);
+    a.H = one_d ? 1 : (int)q.size(2);
+    a.W = (int)q.size(one_d ? 2 : 3);
+    a.C = (int)q.size(one_d ? 3 : 4);
+    a.kernel_size = (int)kernel_size;
+    a.dtype = q.scalar_type() == at::kFloat ? NA2D_F32 : q.scalar_type() == at::kBFloat16 ? NA2D_BF16 : NA2D_F16;
+    a.path = path;
+    a.device = q.device().index();
+    a.scale = (float)scale;
+    a.stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+    return a;
+}
+
+at::DimVector rows_of(const Tensor& q) { return at::DimVector(q.sizes().begin(), q.sizes().end() - 1); }
+
+// Checked q, k, v -> (status, o, lse).
+std::tuple<int, Tensor, Tensor> forward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, int64_t kernel_size,
+                                        int path, double scale) {
+    const Tensor q = in_place_or_copy(q_in), k = in_place_or_copy(k_in), v = in_place_or_copy(v_in);
+    Tensor o = at::empty(q.sizes(), q.options());
+    Tensor lse = at::empty(rows_of(q), q.options().dtype(at::kFloat));
+    int status = NA2D_OK;
+    if (q.numel() != 0) {
+        na2d_args a = arguments(q, kernel_size, path, scale);
+        a.q = describe(q); a.k = describe(k); a.v = describe(v); a.o = describe(o);
+        a.lse = lse.data_ptr<float>();
+        status = abi.forward(&a);
+    }
+    return {status, o, lse};
+}
+
+// Checked operands of whole images -> (status, dQ, dK, dV), None for a half that is not wanted.
+std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in,
+                                                                const MaybeTensor& o_in, const Tensor& lse,
+                                                                const Tensor& d_o_in, int64_t kernel_size, int path,
+                                                                double scale, bool need_dq, bool need_dkdv) {
+    const Tensor q = in_place_or_copy(q_in), k = in_place_or_copy(k_in), v = in_place_or_copy(v_in);
+    const Tensor d_o = in_place_or_copy(d_o_in);
+    MaybeTensor o, d_q, d_k, d_v;
+    if (o_in) o = in_place_or_copy(*o_in);
+    if (need_dq) d_q = at::empty(q.sizes(), q.options());
+    if (need_dkdv) {
+        d_k = at::empty(k.sizes(), q.options());
+        d_v = at::empty(k.sizes(), q.options());
+    }
+    int status = NA2D_OK;
+    if (q.numel() != 0 && (need_dq || need_dkdv)) {
+        Tensor delta = at::empty(rows_of(q), q.options().dtype(at::kFloat)), workspace;
+        na2d_args a = arguments(q, kernel_size, path, scale);
+        a.q = describe(q); a.k = describe(k); a.v = describe(v); a.d_o = describe(d_o);
+        if (o) a.o = describe(*o);
+        if (d_q) a.d_q = describe(*d_q);
+        if (d_k) { a.d_k = describe(*d_k); a.d_v = describe(*d_v); }
+        a.lse = lse.data_ptr<float>();
+        a.delta = delta.data_ptr<float>();
+        if (const size_t bytes = d_k ? abi.backward_workspace(&a) : 0) {
+            try {
+                workspace = at::empty({(int64_t)bytes}, q.options().dtype(at::kByte));
+                a.workspace = workspace.data_ptr();
+                a.workspace_bytes = bytes;
+            } catch (const c10::OutOfMemoryError&) {       // no room: the key half forms the weights again
+            }
+        }
+        status = abi.backward(&a);
+    }
+    return {status, d_q, d_k, d_v};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_na2d_torch, m) {
+    m.def("bind_abi", &bind_abi);
+    m.def("forward", &forward, pybind11::call_guard<pybind11::gil_scoped_release>());
+    m.def("backward", &backward, pybind11::call_guard<pybind11::gil_scoped_release>());
+}

@@ -22,6 +22,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
+from ._lib import torch_ext
 
 _DTYPES = {torch.float32: _lib.DTYPE_F32, torch.bfloat16: _lib.DTYPE_BF16, torch.float16: _lib.DTYPE_F16}
 _PATHS = {"auto": _lib.PATH_AUTO, "simt": _lib.PATH_SIMT, "tensor": _lib.PATH_TENSOR}
@@ -173,26 +174,15 @@ def backward_dkdv_into(q, k, v, lse, d_o, delta, d_k, d_v, kernel_size: int, row
     _lib.check(_lib.lib.na2d_backward_dkdv_ex(C.byref(a)))
 
 
-def _launch_backward(a: _lib.Args, device) -> None:
-    """Both halves of the backward, with the scratch the library asks for; where the allocator has no room
-    for that the key half forms the window weights again."""
-    nbytes = _lib.lib.na2d_backward_workspace(C.byref(a))
-    scratch = None
-    if nbytes:
-        try:
-            scratch = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        except torch.OutOfMemoryError:
-            pass
-        else:
-            a.workspace, a.workspace_bytes = scratch.data_ptr(), nbytes
-    _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
-
-
 # ---- 2D operator ----------------------------------------------------------------------------------------
 def natten2d_forward(q, k, v, kernel_size: int, rows: Optional[_lib.Rows] = None, path: str = "auto",
                      scale: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
     """Raw forward: returns ``(o, lse)``; ``lse`` is fp32 ``(B, heads, H, W)``.  No autograd."""
     _check_inputs(q, k, v, kernel_size, rows)
+    if rows is None:
+        status, o, lse = torch_ext.forward(q, k, v, kernel_size, _PATHS[path], scale)
+        _lib.check(status)
+        return o, lse
     q, k, v = as_kernel_input(q), as_kernel_input(k), as_kernel_input(v)
     B, N, H, W, Cd = q.shape
     o = torch.empty((B, N, H, W, Cd), dtype=q.dtype, device=q.device)
@@ -211,9 +201,13 @@ def natten2d_backward(q, k, v, o, lse, d_o, kernel_size: int, rows: Optional[_li
     query band; ``dkdv_dtype=torch.float32`` keeps those partial sums in fp32.
     """
     _check_inputs(q, k, v, kernel_size, rows)
-    q, k, v, d_o = (as_kernel_input(t) for t in (q, k, v, d_o))
     if d_o.shape != q.shape or d_o.dtype != q.dtype:
         raise ValueError("grad_output must match q in shape and dtype")
+    if rows is None and dkdv_dtype in (None, q.dtype):
+        status, d_q, d_k, d_v = torch_ext.backward(q, k, v, o, lse, d_o, kernel_size, _PATHS[path], scale, need_dq, need_dkdv)
+        _lib.check(status)
+        return d_q, d_k, d_v
+    q, k, v, d_o = (as_kernel_input(t) for t in (q, k, v, d_o))
     if o is not None:
         o = as_kernel_input(o)
     B, N, H, W, Cd = q.shape
@@ -223,10 +217,6 @@ def natten2d_backward(q, k, v, o, lse, d_o, kernel_size: int, rows: Optional[_li
     if q.numel() == 0 or not (need_dq or need_dkdv):
         return d_q, d_k, d_v
     delta = torch.empty((B, N, H, W), dtype=torch.float32, device=q.device)
-    if need_dkdv and rows is None and d_k.dtype == q.dtype:
-        _launch_backward(_args(q, kernel_size, None, path, scale, q=q, k=k, v=v, o=o, lse=lse, d_o=d_o, d_q=d_q, d_k=d_k,
-                               d_v=d_v, delta=delta), q.device)
-        return d_q, d_k, d_v
     # the query half always runs: it produces delta = rowsum(dO * o) for the key half
     backward_dq_into(q, k, v, o, lse, d_o, d_q, delta, kernel_size, rows, path, scale)
     if need_dkdv:
@@ -302,12 +292,8 @@ def _check_inputs_1d(q, k, v, kernel_size):
 def natten1d_forward(q, k, v, kernel_size: int, scale: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
     """Raw 1D forward on ``(B, heads, T, C)``: returns ``(o, lse)``, lse fp32 ``(B, heads, T)``."""
     _check_inputs_1d(q, k, v, kernel_size)
-    q, k, v = as_kernel_input(q), as_kernel_input(k), as_kernel_input(v)
-    o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    lse = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
-    if q.numel() != 0:
-        a = _args(q, kernel_size, None, "auto", scale, q=q, k=k, v=v, o=o, lse=lse)
-        _lib.check(_lib.lib.na2d_forward_ex(C.byref(a)))
+    status, o, lse = torch_ext.forward(q, k, v, kernel_size, _lib.PATH_AUTO, scale)
+    _lib.check(status)
     return o, lse
 
 
@@ -315,18 +301,10 @@ def natten1d_backward(q, k, v, o, lse, d_o, kernel_size: int, need_dq: bool = Tr
                       scale: float = 1.0):
     """Raw 1D backward: ``(dQ, dK, dV)``."""
     _check_inputs_1d(q, k, v, kernel_size)
-    q, k, v, d_o = (as_kernel_input(t) for t in (q, k, v, d_o))
     if d_o.shape != q.shape or d_o.dtype != q.dtype:
         raise ValueError("grad_output must match q in shape and dtype")
-    d_q = torch.empty(q.shape, dtype=q.dtype, device=q.device) if need_dq else None
-    d_k = torch.empty(q.shape, dtype=q.dtype, device=q.device) if need_dkdv else None
-    d_v = torch.empty(q.shape, dtype=q.dtype, device=q.device) if need_dkdv else None
-    if q.numel() == 0 or not (need_dq or need_dkdv):
-        return d_q, d_k, d_v
-    delta = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
-    a = _args(q, kernel_size, None, "auto", scale, q=q, k=k, v=v, lse=lse, d_o=d_o, d_q=d_q, d_k=d_k, d_v=d_v,
-              delta=delta)
-    _launch_backward(a, q.device)
+    status, d_q, d_k, d_v = torch_ext.backward(q, k, v, None, lse, d_o, kernel_size, _lib.PATH_AUTO, scale, need_dq, need_dkdv)
+    _lib.check(status)
     return d_q, d_k, d_v
 
 
