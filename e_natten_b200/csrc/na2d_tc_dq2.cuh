@@ -11,11 +11,12 @@
 // it.  The exact delta is what the kernel writes out for the dK/dV kernel.
 //
 // Two chunks in flight.  With one S / dP buffer the walk is bound by latency: score MMAs, softmax and dQ MMAs run
-// one after the other.  Here a chunk is smaller (dq2_nmax keys), tensor memory holds two S / dP buffers beside dQ and B, and the score
-// MMAs of the next chunk (of the next tile, too) run under a chunk's softmax, its dQ MMAs under the next chunk's.
-// Measured against one chunk in flight, query half with the delta estimate: 32 x 2 x 56 x 56 x 32, window 7, bf16
-// 130 -> 103 us; 16 x 8 x 28 x 28 x 64, window 13, bf16 130 -> 100 us; 2 x 6 x 97 x 131 x 64, window 9, fp16
-// 138 -> 95 us; head dim 128, one 1024 x 1024 image of 8 heads, window 13: whole step 22.3 -> 21.4 ms.
+// one after the other.  Here a chunk is smaller (dq2_nmax keys), tensor memory holds two S / dP buffers beside dQ
+// and B, and the score MMAs of the next chunk (of the next tile, too) run under a chunk's softmax, its dQ MMAs
+// under the next chunk's.  Measured against one chunk in flight, query half with the delta estimate:
+// 32 x 2 x 56 x 56 x 32, window 7, bf16 130 -> 100 us; 16 x 8 x 28 x 28 x 64, window 13, bf16 130 -> 95 us;
+// 2 x 6 x 97 x 131 x 64, window 9, fp16 138 -> 89 us; 1024 x 1024 x 128, window 13, bf16 1.35 -> 0.97 ms (1.24 with
+// two K slots instead of the three or four below).
 #pragma once
 
 namespace na2d_tc {
@@ -36,9 +37,17 @@ struct Dq2Cfg : Cfg<D, KS, dq2_nmax(D)> {
     static constexpr int TMEM_RES = TMEM_S;                            // dS residual: lower half of S
     static constexpr int TMEM_PH = TMEM_S + B::NKP / 2;                // p: upper half of S
     static constexpr int OUT_BYTES = 8 * OutStage<D / 2>::BYTES;       // output staging of the 8 softmax warps
-    static constexpr int FIXED = 2 * B::Q_BYTES + OUT_BYTES + 2 * 2 * 128 * 4 /*delta exchange*/ + 256 + 1024;
-    static constexpr int NST = 2;      // K and V ring slots; scores(n + 1) are issued before outputs(n) frees a K slot
-    static constexpr int SMEM = FIXED + 2 * NST * B::KV_BYTES;
+    static constexpr int FIXED = OUT_BYTES + 2 * 2 * 128 * 4 /*delta exchange*/ + 256 + 1024;
+    // Ring depths.  A K slot is free when the dQ MMAs that read it are done, and the scores of the chunk after next are
+    // the next thing the pipe is given: with two slots it would wait there for a load, with three or four the
+    // chunk is in place.  A second Q / dO tile where it fits beside those.
+    static constexpr bool fits(int nq, int nk, int nv) {
+        return FIXED + nq * 2 * B::Q_BYTES + (nk + nv) * B::KV_BYTES <= kSmemLimit;
+    }
+    static constexpr int NSTK = fits(1, 4, 3) ? 4 : 3;
+    static constexpr int NSTV = fits(1, NSTK, 3) ? 3 : 2;
+    static constexpr int NQ = fits(2, NSTK, NSTV) ? 2 : 1;
+    static constexpr int SMEM = FIXED + NQ * 2 * B::Q_BYTES + (NSTK + NSTV) * B::KV_BYTES;
     static constexpr int NB16 = (B::NKP + 15) / 16;
     static_assert(B::NCH > 1, "several chunks");
     static_assert(SMEM <= kSmemLimit, "dQ kernel shared memory");
@@ -59,25 +68,25 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
-    uint8_t* sDO = sQ + C::Q_BYTES;
-    constexpr int NST = C::NST;
-    uint8_t* sK = sDO + C::Q_BYTES;                   // NST x key chunk   [NKP x D]
-    uint8_t* sV = sK + NST * C::KV_BYTES;             // NST x value chunk [NKP x D]
-    uint8_t* sOut = sV + NST * C::KV_BYTES;           // 8 x output staging (1024-byte aligned)
+    constexpr int NSTK = C::NSTK, NSTV = C::NSTV, NQ = C::NQ;
+    uint8_t* sDO = sQ + NQ * C::Q_BYTES;              // NQ x dO tile (and NQ x Q tile before it)
+    uint8_t* sK = sDO + NQ * C::Q_BYTES;              // NSTK x key chunk   [NKP x D]
+    uint8_t* sV = sK + NSTK * C::KV_BYTES;            // NSTV x value chunk [NKP x D]
+    uint8_t* sOut = sV + NSTV * C::KV_BYTES;          // 8 x output staging (1024-byte aligned)
     float* x_sum = reinterpret_cast<float*>(sOut + C::OUT_BYTES);     // [tile parity][half][row]
     uint64_t* bars = reinterpret_cast<uint64_t*>(x_sum + 2 * 2 * 128);
-    uint64_t* q_full = bars + 0;             // TMA -> MMA (Q and dO tile)
-    uint64_t* q_empty = bars + 1;            // MMA (commit) -> TMA
-    uint64_t* k_full = bars + 2;             // [2]
-    uint64_t* k_empty = bars + 4;            // [2]
-    uint64_t* v_full = bars + 6;             // [2]
-    uint64_t* v_empty = bars + 8;            // [2]
-    uint64_t* s_full = bars + 10;            // [2] MMA (commit) -> softmax: S and dP are complete, per buffer
-    uint64_t* p_full = bars + 12;            // [2] softmax -> MMA: dS and p are in tensor memory, per buffer
-    uint64_t* dq_full = bars + 14;           // MMA (commit) -> softmax (epilogue)
-    uint64_t* dq_free = bars + 15;           // softmax -> MMA
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 17)};
+    uint64_t* q_full = bars + 0;             // [2] TMA -> MMA (Q and dO tile)
+    uint64_t* q_empty = bars + 2;            // [2] MMA (commit) -> TMA
+    uint64_t* k_full = bars + 4;             // [4]
+    uint64_t* k_empty = bars + 8;            // [4]
+    uint64_t* v_full = bars + 12;            // [4]
+    uint64_t* v_empty = bars + 16;           // [4]
+    uint64_t* s_full = bars + 20;            // [2] MMA (commit) -> softmax: S and dP are complete, per buffer
+    uint64_t* p_full = bars + 22;            // [2] softmax -> MMA: dS and p are in tensor memory, per buffer
+    uint64_t* dq_full = bars + 24;           // MMA (commit) -> softmax (epilogue)
+    uint64_t* dq_free = bars + 25;           // softmax -> MMA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 27)};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -85,13 +94,15 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
     if (tid == 0) {
         wait_state_init(wctx.st, err_word, kWaitLimitNs);
-        mbar_init(q_full, 1);
-        mbar_init(q_empty, 1);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             mbar_init(k_full + i, 1);
             mbar_init(k_empty + i, 1);
             mbar_init(v_full + i, 1);
             mbar_init(v_empty + i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(q_full + i, 1);
+            mbar_init(q_empty + i, 1);
             mbar_init(s_full + i, 1);
             mbar_init(p_full + i, 8);
         }
@@ -112,7 +123,7 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // K rows [NK, NKP) of every stage are contraction rows of dQ = dS K that TMA never writes: zero them once.
     if constexpr (C::NKP > C::NK) {
         constexpr int pad16 = (C::NKP - C::NK) * C::ROWB / 16;
-        for (int i = tid; i < NST * C::NS * pad16; i += 384) {
+        for (int i = tid; i < NSTK * C::NS * pad16; i += 384) {
             const int which = i / pad16, off = i - which * pad16;             // which = stage * NS + slab
             st_shared_v4(smem_u32(sK + (which / C::NS) * C::KV_BYTES + (which % C::NS) * C::KV_SLAB + C::NK * C::ROWB +
                                   off * 16), 0u, 0u, 0u, 0u);
@@ -146,26 +157,27 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 split_unit(bn, g, hn, hb);
                 const int box_r0 = na2d_ws(g.q_row0 + r0, g.Hg, KS) - g.kv_row0;
                 const int box_c0 = na2d_ws(c0, g.W, KS);
-                if (!lt.acquire(q_empty, (i & 1) ^ 1, wctx)) break;
-                lt.arm(q_full, i & 1, 2u * C::Q_BYTES);
+                const int qb = i % NQ, qp = (i / NQ) & 1;
+                if (!lt.acquire(q_empty + qb, qp ^ 1, wctx)) break;
+                lt.arm(q_full + qb, qp, 2u * C::Q_BYTES);
 #pragma unroll
                 for (int s = 0; s < C::NS; ++s) {
-                    tma_load_5d(sQ + s * C::Q_SLAB, &tm_q, q_full, s * 64, c0, r0, hn, hb);
-                    tma_load_5d(sDO + s * C::Q_SLAB, &tm_do, q_full, s * 64, c0, r0, hn, hb);
+                    tma_load_5d(sQ + qb * C::Q_BYTES + s * C::Q_SLAB, &tm_q, q_full + qb, s * 64, c0, r0, hn, hb);
+                    tma_load_5d(sDO + qb * C::Q_BYTES + s * C::Q_SLAB, &tm_do, q_full + qb, s * 64, c0, r0, hn, hb);
                 }
                 for (int c = 0; c < NCH; ++c, ++n) {
-                    const uint32_t st = n % NST, par = (n / NST) & 1;
-                    if (!lt.acquire(v_empty + st, par ^ 1, wctx)) break;
-                    lt.arm(v_full + st, par, (uint32_t)C::NS * C::NK * C::ROWB);
+                    const uint32_t sk = n % NSTK, pk = (n / NSTK) & 1, sv = n % NSTV, pv = (n / NSTV) & 1;
+                    if (!lt.acquire(v_empty + sv, pv ^ 1, wctx)) break;
+                    lt.arm(v_full + sv, pv, (uint32_t)C::NS * C::NK * C::ROWB);
 #pragma unroll
                     for (int s = 0; s < C::NS; ++s)
-                        tma_load_5d(sV + st * C::KV_BYTES + s * C::KV_SLAB, &tm_v, v_full + st, s * 64, box_c0,
+                        tma_load_5d(sV + sv * C::KV_BYTES + s * C::KV_SLAB, &tm_v, v_full + sv, s * 64, box_c0,
                                     box_r0 + c * C::RC, hn, hb);
-                    if (!lt.acquire(k_empty + st, par ^ 1, wctx)) break;
-                    lt.arm(k_full + st, par, (uint32_t)C::NS * C::NK * C::ROWB);
+                    if (!lt.acquire(k_empty + sk, pk ^ 1, wctx)) break;
+                    lt.arm(k_full + sk, pk, (uint32_t)C::NS * C::NK * C::ROWB);
 #pragma unroll
                     for (int s = 0; s < C::NS; ++s)
-                        tma_load_5d(sK + st * C::KV_BYTES + s * C::KV_SLAB, &tm_k, k_full + st, s * 64, box_c0,
+                        tma_load_5d(sK + sk * C::KV_BYTES + s * C::KV_SLAB, &tm_k, k_full + sk, s * 64, box_c0,
                                     box_r0 + c * C::RC, hn, hb);
                 }
             }
@@ -177,17 +189,18 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         constexpr uint32_t idesc_s = umma_idesc(TM, C::NKP, IsBf16<DT>::value, IsBf16<DT>::value, false, false);
         constexpr uint32_t idesc_o = umma_idesc(TM, D, IsBf16<DT>::value, IsBf16<DT>::value, false, true);
         constexpr uint32_t hi = smem_desc_hi(C::ATOM, C::SWZ);
-        const uint32_t q_lo = smem_desc_lo(smem_u32(sQ), 16), g_lo = smem_desc_lo(smem_u32(sDO), 16);
         // S(n) = Q K_c^T and dP(n) = dO V_c^T into buffer n & 1
         auto scores = [&](uint32_t n) {
-            const uint32_t i = n / NCH, c = n % NCH, st = n % NST, par = (n / NST) & 1;
+            const uint32_t i = n / NCH, c = n % NCH, sk = n % NSTK, sv = n % NSTV, qb = i % NQ;
             if (lane == 0) NA2D_TR(2, 0, n);
-            if (c == 0) mbar_wait(q_full, i & 1, wctx, kErrLoadWait);
-            mbar_wait(k_full + st, par, wctx, kErrLoadWait);
-            mbar_wait(v_full + st, par, wctx, kErrLoadWait);
+            if (c == 0) mbar_wait(q_full + qb, (i / NQ) & 1, wctx, kErrLoadWait);
+            mbar_wait(k_full + sk, (n / NSTK) & 1, wctx, kErrLoadWait);
+            mbar_wait(v_full + sv, (n / NSTV) & 1, wctx, kErrLoadWait);
             tc_fence_after();
-            const uint32_t k_lo = smem_desc_lo(smem_u32(sK + st * C::KV_BYTES), 16);
-            const uint32_t v_lo = smem_desc_lo(smem_u32(sV + st * C::KV_BYTES), 16);
+            const uint32_t q_lo = smem_desc_lo(smem_u32(sQ + qb * C::Q_BYTES), 16);
+            const uint32_t g_lo = smem_desc_lo(smem_u32(sDO + qb * C::Q_BYTES), 16);
+            const uint32_t k_lo = smem_desc_lo(smem_u32(sK + sk * C::KV_BYTES), 16);
+            const uint32_t v_lo = smem_desc_lo(smem_u32(sV + sv * C::KV_BYTES), 16);
             const uint32_t buf = tmem_base + (n & 1) * C::TMEM_BUF;
             if (elect_one()) {
                 NA2D_TR(2, 1, n);
@@ -206,19 +219,19 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                             desc64(hi, v_lo + ((slab * C::KV_SLAB) >> 4) + 2 * in_slab), idesc_s, kk > 0);
                 }
                 umma_commit(s_full + (n & 1));
-                umma_commit(v_empty + st);
-                if (c == NCH - 1) umma_commit(q_empty);               // last score MMAs of the tile
+                umma_commit(v_empty + sv);
+                if (c == NCH - 1) umma_commit(q_empty + qb);               // last score MMAs of the tile
                 NA2D_TR(2, 2, n);
             }
             __syncwarp();
         };
         // dQ (+)= dS(n) K_c and B (+)= p(n) K_c, both operands read from buffer n & 1
         auto outputs = [&](uint32_t n) {
-            const uint32_t i = n / NCH, c = n % NCH, st = n % NST;
+            const uint32_t i = n / NCH, c = n % NCH, sk = n % NSTK;
             mbar_wait(p_full + (n & 1), (n >> 1) & 1, wctx, kErrMmaWait);
             if (c == 0) mbar_wait(dq_free, (i & 1) ^ 1, wctx, kErrMmaWait);        // the tile before has been read out
             tc_fence_after();
-            const uint32_t km_lo = smem_desc_lo(smem_u32(sK + st * C::KV_BYTES), C::KV_SLAB);
+            const uint32_t km_lo = smem_desc_lo(smem_u32(sK + sk * C::KV_BYTES), C::KV_SLAB);
             const uint32_t buf = tmem_base + (n & 1) * C::TMEM_BUF;
             if (elect_one()) {
                 NA2D_TR(2, 3, n);
@@ -237,7 +250,7 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 for (int kk = 0; kk < C::NKP / 16; ++kk)
                     umma_ts(tmem_base + C::TMEM_BK, buf + C::TMEM_PH + 8 * kk, desc64(hi, km_lo + ((kk * 16 * C::ROWB) >> 4)),
                             idesc_o, acc | (kk > 0));
-                umma_commit(k_empty + st);
+                umma_commit(k_empty + sk);
                 if (c == NCH - 1) umma_commit(dq_full);
                 NA2D_TR(2, 4, n);
             }
