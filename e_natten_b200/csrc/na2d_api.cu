@@ -1,5 +1,5 @@
 // C ABI of libna2d.so (declared in include/na2d.h): argument checking, device selection and
-// dispatch to the SIMT or tcgen05 kernels.  No framework headers; plain pointers and sizes.
+// dispatch to the tcgen05, tiled CUDA-core or warp-per-pixel (SIMT) kernels.  No framework headers; plain pointers and sizes.
 #include <cuda_runtime.h>
 
 #include <atomic>

@@ -9,10 +9,9 @@
 // accumulation is fp32.  The window is kh x kw: ks x ks for the 2D operator, 1 x ks for the 1D
 // operator on a (B, N, 1, T, C) view, so one set of kernels serves both.
 //
-// These kernels are the fp32 path (tensor cores cannot hold 1e-4 relative error), the path for
-// head dims and kernel sizes the tensor-core kernels are not built for, the 1D operator, and the
-// device-side second opinion for shapes the CPU oracle cannot finish.  They are bounds-safe for
-// every grid size and use no atomics, so results are bit-stable from run to run.
+// These kernels serve what the tiled kernels (na2d_tile.cuh) do not: kernel sizes 1 and 15 to 31, and the key half of
+// the backward where no workspace hands it the window weights (row views, fp32 partial sums, callers without
+// scratch).  They are bounds-safe for every grid size and use no atomics, so results are bit-stable from run to run.
 //
 // A block of eight warps works through a compact patch of 64 pixels (8 x 8, or 1 x 64 for a
 // one-row image), warp w taking pixels w, w + 8, ...: neighbouring pixels share most of their

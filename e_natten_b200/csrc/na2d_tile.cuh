@@ -52,8 +52,10 @@ struct Shape {
     static constexpr int kHaloW = kTw + KS - 1;
     static constexpr int kHaloH = kTh + kKh - 1;
     static constexpr int kItems = kTh * kStrips * kKh * kSplit;
-    static constexpr int kThreads = (kItems + 31) / 32 * 32 < 128 ? 128 : (kItems + 31) / 32 * 32;
     static constexpr int kApply = kTh * kStrips * kF;     // (strip, float4 of a chunk) items of the apply loop
+    // a thread per dot item; one more warp where that takes the apply loop from two rounds to one (KS 7)
+    static constexpr int kDotThreads = (kItems + 31) / 32 * 32 < 128 ? 128 : (kItems + 31) / 32 * 32;
+    static constexpr int kThreads = kApply == kDotThreads + 32 ? kApply : kDotThreads;
     // shared memory, in float4
     static constexpr int kWeights = kTh * kStrips * kKh * kU;
     static constexpr int kOwn = kTh * kTw * kF;
@@ -372,6 +374,25 @@ __device__ __forceinline__ void apply_row(float4 (&acc)[kR], const float4* w, co
     }
 }
 
+// The window's rows, odd and even ones in sums of their own: two short sums round less than a long one.
+template <typename S, bool REGULAR>
+__device__ __forceinline__ void apply_rows(float4 (&acc)[kR], const float4* w, const float4* halo, int f, int hy, int hx,
+                                           const Strip& s) {
+    float4 odd[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) odd[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int kW = S::kU * S::kTh, kH = S::kHaloW * kF;
+#pragma unroll 1
+    for (int u = 0; u + 1 < S::kKh; u += 2) {
+        apply_row<S, REGULAR>(acc, w + u * kW, halo + u * kH, f, hy + u, hx, s);
+        apply_row<S, REGULAR>(odd, w + (u + 1) * kW, halo + (u + 1) * kH, f, hy + u + 1, hx, s);
+    }
+    apply_row<S, REGULAR>(acc, w + (S::kKh - 1) * kW, halo + (S::kKh - 1) * kH, f, hy + S::kKh - 1, hx, s);
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+        acc[r] = make_float4(acc[r].x + odd[r].x, acc[r].y + odd[r].y, acc[r].z + odd[r].z, acc[r].w + odd[r].w);
+}
+
 // out = sum over the window of weight * y: all channel chunks, last chunk first (it may be in the halo
 // already: `staged`).  inv: per-pixel factors (float4 over a strip's pixels at [strip * kTh + row]) or null.
 template <typename T, typename S>
@@ -397,17 +418,8 @@ __device__ __forceinline__ void tile_apply(const Operand& out, const Operand& y,
 #pragma unroll
             for (int r = 0; r < kR; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
             const float4* wr = w + strip * S::kKh * S::kU * S::kTh + row;
-            if (s.regular) {
-#pragma unroll 1
-                for (int u = 0; u < S::kKh; ++u)
-                    apply_row<S, true>(acc, wr + u * S::kU * S::kTh, halo + ((hy0 + u) * S::kHaloW + hx) * kF, f, hy0 + u,
-                                       hx, s);
-            } else {
-#pragma unroll 1
-                for (int u = 0; u < S::kKh; ++u)
-                    apply_row<S, false>(acc, wr + u * S::kU * S::kTh, halo + ((hy0 + u) * S::kHaloW + hx) * kF, f, hy0 + u,
-                                        hx, s);
-            }
+            if (s.regular) apply_rows<S, true>(acc, wr, halo + (hy0 * S::kHaloW + hx) * kF, f, hy0, hx, s);
+            else apply_rows<S, false>(acc, wr, halo + (hy0 * S::kHaloW + hx) * kF, f, hy0, hx, s);
             const float4 fac = inv ? inv[strip * S::kTh + row] : make_float4(1.f, 1.f, 1.f, 1.f);
             T* o = os + (t.y0 + row) * out.st.h + (t.x0 + kR * strip) * out.st.w;
 #pragma unroll

@@ -45,7 +45,7 @@ typedef enum na2d_status {
 } na2d_status;
 
 /* Which implementation runs.  AUTO picks the tcgen05 tensor-core kernels for bf16/fp16 with a
- * supported head dim and kernel size, else the fp32-accumulating SIMT kernels. */
+ * supported head dim and kernel size, else the fp32-accumulating CUDA-core kernels. */
 typedef enum na2d_path {
     NA2D_PATH_AUTO = 0,
     NA2D_PATH_SIMT = 1,
