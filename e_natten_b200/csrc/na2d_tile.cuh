@@ -15,8 +15,8 @@
 // issues 16 warp multiply-adds): the strip is what brings the loads per multiply-add down.
 //
 // Measured on one B200 against one warp per pixel with the channels over its lanes (na2d_simt.cuh, four loads and a
-// butterfly of shuffles per 32 products), fp32: forward 4 x 4 x 256 x 256 x 128, window 5, 3.85 -> 0.78 ms;
-// 4 x 4 x 117 x 93 x 64, window 7, 0.75 -> 0.15 ms.
+// butterfly of shuffles per 32 products), fp32: forward 4 x 4 x 256 x 256 x 128, window 5, 3.85 -> 0.79 ms;
+// 4 x 4 x 117 x 93 x 64, window 7, 0.75 -> 0.14 ms.
 //
 // Windows are clamped at the borders, so the four windows of a strip need not be shifted by one
 // column each.  A strip away from the borders ("regular") takes loops whose band is known at compile
@@ -130,21 +130,27 @@ __device__ __forceinline__ void copy4(float* dst, const float* src) {
 }
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Where float4 f of staged pixel (y, x) lies, as an offset from the pixel's first float4: the eight
-// lanes of a quarter warp read the same f of eight rows (or, for one-row tiles, of eight strips) in
-// the dot loop, and the exclusive or puts those on different banks.
+// Where float4 f of staged pixel (y, x) lies, counted from the pixel's first float4: the eight lanes of a quarter
+// warp read the same f of eight rows (or, for one-row tiles, of eight strips) in the dot loop, and the exclusive
+// or puts those on different banks.  With eight-row tiles it does not depend on the column.
 template <int TH>
-__device__ __forceinline__ int bank_of(int y, int x) { return (y + (x >> 2) * TH) & 7; }
+__device__ __forceinline__ int place_of(int f, int y, int x) {
+    static_assert(TH == 1 || TH == 8, "eight rows, or one");
+    if constexpr (TH == 8) return f ^ (y & 7);
+    else return f ^ ((y + (x >> 2)) & 7);
+}
 
-// Four channels from c on of the pixel at p, as fp32, to d; zeros unless `in`, and beyond channel C.
+// Four channels from c on of the pixel at p, as fp32, to d; zeros unless `in`, and beyond channel C.  p is
+// readable either way.
 template <typename T>
 __device__ __forceinline__ void stage_quad(float4* d, const T* p, bool in, int c, int C, bool vec) {
     if (vec) {
         if constexpr (sizeof(T) == 4) {
             copy16(d, p, in);
         } else {
-            using Q = typename Quad<T>::type;
-            *d = in ? widen(__ldg(reinterpret_cast<const Q*>(p)), T{}) : make_float4(0.f, 0.f, 0.f, 0.f);
+            // p can be read in any case: a load without a branch, so that those of an unrolled loop fly together
+            const float4 x = widen(__ldg(reinterpret_cast<const typename Quad<T>::type*>(p)), T{});
+            *d = in ? x : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     } else {
         float v[4];
@@ -171,21 +177,23 @@ __device__ __forceinline__ void stage(float4* dst, const T* src, const Na2dStrid
         const T* p = in ? src + (y0 + yy) * st.h + (x0 + x) * st.w + c : src;
         const long long step = in ? kRows * st.h : 0;
         float4* d = dst + (yy * COLS + x) * kF;
-        const int xb = bank_of<TH>(0, x);
-#pragma unroll 4
+#pragma unroll (sizeof(T) == 2 ? 8 : 4)
         for (int y = yy; y < rows; y += kRows) {
-            stage_quad<T>(d + (f ^ ((y + xb) & 7)), p, in, c, C, vec);
+            stage_quad<T>(d + place_of<TH>(f, y, x), p, in, c, C, vec);
             p += step;
             d += kRows * COLS * kF;
         }
     } else {
         for (int y = 0; y < rows; ++y) {
             const T* p = src + (y0 + y) * st.h + (x0 + px) * st.w + c;
-#pragma unroll 4
-            for (int x = px; x < COLS; x += kPx, p += kPx * st.w) {
+            auto one = [&](int x) {
                 const bool in = x0 + x < W && c < C;
-                stage_quad<T>(dst + (y * COLS + x) * kF + (f ^ bank_of<TH>(y, x)), in ? p : src, in, c, C, vec);
-            }
+                stage_quad<T>(dst + (y * COLS + x) * kF + place_of<TH>(f, y, x), in ? p : src, in, c, C, vec);
+                p += kPx * st.w;
+            };
+#pragma unroll
+            for (int i = 0; i < COLS / kPx; ++i) one(px + i * kPx);
+            if (COLS % kPx != 0 && px < COLS % kPx) one(px + COLS / kPx * kPx);
         }
     }
 }
@@ -252,8 +260,8 @@ __device__ __forceinline__ float sum2(unsigned long long a) {
 // summed in packed pairs first and join acc as one number.  That keeps the running sum short (C / 8 roundings, as
 // few as a sum over the lanes of a warp has) and takes six instructions where eight multiply-adds would stand.
 template <typename S, bool REGULAR>
-__device__ __forceinline__ void dot_chunk(float (&acc)[kR][S::kU], const float4* own, int own_bank, const float4* halo,
-                                          int hy, int hx, int split) {
+__device__ __forceinline__ void dot_chunk(float (&acc)[kR][S::kU], const float4* own, int row, int strip,
+                                          const float4* halo, int hy, int hx, int split) {
     constexpr int kSteps = kF / 2 / S::kSplit;
     const ulonglong2* own2 = reinterpret_cast<const ulonglong2*>(own);
     const ulonglong2* halo2 = reinterpret_cast<const ulonglong2*>(halo);
@@ -263,13 +271,13 @@ __device__ __forceinline__ void dot_chunk(float (&acc)[kR][S::kU], const float4*
         ulonglong2 q0[kR], q1[kR];
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
-            q0[r] = own2[r * kF + (f ^ own_bank)];
-            q1[r] = own2[r * kF + ((f + 1) ^ own_bank)];
+            q0[r] = own2[r * kF + place_of<S::kTh>(f, row, kR * strip)];
+            q1[r] = own2[r * kF + place_of<S::kTh>(f + 1, row, kR * strip)];
         }
 #pragma unroll
         for (int j = 0; j < S::kU; ++j) {
-            const int bank = bank_of<S::kTh>(hy, hx + j);
-            const ulonglong2 x0 = halo2[j * kF + (f ^ bank)], x1 = halo2[j * kF + ((f + 1) ^ bank)];
+            const ulonglong2 x0 = halo2[j * kF + place_of<S::kTh>(f, hy, hx + j)];
+            const ulonglong2 x1 = halo2[j * kF + place_of<S::kTh>(f + 1, hy, hx + j)];
             unsigned long long part[kR];
 #pragma unroll
             for (int r = 0; r < kR; ++r) part[r] = mul2(q0[r].x, x0.x);
@@ -330,15 +338,14 @@ __device__ __forceinline__ void tile_dot(float (&acc)[kR][S::kU], const Operand&
     const T* ys = unit<T>(y, t);
     const float4* own_px = own + (d.row * S::kTw + kR * d.strip) * kF;
     const float4* halo_px = halo + (d.hy * S::kHaloW + d.hx) * kF;
-    const int own_bank = bank_of<S::kTh>(d.row, kR * d.strip);
     for (int c0 = 0; c0 < g.C; c0 += kChunk) {
         stage<T, S::kTh, S::kThreads, S::kTw>(own, xs, x.st, t.y0, t.rows, t.x0, g.W, c0, g.C, x.vec);
         stage<T, S::kTh, S::kThreads, S::kHaloW>(halo, ys, y.st, ky0, halo_rows, kx0, g.W, c0, g.C, y.vec);
         copies_done();
         __syncthreads();
         if (d.active) {
-            if (d.s.regular) dot_chunk<S, true>(acc, own_px, own_bank, halo_px, d.hy, d.hx, d.split);
-            else dot_chunk<S, false>(acc, own_px, own_bank, halo_px, d.hy, d.hx, d.split);
+            if (d.s.regular) dot_chunk<S, true>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split);
+            else dot_chunk<S, false>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split);
         }
         __syncthreads();
     }
@@ -366,7 +373,7 @@ __device__ __forceinline__ void apply_row(float4 (&acc)[kR], const float4* w, co
                                           const Strip& s) {
 #pragma unroll
     for (int j = 0; j < S::kU; ++j) {
-        const float4 x = halo[j * kF + (f ^ bank_of<S::kTh>(hy, hx + j))];
+        const float4 x = halo[j * kF + place_of<S::kTh>(f, hy, hx + j)];
         const float4 wt = w[j * S::kTh];
 #pragma unroll
         for (int r = 0; r < kR; ++r)
@@ -413,13 +420,15 @@ __device__ __forceinline__ void tile_apply(const Operand& out, const Operand& y,
             const int f = it % kF, row = it / kF % S::kTh, strip = it / (kF * S::kTh);
             if (row >= t.rows || kR * strip >= t.cols) continue;
             const Strip s = strip_at<S::kKs>(t.x0 + kR * strip, g.W);
-            const int hy0 = na2d_ws(g.q_row0 + t.y0 + row, g.Hg, S::kKh) - g.kv_row0 - ky0, hx = s.start - kx0;
+            const int hx = s.start - kx0;
+            const int hy0 = na2d_ws(g.q_row0 + t.y0 + row, g.Hg, S::kKh) - g.kv_row0 - ky0;
             float4 acc[kR];
 #pragma unroll
             for (int r = 0; r < kR; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
             const float4* wr = w + strip * S::kKh * S::kU * S::kTh + row;
-            if (s.regular) apply_rows<S, true>(acc, wr, halo + (hy0 * S::kHaloW + hx) * kF, f, hy0, hx, s);
-            else apply_rows<S, false>(acc, wr, halo + (hy0 * S::kHaloW + hx) * kF, f, hy0, hx, s);
+            const float4* hr = halo + (hy0 * S::kHaloW + hx) * kF;
+            if (s.regular) apply_rows<S, true>(acc, wr, hr, f, hy0, hx, s);
+            else apply_rows<S, false>(acc, wr, hr, f, hy0, hx, s);
             const float4 fac = inv ? inv[strip * S::kTh + row] : make_float4(1.f, 1.f, 1.f, 1.f);
             T* o = os + (t.y0 + row) * out.st.h + (t.x0 + kR * strip) * out.st.w;
 #pragma unroll

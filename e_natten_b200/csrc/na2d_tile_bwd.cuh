@@ -1,5 +1,10 @@
 // Tiled CUDA-core kernels of the backward: the query half, which hands the weights P and dS on, and the
 // key-side sum over the inverse neighbourhood.
+//
+// What bounds them: the shared-memory pipe and block barriers in the query half (three loops of the forward's kind),
+// issue slots in the key sums.  Keeping P and dS (2 ks * ks floats per pixel) costs less than the two score loops
+// that would form them again.  Measured on one B200 against the warp-per-pixel kernels, 4 x 4 x 256 x 256 x 128,
+// window 5, fp32: both halves 27.6 -> 2.14 ms; 4 x 8 x 4096 x 64, window 13, bf16, 1D: step 1.72 -> 0.29 ms.
 #pragma once
 
 #include "na2d_tile.cuh"
@@ -153,7 +158,7 @@ __device__ __forceinline__ void stage_columns(float4* dst, const T* src, const N
     const int n = rows * cols;
 #pragma unroll 2
     for (int px = first; px < n; px += kPx) {
-        stage_quad<T>(dst + px * kF + (f ^ bank_of<TH>(y, x)), in ? p : src, in, c, C, vec);
+        stage_quad<T>(dst + px * kF + place_of<TH>(f, y, x), in ? p : src, in, c, C, vec);
         x += kPx;
         p += kPx * st.w;
         while (x >= cols) { x -= cols; ++y; p += wrap; }
@@ -216,8 +221,11 @@ key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ Key
         for (int g0 = 0; g0 < nu; g0 += group) {
             const int gn = min(group, nu - g0);
             __syncthreads();
-            stage_columns<T, S::kTh, K::kThreads>(halo, xs, job.x.st, qy0 + g0, min(row_span + gn, H - qy0 - g0), qx0, cols,
-                                                  ch, g.C, job.x.vec);
+            const int rows = min(row_span + gn, H - qy0 - g0);
+            if (cols == S::kHaloW)                          // away from the column borders
+                stage<T, S::kTh, K::kThreads, S::kHaloW>(halo, xs, job.x.st, qy0 + g0, rows, qx0, W, ch, g.C, job.x.vec);
+            else
+                stage_columns<T, S::kTh, K::kThreads>(halo, xs, job.x.st, qy0 + g0, rows, qx0, cols, ch, g.C, job.x.vec);
             if (ch == 0 || group < nu) {
                 // weights of the group: element (strip, u, j, row, r), four pixels r of eight rows to a warp.  Lane
                 // (row, r) takes the d-th query column of its key, so that a warp's queries lie on a block of
@@ -235,11 +243,16 @@ key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ Key
                     const int qy = first_row + u, uq = y - na2d_ws(qy, H, S::kKh);
                     float* to = wf + (((st * gn + u) * nj + lo - na2d_bws(t.x0 + kR * st, KS)) * S::kTh + ly) * kR + lr;
                     if constexpr (TILED) {
-                        const TW* line = attn + ((long long)(qy / S::kTh) * tiles_w * S::kWeights + uq * (S::kU * S::kTh) + qy % S::kTh) * kR;
+                        // query (qy, qx): tile (qy / kTh, qx / kTw), strip and pixel r of its column, row qy % kTh;
+                        // the key is column col - (window start of the strip) of its halo
+                        const unsigned tile_row = (unsigned)qy / S::kTh, in_row = (unsigned)qy % S::kTh;
+                        const TW* line = attn + ((long long)(tile_row * (unsigned)tiles_w) * S::kWeights + uq * (S::kU * S::kTh) + in_row) * kR;
 #pragma unroll 4
                         for (int i = 0; i < n; ++i, to += S::kTh * kR) {
-                            const int qx = lo + i, strip_q = qx % S::kTw / kR;
-                            copy4(to, line + (qx / S::kTw * S::kWeights + (strip_q * (S::kKh * S::kU) + col - na2d_ws(qx / kR * kR, W, KS)) * S::kTh) * (long long)kR + qx % kR);
+                            const unsigned qx = lo + i, strip_q = qx % S::kTw / kR;
+                            const int j = col - na2d_ws(qx & ~(kR - 1u), W, KS);
+                            copy4(to, line + (long long)(qx / S::kTw) * (S::kWeights * kR) +
+                                          (int)((strip_q * (S::kKh * S::kU) + j) * (S::kTh * kR) + qx % kR));
                         }
                     } else {
                         const TW* line = attn + (long long)qy * W * kTaps + uq * KS + col;
@@ -261,7 +274,7 @@ key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ Key
                         apply_row<S, true>(acc, wr, hr, f, hy, hx, s);
                     } else {
                         for (int j = 0; j < my_nj; ++j) {
-                            const float4 x = hr[j * kF + (f ^ bank_of<S::kTh>(hy, hx + j))];
+                            const float4 x = hr[j * kF + place_of<S::kTh>(f, hy, hx + j)];
                             const float4 wt = wr[j * S::kTh];
 #pragma unroll
                             for (int r = 0; r < kR; ++r)
