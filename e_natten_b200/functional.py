@@ -243,10 +243,13 @@ class Natten2d(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.kernel_size, ctx.scale = kernel_size, scale
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)      # lse's gradient would be a buffer of zeros, filled at each backward
         return o, lse
 
     @staticmethod
     def backward(ctx, grad_output, _grad_lse):
+        if grad_output is None:
+            return None, None, None, None, None
         q, k, v, o, lse = ctx.saved_tensors
         poll_kernels(q.device)            # a wait that gave up in an earlier kernel surfaces here, without a sync
         need_dq = ctx.needs_input_grad[0]
