@@ -26,6 +26,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <float.h>
 #include <math_constants.h>
 #include <stdint.h>
 

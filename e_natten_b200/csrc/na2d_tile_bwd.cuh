@@ -70,11 +70,16 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
     __syncthreads();
     if (d.active) {
         float4 dl4;
-        // p = exp(s - lse) adds up to 1 but for the rounding of lse; taken out here, that rounding does not meet
-        // the cancellation in dP - delta.  (A sum that is not 1 means an lse over more than this window: left alone.)
+        // p = exp(s - lse) over the window that lse was taken over adds up to 1 but for rounding: that of lse, of the
+        // logits beside it (both half an ulp of numbers about as large as lse) and of the exponentials.  Taken out here,
+        // it does not meet the cancellation in dP - delta.  A sum further off than that rounding can bring it is no
+        // rounding but an lse over more than this window, whose weights are what exp(s - lse) says they are.
         const float4 l4 = sum_rows<S>(total + d.strip * S::kKh * S::kTh + d.row);
-        auto rounding = [](float l) { return fabsf(l - 1.f) < 1e-3f ? 1.f / l : 1.f; };
-        const float4 inv = make_float4(rounding(l4.x), rounding(l4.y), rounding(l4.z), rounding(l4.w));
+        auto rounding = [&](int r) {
+            const float l = lane_of(l4, r), limit = 4.f * FLT_EPSILON * (4.f + fabsf(c0 + r < g.W ? lse[stat + r] : 0.f));
+            return fabsf(l - 1.f) < limit ? 1.f / l : 1.f;
+        };
+        const float4 inv = make_float4(rounding(0), rounding(1), rounding(2), rounding(3));
         dl4 = sum_rows<S>(part + d.strip * S::kKh * S::kTh + d.row);
         dl4 = make_float4(dl4.x * inv.x, dl4.y * inv.y, dl4.z * inv.z, dl4.w * inv.w);
 #pragma unroll

@@ -141,7 +141,8 @@ def natten2d_fwd(q, k, v, kernel_size: int, acc_dtype=torch.float64, rows=None, 
     return o, m + torch.log(l)
 
 
-def natten2d_bwd(q, k, v, d_o, kernel_size: int, acc_dtype=torch.float64, rows=None, o=None, scale: float = 1.0):
+def natten2d_bwd(q, k, v, d_o, kernel_size: int, acc_dtype=torch.float64, rows=None, o=None, scale: float = 1.0,
+                 lse=None):
     """Backward in flash form.  Returns (dq, dk, dv) in ``acc_dtype``.
 
     p = exp(s - lse), delta = dO.O, dS = p*(dO.V - delta), dQ = sum dS*K,
@@ -155,12 +156,20 @@ def natten2d_bwd(q, k, v, d_o, kernel_size: int, acc_dtype=torch.float64, rows=N
     the input dtype (e_natten/triton.py:515), so on 16-bit paths the backward's input is the
     rounded o; passing it here makes delta = dO.o use the same rounded values (rounding of an
     input is not an error of the backward).  None uses the exact o.
+
+    ``lse`` other than the window's own (a merged one, over more keys than the window) scales every
+    row's p, and with it delta = sum p dP, by exp(own lse - lse).
     """
     B, N, H, W, C = q.shape
     Hkv = k.shape[2]
     ks = kernel_size
     q, k, v, d_o = (t.to(acc_dtype) for t in (q, k, v, d_o))
-    o_exact, lse = natten2d_fwd(q, k, v, ks, acc_dtype, rows, scale)
+    o_exact, own_lse = natten2d_fwd(q, k, v, ks, acc_dtype, rows, scale)
+    if lse is None:
+        lse = own_lse
+    else:
+        lse = lse.to(acc_dtype)
+        o_exact = o_exact * torch.exp(own_lse - lse).unsqueeze(-1)
     delta = (d_o * (o_exact if o is None else o.to(acc_dtype))).sum(-1)
     wsx, wsy = _row_origins(H, ks, rows), window_start_table(W, ks)
     dq = torch.zeros_like(q)

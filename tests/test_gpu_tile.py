@@ -3,6 +3,7 @@ at the sizes where they can go wrong: image sides around the tile and strip size
 window, head dims that leave a channel chunk part empty or rule out 16-byte loads, backwards that take
 the units in several turns or have no workspace, and values that must not leave their windows."""
 import ctypes as C
+import math
 
 import pytest
 import torch
@@ -126,3 +127,25 @@ def test_infinities_stay_in_their_windows(ks, at):
     assert torch.equal(~torch.isfinite(dv2[0, 0]).all(-1), held)
     assert torch.equal(dv2[0, 0][~held], dv[0, 0][~held])
     assert torch.isfinite(dk2[0, 0][~held]).all()
+
+
+@pytest.mark.parametrize("excess", [2e-5, 5e-4, 0.3])
+@pytest.mark.parametrize("workspace", [True, False])
+def test_merged_lse(excess, workspace):
+    """An lse over more than the window (a merged one): the weights are exp(s - lse), however little the rest adds."""
+    ks, H, W, Cd = 5, 19, 37, 40
+    q, k, v, d_o = _device(*make_inputs((1, 2, H, W, Cd), torch.float32, 31))
+    o, lse = na.natten2d_forward(q, k, v, ks, scale=0.2)
+    lse = (lse.double() + math.log1p(excess)).float()
+    delta, grads = torch.empty_like(lse), [torch.empty_like(q) for _ in range(3)]
+    a = F._args(q, ks, None, "auto", 0.2, q=q, k=k, v=v, o=o, lse=lse, d_o=d_o, d_q=grads[0], d_k=grads[1], d_v=grads[2],
+                delta=delta)
+    scratch = torch.empty(_lib.lib.na2d_backward_workspace(C.byref(a)), dtype=torch.uint8, device=DEV)
+    if workspace:
+        a.workspace, a.workspace_bytes = scratch.data_ptr(), scratch.numel()
+    _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
+    want = orc.natten2d_bwd(q.cpu(), k.cpu(), v.cpu(), d_o.cpu(), ks, scale=0.2, lse=lse.cpu())
+    for g, w, what in zip(grads, want, ("dq", "dk", "dv")):
+        # rounding of s and lse: a few 1e-6 of the norm; a sum brought back to 1 would be off by `excess`
+        err = (g.cpu().double() - w).norm() / w.norm()
+        assert err < 5e-6, f"{what}: {err:.2e}"
