@@ -248,9 +248,9 @@ class Natten2d(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output, _grad_lse):
-        if grad_output is None:
-            return None, None, None, None, None
         q, k, v, o, lse = ctx.saved_tensors
+        if grad_output is None:               # an undefined gradient (a node above returned None) counts as zeros
+            grad_output = torch.zeros_like(q, memory_format=torch.contiguous_format)
         poll_kernels(q.device)            # a wait that gave up in an earlier kernel surfaces here, without a sync
         need_dq = ctx.needs_input_grad[0]
         need_dkdv = ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
