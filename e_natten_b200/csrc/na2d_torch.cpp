@@ -1,7 +1,7 @@
 // The per-call host path between PyTorch tensors and the C ABI: layout tests, output allocation, the
 // argument struct and the call itself, in one native step per direction.  In Python the same steps take
-// longer than the kernels of a small call.  Semantics live in functional.py; this file must not decide
-// anything that differs from it.
+// longer than the kernels of a small call.  The layout rules live here (functional.py calls them for row
+// views); argument checks and autograd live in functional.py.
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
@@ -30,10 +30,11 @@ void bind_abi(uintptr_t forward, uintptr_t backward, uintptr_t backward_workspac
     abi.backward_workspace = reinterpret_cast<size_t (*)(const na2d_args*)>(backward_workspace);
 }
 
-// Whether the kernels can read t in place: contiguous channels, no broadcast or reversed dimension, and for
-// 16-bit types rows on 16-byte boundaries.
+// Whether the kernels can read t in place: contiguous channels, no broadcast dimension, and for 16-bit types (the
+// tensor-core path's TMA tensor maps) a base and strides on 16-byte boundaries.
 bool kernel_ready(const Tensor& t) {
     if (t.numel() == 0) return true;
+    if (t.dim() == 0) return false;
     const auto sizes = t.sizes();
     const auto strides = t.strides();
     const int64_t last = t.dim() - 1;
@@ -51,6 +52,7 @@ Tensor in_place_or_copy(const Tensor& t) { return kernel_ready(t) ? t : t.contig
 // A dimension of extent 1 may report any stride; the library ignores it, but all-zero means dense.
 int64_t at_least_one(int64_t stride) { return stride < 1 ? 1 : stride; }
 na2d_tensor describe(const Tensor& t) {
+    TORCH_CHECK_VALUE(t.dim() == 5 || t.dim() == 4, "expected (B, heads, H, W, C) or (B, heads, T, C); got ", t.dim(), " dimensions");
     const auto s = t.strides();
     if (t.dim() == 5)
         return {t.data_ptr(), at_least_one(s[0]), at_least_one(s[1]), at_least_one(s[2]), at_least_one(s[3])};
@@ -136,6 +138,11 @@ std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_
 
 PYBIND11_MODULE(_na2d_torch, m) {
     m.def("bind_abi", &bind_abi);
+    m.def("kernel_ready", &kernel_ready);
+    m.def("strides", [](const Tensor& t) {      // (batch, heads, row, column), as they go into na2d_tensor
+        const na2d_tensor d = describe(t);
+        return std::make_tuple(d.stride_b, d.stride_n, d.stride_h, d.stride_w);
+    });
     m.def("forward", &forward, pybind11::call_guard<pybind11::gil_scoped_release>());
     m.def("backward", &backward, pybind11::call_guard<pybind11::gil_scoped_release>());
 }

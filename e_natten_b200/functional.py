@@ -75,27 +75,9 @@ def make_rows(q_row0: int, Hq: int, kv_row0: int, Hkv: int, H_global: int) -> _l
 
 
 # ---- layouts ---------------------------------------------------------------------------------------
-def _kernel_ready(t: torch.Tensor) -> bool:
-    """True if the kernels can read ``t`` in place: channels contiguous and, for the 16-bit
-    tensor-core path (TMA tensor maps), a 16-byte aligned base and strides that are multiples
-    of 16 bytes.  fp32 tensors (SIMT kernels) only need contiguous channels."""
-    if t.numel() == 0:
-        return True
-    if t.stride(-1) != 1 and t.shape[-1] != 1:
-        return False
-    if any(s < 0 for s in t.stride()):
-        return False
-    if t.element_size() == 2:
-        if t.data_ptr() % 16:
-            return False
-        for size, stride in zip(t.shape[:-1], t.stride()[:-1]):
-            if size > 1 and (stride % 8 or stride == 0):
-                return False
-    else:
-        for size, stride in zip(t.shape[:-1], t.stride()[:-1]):
-            if size > 1 and stride == 0:
-                return False
-    return True
+# True if the kernels can read a tensor in place: channels contiguous and, for the 16-bit tensor-core path
+# (TMA tensor maps), a 16-byte aligned base and strides that are multiples of 16 bytes.
+_kernel_ready = torch_ext.kernel_ready
 
 
 def as_kernel_input(t: torch.Tensor) -> torch.Tensor:
@@ -107,13 +89,7 @@ def as_kernel_input(t: torch.Tensor) -> torch.Tensor:
 def _desc(t: Optional[torch.Tensor]) -> _lib.TensorDesc:
     if t is None:
         return _lib.TensorDesc(None, 0, 0, 0, 0)
-    if t.dim() == 5:
-        sb, sn, sh, sw, _ = t.stride()
-    else:                                     # (B, N, T, C): the 1D operator, a one-row image
-        sb, sn, sw, _ = t.stride()
-        sh = 0
-    # a dimension of extent 1 may report any stride; the library ignores it, but all-zero means dense
-    return _lib.TensorDesc(t.data_ptr(), max(sb, 1), max(sn, 1), max(sh, 1) if t.dim() == 5 else 0, max(sw, 1))
+    return _lib.TensorDesc(t.data_ptr(), *torch_ext.strides(t))
 
 
 def _args(like, kernel_size: int, rows, path: str, scale: float, **tensors) -> _lib.Args:

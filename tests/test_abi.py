@@ -128,6 +128,19 @@ def test_kernel_ready_layouts():
     assert not _kernel_ready(torch.zeros(1, 1, 8, 1, 32).expand(1, 1, 8, 8, 32))
 
 
+def test_operand_strides():
+    """Strides as the library gets them; ranks that are no operand's are refused, not read past their end."""
+    strides = _lib.torch_ext.strides
+    assert strides(torch.zeros(2, 3, 5, 7, 8)) == (840, 280, 56, 8)
+    assert strides(torch.zeros(2, 3, 7, 8)) == (168, 56, 0, 8)              # (B, heads, T, C)
+    packed = torch.zeros(2, 5, 7, 3, 4, 8)[:, :, :, 1].permute(0, 3, 1, 2, 4)
+    assert strides(packed) == (3360, 8, 672, 96)
+    assert strides(torch.zeros(2, 1, 5, 7, 8).as_strided((2, 1, 5, 7, 8), (280, 0, 56, 8, 1))) == (280, 1, 56, 8)
+    for shape in ((7, 8), (3, 7, 8), (1, 2, 3, 5, 7, 8)):
+        with pytest.raises(ValueError):
+            strides(torch.zeros(shape))
+
+
 def test_python_wrapper_refuses_cpu_tensors_and_bad_shapes():
     q = torch.zeros(1, 1, 8, 8, 32)
     with pytest.raises(ValueError, match="CUDA"):
