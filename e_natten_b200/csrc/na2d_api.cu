@@ -379,15 +379,15 @@ int run_backward_dq(const Problem& p) {
         // With the forward's output at hand, the dQ kernel of the larger windows gets an estimate of
         // the row deltas (dO . o) and walks its key box once; it overwrites the estimate with the
         // exact deltas.
-        const float* delta_in = nullptr;
+        bool have_estimate = false;
         if (g.ks >= 7 && p.o.ptr && p.d_q.ptr) {
             rc = launch_delta(p);
             if (rc != NA2D_OK) return rc;
-            delta_in = p.delta;
+            have_estimate = true;
         }
         rc = p.dtype == NA2D_BF16
-                 ? na2d_tc::backward_dq_bf16(lc, targ(p.q), targ(p.k), targ(p.v), p.lse, targ(p.d_o), targ(p.d_q), p.delta, delta_in)
-                 : na2d_tc::backward_dq_f16(lc, targ(p.q), targ(p.k), targ(p.v), p.lse, targ(p.d_o), targ(p.d_q), p.delta, delta_in);
+                 ? na2d_tc::backward_dq_bf16(lc, targ(p.q), targ(p.k), targ(p.v), p.lse, targ(p.d_o), targ(p.d_q), p.delta, have_estimate)
+                 : na2d_tc::backward_dq_f16(lc, targ(p.q), targ(p.k), targ(p.v), p.lse, targ(p.d_o), targ(p.d_q), p.delta, have_estimate);
         g_launches.fetch_add(launched);
         if (rc == NA2D_ERR_CUDA) return tc_fail("tcgen05 dQ launch");
         return rc;

@@ -20,7 +20,8 @@
 namespace na2d_tc {
 
 // Keys per chunk at most: the whole box where it fits 256 columns (a single unit); else what
-// leaves room in tensor memory for S, dP and the two output accumulators dQ and B.
+// leaves room in tensor memory for S, dP and dQ (192), or at D = 128 in shared memory for two K and
+// two V chunks beside Q and dO (128).
 constexpr int dq_nmax(int d, int ks) {
     return (TH + ks - 1) * (TW + ks - 1) <= 256 ? 256 : (d == 128 ? 128 : 192);
 }
@@ -441,17 +442,17 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
     }
 }
 
-// delta_in: row deltas formed beforehand (or null: the kernel forms them itself and writes `delta`).
+// have_estimate: `delta` holds an estimate of the row deltas, which the exact ones replace.
 template <typename DT, int D, int KS>
 int launch_dq(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
-              const TensorArg& d_o, const TensorArg& d_q, float* delta, const float* delta_in) {
+              const TensorArg& d_o, const TensorArg& d_q, float* delta, bool have_estimate) {
     // kernel sizes 3 and 5 with a dQ output go to the strip kernel, larger ones with an estimate of delta to the
     // pipelined kernel; this one keeps two walks and the delta-only call
     if constexpr (KS <= 5) {
         if (d_q.ptr != nullptr) return launch_dq1<DT, D, KS>(lc, q, k, v, lse, d_o, d_q, delta);
     } else {
-        if (d_q.ptr != nullptr && delta_in != nullptr)
-            return launch_dq2<DT, D, KS>(lc, q, k, v, lse, d_o, d_q, delta, delta_in);
+        if (d_q.ptr != nullptr && have_estimate)
+            return launch_dq2<DT, D, KS>(lc, q, k, v, lse, d_o, d_q, delta);
     }
     using C = DqCfg<D, KS, IsBf16<DT>::value>;
     const Na2dGeom& g = lc.g;

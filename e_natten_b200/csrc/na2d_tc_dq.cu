@@ -19,9 +19,9 @@ namespace na2d_tc {
 
 int NA2D_TC_NAME(backward_dq)(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v,
                               const float* lse, const TensorArg& d_o, const TensorArg& d_q, float* delta,
-                              const float* delta_in) {
+                              bool have_estimate) {
     const Na2dGeom& g = lc.g;
-    NA2D_TC_DISPATCH_D(launch_dq, NA2D_TC_TYPE, lc, q, k, v, lse, d_o, d_q, delta, delta_in)
+    NA2D_TC_DISPATCH_D(launch_dq, NA2D_TC_TYPE, lc, q, k, v, lse, d_o, d_q, delta, have_estimate)
 }
 
 }  // namespace na2d_tc

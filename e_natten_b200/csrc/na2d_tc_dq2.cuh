@@ -3,7 +3,7 @@
 // tile's chunks are walked once, and two chunks are in flight.
 //
 // One walk.  delta needs every chunk before any dS can be formed exactly.  The caller hands in an estimate d~ of it
-// (dO . o from the stored output, see na2d_delta.cuh; off by the rounding of o, a few 1e-2 at most).  Every
+// (in `delta`: dO . o from the stored output, see na2d_delta.cuh; off by the rounding of o, a few 1e-2 at most).  Every
 // unit forms dS~ = p (dP - d~), adds dS~ K_c to dQ and, with one more MMA, p K_c to a second accumulator B, while
 // the exact delta = sum_j p dP builds up in registers.  Since
 // sum_j p (dP - delta) k = sum_j p (dP - d~) k - (delta - d~) sum_j p k, the epilogue stores
@@ -59,8 +59,7 @@ template <typename DT, int D, int KS>
 __global__ void __launch_bounds__(384, 1)
 dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
            const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* __restrict__ delta,
-           const float* __restrict__ delta_in, unsigned int* __restrict__ err_word,
+           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* delta, unsigned int* __restrict__ err_word,
            const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = Dq2Cfg<D, KS>;
@@ -295,10 +294,10 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             const float lse2 = lse[qi] * kLog2e;
             float dl_part = 0.f;                             // this half's part of delta
             float dl = 0.f;                                  // delta, once every chunk has been seen
-            // The estimate is read before this tile's first partner barrier and the exact value
-            // written (by the partner warp of half 0, to the same address when delta_in == delta)
-            // after its last one, so the read never sees the new value.
-            const float d_est = delta_in[qi];
+            // delta holds the estimate here and the exact value afterwards.  It is read before this tile's first
+            // partner barrier and written (by the partner warp of half 0) after its last one, so the read never sees
+            // the new value: `delta` must not be declared __restrict__, which would let the read sink past those.
+            const float d_est = delta[qi];
 
             for (int ch = 0; ch < NCH; ++ch, ++n) {
                 const uint32_t tmem_buf = tmem_lane + (n & 1) * C::TMEM_BUF;
@@ -453,7 +452,7 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
 template <typename DT, int D, int KS>
 int launch_dq2(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
-               const TensorArg& d_o, const TensorArg& d_q, float* delta, const float* delta_in) {
+               const TensorArg& d_o, const TensorArg& d_q, float* delta) {
     using C = Dq2Cfg<D, KS>;
     const Na2dGeom& g = lc.g;
     CUtensorMap tq, tg, tk, tv, tdq;
@@ -470,7 +469,7 @@ int launch_dq2(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, cons
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, delta_in, lc.err_word, g, tiles_r, tiles_c,
+    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, lc.err_word, g, tiles_r, tiles_c,
                                         (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;

@@ -12,13 +12,13 @@ int forward_bf16(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, co
 int forward_f16(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const TensorArg& o,
                 float* lse);
 
-// dQ (d_q.ptr may be null: delta only).  The exact row deltas are written to `delta`.  delta_in, if
-// not null (it may be `delta` itself), holds an estimate of them (dO . o); the kernels of the
-// larger windows then walk their key box once and correct the result, instead of walking twice.
+// dQ (d_q.ptr may be null: delta only).  The exact row deltas are written to `delta`.  have_estimate: `delta`
+// holds an estimate of them (dO . o) beforehand; the kernels of the larger windows then walk their key box
+// once and correct the result, instead of walking twice.
 int backward_dq_bf16(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
-                     const TensorArg& d_o, const TensorArg& d_q, float* delta, const float* delta_in);
+                     const TensorArg& d_o, const TensorArg& d_q, float* delta, bool have_estimate);
 int backward_dq_f16(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
-                    const TensorArg& d_o, const TensorArg& d_q, float* delta, const float* delta_in);
+                    const TensorArg& d_o, const TensorArg& d_q, float* delta, bool have_estimate);
 
 int backward_dkdv_bf16(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v,
                        const float* lse, const TensorArg& d_o, const float* delta, const TensorArg& d_k,
