@@ -5,11 +5,14 @@
 The library is plain CUDA C++ behind a C ABI (include/na2d.h); it needs no framework headers.
 Its kernels are compiled as ten translation units in parallel (the API with the SIMT kernels, the
 tiled CUDA-core kernels once per element type, and each of the three tcgen05 kernel families once per
-16-bit element type) and linked into one shared object.
+16-bit element type) and linked into one shared object.  The Python package's extension module
+(_na2d_torch.so, host code over PyTorch's C++ API) is compiled beside it with g++; it belongs to one
+PyTorch and one Python version and is compiled again when either changes.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -44,17 +47,35 @@ def _nvcc() -> str:
     return exe
 
 
-def _deps():
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+EXT_SOURCE = "na2d_torch.cpp"
+
+
+def _deps(ext: bool):
+    """Sources of the extension module, or of the library."""
+    names = [EXT_SOURCE] if ext else [f for f in os.listdir(CSRC) if f != EXT_SOURCE]
+    deps = [os.path.join(CSRC, f) for f in names]
     deps.append(os.path.join(os.path.dirname(PKG_DIR), "include", "na2d.h"))
     return [d for d in deps if os.path.isfile(d)]
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(EXT_PATH):
+def _older(path: str, ext: bool) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in _deps(ext))
+
+
+def _ext_tag() -> str:
+    """What the extension module is compiled for; the module carries it as a string."""
+    return f"na2d_torch for torch {importlib.metadata.version('torch')}, {sys.implementation.cache_tag}"
+
+
+def _lib_stale() -> bool:
+    return _older(LIB_PATH, ext=False)
+
+
+def _ext_stale() -> bool:
+    if _older(EXT_PATH, ext=True):
         return True
-    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(EXT_PATH))
-    return any(os.path.getmtime(d) > built for d in _deps())
+    with open(EXT_PATH, "rb") as f:
+        return _ext_tag().encode() not in f.read()
 
 
 def _compile(unit, verbose: bool, extra, obj_dir):
@@ -69,10 +90,10 @@ def _compile_torch_ext():
     """The Python extension module over PyTorch's C++ API (host code only)."""
     import torch
     from torch.utils import cpp_extension
-    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[f"-I{p}" for p in (*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"])],
-           os.path.join(CSRC, "na2d_torch.cpp"), "-o", EXT_PATH,
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DNA2D_EXT_TAG="{_ext_tag()}"',
+           *[f"-isystem{p}" for p in (*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"])],
+           os.path.join(CSRC, EXT_SOURCE), "-o", EXT_PATH,
            *[f"-L{p}" for p in cpp_extension.library_paths("cuda")],
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
@@ -80,23 +101,29 @@ def _compile_torch_ext():
 
 
 def build(force: bool = False, verbose: bool = False, extra_flags=(), lib_path: str = LIB_PATH) -> str:
-    """Compile the library if it is missing or older than its sources; return its path."""
-    if not force and lib_path == LIB_PATH and not _stale():
-        return LIB_PATH
-    # a library built elsewhere with other flags (a development build) keeps its objects apart
-    obj_dir = OBJ_DIR if lib_path == LIB_PATH else lib_path + ".objs"
+    """Compile the library and the extension module where they are missing or out of date; return
+    the library's path."""
+    own = lib_path == LIB_PATH         # a library built elsewhere (a development build) has no extension module
+    build_lib = force or not own or _lib_stale()
+    build_ext = own and (force or _ext_stale())
+    if not (build_lib or build_ext):
+        return lib_path
+    # one with other flags keeps its objects apart
+    obj_dir = OBJ_DIR if own else lib_path + ".objs"
     os.makedirs(obj_dir, exist_ok=True)
-    workers = max(1, min(len(UNITS), os.cpu_count() or 1))
-    with concurrent.futures.ThreadPoolExecutor(workers) as pool:
-        ext = pool.submit(_compile_torch_ext) if lib_path == LIB_PATH else None
-        results = list(pool.map(lambda u: _compile(u, verbose, list(extra_flags), obj_dir), UNITS))
+    units = UNITS if build_lib else []
+    with concurrent.futures.ThreadPoolExecutor(max(1, min(len(UNITS), os.cpu_count() or 1))) as pool:
+        ext = pool.submit(_compile_torch_ext) if build_ext else None
+        results = list(pool.map(lambda u: _compile(u, verbose, list(extra_flags), obj_dir), units))
         if ext is not None:
             results.append(ext.result())
     for obj, rc, out, cmd in results:
         if verbose or rc != 0:
             sys.stderr.write(f"--- {obj}\n{out}")
         if rc != 0:
-            raise RuntimeError("nvcc failed building %s (command: %s)" % (obj, cmd))
+            raise RuntimeError("failed compiling %s (command: %s)" % (obj, cmd))
+    if not build_lib:
+        return lib_path
     link = [_nvcc(), "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a",
             *[os.path.join(obj_dir, u[2]) for u in UNITS], "-o", lib_path]
     proc = subprocess.run(link, capture_output=True, text=True)

@@ -137,6 +137,7 @@ std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_
 }  // namespace
 
 PYBIND11_MODULE(_na2d_torch, m) {
+    m.attr("built_for") = NA2D_EXT_TAG;         // looked for in the file by build.py
     m.def("bind_abi", &bind_abi);
     m.def("kernel_ready", &kernel_ready);
     m.def("strides", [](const Tensor& t) {      // (batch, heads, row, column), as they go into na2d_tensor

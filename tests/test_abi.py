@@ -157,3 +157,12 @@ def test_check_maps_status_to_exceptions():
     with pytest.raises(RuntimeError):
         _lib.check(_lib.ERR_KERNEL_WAIT)
     _lib.check(0)
+
+
+def test_build_is_stale_after_a_pytorch_change(monkeypatch):
+    """The extension module belongs to one PyTorch; the library does not."""
+    from e_natten_b200 import build
+    assert not build._lib_stale() and not build._ext_stale()
+    assert _lib.torch_ext.built_for == build._ext_tag()
+    monkeypatch.setattr(build.importlib.metadata, "version", lambda name: "9.9.9")
+    assert build._ext_stale() and not build._lib_stale()
