@@ -1,8 +1,6 @@
 // Launchers of the tiled CUDA-core kernels for one element type.
 #include "na2d_tile_entry.h"
 
-#include <type_traits>
-
 #include "../../include/na2d.h"
 #include "na2d_tile.cuh"
 #include "na2d_tile_bwd.cuh"
@@ -22,9 +20,6 @@ using Elem = __half;
 namespace na2d_tile {
 namespace {
 
-template <int V> using IntTag = std::integral_constant<int, V>;
-template <bool V> using BoolTag = std::integral_constant<bool, V>;
-
 // Four neighbouring channels can be moved at once: rows start on a boundary of four elements and hold a
 // multiple of four.
 Operand operand(const Tensor& t, int C) {
@@ -34,19 +29,22 @@ Operand operand(const Tensor& t, int C) {
     return Operand{t.ptr, t.st, vec ? 1 : 0};
 }
 
-// Calls f(kernel size tag, one-row tag).
-template <typename F>
-int by_window(const Na2dGeom& g, F&& f) {
-    auto with = [&](auto ks) -> int { return g.kh == 1 ? f(ks, BoolTag<true>{}) : f(ks, BoolTag<false>{}); };
+// Calls f(Shape) for the window size, of the 2D operator and the pair or of one-row images.
+template <bool ONE_D, typename F>
+int by_size(const Na2dGeom& g, F&& f) {
     switch (g.ks) {
-        case 3: return with(IntTag<3>{});
-        case 5: return with(IntTag<5>{});
-        case 7: return with(IntTag<7>{});
-        case 9: return with(IntTag<9>{});
-        case 11: return with(IntTag<11>{});
-        case 13: return with(IntTag<13>{});
+        case 3: return f(Shape<3, ONE_D>{});
+        case 5: return f(Shape<5, ONE_D>{});
+        case 7: return f(Shape<7, ONE_D>{});
+        case 9: return f(Shape<9, ONE_D>{});
+        case 11: return f(Shape<11, ONE_D>{});
+        case 13: return f(Shape<13, ONE_D>{});
         default: return NA2D_ERR_UNSUPPORTED;
     }
+}
+template <typename F>
+int by_window(const Na2dGeom& g, F&& f) {
+    return g.kh == 1 ? by_size<true>(g, f) : by_size<false>(g, f);
 }
 
 template <typename S>
@@ -71,8 +69,8 @@ int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream
 #if NA2D_TILE_DT == 0
 long long workspace_floats(const Na2dGeom& g) {
     long long floats = 0;
-    by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    by_window(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         floats = 2ll * ((g.Hq + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw) * S::kWeights * kR;
         return NA2D_OK;
     });
@@ -82,8 +80,8 @@ long long workspace_floats(const Na2dGeom& g) {
 
 int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
                        const Tensor& o, float* lse) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_window(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
         return launch(fwd_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
@@ -93,8 +91,8 @@ int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, cons
 
 int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
                            const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_window(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
         return launch(dq_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
@@ -106,8 +104,8 @@ int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, 
 int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
                         const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v, const float* lse,
                         float* delta, float* workspace, int units, int* launches) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_window(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         using K = KeyShape<S>;
         for (int unit0 = 0; unit0 < g.BN; unit0 += units) {
             const int here = g.BN - unit0 < units ? g.BN - unit0 : units;
@@ -130,33 +128,33 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
 }
 
 int NA2D_NAME(pair_dot)(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_size<false>(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(window_dot_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(x, g.C),
+        return launch(window_dot_kernel<Elem, S::kKs>, n, S::kThreads, S::kSmem, st, operand(x, g.C),
                       operand(y, g.C), (Elem*)attn, g);
     });
 }
 
 int NA2D_NAME(pair_apply)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_size<false>(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(window_apply_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, (const Elem*)attn,
+        return launch(window_apply_kernel<Elem, S::kKs>, n, S::kThreads, S::kSmem, st, (const Elem*)attn,
                       operand(y, g.C), operand(out, g.C), g);
     });
 }
 
 int NA2D_NAME(pair_inverse)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out) {
-    return by_window(g, [&](auto ks, auto one_d) -> int {
-        using S = Shape<decltype(ks)::value, decltype(one_d)::value>;
+    return by_size<false>(g, [&](auto shape) -> int {
+        using S = decltype(shape);
         using K = KeyShape<S>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hkv, &n)) return rc;
         const KeySum sum{attn, operand(x, g.C), operand(out, g.C)};
-        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, S::kOneD>, n, K::kThreads, K::kSmem, st, sum, sum, 0, g);
+        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, false>, n, K::kThreads, K::kSmem, st, sum, sum, 0, g);
     });
 }
 

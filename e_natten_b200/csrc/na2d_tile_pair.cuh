@@ -9,11 +9,11 @@ namespace na2d_tile {
 
 // ------------------------------------------------------------------------------------ unfused pair
 // attn[pixel, member] = x[pixel] . y[member of the pixel's window]
-template <typename T, int KS, bool ONE_D>
-__global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
+template <typename T, int KS>
+__global__ void __launch_bounds__(Shape<KS, false>::kThreads, Shape<KS, false>::kBlocks)
 window_dot_kernel(const __grid_constant__ Operand x, const __grid_constant__ Operand y, T* __restrict__ attn,
                   const __grid_constant__ Na2dGeom g) {
-    using S = Shape<KS, ONE_D>;
+    using S = Shape<KS, false>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *own = w + S::kWeights, *halo = own + S::kOwn;
     const Tile t = tile_of_block<S>(g, g.Hq, 0);
@@ -34,11 +34,11 @@ window_dot_kernel(const __grid_constant__ Operand x, const __grid_constant__ Ope
 }
 
 // out[pixel] = sum over the window of attn[pixel, member] * y[member]
-template <typename T, int KS, bool ONE_D>
-__global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
+template <typename T, int KS>
+__global__ void __launch_bounds__(Shape<KS, false>::kThreads, Shape<KS, false>::kBlocks)
 window_apply_kernel(const T* __restrict__ attn, const __grid_constant__ Operand y, const __grid_constant__ Operand out,
                     const __grid_constant__ Na2dGeom g) {
-    using S = Shape<KS, ONE_D>;
+    using S = Shape<KS, false>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *halo = w + S::kWeights + S::kOwn;
     const Tile t = tile_of_block<S>(g, g.Hq, 0);
