@@ -82,9 +82,10 @@ int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, cons
                        const Tensor& o, float* lse) {
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
+        const auto kernel = g.C > kParkAbove<S> ? fwd_kernel<Elem, S::kKs, S::kOneD, true> : fwd_kernel<Elem, S::kKs, S::kOneD, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(fwd_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(o, g.C), lse, g);
     });
 }
@@ -93,9 +94,10 @@ int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, 
                            const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta) {
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
+        const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(dq_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float4*)nullptr,
                       (float4*)nullptr, 0, g);
     });
@@ -106,13 +108,14 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
                         float* delta, float* workspace, int units, int* launches) {
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
+        const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
         using K = KeyShape<S>;
         for (int unit0 = 0; unit0 < g.BN; unit0 += units) {
             const int here = g.BN - unit0 < units ? g.BN - unit0 : units;
             float4 *p = reinterpret_cast<float4*>(workspace), *ds = p + workspace_floats(g) / 8 * here;
             unsigned n = 0;
             if (int rc = tiles<S>(g, here, g.Hq, &n)) return rc;
-            if (int rc = launch(dq_kernel<Elem, S::kKs, S::kOneD>, n, S::kThreads, S::kSmem, st, operand(q, g.C),
+            if (int rc = launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C),
                                 operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, p, ds,
                                 unit0, g))
                 return rc;
@@ -130,9 +133,10 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
 int NA2D_NAME(pair_dot)(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn) {
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
+        const auto kernel = g.C > kParkAbove<S> ? window_dot_kernel<Elem, S::kKs, true> : window_dot_kernel<Elem, S::kKs, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(window_dot_kernel<Elem, S::kKs>, n, S::kThreads, S::kSmem, st, operand(x, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(x, g.C),
                       operand(y, g.C), (Elem*)attn, g);
     });
 }

@@ -6,8 +6,8 @@
 // through shared memory 32 at a time (always as fp32): the tile's own rows and the halo of rows its
 // windows reach.  Two loops do all the work:
 //   dot    a thread holds the scores of a strip of four neighbouring pixels against one window row:
-//          4 own and ks + 3 halo float4 loads feed 16 * ks multiply-adds.  No cross-lane sums: the
-//          scores stay in registers over all channel chunks.
+//          4 own and ks + 3 halo float4 loads feed 16 * ks multiply-adds.  No cross-lane sums: a score
+//          is summed by one thread (four in 1D) over all channels.
 //   apply  a thread holds 4 pixels x 4 channels of an output; per window row, ks + 3 halo float4 and as
 //          many weight float4 (the strip's four weights for that halo column; a broadcast to the
 //          eight lanes that share the strip) feed the same 16 * ks multiply-adds.
@@ -15,8 +15,8 @@
 // issues 16 warp multiply-adds): the strip is what brings the loads per multiply-add down.
 //
 // Measured on one B200 against one warp per pixel with the channels over its lanes (na2d_simt.cuh, four loads and a
-// butterfly of shuffles per 32 products), fp32: forward 4 x 4 x 256 x 256 x 128, window 5, 3.85 -> 0.79 ms;
-// 4 x 4 x 117 x 93 x 64, window 7, 0.75 -> 0.14 ms.
+// butterfly of shuffles per 32 products), fp32: forward 4 x 4 x 256 x 256 x 128, window 5, 3.85 -> 0.84 ms;
+// 4 x 4 x 117 x 93 x 64, window 7, 0.75 -> 0.15 ms.
 //
 // Windows are clamped at the borders, so the four windows of a strip need not be shifted by one
 // column each.  A strip away from the borders ("regular") takes loops whose band is known at compile
@@ -257,18 +257,74 @@ __device__ __forceinline__ float sum2(unsigned long long a) {
     return __uint_as_float((unsigned)a) + __uint_as_float((unsigned)(a >> 32));
 }
 
-// acc[r][j] += own pixel r . halo column j over one staged chunk, eight channels at a time: their products are
-// summed in packed pairs first and join acc as one number.  That keeps the running sum short (C / 8 roundings, as
-// few as a sum over the lanes of a warp has) and takes six instructions where eight multiply-adds would stand.
+// Scores of a thread over the channels so far, parked in its local memory (PARK kernels).  A running sum over all C
+// channels would round at every step at its full size: 1.25 times the error of a sum over the lanes of a warp
+// (na2d_simt.cuh) at C = 128, 1.44 times at 256.  Instead the registers sum at most 32 channels (64 where a strip's channels
+// lie over four threads); their sum then joins the parked one, and what that addition rounds off starts the next.  Error
+// on normal rows against the lanes' sum: at most 0.99 times up to C = 96, 0.95 at 128, 0.86 at 256.  Registers or shared
+// memory for both sums would take a block per SM.  In local memory they cost 4 to 12 % of a kernel's time, in tensor
+// memory (allocated and freed by every block) 7 to 20 %.
+// Where the lines lie: up to 32 channels (64 with four threads to a strip) the running sum rounds no more than the
+// lanes' sum, 0.96 (0.99) times, and the kernels without parking are 1 to 5 % (8 to 11 %) faster there.
+template <typename S>
+constexpr int kParkAbove = S::kSplit > 1 ? 2 * kChunk : kChunk;
 template <typename S, bool REGULAR>
+__device__ __forceinline__ float& score(float (&acc)[kR][S::kU], int i) {      // a regular strip has a band of them
+    return REGULAR ? acc[i / S::kKs][i / S::kKs + i % S::kKs] : acc[i / S::kU][i % S::kU];
+}
+template <typename S, bool REGULAR>
+constexpr int kScores = kR * (REGULAR ? S::kKs : S::kU);
+template <typename S, bool REGULAR>
+__device__ __forceinline__ void park(float (&acc)[kR][S::kU], float4* parked, bool first) {
+#pragma unroll
+    for (int i = 0; i < kScores<S, REGULAR>; i += 4) {
+        const float4 old = first ? make_float4(0.f, 0.f, 0.f, 0.f) : parked[i / 4];
+        float sum[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float& a = score<S, REGULAR>(acc, i + e);
+            const float total = __fadd_rn(sum[e], a);
+            a = fabsf(total) <= FLT_MAX ? __fsub_rn(a, __fsub_rn(total, sum[e])) : 0.f;      // an infinite sum stays one
+            sum[e] = total;
+        }
+        parked[i / 4] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+    }
+}
+template <typename S, bool REGULAR>
+__device__ __forceinline__ void unpark(float (&acc)[kR][S::kU], const float4* parked) {
+#pragma unroll
+    for (int i = 0; i < kScores<S, REGULAR>; i += 4) {
+        const float4 sum = parked[i / 4];
+        score<S, REGULAR>(acc, i) += sum.x;
+        score<S, REGULAR>(acc, i + 1) += sum.y;
+        score<S, REGULAR>(acc, i + 2) += sum.z;
+        score<S, REGULAR>(acc, i + 3) += sum.w;
+    }
+}
+// Steps (of eight channels) of the chunk at channel c0 after which a PARK kernel parks, 0 for none: as few times as the error
+// allows.  Up to 64 channels that is the middle of each chunk, since 16 + 32 + 16 round less than 32 + 32, beyond
+// that its end; where a strip's channels lie over four threads, every other chunk from 128 on.
+template <typename S>
+constexpr int kSteps = kF / 2 / S::kSplit;
+template <typename S>
+__device__ __forceinline__ int park_after(int c0, int C) {
+    if (C <= 2 * kChunk) return c0 + kChunk / 2 < C ? kSteps<S> / 2 : 0;
+    const bool every = S::kSplit == 1 || C < 4 * kChunk;
+    return c0 + kChunk < C && (every || c0 % (2 * kChunk) != 0) ? kSteps<S> : 0;
+}
+
+// acc[r][j] += own pixel r . halo column j over one staged chunk, eight channels at a time: their products are
+// summed in packed pairs first and join acc as one number: six instructions where eight multiply-adds would stand, and
+// one rounding of acc.
+template <typename S, bool REGULAR, bool PARK>
 __device__ __forceinline__ void dot_chunk(float (&acc)[kR][S::kU], const float4* own, int row, int strip,
-                                          const float4* halo, int hy, int hx, int split) {
-    constexpr int kSteps = kF / 2 / S::kSplit;
+                                          const float4* halo, int hy, int hx, int split, float4* parked, int park_at,
+                                          bool first) {
     const ulonglong2* own2 = reinterpret_cast<const ulonglong2*>(own);
     const ulonglong2* halo2 = reinterpret_cast<const ulonglong2*>(halo);
 #pragma unroll 1
-    for (int i = 0; i < kSteps; ++i) {
-        const int f = 2 * (split * kSteps + i);
+    for (int i = 0; i < kSteps<S>; ++i) {
+        const int f = 2 * (split * kSteps<S> + i);
         ulonglong2 q0[kR], q1[kR];
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
@@ -292,7 +348,9 @@ __device__ __forceinline__ void dot_chunk(float (&acc)[kR][S::kU], const float4*
             for (int r = 0; r < kR; ++r)
                 if (!REGULAR || (j >= r && j - r < S::kKs)) acc[r][j] += sum2(part[r]);
         }
+        if (PARK && S::kSplit == 1 && i + 1 == park_at) park<S, REGULAR>(acc, parked, first);
     }
+    if (PARK && S::kSplit > 1 && park_at != 0) park<S, REGULAR>(acc, parked, first);
 }
 
 // What a thread does in the dot loop: window row u of the strip `strip` of tile row `row`.
@@ -327,7 +385,7 @@ __device__ __forceinline__ float4* weight_slots(float4* w, const DotItem& d) {
 
 // Scores of the whole tile: own tensor x (tile pixels) against tensor y (halo), all channel chunks.
 // Ends with the halo holding y's last chunk and every thread past its reads.
-template <typename T, typename S>
+template <typename T, typename S, bool PARK>
 __device__ __forceinline__ void tile_dot(float (&acc)[kR][S::kU], const Operand& x, const Operand& y, float4* own,
                                          float4* halo, const Tile& t, const DotItem& d, const Na2dGeom& g, int ky0,
                                          int kx0, int halo_rows) {
@@ -339,16 +397,26 @@ __device__ __forceinline__ void tile_dot(float (&acc)[kR][S::kU], const Operand&
     const T* ys = unit<T>(y, t);
     const float4* own_px = own + (d.row * S::kTw + kR * d.strip) * kF;
     const float4* halo_px = halo + (d.hy * S::kHaloW + d.hx) * kF;
+    float4 local[PARK ? S::kU : 1];
+    float4* parked = local;
+    if constexpr (PARK) asm volatile("" : "+l"(parked));    // not in registers: those are needed for the loop
+    bool first = true;
     for (int c0 = 0; c0 < g.C; c0 += kChunk) {
         stage<T, S::kTh, S::kThreads, S::kTw>(own, xs, x.st, t.y0, t.rows, t.x0, g.W, c0, g.C, x.vec);
         stage<T, S::kTh, S::kThreads, S::kHaloW>(halo, ys, y.st, ky0, halo_rows, kx0, g.W, c0, g.C, y.vec);
         copies_done();
         __syncthreads();
         if (d.active) {
-            if (d.s.regular) dot_chunk<S, true>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split);
-            else dot_chunk<S, false>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split);
+            const int park_at = PARK ? park_after<S>(c0, g.C) : 0;
+            if (d.s.regular) dot_chunk<S, true, PARK>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split, parked, park_at, first);
+            else dot_chunk<S, false, PARK>(acc, own_px, d.row, d.strip, halo_px, d.hy, d.hx, d.split, parked, park_at, first);
+            first = first && park_at == 0;
         }
         __syncthreads();
+    }
+    if (PARK && !first) {
+        if (d.s.regular) unpark<S, true>(acc, parked);
+        else unpark<S, false>(acc, parked);
     }
     if constexpr (S::kSplit > 1) {
 #pragma unroll
@@ -467,17 +535,14 @@ __device__ __forceinline__ void for_each_weight(const Tile& t, const Na2dGeom& g
     }
 }
 
-// Sum of a strip's per-window-row values, in two partial sums.
+// Sum of a strip's per-window-row values, in four partial sums.
 template <typename S>
 __device__ __forceinline__ float4 sum_rows(const float4* v) {
-    float4 s[2] = {};
+    float4 s[4] = {};
+    auto add = [](float4 a, float4 x) { return make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w); };
 #pragma unroll
-    for (int u = 0; u < S::kKh; ++u) {
-        const float4 x = v[u * S::kTh];
-        float4& a = s[u & 1];
-        a = make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w);
-    }
-    return make_float4(s[0].x + s[1].x, s[0].y + s[1].y, s[0].z + s[1].z, s[0].w + s[1].w);
+    for (int u = 0; u < S::kKh; ++u) s[u & 3] = add(s[u & 3], v[u * S::kTh]);
+    return add(add(s[0], s[1]), add(s[2], s[3]));
 }
 
 // Rows and columns of the halo of a tile of queries.
@@ -489,7 +554,7 @@ __device__ __forceinline__ void query_halo(const Tile& t, const Na2dGeom& g, int
 }
 
 // ------------------------------------------------------------------------------------ forward
-template <typename T, int KS, bool ONE_D>
+template <typename T, int KS, bool ONE_D, bool PARK>
 __global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
 fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, const __grid_constant__ Operand v,
            const __grid_constant__ Operand o, float* __restrict__ lse, const __grid_constant__ Na2dGeom g) {
@@ -501,7 +566,7 @@ fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k,
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     const DotItem d = dot_item<S>(t, g, ky0, kx0);
     float s[kR][S::kU];
-    tile_dot<T, S>(s, q, k, own, halo, t, d, g, ky0, kx0, halo_rows);
+    tile_dot<T, S, PARK>(s, q, k, own, halo, t, d, g, ky0, kx0, halo_rows);
 
     // Softmax over the kKh threads that share a strip, through the own-pixel buffer: row maxima and sums.
     float4 *mx = own, *sum = own + S::kTh * S::kStrips * S::kKh, *inv = sum + S::kTh * S::kStrips * S::kKh;
@@ -527,7 +592,7 @@ fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k,
             const float4 x = mx[(d.strip * S::kKh + u) * S::kTh + d.row];
             m4 = make_float4(fmaxf(m4.x, x.x), fmaxf(m4.y, x.y), fmaxf(m4.z, x.z), fmaxf(m4.w, x.w));
         }
-        float l[2][kR] = {};                                // two short sums instead of a long one
+        float l[4][kR] = {};                                // four short sums instead of a long one
         float4* slots = weight_slots<S>(w, d);
 #pragma unroll
         for (int j = 0; j < S::kU; ++j) {
@@ -535,11 +600,12 @@ fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k,
 #pragma unroll
             for (int r = 0; r < kR; ++r) {
                 e[r] = in_window<KS>(d.s, r, j) ? expf(s[r][j] - lane_of(m4, r)) : 0.f;
-                l[j & 1][r] += e[r];
+                l[j & 3][r] += e[r];
             }
             if (j % S::kSplit == d.split) slots[j * S::kTh] = make_float4(e[0], e[1], e[2], e[3]);
         }
-        if (d.split == 0) sum[slot] = make_float4(l[0][0] + l[1][0], l[0][1] + l[1][1], l[0][2] + l[1][2], l[0][3] + l[1][3]);
+        auto total = [&](int r) { return (l[0][r] + l[1][r]) + (l[2][r] + l[3][r]); };
+        if (d.split == 0) sum[slot] = make_float4(total(0), total(1), total(2), total(3));
     }
     __syncthreads();
     if (d.active && d.u == 0 && d.split == 0) {

@@ -4,7 +4,7 @@
 // What bounds them: the shared-memory pipe and block barriers in the query half (three loops of the forward's kind),
 // issue slots in the key sums.  Keeping P and dS (2 ks * ks floats per pixel) costs less than the two score loops
 // that would form them again.  Measured on one B200 against the warp-per-pixel kernels, 4 x 4 x 256 x 256 x 128,
-// window 5, fp32: both halves 27.6 -> 2.14 ms; 4 x 8 x 4096 x 64, window 13, bf16, 1D: step 1.72 -> 0.29 ms.
+// window 5, fp32: both halves 27.6 -> 2.24 ms; 4 x 8 x 4096 x 64, window 13, bf16, 1D: step 1.72 -> 0.29 ms.
 #pragma once
 
 #include "na2d_tile.cuh"
@@ -15,7 +15,7 @@ namespace na2d_tile {
 // delta = sum_j p_j dp_j, which equals dO . o exactly and does not depend on how o was rounded when it
 // was stored.  d_q may be null: then only delta (and the weights) are produced.  p_out / ds_out, both or
 // neither: the tiles' weight slots for the key half, as they lie in shared memory, tile after tile.
-template <typename T, int KS, bool ONE_D>
+template <typename T, int KS, bool ONE_D, bool PARK>
 __global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
 dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, const __grid_constant__ Operand v,
           const __grid_constant__ Operand d_o, const __grid_constant__ Operand d_q, const float* __restrict__ lse,
@@ -34,13 +34,13 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
     float s[kR][S::kU];
     // dP first, parked in the thread's own weight slots; the scores second, so that the halo ends up
     // holding a chunk of k, which dQ needs next
-    tile_dot<T, S>(s, d_o, v, own, halo, t, d, g, ky0, kx0, halo_rows);
+    tile_dot<T, S, PARK>(s, d_o, v, own, halo, t, d, g, ky0, kx0, halo_rows);
     if (d.active) {
 #pragma unroll
         for (int j = 0; j < S::kU; ++j)
             if (j % S::kSplit == d.split) slots[j * S::kTh] = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
     }
-    tile_dot<T, S>(s, q, k, own, halo, t, d, g, ky0, kx0, halo_rows);
+    tile_dot<T, S, PARK>(s, q, k, own, halo, t, d, g, ky0, kx0, halo_rows);
     float4 *part = own, *total = own + S::kTh * S::kStrips * S::kKh;
     if (d.active) {
         float dl[2][kR], l[2][kR];                          // two short sums instead of a long one

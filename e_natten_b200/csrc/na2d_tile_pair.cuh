@@ -1,6 +1,6 @@
 // Tiled CUDA-core kernels of the unfused pair (scores, apply); its key-side gradients are key sums.
 // Measured on one B200 against the warp-per-pixel kernels: step of 4 x 4 x 64 x 64 x 128, window 5, fp32
-// 0.80 -> 0.41 ms, the softmax between the two calls included.
+// 0.80 -> 0.43 ms, the softmax between the two calls included.
 #pragma once
 
 #include "na2d_tile.cuh"
@@ -9,7 +9,7 @@ namespace na2d_tile {
 
 // ------------------------------------------------------------------------------------ unfused pair
 // attn[pixel, member] = x[pixel] . y[member of the pixel's window]
-template <typename T, int KS>
+template <typename T, int KS, bool PARK>
 __global__ void __launch_bounds__(Shape<KS, false>::kThreads, Shape<KS, false>::kBlocks)
 window_dot_kernel(const __grid_constant__ Operand x, const __grid_constant__ Operand y, T* __restrict__ attn,
                   const __grid_constant__ Na2dGeom g) {
@@ -21,7 +21,7 @@ window_dot_kernel(const __grid_constant__ Operand x, const __grid_constant__ Ope
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     const DotItem d = dot_item<S>(t, g, ky0, kx0);
     float s[kR][S::kU];
-    tile_dot<T, S>(s, x, y, own, halo, t, d, g, ky0, kx0, halo_rows);
+    tile_dot<T, S, PARK>(s, x, y, own, halo, t, d, g, ky0, kx0, halo_rows);
     if (d.active) {
         float4* slots = weight_slots<S>(w, d);
 #pragma unroll
