@@ -55,6 +55,12 @@ int tiles(const Na2dGeom& g, int units, int H, unsigned* n) {
     return NA2D_OK;
 }
 
+template <typename S>
+Band whole_images(const Na2dGeom& g, int H) {
+    const int rows = (H + S::kTh - 1) / S::kTh;
+    return Band{0, 0, rows, rows};
+}
+
 template <typename... P, typename... A>
 int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
     if (smem > 48 * 1024 &&
@@ -66,15 +72,63 @@ int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream
 
 }  // namespace
 
+// ---- how the backward's workspace is shared out -------------------------------------------------------
+namespace {
+
+template <typename S> int tile_rows(const Na2dGeom& g) { return (g.Hq + S::kTh - 1) / S::kTh; }
+// fp32 values of P and dS of a row of tiles.
+template <typename S> long long row_floats(const Na2dGeom& g) {
+    return 2ll * ((g.W + S::kTw - 1) / S::kTw) * S::kWeights * kR;
+}
+// First and last row of query tiles that a row of key tiles reads.
+template <typename S> int first_query_row(int row) { return na2d_bws(row * S::kTh, S::kKh) / S::kTh; }
+template <typename S> int last_query_row(const Na2dGeom& g, int row) {
+    const int last_key = (row + 1) * S::kTh < g.Hkv ? (row + 1) * S::kTh - 1 : g.Hkv - 1;
+    return (na2d_bwe(last_key, g.Hg, S::kKh) - 1) / S::kTh;
+}
+// Tile rows that the weights need at least, one unit at a time.
+template <typename S> int least_rows(const Na2dGeom& g) {
+    int least = 1;
+    for (int row = 0; row < tile_rows<S>(g); ++row) {
+        const int n = last_query_row<S>(g, row) - first_query_row<S>(row) + 1;
+        if (n > least) least = n;
+    }
+    return least;
+}
+
+}  // namespace
+
 #if NA2D_TILE_DT == 0
-long long workspace_floats(const Na2dGeom& g) {
+long long workspace_floats(const Na2dGeom& g, long long limit) {
     long long floats = 0;
     by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
-        floats = 2ll * ((g.Hq + S::kTh - 1) / S::kTh) * ((g.W + S::kTw - 1) / S::kTw) * S::kWeights * kR;
+        const long long row = row_floats<S>(g), unit = row * tile_rows<S>(g);
+        const long long units = limit / unit < g.BN ? limit / unit : g.BN;
+        if (units > 0) {
+            floats = units * unit;
+        } else {
+            const long long rows = limit / row, least = least_rows<S>(g);
+            floats = row * (rows > least ? rows : least);
+        }
         return NA2D_OK;
     });
     return floats;
+}
+
+Turns workspace_turns(const Na2dGeom& g, long long floats) {
+    Turns t{0, 0};
+    by_window(g, [&](auto shape) -> int {
+        using S = decltype(shape);
+        const long long row = row_floats<S>(g), unit = row * tile_rows<S>(g);
+        if (floats >= unit) {
+            t = Turns{(int)(floats / unit < g.BN ? floats / unit : g.BN), tile_rows<S>(g)};
+        } else if (floats / row >= least_rows<S>(g)) {
+            t = Turns{1, (int)(floats / row)};
+        }
+        return NA2D_OK;
+    });
+    return t;
 }
 #endif
 
@@ -99,32 +153,47 @@ int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, 
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
         return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float4*)nullptr,
-                      (float4*)nullptr, 0, g);
+                      (float4*)nullptr, whole_images<S>(g, g.Hq), g);
     });
 }
 
 int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
                         const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v, const float* lse,
-                        float* delta, float* workspace, int units, int* launches) {
+                        float* delta, float* workspace, Turns turns, int* launches) {
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
         const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
         using K = KeyShape<S>;
-        for (int unit0 = 0; unit0 < g.BN; unit0 += units) {
-            const int here = g.BN - unit0 < units ? g.BN - unit0 : units;
-            float4 *p = reinterpret_cast<float4*>(workspace), *ds = p + workspace_floats(g) / 8 * here;
-            unsigned n = 0;
-            if (int rc = tiles<S>(g, here, g.Hq, &n)) return rc;
-            if (int rc = launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C),
-                                operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, p, ds,
-                                unit0, g))
-                return rc;
-            ++*launches;
+        const int all_rows = tile_rows<S>(g), tiles_w = (g.W + S::kTw - 1) / S::kTw;
+        for (long long unit0 = 0; unit0 < g.BN; unit0 += turns.units) {
+            const int units = (int)(g.BN - unit0 < turns.units ? g.BN - unit0 : turns.units);
+            float4 *p = reinterpret_cast<float4*>(workspace), *ds = p + (long long)units * turns.rows * tiles_w * S::kWeights;
             const KeySum for_dk{ds, operand(q, g.C), operand(d_k, g.C)}, for_dv{p, operand(d_o, g.C), operand(d_v, g.C)};
-            if (int rc = launch(key_sum_kernel<Elem, float, true, S::kKs, S::kOneD>, dim3(n, 2), K::kThreads, K::kSmem, st, for_dk,
-                                for_dv, unit0, g))
-                return rc;
-            ++*launches;
+            // Query tiles as far as the ring has room without losing a row that the next key tiles read, then the
+            // key tiles that have all their queries; in one go where the ring holds the whole image.
+            for (int keys = 0, queries = 0; keys < all_rows;) {
+                const int room = first_query_row<S>(keys) + turns.rows, query_end = room < all_rows ? room : all_rows;
+                int key_end = keys;
+                while (key_end < all_rows && last_query_row<S>(g, key_end) < query_end) ++key_end;
+                if (key_end == keys) return NA2D_ERR_BAD_ARG;              // a ring below least_rows()
+                const Band query_band{(int)unit0, queries, query_end - queries, turns.rows};
+                const Band key_band{(int)unit0, keys, key_end - keys, turns.rows};
+                unsigned n = 0;
+                if (query_band.rows > 0) {
+                    if (int rc = tiles<S>(g, units, query_band.rows * S::kTh, &n)) return rc;
+                    if (int rc = launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C), operand(v, g.C),
+                                        operand(d_o, g.C), operand(d_q, g.C), lse, delta, p, ds, query_band, g))
+                        return rc;
+                    ++*launches;
+                }
+                if (int rc = tiles<S>(g, units, key_band.rows * S::kTh, &n)) return rc;
+                if (int rc = launch(key_sum_kernel<Elem, float, true, S::kKs, S::kOneD>, dim3(n, 2), K::kThreads, K::kSmem, st,
+                                    for_dk, for_dv, key_band, g))
+                    return rc;
+                ++*launches;
+                keys = key_end;
+                queries = query_end;
+            }
         }
         return NA2D_OK;
     });
@@ -158,7 +227,7 @@ int NA2D_NAME(pair_inverse)(const Na2dGeom& g, cudaStream_t st, const void* attn
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hkv, &n)) return rc;
         const KeySum sum{attn, operand(x, g.C), operand(out, g.C)};
-        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, false>, n, K::kThreads, K::kSmem, st, sum, sum, 0, g);
+        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, false>, n, K::kThreads, K::kSmem, st, sum, sum, whole_images<S>(g, g.Hkv), g);
     });
 }
 

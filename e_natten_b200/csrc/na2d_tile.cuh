@@ -199,24 +199,34 @@ __device__ __forceinline__ void stage(float4* dst, const T* src, const Na2dStrid
     }
 }
 
-// Tile of this block in a (BN, H, W) grid of pixels; the launch covers the units from `unit0` on.
+// The tiles of a launch: tile rows [row0, row0 + rows) of each unit from `unit0` on.  `ring`: tile rows of a unit that the
+// weights handed from the query half to the key half have room for; row r lies in place r % ring.
+struct Band {
+    int unit0, row0, rows, ring;
+};
+
+// Tile of this block in a (BN, H, W) grid of pixels.
 struct Tile {
     int bn, b, n, y0, x0, rows, cols;
 };
 template <typename S>
-__device__ __forceinline__ Tile tile_of_block(const Na2dGeom& g, int H, int unit0) {
-    const unsigned tw = (unsigned)(g.W + S::kTw - 1) / S::kTw, th = (unsigned)(H + S::kTh - 1) / S::kTh;
+__device__ __forceinline__ Tile tile_of_block(const Na2dGeom& g, int H, int unit0, unsigned row0, unsigned th) {
+    const unsigned tw = (unsigned)(g.W + S::kTw - 1) / S::kTw;
     unsigned blk = blockIdx.x;
     Tile t;
     t.x0 = (int)(blk % tw) * S::kTw;
     blk /= tw;
-    t.y0 = (int)(blk % th) * S::kTh;
+    t.y0 = (int)(row0 + blk % th) * S::kTh;
     t.bn = unit0 + (int)(blk / th);
     t.b = t.bn / g.N;
     t.n = t.bn - t.b * g.N;
     t.rows = min(S::kTh, H - t.y0);
     t.cols = min(S::kTw, g.W - t.x0);
     return t;
+}
+template <typename S>
+__device__ __forceinline__ Tile tile_of_block(const Na2dGeom& g, int H) {
+    return tile_of_block<S>(g, H, 0, 0, (unsigned)(H + S::kTh - 1) / S::kTh);
 }
 template <typename T>
 __device__ __forceinline__ T* unit(const Operand& o, const Tile& t) {
@@ -561,7 +571,7 @@ fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k,
     using S = Shape<KS, ONE_D>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *own = w + S::kWeights, *halo = own + S::kOwn;
-    const Tile t = tile_of_block<S>(g, g.Hq, 0);
+    const Tile t = tile_of_block<S>(g, g.Hq);
     int ky0, kx0, halo_rows;
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     const DotItem d = dot_item<S>(t, g, ky0, kx0);

@@ -14,17 +14,18 @@ namespace na2d_tile {
 // ------------------------------------------------------------------------------------ dQ (+ delta, P, dS)
 // delta = sum_j p_j dp_j, which equals dO . o exactly and does not depend on how o was rounded when it
 // was stored.  d_q may be null: then only delta (and the weights) are produced.  p_out / ds_out, both or
-// neither: the tiles' weight slots for the key half, as they lie in shared memory, tile after tile.
+// neither: the tiles' weight slots for the key half, as they lie in shared memory, tile after tile in the rows of
+// `band`'s ring.
 template <typename T, int KS, bool ONE_D, bool PARK>
 __global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
 dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, const __grid_constant__ Operand v,
           const __grid_constant__ Operand d_o, const __grid_constant__ Operand d_q, const float* __restrict__ lse,
-          float* __restrict__ delta, float4* __restrict__ p_out, float4* __restrict__ ds_out, const int unit0,
-          const __grid_constant__ Na2dGeom g) {
+          float* __restrict__ delta, float4* __restrict__ p_out, float4* __restrict__ ds_out,
+          const __grid_constant__ Band band, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS, ONE_D>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *own = w + S::kWeights, *halo = own + S::kOwn;
-    const Tile t = tile_of_block<S>(g, g.Hq, unit0);
+    const Tile t = tile_of_block<S>(g, g.Hq, band.unit0, band.row0, band.rows);
     int ky0, kx0, halo_rows;
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     const DotItem d = dot_item<S>(t, g, ky0, kx0);
@@ -101,9 +102,11 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
             for (int r = 0; r < kR; ++r) s[r][j] = g.scale * s[r][j] * (lane_of(dp, r) - lane_of(dl4, r));
         }
     }
+    const long long place = (((long long)(t.bn - band.unit0) * band.ring + t.y0 / S::kTh % band.ring) *
+                                 ((g.W + S::kTw - 1) / S::kTw) + t.x0 / S::kTw) * S::kWeights;
     if (p_out) {
         __syncthreads();
-        for (int i = threadIdx.x; i < S::kWeights; i += S::kThreads) p_out[(long long)blockIdx.x * S::kWeights + i] = w[i];
+        for (int i = threadIdx.x; i < S::kWeights; i += S::kThreads) p_out[place + i] = w[i];
         __syncthreads();
     }
     if (d.active) {
@@ -113,7 +116,7 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
     }
     if (ds_out) {
         __syncthreads();
-        for (int i = threadIdx.x; i < S::kWeights; i += S::kThreads) ds_out[(long long)blockIdx.x * S::kWeights + i] = w[i];
+        for (int i = threadIdx.x; i < S::kWeights; i += S::kThreads) ds_out[place + i] = w[i];
     }
     if (d_q.ptr) tile_apply<T, S>(d_q, k, w, nullptr, halo, t, g, ky0, kx0, halo_rows, true);
 }
@@ -121,8 +124,8 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
 // ------------------------------------------------------------------------------------ key side
 // out[key] = sum over the queries i whose window holds the key of attn[i, position of the key in i's window]
 // * x[i]: dK (attn = dS, x = q) and dV (attn = P, x = dO).  Two such sums run in one launch (blockIdx.y).
-// Whole images only; attn starts at unit `unit0`, the launch's first: the dense (units, H, W, kh * ks) array of the
-// unfused pair, or (TILED) the weight slots of query tiles that dq_kernel wrote.
+// Whole images only; attn starts at the launch's first unit: the dense (units, H, W, kh * ks) array of the
+// unfused pair, or (TILED) the weight slots of query tiles that dq_kernel wrote, in the rows of `band`'s ring.
 //
 // The queries that see a key are a product of a row range and a column range: ks x ks away from the
 // borders, up to (3 * ks / 2) on a side near them.  A strip of four keys away from the borders meets a band
@@ -177,15 +180,15 @@ struct KeySum {
 
 template <typename T, typename TW, bool TILED, int KS, bool ONE_D>
 __global__ void __launch_bounds__(KeyShape<Shape<KS, ONE_D>>::kThreads, KeyShape<Shape<KS, ONE_D>>::kBlocks)
-key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ KeySum second, const int unit0,
-               const __grid_constant__ Na2dGeom g) {
+key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ KeySum second,
+               const __grid_constant__ Band band, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS, ONE_D>;
     using K = KeyShape<S>;
     constexpr int kTaps = S::kKh * KS;
     extern __shared__ float4 smem[];
     float4 *w = smem, *halo = w + K::kWeights;
     const KeySum& job = blockIdx.y == 0 ? first : second;
-    const Tile t = tile_of_block<S>(g, g.Hkv, unit0);
+    const Tile t = tile_of_block<S>(g, g.Hkv, band.unit0, band.row0, band.rows);
     const int H = g.Hg, W = g.W;
     // query rows and columns the tile's keys meet
     const int qy0 = na2d_bws(t.y0, S::kKh), qx0 = na2d_bws(t.x0, KS);
@@ -214,9 +217,10 @@ key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ Key
     const int my_u0 = na2d_bws(t.y0 + min(row, t.rows - 1), S::kKh), my_nu = na2d_bwe(t.y0 + min(row, t.rows - 1), H, S::kKh) - my_u0;
     const int hx = s.start - qx0;
 
-    const int tiles_w = (W + S::kTw - 1) / S::kTw, tiles_h = (H + S::kTh - 1) / S::kTh;
+    const int tiles_w = (W + S::kTw - 1) / S::kTw;
+    const unsigned first_tile_row = (unsigned)qy0 / S::kTh, first_place = first_tile_row % (unsigned)band.ring;
     const TW* attn = static_cast<const TW*>(job.attn) +
-                     (t.bn - unit0) * (TILED ? (long long)tiles_h * tiles_w * S::kWeights * kR : (long long)H * W * kTaps);
+                     (t.bn - band.unit0) * (TILED ? (long long)band.ring * tiles_w * S::kWeights * kR : (long long)H * W * kTaps);
     const T* xs = unit<T>(job.x, t);
     T* os = unit<T>(job.out, t);
     for (int ch = 0; ch < g.C; ch += kChunk) {
@@ -250,8 +254,10 @@ key_sum_kernel(const __grid_constant__ KeySum first, const __grid_constant__ Key
                     if constexpr (TILED) {
                         // query (qy, qx): tile (qy / kTh, qx / kTw), strip and pixel r of its column, row qy % kTh;
                         // the key is column col - (window start of the strip) of its halo
-                        const unsigned tile_row = (unsigned)qy / S::kTh, in_row = (unsigned)qy % S::kTh;
-                        const TW* line = attn + ((long long)(tile_row * (unsigned)tiles_w) * S::kWeights + uq * (S::kU * S::kTh) + in_row) * kR;
+                        const unsigned in_row = (unsigned)qy % S::kTh;
+                        unsigned place = first_place + (unsigned)qy / S::kTh - first_tile_row;
+                        if (place >= (unsigned)band.ring) place -= band.ring;
+                        const TW* line = attn + ((long long)(place * (unsigned)tiles_w) * S::kWeights + uq * (S::kU * S::kTh) + in_row) * kR;
 #pragma unroll 4
                         for (int i = 0; i < n; ++i, to += S::kTh * kR) {
                             const unsigned qx = lo + i, strip_q = qx % S::kTw / kR;

@@ -19,11 +19,20 @@ struct Tensor {
 // wants another shape, which is not built.
 inline bool supported(int ks) { return ks == 3 || ks == 5 || ks == 7 || ks == 9 || ks == 11 || ks == 13; }
 
-// fp32 values of P and dS that the backward of one unit hands from its query half to its key half.
-long long workspace_floats(const Na2dGeom& g);
+// How the backward hands P and dS from its query half to its key half: `units` (batch, head) units at a time, for each of
+// which a workspace has room for `rows` rows of tiles.  Where that is not the whole image, units is 1, and the halves
+// take turns, the rows of the workspace being used again as the key half is done with them.
+struct Turns {
+    int units, rows;
+};
+// fp32 values of workspace that the backward asks for: all of P and dS up to `limit` values, else as many whole
+// units, or whole rows of tiles of one unit, as fit (but no fewer than a row of key tiles reads: the weights of at most
+// 32 image rows; a one-row image cannot be cut).
+long long workspace_floats(const Na2dGeom& g, long long limit);
+// The turns a workspace of so many values allows; units is 0 if it is too small for any.
+Turns workspace_turns(const Na2dGeom& g, long long floats);
 
-// backward: both halves, for whole images; the workspace holds workspace_floats() of `units` units, which
-// are taken that many at a time.
+// backward: both halves, for whole images.
 // Status: 0, NA2D_ERR_TOO_LARGE (grid), or NA2D_ERR_CUDA (the launch's error is left for cudaGetLastError).
 #define NA2D_TILE_ENTRIES(suffix)                                                                                     \
     int forward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,       \
@@ -32,7 +41,7 @@ long long workspace_floats(const Na2dGeom& g);
                              const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta);                   \
     int backward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,      \
                           const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v,                 \
-                          const float* lse, float* delta, float* workspace, int units, int* launches);                \
+                          const float* lse, float* delta, float* workspace, Turns turns, int* launches);                \
     int pair_dot_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn);          \
     int pair_apply_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out); \
     int pair_inverse_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out);

@@ -16,7 +16,7 @@ window_dot_kernel(const __grid_constant__ Operand x, const __grid_constant__ Ope
     using S = Shape<KS, false>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *own = w + S::kWeights, *halo = own + S::kOwn;
-    const Tile t = tile_of_block<S>(g, g.Hq, 0);
+    const Tile t = tile_of_block<S>(g, g.Hq);
     int ky0, kx0, halo_rows;
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     const DotItem d = dot_item<S>(t, g, ky0, kx0);
@@ -41,7 +41,7 @@ window_apply_kernel(const T* __restrict__ attn, const __grid_constant__ Operand 
     using S = Shape<KS, false>;
     extern __shared__ float4 smem[];
     float4 *w = smem, *halo = w + S::kWeights + S::kOwn;
-    const Tile t = tile_of_block<S>(g, g.Hq, 0);
+    const Tile t = tile_of_block<S>(g, g.Hq);
     int ky0, kx0, halo_rows;
     query_halo<S>(t, g, ky0, kx0, halo_rows);
     float* wf = reinterpret_cast<float*>(w);

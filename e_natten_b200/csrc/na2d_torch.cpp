@@ -121,12 +121,16 @@ std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_
         if (d_k) { a.d_k = describe(*d_k); a.d_v = describe(*d_v); }
         a.lse = lse.data_ptr<float>();
         a.delta = delta.data_ptr<float>();
-        if (const size_t bytes = d_k ? abi.backward_workspace(&a) : 0) {
+        // Where memory is short, the halves take more turns with a smaller workspace; without any, the key half forms
+        // the weights again.
+        constexpr size_t kLeast = 1 << 20;
+        for (size_t bytes = d_k ? abi.backward_workspace(&a) : 0; bytes != 0; bytes = bytes / 2 < kLeast ? 0 : bytes / 2) {
             try {
                 workspace = at::empty({(int64_t)bytes}, q.options().dtype(at::kByte));
                 a.workspace = workspace.data_ptr();
                 a.workspace_bytes = bytes;
-            } catch (const c10::OutOfMemoryError&) {       // no room: the key half forms the weights again
+                break;
+            } catch (const c10::OutOfMemoryError&) {
             }
         }
         status = abi.backward(&a);

@@ -207,9 +207,12 @@ int na2d_backward_dkdv_ex(const na2d_args* a);
 int na2d_backward_ex(const na2d_args* a);
 /* Bytes of scratch that na2d_backward_ex can use for this problem as a->workspace / a->workspace_bytes, 0 where it
  * has no use for any.  Problems that run on CUDA cores (fp32, the 1D operator, head dims without tensor-core
- * kernels) keep their window weights P and dS there, in fp32, instead of forming them again in the key half;
- * without a workspace, or with one smaller than a single (batch, head) image needs, they form them again.  The
- * contents are of no use after the call.  No reference counterpart. */
+ * kernels) keep their window weights P and dS there, in fp32, instead of forming them again in the key half.
+ * At most 512 MiB, or the weights of 32 image rows (of a whole sequence in 1D) where those are more.  With less than
+ * this, the halves take turns over fewer images, or fewer rows of one image; the results are the same bit for bit.
+ * Without a workspace, or with one that does not hold the rows that 8 rows of keys meet (at most 32), the key half
+ * forms the weights again: slower, and other last bits of d_k and d_v.
+ * The contents are of no use after the call.  No reference counterpart. */
 size_t na2d_backward_workspace(const na2d_args* a);
 
 /* ---- 1D operator, dense tensors (B, N, T, C) ------------------------------------------------

@@ -106,6 +106,26 @@ def test_ex_entry_points_refuse_bad_arguments_without_touching_cuda():
     assert fwd(_args()) in (_lib.ERR_CUDA, _lib.ERR_NO_DEVICE)      # past validation: needs a GPU
 
 
+def test_header_without_workspace_fields():
+    """A struct_size that ends before the workspace fields is accepted, one byte less is not."""
+    base = _lib.Args.workspace.offset
+    assert _lib.lib.na2d_forward_ex(C.byref(_args(struct_size=base))) in (_lib.ERR_CUDA, _lib.ERR_NO_DEVICE)
+    assert _lib.lib.na2d_forward_ex(C.byref(_args(struct_size=base - 1))) == _lib.ERR_BAD_ARG
+
+
+def test_workspace_is_bounded():
+    """What the backward asks for: all weights where they are few, at most 512 MiB else (32 image rows if those are more)."""
+    ask = lambda **kw: _lib.lib.na2d_backward_workspace(C.byref(_args(**kw)))
+    weights = lambda H, W, ks: 2 * H * W * ks * (ks + 3) * 4           # P and dS, ks + 3 columns for four pixels
+    assert ask(dtype=0, H=64, W=64, B=2, N=3) == 6 * weights(64, 64, 5)
+    assert ask(dtype=0, H=64, W=64, B=200, N=3) <= 512 << 20
+    assert ask(dtype=0, op=_lib.OP_1D, H=1, W=4096, kernel_size=13) == 2 * 4096 * 16 * 4
+    for H, W, ks in ((1024, 1024, 13), (4096, 4096, 13), (16384, 2048, 3), (2000, 3000, 9)):
+        assert 128 << 20 <= ask(dtype=0, H=H, W=W, kernel_size=ks, B=2) <= 512 << 20
+    assert ask(dtype=0, H=1024, W=1 << 17, kernel_size=13) <= weights(32, 1 << 17, 13)
+    assert ask(C=64, H=64, W=64) == 0                                  # bf16 on tensor cores has no use for one
+
+
 def test_unfused_pair_and_1d_refuse_bad_arguments_without_touching_cuda():
     p = C.c_void_p(256)
     assert _lib.lib.na2d_qk_forward(None, p, p, 1, 1, 8, 8, 32, 5, 0, 0, None) == _lib.ERR_BAD_ARG

@@ -102,6 +102,76 @@ def test_workspace_of_any_size(ks, H, W):
         assert_close(g, w, torch.float32, what + " without workspace")
 
 
+def _backward(q, k, v, o, lse, d_o, ks, scale, bytes_of, path="auto"):
+    """Gradients with a workspace of bytes_of(what is asked for) bytes; nothing beyond it may be written."""
+    delta = torch.empty_like(lse)
+    grads = [torch.full_like(q, float("nan")) for _ in range(3)]
+    a = F._args(q, ks, None, path, scale, q=q, k=k, v=v, o=o, lse=lse, d_o=d_o, d_q=grads[0], d_k=grads[1], d_v=grads[2],
+                delta=delta)
+    n = bytes_of(_lib.lib.na2d_backward_workspace(C.byref(a))) // 4
+    scratch = torch.full((n + 4,), -1.0, device=DEV)
+    a.workspace, a.workspace_bytes = scratch.data_ptr(), 4 * n
+    before = na.launch_count()
+    _lib.check(_lib.lib.na2d_backward_ex(C.byref(a)))
+    assert bool((scratch[n:] == -1.0).all())
+    return grads, na.launch_count() - before
+
+
+@pytest.mark.parametrize("ks,H,W,dtype", [(3, 41, 9, torch.float32), (5, 67, 18, torch.bfloat16), (9, 50, 19, torch.float32),
+                                          (13, 75, 14, torch.float32)])
+def test_workspace_of_some_rows(ks, H, W, dtype):
+    """A workspace below one image: rows of tiles are used again as the key half is done with them."""
+    Cd, scale = 40, 0.2
+    q, k, v, d_o = _device(*make_inputs((1, 2, H, W, Cd), dtype, 78))
+    o, lse = na.natten2d_forward(q, k, v, ks, path="simt", scale=scale)
+    run = lambda bytes_of: _backward(q, k, v, o, lse, d_o, ks, scale, bytes_of, path="simt")
+    whole, launches = run(lambda n: n)
+    assert launches == 2
+    tile_rows = -(-H // 8)
+    least = 3 if ks <= 9 else 4                                  # tile rows that 8 rows of keys meet
+    for rows in range(least, tile_rows):
+        got, launches = run(lambda n: n // (2 * tile_rows) * rows + 60)
+        assert launches >= 2 * 3 - 1 and all(torch.equal(x, y) for x, y in zip(got, whole)), rows
+    want = orc.natten2d_bwd(q.cpu(), k.cpu(), v.cpu(), d_o.cpu(), ks, scale=scale)
+    short, launches = run(lambda n: n // (2 * tile_rows) * (least - 1))
+    assert launches == 2                                         # too short: without it
+    for g, w, what in zip(short, want, ("dq", "dk", "dv")):
+        assert_close(g, w, dtype, what)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_workspace_of_some_sequences(dtype):
+    g = torch.Generator().manual_seed(4)
+    q, k, v, d_o = _device(*(torch.randn((1, 5, 300, 48), generator=g).to(dtype) for _ in range(4)))
+    o, lse = F.natten1d_forward(q, k, v, 7, 0.2)
+    run = lambda bytes_of: _backward(q, k, v, None, lse, d_o, 7, 0.2, bytes_of)
+    whole, _ = run(lambda n: n)
+    for units in (1, 2, 4):
+        got, launches = run(lambda n: n // 5 * units + 12)
+        assert launches == 2 * -(-5 // units) and all(torch.equal(x, y) for x, y in zip(got, whole))
+
+
+def test_short_memory():
+    """No room for the whole workspace: the extension asks for half as much, and the result stays the same."""
+    q, k, v, d_o = (torch.randn(1, 4, 256, 256, 32, device=DEV) for _ in range(4))
+    o, lse = na.natten2d_forward(q, k, v, 5, scale=0.2)
+    before = na.launch_count()
+    want = na.natten2d_backward(q, k, v, o, lse, d_o, 5, scale=0.2)
+    assert na.launch_count() - before == 2                       # 84 MB of weights, 21 per image
+    want = [t.cpu() for t in want]
+    torch.cuda.empty_cache()
+    outputs = 3 * q.numel() * 4
+    limit = torch.cuda.memory_reserved() + outputs + (72 << 20)
+    try:
+        torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
+        before = na.launch_count()
+        got = na.natten2d_backward(q, k, v, o, lse, d_o, 5, scale=0.2)
+        assert na.launch_count() - before == 4
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert all(torch.equal(x.cpu(), y) for x, y in zip(got, want))
+
+
 @pytest.mark.parametrize("ks", [3, 5, 9])
 @pytest.mark.parametrize("at", [(0, 0), (7, 7), (8, 16), (23, 30)])
 def test_infinities_stay_in_their_windows(ks, at):
