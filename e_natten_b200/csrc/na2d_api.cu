@@ -16,6 +16,7 @@
 #include "na2d_simt.cuh"
 #include "na2d_tc_entry.h"
 #include "na2d_tile_entry.h"
+#include "na2d_tile_rule.h"
 
 namespace {
 
@@ -143,6 +144,7 @@ struct Problem {
     Tensor q, k, v, o, d_o, d_q, d_k, d_v;
     float* lse = nullptr;
     float* delta = nullptr;
+    float* row_factor = nullptr;   // CUDA-core backward: factors of exp(s - lse) on their way to the key half
 };
 
 // Strides of one operand: the caller's, or dense (B, N, rows, W, C) when all four are zero.  The
@@ -292,6 +294,17 @@ int after_launch() {
     return NA2D_OK;
 }
 
+// Whether the tiled kernels take this part of a CUDA-core call.  It goes by the whole image's rows, so that a band of them
+// is computed as the image is, bit for bit.
+bool in_tiles(na2d_tile::Work work, const Na2dGeom& g, int dtype) {
+    return na2d_tile::supported(g.ks) &&
+           na2d_tile::faster_in_tiles(work, g.kh == 1, dtype != NA2D_F32, (long long)g.BN * g.Hg * g.W, g.C, g.ks);
+}
+// The query half by itself; in 2D as the whole backward runs it, for the same reason.
+bool query_half_in_tiles(const Na2dGeom& g, int dtype) {
+    return in_tiles(na2d_tile::Work::kQueryHalf, g, dtype) || (g.kh > 1 && in_tiles(na2d_tile::Work::kBackward, g, dtype));
+}
+
 na2d_tile::Tensor tile(const Tensor& t) { return na2d_tile::Tensor{t.ptr, t.st}; }
 
 // The launcher of the element type.
@@ -329,7 +342,7 @@ int run_forward(const Problem& p) {
         if (rc == NA2D_ERR_CUDA) return tc_fail("tcgen05 forward launch");
         return rc;
     }
-    if (na2d_tile::supported(g.ks)) {
+    if (in_tiles(na2d_tile::Work::kForward, g, p.dtype)) {
         const auto run = NA2D_TILE_PICK(p.dtype, forward);
         return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.o), p.lse), 1);
     }
@@ -392,9 +405,9 @@ int run_backward_dq(const Problem& p) {
         if (rc == NA2D_ERR_CUDA) return tc_fail("tcgen05 dQ launch");
         return rc;
     }
-    if (na2d_tile::supported(g.ks)) {
+    if (query_half_in_tiles(g, p.dtype)) {
         const auto run = NA2D_TILE_PICK(p.dtype, backward_dq);
-        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), p.lse, p.delta), 1);
+        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), p.lse, p.delta, p.row_factor), 1);
     }
     unsigned grid = 0;
     int rc = grid_for(g.BN, g.Hq, g.W, g.patch, &grid);
@@ -404,7 +417,7 @@ int run_backward_dq(const Problem& p) {
         na2d_simt::dq_kernel<T, decltype(cpl)::value>
             <<<grid, kSimtThreads, na2d_simt::window_smem_bytes(g.kh, g.ks, 2), p.st>>>(
                 (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, p.lse, (const T*)p.d_o.ptr, (T*)p.d_q.ptr,
-                p.delta, p.q.st, p.k.st, p.v.st, p.d_o.st, p.d_q.st, g);
+                p.delta, p.row_factor, p.q.st, p.k.st, p.v.st, p.d_o.st, p.d_q.st, g);
         return after_launch();
     });
 }
@@ -429,7 +442,7 @@ int run_backward_dkdv(const Problem& p) {
     return simt_dispatch(p.dtype, g.C, [&](auto tt, auto cpl) -> int {
         using T = typename decltype(tt)::type;
         na2d_simt::dkdv_kernel<T, decltype(cpl)::value><<<grid, kSimtThreads, 0, p.st>>>(
-            (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, p.lse, (const T*)p.d_o.ptr, p.delta,
+            (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, p.lse, (const T*)p.d_o.ptr, p.delta, p.row_factor,
             p.d_k.ptr, p.d_v.ptr, p.dkdv_f32 ? 1 : 0, p.q.st, p.k.st, p.v.st, p.d_o.st, p.d_k.st, p.d_v.st, g);
         return after_launch();
     });
@@ -441,11 +454,12 @@ int run_backward_dkdv(const Problem& p) {
 // 2048 x 2048 12.9 -> 13.9 ms for 0.5 in place of 6.5 GiB).
 constexpr long long kWorkspaceBytes = 512ll << 20;
 
-// Whether the backward can keep P and dS for its key half: the tensor-core kernels form them again, faster than
-// they could be read, and row views and fp32 partial sums stay with the kernels that take them.
-bool uses_workspace(const Problem& p, const na2d_args* a) {
-    return !p.tensor && !a->rows && !p.dkdv_f32 && na2d_tile::supported(p.g.ks);
-}
+// Whether the backward hands something on to its key half: the tensor-core kernels form P and dS again, faster than
+// they could be read, and row views and fp32 partial sums stay with the halves that can be called by themselves.
+bool uses_workspace(const Problem& p, const na2d_args* a) { return !p.tensor && !a->rows && !p.dkdv_f32; }
+// P and dS, or else the factors that make P of exp(s - lse): small problems, and windows without tiled kernels.
+bool hands_on_weights(const Problem& p) { return in_tiles(na2d_tile::Work::kBackward, p.g, p.dtype); }
+size_t row_factor_bytes(const Problem& p) { return (size_t)p.g.BN * p.g.Hq * p.g.W * sizeof(float); }
 
 // Both halves of the backward, sharing a workspace.
 int run_backward_shared(const Problem& p, void* workspace, na2d_tile::Turns turns) {
@@ -554,7 +568,7 @@ na2d_tile::Tensor tile_dense(const PairProblem& p, const void* ptr) { return na2
 
 // x . y over the window -> attn
 int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
-    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_dot)(p.g, p.stream, tile_dense(p, x), tile_dense(p, y), attn), 1);
+    if (in_tiles(na2d_tile::Work::kDot, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_dot)(p.g, p.stream, tile_dense(p, x), tile_dense(p, y), attn), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -567,7 +581,7 @@ int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
 }
 // sum_j attn_j y_j -> out
 int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out) {
-    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_apply)(p.g, p.stream, attn, tile_dense(p, y), tile_dense(p, out)), 1);
+    if (in_tiles(na2d_tile::Work::kApply, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_apply)(p.g, p.stream, attn, tile_dense(p, y), tile_dense(p, out)), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -581,7 +595,7 @@ int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out)
 }
 // key-side sum over the inverse neighbourhood of attn x -> out
 int pair_inverse(const PairProblem& p, const void* attn, const void* x, void* out) {
-    if (na2d_tile::supported(p.g.ks)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_inverse)(p.g, p.stream, attn, tile_dense(p, x), tile_dense(p, out)), 1);
+    if (in_tiles(na2d_tile::Work::kKeySum, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_inverse)(p.g, p.stream, attn, tile_dense(p, x), tile_dense(p, out)), 1);
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hkv, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -663,6 +677,7 @@ int na2d_backward_dkdv_ex(const na2d_args* a) {
 size_t na2d_backward_workspace(const na2d_args* a) {
     Problem p;
     if (make_problem(a, &p) != NA2D_OK || !uses_workspace(p, a)) return 0;
+    if (!hands_on_weights(p)) return row_factor_bytes(p);
     return sizeof(float) * (size_t)na2d_tile::workspace_floats(p.g, kWorkspaceBytes / (long long)sizeof(float));
 }
 
@@ -673,14 +688,17 @@ int na2d_backward_ex(const na2d_args* a) {
     if (a->d_k.ptr && a->struct_size >= sizeof(na2d_args) && a->workspace) {
         if (!a->q.ptr || !a->k.ptr || !a->v.ptr || !a->lse || !a->d_o.ptr || !a->delta) return NA2D_ERR_BAD_ARG;
         if (reinterpret_cast<uintptr_t>(a->workspace) % 16) return NA2D_ERR_BAD_ARG;
-        bool shared = false;
-        const int rc = enter(a, [&](const Problem& p) -> int {
-            if (!uses_workspace(p, a)) return NA2D_OK;
-            const na2d_tile::Turns turns = na2d_tile::workspace_turns(p.g, (long long)(a->workspace_bytes / sizeof(float)));
-            shared = turns.units > 0;
-            return shared ? run_backward_shared(p, a->workspace, turns) : NA2D_OK;
+        return enter(a, [&](const Problem& problem) -> int {
+            Problem p = problem;
+            if (uses_workspace(p, a)) {
+                const long long floats = (long long)(a->workspace_bytes / sizeof(float));
+                const na2d_tile::Turns turns = hands_on_weights(p) ? na2d_tile::workspace_turns(p.g, floats) : na2d_tile::Turns{0, 0};
+                if (turns.units > 0) return run_backward_shared(p, a->workspace, turns);
+                if (a->workspace_bytes >= row_factor_bytes(p)) p.row_factor = (float*)a->workspace;
+            }
+            const int rc = run_backward_dq(p);
+            return rc != NA2D_OK ? rc : run_backward_dkdv(p);
         });
-        if (rc != NA2D_OK || shared) return rc;
     }
     // the query half always runs: it produces delta, which the key half needs
     int rc = na2d_backward_dq_ex(a);

@@ -9,9 +9,9 @@
 // accumulation is fp32.  The window is kh x kw: ks x ks for the 2D operator, 1 x ks for the 1D
 // operator on a (B, N, 1, T, C) view, so one set of kernels serves both.
 //
-// These kernels serve what the tiled kernels (na2d_tile.cuh) do not: kernel sizes 1 and 15 to 31, and the key half of
-// the backward where no workspace hands it the window weights (row views, fp32 partial sums, callers without
-// scratch).  They are bounds-safe for every grid size and use no atomics, so results are bit-stable from run to run.
+// These kernels serve what the tiled kernels (na2d_tile.cuh) do not: kernel sizes 1 and 15 to 31, problems of few pixels
+// (na2d_tile_rule.h), and the key half of the backward where no workspace hands it the window weights (row
+// views, fp32 partial sums, callers without scratch).  They are bounds-safe for every grid size and use no atomics, so results are bit-stable from run to run.
 //
 // A block of eight warps works through a compact patch of 64 pixels (8 x 8, or 1 x 64 for a
 // one-row image), warp w taking pixels w, w + 8, ...: neighbouring pixels share most of their
@@ -30,6 +30,7 @@
 #include <math_constants.h>
 
 #include "na2d_index.cuh"
+#include "na2d_softmax.cuh"
 
 namespace na2d_simt {
 
@@ -147,13 +148,23 @@ __device__ __forceinline__ float dot_members32(const float (&x)[CPL], const T* o
 }
 
 // acc[e] += sum_j weight[j] * row_j[lane + 32 e] over all nk members of the window at `origin`;
-// the weights are read from shared memory (a broadcast).
+// the weights are read from shared memory (a broadcast).  Odd and even window rows in sums of their own:
+// two short sums round less than a long one.
 template <typename T, int CPL>
 __device__ __forceinline__ void add_weighted_rows(float (&acc)[CPL], const float* weight, const T* origin, long long sh,
                                                   long long sw, int kh, int kw, int C, int lane) {
     int j = 0;
+    float other[CPL];
+#pragma unroll
+    for (int e = 0; e < CPL; ++e) other[e] = 0.f;
     for (int u = 0; u < kh; ++u) {
         const T* row = origin + u * sh;
+#pragma unroll
+        for (int e = 0; e < CPL; ++e) {
+            const float x = acc[e];
+            acc[e] = other[e];
+            other[e] = x;
+        }
         for (int w = 0; w < kw; ++w, ++j, row += sw) {
             const float wt = weight[j];
 #pragma unroll
@@ -163,6 +174,8 @@ __device__ __forceinline__ void add_weighted_rows(float (&acc)[CPL], const float
             }
         }
     }
+#pragma unroll
+    for (int e = 0; e < CPL; ++e) acc[e] += other[e];
 }
 
 template <typename T, int CPL>
@@ -228,12 +241,13 @@ fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict
 // ------------------------------------------------------------------------------------ dQ (+ delta)
 // delta = sum_j p_j dp_j, which equals dO . o exactly and does not depend on how o was rounded
 // when it was stored (the reference's backward does not read o either, e_natten/triton.py:522).
-// d_q may be null: then only delta is produced.
+// d_q may be null: then only delta is produced.  row_factor (or null): what each row's exp(s - lse) is multiplied by
+// to be P, for the key half.
 template <typename T, int CPL>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ lse,
-          const T* __restrict__ d_o, T* __restrict__ d_q, float* __restrict__ delta, const Na2dStride sq,
-          const Na2dStride sk, const Na2dStride sv, const Na2dStride sg, const Na2dStride sdq, const Na2dGeom g) {
+          const T* __restrict__ d_o, T* __restrict__ d_q, float* __restrict__ delta, float* __restrict__ row_factor,
+          const Na2dStride sq, const Na2dStride sk, const Na2dStride sv, const Na2dStride sg, const Na2dStride sdq, const Na2dGeom g) {
     extern __shared__ float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kh = g.kh, kw = g.ks, nk = kh * kw;
@@ -252,7 +266,7 @@ dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict_
     const T* k0 = k + offset_of(sk, px.b, px.n, oh, ow);
     const T* v0 = v + offset_of(sv, px.b, px.n, oh, ow);
     const float row_lse = lse[qi];
-    float dl = 0.f;
+    float dl = 0.f, l = 0.f;
     for (int j0 = 0; j0 < nk; j0 += 32) {
         const float s = dot_members32<T, CPL>(x, k0, sk.h, sk.w, kw, j0, nk, g.C, lane) * g.scale;
         const float dp = dot_members32<T, CPL>(gx, v0, sv.h, sv.w, kw, j0, nk, g.C, lane);
@@ -261,12 +275,17 @@ dq_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict_
             ps[j0 + lane] = p;
             dps[j0 + lane] = dp;
             dl = fmaf(p, dp, dl);
+            l += p;
         }
     }
-    dl = warp_sum(dl);
-    if (lane == 0) delta[qi] = dl;
+    const float factor = na2d_row_factor(warp_sum(l), row_lse);
+    dl = warp_sum(dl) * factor;
+    if (lane == 0) {
+        delta[qi] = dl;
+        if (row_factor != nullptr) row_factor[qi] = factor;
+    }
     if (d_q != nullptr) {
-        for (int j = lane; j < nk; j += 32) ps[j] = g.scale * ps[j] * (dps[j] - dl);
+        for (int j = lane; j < nk; j += 32) ps[j] = g.scale * (ps[j] * factor) * (dps[j] - dl);
         __syncwarp();
         float acc[CPL];
 #pragma unroll
@@ -298,11 +317,12 @@ __device__ __forceinline__ Inverse inverse_neighbourhood(int key_row_global, int
 // ------------------------------------------------------------------------------------ dK, dV
 // One warp per key pixel of the key band; sums over the queries of the local query band whose
 // window holds the key (the inverse neighbourhood, a product of two index ranges), 32 at a time.
+// row_factor (or null): see dq_kernel.
 template <typename T, int CPL>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ lse,
-            const T* __restrict__ d_o, const float* __restrict__ delta, void* __restrict__ d_k, void* __restrict__ d_v,
-            const int f32_out, const Na2dStride sq, const Na2dStride sk, const Na2dStride sv, const Na2dStride sg,
+            const T* __restrict__ d_o, const float* __restrict__ delta, const float* __restrict__ row_factor,
+            void* __restrict__ d_k, void* __restrict__ d_v, const int f32_out, const Na2dStride sq, const Na2dStride sk, const Na2dStride sv, const Na2dStride sg,
             const Na2dStride sdk, const Na2dStride sdv, const Na2dGeom g) {
     __shared__ float s_p[kWarps][32], s_ds[kWarps][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -330,6 +350,7 @@ dkdv_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restric
             const int rr = (j0 + lane) / iv.nc, cc = (j0 + lane) - rr * iv.nc;
             const long long si = stat0 + (long long)rr * g.W + cc;
             p = expf(s - lse[si]);
+            if (row_factor != nullptr) p *= row_factor[si];
             ds = g.scale * p * (dp - delta[si]);
         }
         s_p[warp][lane] = p;

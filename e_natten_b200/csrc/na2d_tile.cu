@@ -145,14 +145,14 @@ int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, cons
 }
 
 int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
-                           const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta) {
+                           const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta, float* row_factor) {
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
         const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
         return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
-                      operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float4*)nullptr,
+                      operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, row_factor, (float4*)nullptr,
                       (float4*)nullptr, whole_images<S>(g, g.Hq), g);
     });
 }
@@ -182,7 +182,7 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
                 if (query_band.rows > 0) {
                     if (int rc = tiles<S>(g, units, query_band.rows * S::kTh, &n)) return rc;
                     if (int rc = launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C), operand(v, g.C),
-                                        operand(d_o, g.C), operand(d_q, g.C), lse, delta, p, ds, query_band, g))
+                                        operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float*)nullptr, p, ds, query_band, g))
                         return rc;
                     ++*launches;
                 }

@@ -31,6 +31,7 @@
 #include <stdint.h>
 
 #include "na2d_index.cuh"
+#include "na2d_softmax.cuh"
 
 namespace na2d_tile {
 

@@ -15,12 +15,12 @@ namespace na2d_tile {
 // delta = sum_j p_j dp_j, which equals dO . o exactly and does not depend on how o was rounded when it
 // was stored.  d_q may be null: then only delta (and the weights) are produced.  p_out / ds_out, both or
 // neither: the tiles' weight slots for the key half, as they lie in shared memory, tile after tile in the rows of
-// `band`'s ring.
+// `band`'s ring.  row_factor (or null): what each row's exp(s - lse) is multiplied by to be P.
 template <typename T, int KS, bool ONE_D, bool PARK>
 __global__ void __launch_bounds__(Shape<KS, ONE_D>::kThreads, Shape<KS, ONE_D>::kBlocks)
 dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, const __grid_constant__ Operand v,
           const __grid_constant__ Operand d_o, const __grid_constant__ Operand d_q, const float* __restrict__ lse,
-          float* __restrict__ delta, float4* __restrict__ p_out, float4* __restrict__ ds_out,
+          float* __restrict__ delta, float* __restrict__ row_factor, float4* __restrict__ p_out, float4* __restrict__ ds_out,
           const __grid_constant__ Band band, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS, ONE_D>;
     extern __shared__ float4 smem[];
@@ -71,16 +71,9 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
     __syncthreads();
     if (d.active) {
         float4 dl4;
-        // p = exp(s - lse) over the window that lse was taken over adds up to 1 but for rounding: that of lse, of the
-        // logits beside it (both half an ulp of numbers about as large as lse) and of the exponentials.  Taken out here,
-        // it does not meet the cancellation in dP - delta.  A sum further off than that rounding can bring it is no
-        // rounding but an lse over more than this window, whose weights are what exp(s - lse) says they are.
         const float4 l4 = sum_rows<S>(total + d.strip * S::kKh * S::kTh + d.row);
-        auto rounding = [&](int r) {
-            const float l = lane_of(l4, r), limit = 4.f * FLT_EPSILON * (4.f + fabsf(c0 + r < g.W ? lse[stat + r] : 0.f));
-            return fabsf(l - 1.f) < limit ? 1.f / l : 1.f;
-        };
-        const float4 inv = make_float4(rounding(0), rounding(1), rounding(2), rounding(3));
+        auto factor = [&](int r) { return na2d_row_factor(lane_of(l4, r), c0 + r < g.W ? lse[stat + r] : 0.f); };
+        const float4 inv = make_float4(factor(0), factor(1), factor(2), factor(3));
         dl4 = sum_rows<S>(part + d.strip * S::kKh * S::kTh + d.row);
         dl4 = make_float4(dl4.x * inv.x, dl4.y * inv.y, dl4.z * inv.z, dl4.w * inv.w);
 #pragma unroll
@@ -90,7 +83,10 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
         if (d.u == 0 && d.split == 0) {
 #pragma unroll
             for (int r = 0; r < kR; ++r)
-                if (c0 + r < g.W) delta[stat + r] = lane_of(dl4, r);
+                if (c0 + r < g.W) {
+                    delta[stat + r] = lane_of(dl4, r);
+                    if (row_factor) row_factor[stat + r] = lane_of(inv, r);
+                }
         }
         // the slots turn from dP into P, the registers from P into dS
 #pragma unroll

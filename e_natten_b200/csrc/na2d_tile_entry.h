@@ -14,9 +14,8 @@ struct Tensor {
     Na2dStride st;
 };
 
-// Kernel sizes the tiled kernels are built for.  They are the faster ones at every size of these, down to a few tiles
-// (1 x 2 x 16 x 16 x 32, window 5, fp32: forward 23 -> 19 us).  From 15 on a tile would take 139 KB and leave one block per SM: that
-// wants another shape, which is not built.
+// Kernel sizes the tiled kernels are built for; na2d_tile_rule.h says which calls of these they take.  From 15 on a tile
+// would take 139 KB and leave one block per SM: that wants another shape, which is not built.
 inline bool supported(int ks) { return ks == 3 || ks == 5 || ks == 7 || ks == 9 || ks == 11 || ks == 13; }
 
 // How the backward hands P and dS from its query half to its key half: `units` (batch, head) units at a time, for each of
@@ -32,13 +31,14 @@ long long workspace_floats(const Na2dGeom& g, long long limit);
 // The turns a workspace of so many values allows; units is 0 if it is too small for any.
 Turns workspace_turns(const Na2dGeom& g, long long floats);
 
+// backward_dq: row_factor (or null) takes what the key half multiplies each row's exp(s - lse) by.
 // backward: both halves, for whole images.
 // Status: 0, NA2D_ERR_TOO_LARGE (grid), or NA2D_ERR_CUDA (the launch's error is left for cudaGetLastError).
 #define NA2D_TILE_ENTRIES(suffix)                                                                                     \
     int forward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,       \
                          const Tensor& o, float* lse);                                                                \
     int backward_dq_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,   \
-                             const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta);                   \
+                             const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta, float* row_factor);                   \
     int backward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,      \
                           const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v,                 \
                           const float* lse, float* delta, float* workspace, Turns turns, int* launches);                \

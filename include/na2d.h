@@ -210,8 +210,10 @@ int na2d_backward_ex(const na2d_args* a);
  * kernels) keep their window weights P and dS there, in fp32, instead of forming them again in the key half.
  * At most 512 MiB, or the weights of 32 image rows (of a whole sequence in 1D) where those are more.  With less than
  * this, the halves take turns over fewer images, or fewer rows of one image; the results are the same bit for bit.
- * Without a workspace, or with one that does not hold the rows that 8 rows of keys meet (at most 32), the key half
- * forms the weights again: slower, and other last bits of d_k and d_v.
+ * Where a workspace does not hold the rows that 8 rows of keys meet (at most 32), the key half forms the weights again:
+ * slower, and other last bits of d_k and d_v.  So it does for small problems and windows of 1 and 15 to 31, which only
+ * ask for a value per row, 4 * B * N * H * W bytes: a factor of exp(logit - lse) that takes out the rounding of
+ * lse.  Without any workspace that rounding stays in d_k and d_v.
  * The contents are of no use after the call.  No reference counterpart. */
 size_t na2d_backward_workspace(const na2d_args* a);
 

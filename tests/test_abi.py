@@ -123,6 +123,8 @@ def test_workspace_is_bounded():
     for H, W, ks in ((1024, 1024, 13), (4096, 4096, 13), (16384, 2048, 3), (2000, 3000, 9)):
         assert 128 << 20 <= ask(dtype=0, H=H, W=W, kernel_size=ks, B=2) <= 512 << 20
     assert ask(dtype=0, H=1024, W=1 << 17, kernel_size=13) <= weights(32, 1 << 17, 13)
+    assert ask(dtype=0, C=128, H=16, W=16, kernel_size=3) == 16 * 16 * 4    # few pixels, no tiles: a factor per row
+    assert ask(dtype=0, H=64, W=64, kernel_size=15) == 64 * 64 * 4
     assert ask(C=64, H=64, W=64) == 0                                  # bf16 on tensor cores has no use for one
 
 
