@@ -414,8 +414,11 @@ int run_backward_dq(const Problem& p) {
     if (rc != NA2D_OK) return rc;
     return simt_dispatch(p.dtype, g.C, [&](auto tt, auto cpl) -> int {
         using T = typename decltype(tt)::type;
-        na2d_simt::dq_kernel<T, decltype(cpl)::value>
-            <<<grid, kSimtThreads, na2d_simt::window_smem_bytes(g.kh, g.ks, 2), p.st>>>(
+        const auto kernel = na2d_simt::dq_kernel<T, decltype(cpl)::value>;
+        const size_t smem = na2d_simt::window_smem_bytes(g.kh, g.ks, 2);
+        if (smem > 48 * 1024)                      // kernel sizes 29 and 31
+            NA2D_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, kSimtThreads, smem, p.st>>>(
                 (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, p.lse, (const T*)p.d_o.ptr, (T*)p.d_q.ptr,
                 p.delta, p.row_factor, p.q.st, p.k.st, p.v.st, p.d_o.st, p.d_q.st, g);
         return after_launch();

@@ -292,3 +292,18 @@ def test_few_pixels_keep_the_rounding_of_lse_out(Cd, ks):
     assert all(torch.isfinite(t).all() for t in given + without) and torch.equal(given[0], without[0])
     for i, most, what in ((1, 1.0, "dk"), (2, 0.8, "dv")):       # dK also has the scores' own rounding in dP - delta
         assert err(given[i], want[i]) < most * err(without[i], want[i]), what
+
+
+@pytest.mark.parametrize("ks", [15, 27, 29, 31])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_windows_beyond_the_tiles(ks, dtype):
+    """Kernel sizes up to the largest; from 29 on the query half needs more than 48 KB of shared memory."""
+    q, k, v, d_o = make_inputs((1, 2, 31, 34, 40), dtype, ks, q_scale=0.16)
+    ro, rlse = orc.natten2d_fwd(q, k, v, ks)
+    want = orc.natten2d_bwd(q, k, v, d_o, ks)
+    qd, kd, vd, gd = _device(q, k, v, d_o)
+    o, lse = na.natten2d_forward(qd, kd, vd, ks)
+    assert_close(o, ro, dtype, "o")
+    assert_close(lse, rlse, torch.float32, "lse")
+    for got, w, what in zip(na.natten2d_backward(qd, kd, vd, o, lse, gd, ks), want, ("dq", "dk", "dv")):
+        assert_close(got, w, dtype, what)
