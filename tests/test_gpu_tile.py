@@ -307,3 +307,56 @@ def test_windows_beyond_the_tiles(ks, dtype):
     assert_close(lse, rlse, torch.float32, "lse")
     for got, w, what in zip(na.natten2d_backward(qd, kd, vd, o, lse, gd, ks), want, ("dq", "dk", "dv")):
         assert_close(got, w, dtype, what)
+
+
+@pytest.mark.parametrize("shape,ks,dtype", [((1, 24, 20, 21, 40), 5, torch.float32), ((1, 2, 30, 33, 64), 9, torch.bfloat16),
+                                            ((2, 40, 300, 64), 7, torch.bfloat16)])
+def test_on_another_stream(shape, ks, dtype):
+    """The native path launches on the current stream, behind the work that makes its inputs, and its outputs and
+    scratch belong to that stream."""
+    g = torch.Generator().manual_seed(9)
+    inputs = [torch.randn(shape, generator=g).to(dtype).to(DEV) for _ in range(4)]
+    forward, backward = ((na.natten2d_forward, na.natten2d_backward) if len(shape) == 5 else
+                         (F.natten1d_forward, F.natten1d_backward))
+    o, lse = forward(*inputs[:3], ks)
+    want = (o, lse, *backward(*inputs[:3], o, lse, inputs[3], ks))
+    torch.cuda.synchronize()
+    busy = torch.randn(4096, 4096, device=DEV)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        late = [torch.full_like(t, float("nan")) for t in inputs]
+        for _ in range(20):
+            busy = (busy @ busy).clamp_(-1, 1)
+        for t, x in zip(late, inputs):
+            t.copy_(x)                                           # the inputs are there once `busy` is done
+        o2, lse2 = forward(*late[:3], ks)
+        got = (o2, lse2, *backward(*late[:3], o2, lse2, late[3], ks))
+        [torch.full_like(t, float("nan")) for t in got]          # takes freed scratch of this stream again
+    stream.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("ks,Cd", [(7, 32), (9, 64), (13, 128)])
+def test_infinities_in_the_chunked_query_half(ks, Cd):
+    """An infinite value and an infinite gradient in the query half of the larger windows on tensor cores, which walks the
+    key box in chunks: dQ of the pixels whose windows hold them, and no others, is not finite.  (o is that of
+    finite values: the forward's P V leaves the window's bounds to zeros of P, so there an infinity spreads over a tile.)"""
+    H, W, at = 40, 37, (17, 9)
+    q, k, v, d_o = _device(*make_inputs((1, 2, H, W, Cd), torch.bfloat16, 6, q_scale=0.2))
+    o, lse = na.natten2d_forward(q, k, v, ks, path="tensor")
+    clean, _, _ = na.natten2d_backward(q, k, v, o, lse, d_o, ks, path="tensor", need_dkdv=False)
+    v2 = v.clone()
+    v2[0, 0, at[0], at[1]] = float("inf")
+    dirty, _, _ = na.natten2d_backward(q, k, v2, o, lse, d_o, ks, path="tensor", need_dkdv=False)
+    holds = lambda n, i: [na.get_window_start(y, n, ks) <= i < na.get_window_start(y, n, ks) + ks for y in range(n)]
+    reached = (torch.tensor(holds(H, at[0]))[:, None] & torch.tensor(holds(W, at[1]))[None, :]).to(DEV)
+    assert torch.equal(~torch.isfinite(dirty[0, 0]).all(-1), reached)
+    assert torch.equal(dirty[0, 0][~reached], clean[0, 0][~reached]) and torch.equal(dirty[0, 1], clean[0, 1])
+    g2 = d_o.clone()
+    g2[0, 0, at[0], at[1]] = float("inf")
+    dirty, _, _ = na.natten2d_backward(q, k, v, o, lse, g2, ks, path="tensor", need_dkdv=False)
+    itself = torch.zeros(H, W, dtype=torch.bool, device=DEV)
+    itself[at] = True
+    assert torch.equal(~torch.isfinite(dirty[0, 0]).all(-1), itself)
+    assert torch.equal(dirty[0, 0][~itself], clean[0, 0][~itself])
