@@ -53,12 +53,19 @@ fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     uint64_t* q_empty = bars + 1;            //      MMA (commit) -> TMA
     uint64_t* o_full = bars + 2;             //      MMA (commit) -> softmax
     uint64_t* o_free = bars + 3;             //      softmax -> MMA
-    uint64_t* s_full = bars + 4;             // [2]  MMA (commit) -> softmax: S_x is complete
-    uint64_t* p_full = bars + 6;             // [2]  softmax -> MMA: P_x is in tensor memory
-    uint64_t* kv_full = bars + 8;            // [4]  TMA -> MMA: K_A, K_B, V_A, V_B
-    uint64_t* kv_empty = bars + 12;          // [4]  MMA (commit) -> TMA
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 17)};
+    uint64_t* s_full = bars + 4;             // [3]  MMA (commit) -> softmax: S_A of even tiles, S_A of odd tiles, S_B
+    uint64_t* p_full = bars + 7;             // [2]  softmax -> MMA: P_x is in tensor memory
+    uint64_t* kv_full = bars + 9;            // [4]  TMA -> MMA: K_A, K_B, V_A, V_B
+    uint64_t* kv_empty = bars + 13;          // [4]  MMA (commit) -> TMA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 18)};
+    // S_A of tile i + 1 is issued before anything of tile i is waited for, so it may be complete before a softmax warp
+    // has looked for S_A of tile i: on one barrier that would be two phases ahead, which a wait by parity takes for
+    // none and waits for ever.  With a barrier for either parity of i, the next use of a barrier (tile i + 2) comes
+    // after the wait for P_A of tile i, to which every softmax warp arrives behind its wait here.  S_B of tile i + 1
+    // comes after that wait as it is.
+    auto s_bar = [](int i, int x) { return x ? 2 : i & 1; };
+    auto s_par = [](int i, int x) { return x ? i & 1 : (i >> 1) & 1; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -69,10 +76,8 @@ fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         mbar_init(q_empty, 1);
         mbar_init(o_full, 1);
         mbar_init(o_free, 4);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(s_full + i, 1);
-            mbar_init(p_full + i, 8);
-        }
+        for (int i = 0; i < 3; ++i) mbar_init(s_full + i, 1);
+        for (int i = 0; i < 2; ++i) mbar_init(p_full + i, 8);
         for (int i = 0; i < 4; ++i) {
             mbar_init(kv_full + i, 1);
             mbar_init(kv_empty + i, 1);
@@ -183,7 +188,7 @@ fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     umma_ss(t_s, desc64(hi, q_lo + ((slab * C::Q_SLAB) >> 4) + 2 * in_slab),
                             desc64(hi, k_lo + ((slab * C::KV_SLAB) >> 4) + 2 * in_slab), idesc_s, kk > 0);
                 }
-                umma_commit(s_full + x);
+                umma_commit(s_full + s_bar(i, x));
                 umma_commit(kv_empty + x);
                 if (x == 1) umma_commit(q_empty);                    // last reader of the Q tile
                 NA2D_TR(2, x ? 3 : 1, i);
@@ -314,7 +319,7 @@ fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     }
                 }
                 if (tid == 0) NA2D_TR(3, x ? 2 : 0, i);
-                mbar_wait(s_full + x, par, wctx, kErrMmaWait);
+                mbar_wait(s_full + s_bar(i, x), s_par(i, x), wctx, kErrMmaWait);
                 tc_fence_after();
                 if (tid == 0) NA2D_TR(3, x ? 3 : 1, i);
 #pragma unroll

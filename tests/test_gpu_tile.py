@@ -360,3 +360,21 @@ def test_infinities_in_the_chunked_query_half(ks, Cd):
     itself[at] = True
     assert torch.equal(~torch.isfinite(dirty[0, 0]).all(-1), itself)
     assert torch.equal(dirty[0, 0][~itself], clean[0, 0][~itself])
+
+
+@pytest.mark.parametrize("ks,Cd,dtype", [(3, 32, torch.float16), (5, 64, torch.bfloat16), (5, 128, torch.bfloat16)])
+def test_strip_forward_hand_overs(ks, Cd, dtype):
+    """Many tiles per block and many launches beside a kernel that takes instruction slots and memory bandwidth from the
+    softmax warps at odd moments: every hand-over between the warps takes place (no bounded wait runs out), and the
+    results stay the same."""
+    q, k, v, _ = _device(*make_inputs((2, 4, 96, 200, Cd), dtype, 12, q_scale=0.2))
+    o, lse = na.natten2d_forward(q, k, v, ks)
+    other, noise = torch.cuda.Stream(), torch.randn(1 << 22, device=DEV)
+    torch.cuda.synchronize()
+    for _ in range(40):
+        with torch.cuda.stream(other):
+            noise = torch.sin(noise)
+        for _ in range(20):
+            o2, lse2 = na.natten2d_forward(q, k, v, ks)
+        assert torch.equal(o2, o) and torch.equal(lse2, lse)
+    na.check_kernels(DEV)
