@@ -398,6 +398,27 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
         : "memory");
 }
 
+// ------------------------------------------------------------------------------------ packed fp32 pairs
+__device__ __forceinline__ uint64_t pair2(uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; }
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) { return pair2(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ float lo2(uint64_t a) { return __uint_as_float(static_cast<uint32_t>(a)); }
+__device__ __forceinline__ float hi2(uint64_t a) { return __uint_as_float(static_cast<uint32_t>(a >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // ------------------------------------------------------------------------------------ descriptors
 // Shared-memory matrix descriptor (64 bit) for a swizzled canonical layout.
 //   bits  0-13  start address >> 4          bits 16-29  leading byte offset >> 4

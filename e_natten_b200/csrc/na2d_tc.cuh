@@ -46,6 +46,34 @@ __device__ __forceinline__ void split_unit(int bn, const Na2dGeom& g, int& hn, i
     hn = bn - hb * g.N;
 }
 
+// The tiles first, first + step, first + 2 step, ... of a (unit, tile row, tile column) grid, divided out once and then
+// stepped with carries: a role of a persistent kernel that works out every tile's place by division spends some 400 cycles of
+// each tile on it, with nothing to overlap.
+struct TileWalk {
+    int tiles_r, tiles_c;
+    int bn, tr, tc;            // unit, tile row, tile column of the present tile
+    int d_bn, d_tr, d_tc;      // the step
+    __device__ __forceinline__ TileWalk(int first, int step, int rows, int cols) : tiles_r(rows), tiles_c(cols) {
+        split(first, bn, tr, tc);
+        split(step, d_bn, d_tr, d_tc);
+    }
+    __device__ __forceinline__ void split(int t, int& b, int& r, int& c) const {
+        const int q = t / tiles_c;
+        c = t - q * tiles_c;
+        b = q / tiles_r;
+        r = q - b * tiles_r;
+    }
+    __device__ __forceinline__ void next() {
+        bn += d_bn;
+        tr += d_tr;
+        tc += d_tc;
+        if (tc >= tiles_c) { tc -= tiles_c; ++tr; }
+        if (tr >= tiles_r) { tr -= tiles_r; ++bn; }
+    }
+    __device__ __forceinline__ int row() const { return tr * TH; }
+    __device__ __forceinline__ int col() const { return tc * TW; }
+};
+
 // Compile-time geometry of one (head dim, kernel size) instantiation.
 // NMAX caps the keys (forward, dQ) or queries (dK/dV) of one chunk; it is set by how many
 // tensor-memory columns the kernel can spare for the S-shaped accumulators.
@@ -91,6 +119,17 @@ __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {       // a NaN counts for nothing
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
 }
 
 template <typename DT> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
@@ -162,6 +201,13 @@ __device__ __forceinline__ uint32_t block_mask16(int blk, int wr_rel, int wc) {
     return static_cast<uint32_t>(w >> c0) & 0xffffu;
 }
 
+// Bits [lo, hi) of a block of N columns that starts at column `at`.
+template <int N>
+__device__ __forceinline__ uint32_t range_bits(int lo, int hi, int at) {
+    const int a = min(max(lo - at, 0), N), b = min(max(hi - at, 0), N);
+    return ((1u << b) - 1u) & ~((1u << a) - 1u);
+}
+
 // Output rows leave through TMA: a thread that wrote its own 16-byte pieces straight to global
 // memory would touch 32 different 128-byte lines per warp instruction.  Each softmax warp owns a
 // staging buffer of 32 pixels (32 / TW tile rows x TW columns) x OUT_RW channels, laid out as the
@@ -210,6 +256,20 @@ __device__ __forceinline__ void stage_and_store(const CUtensorMap* map, uint8_t*
             tma_store_5d(map, base, ch0 + r * S::RW, w0, h0, n, b);
             bulk_commit();
         }
+    }
+}
+
+// Writes 32 columns held as fp32 bit patterns (times `scale`) as the lane's 16-bit row of a staging buffer.
+template <typename DT>
+__device__ __forceinline__ void stage_rows(uint8_t* stage, const uint32_t (&v)[32], float scale, int lane) {
+    const uint32_t row = smem_u32(stage) + lane * OutStage<32>::ROWB;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            w[e] = pack2<DT>(__uint_as_float(v[8 * c + 2 * e]) * scale, __uint_as_float(v[8 * c + 2 * e + 1]) * scale);
+        st_shared_v4(row + ((c ^ ((lane >> 1) & 3)) << 4), w[0], w[1], w[2], w[3]);
     }
 }
 

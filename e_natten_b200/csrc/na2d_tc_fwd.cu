@@ -2,6 +2,8 @@
 // (-DNA2D_TC_DT=1: bf16, 2: fp16).
 #include "na2d_tc_entry.h"
 #include "na2d_tc_fwd1.cuh"
+#include "na2d_tc_strip.cuh"
+#include "na2d_tc_fwd2.cuh"
 #include "na2d_tc_fwd.cuh"
 
 namespace na2d_tc {

@@ -473,15 +473,16 @@ int launch_forward(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, 
     } else {
     using C = FwdCfg<D, KS>;
     const Na2dGeom& g = lc.g;
+    const int tiles_r = (g.Hq + TH - 1) / TH, tiles_c = (g.W + TW - 1) / TW;
+    const long long tiles = (long long)g.BN * tiles_r * tiles_c;
+    if (tiles > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
+    if (tiles > sm_count(lc.device)) return launch_forward2<DT, D, KS>(lc, q, k, v, o, lse, tiles, tiles_r, tiles_c);
     CUtensorMap tq, tk, tv, to;
     int rc = make_map(&tq, q, lc.dtype, lc.B, g.N, g.Hq, g.W, D, TW, TH);
     if (rc == NA2D_OK) rc = make_map(&to, o, lc.dtype, lc.B, g.N, g.Hq, g.W, D, TW, 32 / TW, OutStage<D / 2>::RW);
     if (rc == NA2D_OK) rc = make_map(&tk, k, lc.dtype, lc.B, g.N, g.Hkv, g.W, D, C::HW, C::RC);
     if (rc == NA2D_OK) rc = make_map(&tv, v, lc.dtype, lc.B, g.N, g.Hkv, g.W, D, C::HW, C::RC);
     if (rc != NA2D_OK) return rc;
-    const int tiles_r = (g.Hq + TH - 1) / TH, tiles_c = (g.W + TW - 1) / TW;
-    const long long tiles = (long long)g.BN * tiles_r * tiles_c;
-    if (tiles > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
     auto kern = fwd_kernel<DT, D, KS>;
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
