@@ -2,6 +2,7 @@
 // (-DNA2D_TC_DT=1: bf16, 2: fp16).
 #include "na2d_tc_entry.h"
 #include "na2d_tc_dq1.cuh"
+#include "na2d_tc_strip.cuh"
 #include "na2d_tc_dq2.cuh"
 #include "na2d_tc_bwd.cuh"
 
