@@ -3,21 +3,29 @@
 // One CTA per SM walks key tiles (TH x TW keys, row r of every MMA = key r = tensor-memory lane
 // r).  The queries that can see a tile form a box (the union of the keys' inverse
 // neighbourhoods, clipped to the local query band), walked in chunks of RC rows x HW columns
-// (at most 64 queries):
+// (at most NMAX queries).  From kernel size 7 on a chunk is a column strip as tall as the box of an inner tile: a
+// warp's 32 keys (four image rows) are seen from ks + 3 of its rows, the same share of every chunk, while of
+// a group of rows some warps see everything and others nothing, and a chunk lasts as long as its busiest warp.
 //     S^T = K Q_c^T,  dP^T = V dO_c^T                      (tensor memory, fp32)
 //     P^T = exp(S^T - lse),  dS^T = scale P^T (dP^T - delta)   (softmax warps, registers; the scale is dK's)
 //     dV += P^T dO_c,  dK += dS^T Q_c                      (P^T, dS^T read from tensor memory)
 // P^T and dS^T are written back over S^T / dP^T as packed 16-bit pairs; on the bf16 path dS^T
 // is written as head + residual (two MMAs), because one bf16 keeps too few bits for dK.
 //
-// Tensor memory holds two chunk stages (S^T, dP^T of 64 columns each) next to the dV and dK
+// Tensor memory holds two chunk stages (S^T, dP^T of NMAX columns each) next to the dV and dK
 // accumulators, so the score MMAs of one chunk run while the softmax warps work on the previous
 // one.  Sixteen warps: 0-7 softmax (warps w and w + 4 own the same 32 keys of a lane quarter and split
-// the 8-column blocks of every chunk between them), 8 TMA producer of the Q / dO chunk ring, 11 TMA
-// producer of the K, V tile, 9 issues the score MMAs, 10 the output MMAs, 12-15 epilogue (dV, dK rows ->
+// the 8-column blocks of every chunk between them), 8 producer of the Q / dO chunk ring and of the chunks' lse and
+// delta, 11 TMA producer of the K, V tile, 9 issues the score MMAs, 10 the output MMAs, 12-15 epilogue (dV, dK rows ->
 // staging -> TMA store), which
 // overlaps the next tile.  dK and dV accumulate in tensor memory over all chunks of a tile; no
 // atomics.
+//
+// What bounds it: the chain score MMAs -> softmax warps -> output MMAs -> stage free, of which tensor memory holds two; the
+// softmax part of it was cut by strips, packed fp32 pairs, and lse and delta handed over by the producer.  Measured on one B200
+// against chunks of box rows: 32 x 2 x 56 x 56 x 32, window 7, bf16 104 -> 62 us; 16 x 8 x 28 x 28 x 64, window 13, bf16
+// 135 -> 100 us; 16 x 16 x 14 x 14 x 64, window 13, fp16 39 -> 29 us; 8 heads of 1024 x 1024 x 128, window 13, bf16 7.8 -> 6.6 ms;
+// 4 x 4 x 256 x 256 x 128, window 5, bf16 (the same chunks as before) 0.39 -> 0.375 ms.
 #pragma once
 
 namespace na2d_tc {
@@ -32,6 +40,7 @@ constexpr int dkv_chunks(int ks, int split) {
 // Fewest chunks wins; on a tie the narrower strips, which spread the work evenly over the lane
 // quarters (a key row group sees the same number of queries in every strip).
 constexpr int dkv_w_split(int ks) {
+    if (ks >= 7) return (TW + ks - 1) / 2;
     const int c1 = dkv_chunks(ks, 1), c2 = dkv_chunks(ks, 2), c4 = dkv_chunks(ks, 4);
     return (c4 <= c2 && c4 <= c1) ? 4 : (c2 <= c1 ? 2 : 1);
 }
@@ -42,23 +51,47 @@ constexpr unsigned long long row_repeat(int hw, int rc) {
     return m;
 }
 
-template <int D, int KS, bool SPLIT>
-struct DkvCfg : Cfg<D, KS, 64, 0, dkv_w_split(KS)> {
-    using B = Cfg<D, KS, 64, 0, dkv_w_split(KS)>;
+// Queries per chunk at most: 2 x (S^T + dP^T) + dV + dK in 512 columns.  (Kernel sizes 3 and 5 keep chunks of 64.)
+constexpr int dkv_nmax(int d, int ks) { return ks < 7 || d == 128 ? 64 : (512 - 2 * d) / 4 / 16 * 16; }
+// Columns of a chunk from kernel size 7 on: 4 or 2, so that a column pattern repeats every 8 queries.
+constexpr int dkv_strip(int d, int ks) { return (TH + ks - 1) * 4 <= dkv_nmax(d, ks) ? 4 : 2; }
+
+// (Cfg wants strips that tile the box: it is taken as wide as the next multiple of 8.)
+constexpr int dkv_box_w(int ks) { return (TW + ks - 1 + 7) / 8 * 8; }
+template <int D, int KS>
+using DkvCfgBase = Cfg<D, KS, dkv_nmax(D, KS), KS < 7 ? 0 : dkv_box_w(KS) - (TW + KS - 1), KS < 7 ? dkv_w_split(KS) : dkv_box_w(KS) / dkv_strip(D, KS)>;
+
+template <int D, int KS>
+struct DkvCfg : DkvCfgBase<D, KS> {
+    using B = DkvCfgBase<D, KS>;
     // names of the base read as "queries per chunk" here: NK = queries in a chunk, NKP padded
-    static constexpr int TMEM_STAGE = 128;                                 // columns per chunk stage
-    static constexpr int TMEM_ST = 0, TMEM_DPT = 64, TMEM_DV = 256, TMEM_DK = 384;
-    static constexpr int TMEM_PT = 0, TMEM_DST = 32, TMEM_RES = 64;       // 16-bit operands over S^T / dP^T
+    static constexpr bool PATTERN = KS >= 7;                               // masks by pattern (HW divides 8)
+    static constexpr int NMAX = dkv_nmax(D, KS);
+    static constexpr int TMEM_STAGE = 2 * NMAX;                            // columns per chunk stage
+    static constexpr int TMEM_ST = 0, TMEM_DPT = NMAX, TMEM_DV = 512 - 2 * D, TMEM_DK = TMEM_DV + D;
+    static constexpr int TMEM_PT = 0, TMEM_DST = NMAX / 2, TMEM_RES = NMAX;   // 16-bit operands over S^T / dP^T
     static constexpr int STAGE = 2 * B::KV_BYTES;                          // Q chunk then dO chunk
     static constexpr int OUT_BYTES = 4 * 2 * OutStage<32>::BYTES;          // two staging buffers for each of the 4 epilogue warps
-    static constexpr int XCHG_BYTES = 2 * 2 * 2 * 64 * 4;                  // [group][parity]{lse, delta}[64]
+    static constexpr int XCHG_BYTES = 4 * 2 * B::NKP * 4;                  // [ring slot]{-lse * log2(e), -delta * scale}[NKP]
     static constexpr int FIXED = 2 * B::Q_BYTES /*K, V tile*/ + OUT_BYTES + XCHG_BYTES + 256 + 1024;
     static constexpr int NSTQ = (FIXED + 4 * STAGE <= kSmemLimit) ? 4 : 3;
     static constexpr int SMEM = FIXED + NSTQ * STAGE;
     static constexpr int NB8 = B::NKP / 8;
-    static constexpr unsigned long long ROW_REP = row_repeat(B::HW, B::RC);
+    // A warp pair works on blocks b_lo .. b_lo + 2 NOWN - 1 in any case (what an inner tile needs), and on those beyond where a
+    // tile at a border needs them: a warp's 32 / TW key rows are seen from at most that many + 2 ks - 2 query rows.
+    static constexpr int kInner = (32 / TW - 1 + KS) < B::RC ? (32 / TW - 1 + KS) : B::RC;
+    static constexpr int kMost = (32 / TW - 1 + 2 * KS - 1) < B::RC ? (32 / TW - 1 + 2 * KS - 1) : B::RC;
+    static constexpr int half_blocks(int rows, bool aligned) {
+        const int n = (rows * B::HW + 7) / 8 + (aligned ? 0 : 1);
+        return ((n < NB8 ? n : NB8) + 1) / 2;
+    }
+    static constexpr int NOWN = half_blocks(kInner, PATTERN), NALL = half_blocks(kMost, false);
+    static constexpr unsigned long long ROW_REP = PATTERN ? 0ull : row_repeat(B::HW, B::RC);
+    static constexpr uint32_t REP8 = B::HW == 4 ? 0x11u : 0x55u;
     static_assert(SMEM <= kSmemLimit, "dK/dV kernel shared memory");
-    static_assert(B::NKP <= 64 && D <= 128 && D % 32 == 0, "tensor memory layout");
+    static_assert(!PATTERN || B::HW == 2 || B::HW == 4, "strips of 2 or 4 columns");
+    static_assert(B::NKP <= NMAX && 2 * TMEM_STAGE <= TMEM_DV && TMEM_DK + D <= 512 && D % 32 == 0, "tensor memory layout");
+    static_assert(NMAX % 16 == 0 && NB8 % 2 == 0 && NOWN <= NALL, "blocks in pairs");
 };
 
 template <typename DT, int D, int KS>
@@ -70,7 +103,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             unsigned int* __restrict__ err_word, const Na2dGeom g, const int tiles_r, const int tiles_c,
             const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
-    using C = DkvCfg<D, KS, SPLIT>;
+    using C = DkvCfg<D, KS>;
     constexpr int NSTQ = C::NSTQ;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -78,7 +111,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     uint8_t* sV = sK + C::Q_BYTES;                    // value tile [128 x D]
     uint8_t* sQD = sV + C::Q_BYTES;                   // NSTQ x (query chunk, dO chunk), each [NKP x D]
     uint8_t* sOut = sQD + NSTQ * C::STAGE;            // 4 x output staging (1024-byte aligned)
-    float* s_x = reinterpret_cast<float*>(sOut + C::OUT_BYTES);   // [group][parity]{lse * log2(e), delta}[64]
+    float* s_x = reinterpret_cast<float*>(sOut + C::OUT_BYTES);   // [ring slot]{-lse * log2(e), -delta * scale}[NKP]
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_x + C::XCHG_BYTES / 4);
     uint64_t* kv_full = bars + 0;            //       TMA -> MMA
     uint64_t* kv_empty = bars + 1;           //       MMA (commit) -> TMA
@@ -90,8 +123,9 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     uint64_t* qd_empty = bars + 12;          // [4]   MMA (commit) -> TMA
     uint64_t* st_free = bars + 16;           // [2]   output MMAs (commit) -> score MMAs: the stage is free
     uint64_t* accv_free = bars + 18;         //       epilogue -> MMA: dV has been read (dK follows)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
-    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 20)};
+    uint64_t* x_full = bars + 19;            // [4]   producer -> score MMAs (and through them softmax): lse and delta
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
+    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 24)};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -111,6 +145,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         for (int i = 0; i < 4; ++i) {
             mbar_init(qd_full + i, 1);
             mbar_init(qd_empty + i, 1);
+            mbar_init(x_full + i, 1);
         }
         mbar_fence_init();
         tma_prefetch_desc(&tm_k);
@@ -144,14 +179,13 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
 
     // Geometry of my i-th tile: key tile origin and the query box it is seen from.
     struct TileGeo { int bn, hn, hb, kr0, kc0, qb_r0, q_local_r0, n_rows, qb_c0, n_cc, n_ch; };
-    auto tile_geo = [&](int i) {
+    // (each role steps through the tiles by itself)
+    TileWalk walk((int)blockIdx.x, (int)gridDim.x, tiles_r, tiles_c);
+    auto tile_geo = [&](const TileWalk& at) {
         TileGeo t;
-        int x = (int)blockIdx.x + i * (int)gridDim.x;
-        const int tc = x % tiles_c;
-        x /= tiles_c;
-        t.kr0 = (x % tiles_r) * TH;
-        t.kc0 = tc * TW;
-        t.bn = x / tiles_r;
+        t.kr0 = at.row();
+        t.kc0 = at.col();
+        t.bn = at.bn;
         split_unit(t.bn, g, t.hn, t.hb);
         const int kg_first = g.kv_row0 + t.kr0;
         const int kg_last = g.kv_row0 + min(t.kr0 + TH, g.Hkv) - 1;
@@ -162,7 +196,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         t.qb_c0 = na2d_bws(t.kc0, KS);
         const int n_cols = na2d_bwe(min(t.kc0 + TW, g.W) - 1, g.W, KS) - t.qb_c0;
         t.n_cc = (n_cols + C::HW - 1) / C::HW;           // strips; more where both borders stretch the box
-        t.n_ch = ((t.n_rows + C::RC - 1) / C::RC) * t.n_cc;
+        t.n_ch = ((t.n_rows + C::RC - 1) / C::RC) * t.n_cc;       // (divisions by constants)
         return t;
     };
 
@@ -170,16 +204,33 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         // ------------------------------------------------------------------ producer of the Q / dO chunk ring
         // (the K, V tile has a producer of its own, warp 11: a chunk of the next tile can be
         // fetched as soon as a ring slot is free, long before the K, V buffers are)
+        // The chunk's lse and delta go with it, as the softmax warps use them: lane l has queries l, l + 32, ...; they are read
+        // one chunk ahead, so that their latency runs under the wait for a ring slot.
         reg_dec<kDkvRegsCtl>();
-        if (lane == 0) {
-            uint32_t n = 0;
-            LoadTracker lt(bars);
-            for (int i = 0; i < n_my && lt.ok; ++i) {
-                const TileGeo t = tile_geo(i);
-                for (int ch = 0; ch < t.n_ch; ++ch, ++n) {
-                    const int rc = ch / t.n_cc, cc = ch - rc * t.n_cc;
-                    const uint32_t st = n % NSTQ;
-                    if (!lt.acquire(qd_empty + st, ((n / NSTQ) & 1) ^ 1, wctx)) break;
+        constexpr int kPer = (C::NKP + 31) / 32;
+        float pre_l2[kPer], pre_dl[kPer];
+        auto fetch = [&](const TileGeo& t, int rc, int cc) {
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int j = lane + 32 * u, br = rc * C::RC + j / C::HW, qc = t.qb_c0 + cc * C::HW + j % C::HW;
+                pre_l2[u] = pre_dl[u] = 0.f;                     // zero outside the band
+                if (j < C::NK && br < t.n_rows && qc < g.W) {
+                    const size_t qi = (static_cast<size_t>(t.bn) * g.Hq + (t.q_local_r0 + br)) * g.W + qc;
+                    pre_l2[u] = -(lse[qi] * kLog2e);
+                    pre_dl[u] = -(delta[qi] * g.scale);          // dS^T carries the softmax scale of dK: scale p (dP - delta)
+                }
+            }
+        };
+        uint32_t n = 0;
+        LoadTracker lt(bars);
+        for (int i = 0; i < n_my && lt.ok; ++i, walk.next()) {
+            const TileGeo t = tile_geo(walk);
+            if (t.n_ch == 0) continue;
+            fetch(t, 0, 0);
+            for (int ch = 0, rc = 0, cc = 0; ch < t.n_ch; ++ch, ++n) {
+                const uint32_t st = n % NSTQ;
+                if (!lt.acquire(qd_empty + st, ((n / NSTQ) & 1) ^ 1, wctx)) break;
+                if (lane == 0) {
                     NA2D_TR(2, 7, n);
                     lt.arm(qd_full + st, (n / NSTQ) & 1, 2u * C::NS * C::NK * C::ROWB);
                     uint8_t* dst = sQD + st * C::STAGE;
@@ -191,9 +242,25 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                                     t.qb_c0 + cc * C::HW, t.q_local_r0 + rc * C::RC, t.hn, t.hb);
                     }
                 }
+                float* x = s_x + st * 2 * C::NKP;
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    const int j = lane + 32 * u;
+                    if (j < C::NKP) {
+                        x[j] = pre_l2[u];
+                        x[C::NKP + j] = pre_dl[u];
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(x_full + st);
+                if (++cc == t.n_cc) {
+                    cc = 0;
+                    ++rc;
+                }
+                if (ch + 1 < t.n_ch) fetch(t, rc, cc);
             }
-            lt.drain(wctx);
         }
+        if (lane == 0) lt.drain(wctx);
     } else if (warp == 9) {
         // ------------------------------------------------------------------ MMA issue: scores
         // Two warps issue MMAs, so that the bookkeeping of one runs under the MMAs of the other:
@@ -206,8 +273,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         const uint32_t k_lo = smem_desc_lo(smem_u32(sK), 16), v_lo = smem_desc_lo(smem_u32(sV), 16);
         const uint32_t qd_base = smem_u32(sQD);
         uint32_t n = 0, it = 0;
-        for (int i = 0; i < n_my; ++i) {
-            const TileGeo t = tile_geo(i);
+        for (int i = 0; i < n_my; ++i, walk.next()) {
+            const TileGeo t = tile_geo(walk);
             if (t.n_ch == 0) continue;
             for (int ch = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t q_addr = qd_base + (n % NSTQ) * C::STAGE, g_addr = q_addr + C::KV_BYTES;
@@ -217,6 +284,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                 if (ch == 0) mbar_wait(kv_full, it & 1, wctx, kErrLoadWait);
                 if (lane == 0) NA2D_TR(2, 1, n);
                 mbar_wait(qd_full + n % NSTQ, (n / NSTQ) & 1, wctx, kErrLoadWait);
+                mbar_wait(x_full + n % NSTQ, (n / NSTQ) & 1, wctx, kErrLoadWait);
                 if (lane == 0) NA2D_TR(2, 3, n);
                 mbar_wait(st_free + (n & 1), ((n >> 1) & 1) ^ 1, wctx, kErrMmaWait);
                 if (lane == 0) NA2D_TR(2, 5, n);
@@ -250,8 +318,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         constexpr uint32_t hi = smem_desc_hi(C::ATOM, C::SWZ);
         const uint32_t qd_base = smem_u32(sQD);
         uint32_t n = 0, it = 0;
-        for (int i = 0; i < n_my; ++i) {
-            const TileGeo t = tile_geo(i);
+        for (int i = 0; i < n_my; ++i, walk.next()) {
+            const TileGeo t = tile_geo(walk);
             if (t.n_ch == 0) continue;
             for (int ch = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t q_addr = qd_base + (n % NSTQ) * C::STAGE, g_addr = q_addr + C::KV_BYTES;
@@ -305,8 +373,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         if (lane == 0) {
             uint32_t it = 0;                            // non-empty tile counter
             LoadTracker lt(bars);
-            for (int i = 0; i < n_my; ++i) {
-                const TileGeo t = tile_geo(i);
+            for (int i = 0; i < n_my; ++i, walk.next()) {
+                const TileGeo t = tile_geo(walk);
                 if (t.n_ch == 0) continue;
                 if (!lt.acquire(kv_empty, (it & 1) ^ 1, wctx)) break;
                 lt.arm(kv_full, it & 1, 2u * C::Q_BYTES);
@@ -320,7 +388,9 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                 // load from HBM issued then is what the next tile would wait for: bring the next
                 // tile's K, V into L2 now.
                 if (i + 1 < n_my) {
-                    const TileGeo tn = tile_geo(i + 1);
+                    TileWalk ahead = walk;
+                    ahead.next();
+                    const TileGeo tn = tile_geo(ahead);
 #pragma unroll
                     for (int s = 0; s < C::NS; ++s) {
                         tma_prefetch_5d(&tm_k, s * 64, tn.kc0, tn.kr0, tn.hn, tn.hb);
@@ -338,8 +408,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         uint8_t* stage = sOut + quarter * 2 * OutStage<32>::BYTES;
         constexpr int RPO = D / 32;                          // 32-channel rounds per output
         uint32_t it = 0, seq = 0;
-        for (int i = 0; i < n_my; ++i) {
-            const TileGeo t = tile_geo(i);
+        for (int i = 0; i < n_my; ++i, walk.next()) {
+            const TileGeo t = tile_geo(walk);
             if (t.n_ch == 0) {                               // no local query sees this tile: zeros
                 uint32_t z[32];
 #pragma unroll
@@ -397,49 +467,19 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         // Both groups work on every chunk: warps w and w + 4 own the same 32 keys (tensor-memory
         // lanes) and take alternate 8-column blocks of the warp's active range, so a chunk's S^T and
         // dP^T spend half as long in registers before the output MMAs may start - that time is part
-        // of the chain that bounds the kernel (score MMAs -> this -> output MMAs -> stage free).
+        // of the chain that bounds the kernel (score MMAs -> this -> output MMAs -> stage free).  The blocks an inner tile
+        // needs are done without a branch between them: their chains of loads, exponentials and conversions overlap.
         reg_inc<kDkvRegsSoftmax>();
         const int quarter = warp & 3, group = warp >> 2;
         const int row = quarter * 32 + lane;                 // key of the tile = tensor-memory lane
-        const int gtid = quarter * 32 + lane;                // 0..127 inside the group
         const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-        // a warp's 32 / TW key rows are seen from at most that many + 2 ks - 2 query rows
-        constexpr int kRows = (32 / TW - 1 + 2 * KS - 1) < C::RC ? (32 / TW - 1 + 2 * KS - 1) : C::RC;
-        constexpr int kBlocks = (kRows * C::HW - 1) / 8 + 2;
-        constexpr int NACT = kBlocks < C::NB8 ? kBlocks : C::NB8;   // 8-column blocks a warp pair can have in range
-        constexpr int NOWN = (NACT + 1) / 2;                        // of which one warp takes at most
-        constexpr unsigned long long kRowRep = C::ROW_REP;          // bit r * HW set for every chunk row r
-
-        // lse and delta of this thread's query of chunk (rc, cc) of tile t (zero outside the band); the
-        // values are fetched one chunk ahead, so that their latency runs under the wait for the
-        // chunk's scores instead of before it
-        auto fetch = [&](const TileGeo& t, int rc, int cc, float& l2, float& dl) {
-            l2 = 0.f;
-            dl = 0.f;
-            if (gtid < C::NK) {
-                const int br = rc * C::RC + gtid / C::HW, qc = t.qb_c0 + cc * C::HW + gtid % C::HW;
-                if (br < t.n_rows && qc < g.W) {
-                    const size_t qi = (static_cast<size_t>(t.bn) * g.Hq + (t.q_local_r0 + br)) * g.W + qc;
-                    l2 = lse[qi];
-                    dl = delta[qi];
-                }
-            }
-        };
-        // first tile with chunks at or after i
-        auto next_tile = [&](int i, TileGeo& t) {
-            for (; i < n_my; ++i) {
-                t = tile_geo(i);
-                if (t.n_ch > 0) break;
-            }
-            return i;
-        };
+        const uint64_t sl2 = pair2(g.sl2, g.sl2), scale2 = pair2(g.scale, g.scale);
+        constexpr int NOWN = C::NOWN, NALL = C::NALL;
 
         uint32_t n = 0;
-        TileGeo t;
-        int i = next_tile(0, t);
-        float pre_l2 = 0.f, pre_dl = 0.f;
-        if (i < n_my) fetch(t, 0, 0, pre_l2, pre_dl);
-        while (i < n_my) {
+        for (int i = 0; i < n_my; ++i, walk.next()) {
+            const TileGeo t = tile_geo(walk);
+            if (t.n_ch == 0) continue;
             const int kr = min(t.kr0 + (row / TW), g.Hkv - 1), kc = min(t.kc0 + (row % TW), g.W - 1);
             // the queries that see this thread's key: box rows [row_lo, row_hi), box columns [col_lo, col_hi)
             const int kg = g.kv_row0 + kr;
@@ -449,63 +489,52 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             const int col_hi = na2d_bwe(kc, g.W, KS) - t.qb_c0;
             const int wrow_lo = __shfl_sync(0xffffffffu, row_lo, 0);
             const int wrow_hi = __shfl_sync(0xffffffffu, row_hi, 31);
-            TileGeo t_next = t;
-            int i_next = n_my;
+
+            // of the chunk rows from r_off on: the warp's active blocks, the first one it takes, and this key's rows in
+            // them (one bit a query)
+            int b_hi = 0, b0 = 0;
+            uint32_t rows8[NALL];                            // of the blocks b0 + 2 a + group
+            unsigned long long rows64 = 0;                   // (general strips: of the chunk)
+            auto row_part = [&](int r_off) {
+                const int ra = max(wrow_lo - r_off, 0), rb = min(wrow_hi - r_off, C::RC);
+                b_hi = rb > ra ? (min(rb * C::HW, C::NK) + 7) >> 3 : 0;
+                b0 = min(rb > ra ? (ra * C::HW) >> 3 : 0, C::NB8 - 2 * NOWN);
+                const int ta = max(row_lo - r_off, 0) * C::HW, tb = max(min(row_hi - r_off, C::RC), 0) * C::HW;
+                if constexpr (C::PATTERN) {
+#pragma unroll
+                    for (int a = 0; a < NALL; ++a) rows8[a] = range_bits<8>(ta, tb, 8 * (b0 + 2 * a + group));
+                } else {
+                    rows64 = tb > ta ? (tb >= 64 ? ~0ull : (1ull << tb) - 1ull) & ~((1ull << ta) - 1ull) : 0ull;      // ta < 64
+                }
+            };
+            row_part(0);
 
             for (int ch = 0, rc = 0, cc = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t stage = n & 1u, k = n >> 1;  // tensor-memory stage and its use counter
                 const uint32_t t_stage = tmem_lane + stage * C::TMEM_STAGE;
-                const int r_off = rc * C::RC, c_off = cc * C::HW;       // chunk ch = rc * n_cc + cc
+                const int c_off = cc * C::HW;               // chunk ch = rc * n_cc + cc
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 0, n);
-                // each group keeps its own copy of the chunk's lse * log2(e) and delta (two buffers: a
-                // warp may be one chunk ahead of the others of its group, the barrier below keeps it
-                // from two)
-                float* x_lse = s_x + ((group * 2 + stage) * 2) * 64;
-                float* x_delta = x_lse + 64;
-                if (gtid < C::NK) {
-                    x_lse[gtid] = pre_l2 * kLog2e;
-                    x_delta[gtid] = pre_dl * g.scale;       // dS^T carries the softmax scale of dK: scale p (dP - delta)
-                }
-                // the warp's keys are seen from chunk rows [ra, rb): its active column range
-                const int ra = max(wrow_lo - r_off, 0), rb = min(wrow_hi - r_off, C::RC);
-                const int j_lo = ra * C::HW;
-                const int j_hi = rb > ra ? min(rb * C::HW, C::NK) : 0;
-                const int b_hi = (j_hi + 7) >> 3;
-                const int b_lo = j_hi > 0 ? (j_lo >> 3) : 0;
-                // this thread's column segment inside a chunk row
-                const int cl = max(col_lo - c_off, 0), chi = min(col_hi - c_off, C::HW);
-                const int seg_len = chi - cl;
+                const float* x_lse = s_x + (n % NSTQ) * 2 * C::NKP;
+                const float* x_delta = x_lse + C::NKP;
+                // this thread's column segment inside a chunk row; the chunk's queries that see its key
+                const int cl = max(col_lo - c_off, 0), seg_len = min(col_hi - c_off, C::HW) - cl;
                 const uint32_t seg = seg_len > 0 ? ((1u << seg_len) - 1u) : 0u;
-                // validity of the chunk's (at most 64) columns for this thread's key, one bit each:
-                // its column segment repeated in every chunk row, cut to its row range
-                unsigned long long m64 = 0ull;
-                {
-                    const int ta = max(row_lo - r_off, 0), tb = min(row_hi - r_off, C::RC);
-                    const unsigned long long rows_hi = tb * C::HW >= 64 ? ~0ull : ((1ull << (max(tb, 0) * C::HW)) - 1ull);
-                    const unsigned long long rows_lo = (1ull << (ta * C::HW)) - 1ull;       // ta * HW < 64
-                    if (tb > ta) m64 = ((kRowRep * seg) << cl) & rows_hi & ~rows_lo;
-                }
-                bar_sync(5 + group, 128);                                   // lse / delta are in place
-                if (++cc == t.n_cc) {
-                    cc = 0;
-                    ++rc;
-                }
-                if (ch + 1 < t.n_ch) {
-                    fetch(t, rc, cc, pre_l2, pre_dl);
-                } else {
-                    i_next = next_tile(i + 1, t_next);
-                    if (i_next < n_my) fetch(t_next, 0, 0, pre_l2, pre_dl);
-                }
-                if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 1, n);
+                uint32_t cols8 = 0;
+                unsigned long long m64 = 0;
+                if constexpr (C::PATTERN) cols8 = (seg << cl) * C::REP8;
+                else m64 = ((C::ROW_REP * seg) << cl) & rows64;
+                auto seen = [&](int a) {                    // of block b0 + 2 a + group
+                    return C::PATTERN ? rows8[a] & cols8 : static_cast<uint32_t>(m64 >> (8 * (b0 + 2 * a + group))) & 0xffu;
+                };
 
                 mbar_wait(s_full + stage, k & 1, wctx, kErrMmaWait);
                 tc_fence_after();
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 2, n);
-                uint32_t s[NOWN][8], dp[NOWN][8];
+                uint32_t s[NALL][8], dp[NALL][8];
 #pragma unroll
-                for (int a = 0; a < NOWN; ++a) {
-                    const int blk = b_lo + 2 * a + group;
-                    if (blk < b_hi) {                                       // warp-uniform
+                for (int a = 0; a < NALL; ++a) {
+                    const int blk = b0 + 2 * a + group;
+                    if (a < NOWN || blk < b_hi) {                           // warp-uniform
                         tmem_ld_32x8(t_stage + C::TMEM_ST + 8 * blk, s[a]);
                         tmem_ld_32x8(t_stage + C::TMEM_DPT + 8 * blk, dp[a]);
                     }
@@ -515,12 +544,40 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                 // partner warp must have its blocks in registers too before either of them writes.
                 bar_sync(1 + quarter, 64);
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 3, n);
+                auto block = [&](int a, uint32_t (&wp)[4], uint32_t (&wd)[4], uint32_t (&wr2)[4]) {
+                    const int blk = b0 + 2 * a + group;
+                    const uint32_t vmask = seen(a);
+#pragma unroll
+                    for (int e4 = 0; e4 < 2; ++e4) {
+                        const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(x_lse + 8 * blk + 4 * e4);
+                        const ulonglong2 nd = *reinterpret_cast<const ulonglong2*>(x_delta + 8 * blk + 4 * e4);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int e = 4 * e4 + 2 * h, e2 = e / 2;
+                            const bool ok0 = (vmask >> e) & 1u, ok1 = (vmask >> (e + 1)) & 1u;
+                            const uint64_t x = fma2(pair2(s[a][e], s[a][e + 1]), sl2, h ? nl.y : nl.x);
+                            const uint64_t pe = pair2(fast_exp2(lo2(x)), fast_exp2(hi2(x)));
+                            const uint64_t de = mul2(pe, fma2(pair2(dp[a][e], dp[a][e + 1]), scale2, h ? nd.y : nd.x));
+                            const float ds0 = ok0 ? lo2(de) : 0.f, ds1 = ok1 ? hi2(de) : 0.f;    // select, never multiply by zero
+                            wp[e2] = pack2<DT>(ok0 ? lo2(pe) : 0.f, ok1 ? hi2(pe) : 0.f);
+                            wd[e2] = pack2<DT>(ds0, ds1);
+                            wr2[e2] = SPLIT ? pack2_residual_bf16(ds0, ds1, wd[e2]) : 0u;
+                        }
+                    }
+                };
+                auto store = [&](int a, const uint32_t (&wp)[4], const uint32_t (&wd)[4], const uint32_t (&wr2)[4]) {
+                    const int blk = b0 + 2 * a + group;
+                    tmem_st_32x4(t_stage + C::TMEM_PT + 4 * blk, wp);
+                    tmem_st_32x4(t_stage + C::TMEM_DST + 4 * blk, wd);
+                    if (SPLIT) tmem_st_32x4(t_stage + C::TMEM_RES + 4 * blk, wr2);
+                };
                 {   // blocks outside the active range hold zeros (this warp: every other one of them)
                     const uint32_t z[4] = {0u, 0u, 0u, 0u};
+                    const int b_end = max(b_hi, b0 + 2 * NOWN);
 #pragma unroll
-                    for (int blk = 0; blk < C::NB8; ++blk) {
-                        const bool in_range = blk >= b_lo && blk < b_lo + NACT && blk < b_hi;
-                        if (!in_range && ((blk & 1) == group)) {
+                    for (int b = 0; b < C::NB8 / 2; ++b) {
+                        const int blk = 2 * b + ((group ^ b0) & 1);         // the blocks of b0's parity are group 0's
+                        if (blk < b0 || blk >= b_end) {
                             tmem_st_32x4(t_stage + C::TMEM_PT + 4 * blk, z);
                             tmem_st_32x4(t_stage + C::TMEM_DST + 4 * blk, z);
                             if (SPLIT) tmem_st_32x4(t_stage + C::TMEM_RES + 4 * blk, z);
@@ -528,49 +585,29 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                     }
                 }
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 6, n);
+                // (all blocks first, then their stores: a store waits for its block's conversions)
+                uint32_t wp[NOWN][4], wd[NOWN][4], wr2[NOWN][4];
 #pragma unroll
-                for (int a = 0; a < NOWN; ++a) {
-                    const int blk = b_lo + 2 * a + group;
-                    if (blk < b_hi) {
-                        const uint32_t vmask = static_cast<uint32_t>(m64 >> (8 * blk)) & 0xffu;
-                        float l2[8], dl[8];
+                for (int a = 0; a < NOWN; ++a) block(a, wp[a], wd[a], wr2[a]);
 #pragma unroll
-                        for (int v4 = 0; v4 < 2; ++v4) {
-                            const float4 x = *reinterpret_cast<const float4*>(x_lse + 8 * blk + 4 * v4);
-                            const float4 y = *reinterpret_cast<const float4*>(x_delta + 8 * blk + 4 * v4);
-                            l2[4 * v4] = x.x; l2[4 * v4 + 1] = x.y; l2[4 * v4 + 2] = x.z; l2[4 * v4 + 3] = x.w;
-                            dl[4 * v4] = y.x; dl[4 * v4 + 1] = y.y; dl[4 * v4 + 2] = y.z; dl[4 * v4 + 3] = y.w;
-                        }
-                        uint32_t wp[4], wd[4], wr2[4];
+                for (int a = 0; a < NOWN; ++a) store(a, wp[a], wd[a], wr2[a]);
 #pragma unroll
-                        for (int e2 = 0; e2 < 4; ++e2) {
-                            float p[2], ds[2];
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const int e = 2 * e2 + h;
-                                const float pe = fast_exp2(fmaf(__uint_as_float(s[a][e]), g.sl2, -l2[e]));
-                                const bool ok = (vmask >> e) & 1u;         // select, never multiply by zero
-                                p[h] = ok ? pe : 0.f;
-                                ds[h] = ok ? pe * fmaf(__uint_as_float(dp[a][e]), g.scale, -dl[e]) : 0.f;
-                            }
-                            wp[e2] = pack2<DT>(p[0], p[1]);
-                            wd[e2] = pack2<DT>(ds[0], ds[1]);
-                            wr2[e2] = SPLIT ? pack2_residual_bf16(ds[0], ds[1], wd[e2]) : 0u;
-                        }
-                        tmem_st_32x4(t_stage + C::TMEM_PT + 4 * blk, wp);
-                        tmem_st_32x4(t_stage + C::TMEM_DST + 4 * blk, wd);
-                        if (SPLIT) tmem_st_32x4(t_stage + C::TMEM_RES + 4 * blk, wr2);
+                for (int a = NOWN; a < NALL; ++a)
+                    if (b0 + 2 * a + group < b_hi) {
+                        block(a, wp[0], wd[0], wr2[0]);
+                        store(a, wp[0], wd[0], wr2[0]);
                     }
-                }
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 4, n);
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full + stage);
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 5, n);
+                if (++cc == t.n_cc) {
+                    cc = 0;
+                    if (ch + 1 < t.n_ch) row_part(++rc * C::RC);
+                }
             }
-            i = i_next;
-            t = t_next;
         }
     }
 
@@ -585,7 +622,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
 template <typename DT, int D, int KS>
 int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
                 const TensorArg& d_o, const float* delta, const TensorArg& d_k, const TensorArg& d_v) {
-    using C = DkvCfg<D, KS, IsBf16<DT>::value>;
+    using C = DkvCfg<D, KS>;
     const Na2dGeom& g = lc.g;
     CUtensorMap tk, tv, tq, tg, tdk, tdv;
     int rc = make_map(&tk, k, lc.dtype, lc.B, g.N, g.Hkv, g.W, D, TW, TH);
