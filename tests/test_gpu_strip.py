@@ -1,0 +1,60 @@
+"""GPU tests of the tensor-core kernels of the larger windows: column strips, two query tiles in flight."""
+import pytest
+import torch
+
+import e_natten_b200 as na
+from oracle import na2d_oracle as orc
+from helpers import assert_close, make_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def step(q, k, v, d_o, ks):
+    qd, kd, vd, gd = (t.to(DEV) for t in (q, k, v, d_o))
+    o, lse = na.natten2d_forward(qd, kd, vd, ks)
+    grads = na.natten2d_backward(qd, kd, vd, o, lse, gd, ks)
+    na.check_kernels(DEV)
+    return (o, lse, *grads)
+
+
+# Units of 2 x 2 and 2 x 3 tiles, enough of them for two tiles on some CTAs and one on others (the forward takes pairs of tiles from
+# 149 tiles on); the second tile row and the last column hold one to nine pixels, every border clamps.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("ks,H,W", [(7, 17, 17), (9, 21, 16), (11, 25, 23), (13, 17, 13)])
+def test_odd_and_even_tiles_of_a_cta(ks, H, W, D, dtype):
+    shape = (2, 20, H, W, D)
+    q, k, v, d_o = make_inputs(shape, dtype, ks, q_scale=D ** -0.5)
+    got = step(q, k, v, d_o, ks)
+    want = orc.natten2d_fwd_bwd(q, k, v, d_o, ks)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), got, want):
+        assert_close(g, w, dtype, f"{name} {shape} ks={ks}")
+
+
+# Three tile rows, the middle one away from both borders, at the sizes on either side of where the forward changes kernels.
+@pytest.mark.parametrize("units", [1, 13])
+@pytest.mark.parametrize("ks,D", [(7, 32), (9, 64), (13, 128)])
+def test_inner_and_border_tiles(ks, D, units):
+    shape = (1, units, 48, 30, D)
+    q, k, v, d_o = make_inputs(shape, torch.bfloat16, 5, q_scale=D ** -0.5)
+    got = step(q, k, v, d_o, ks)
+    want = orc.natten2d_fwd_bwd(q, k, v, d_o, ks)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), got, want):
+        assert_close(g, w, torch.bfloat16, f"{name} {shape} ks={ks}")
+
+
+@pytest.mark.parametrize("bad", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("ks,D,at", [(7, 32, (8, 9)), (13, 128, (0, 15)), (9, 64, (16, 7))])
+def test_a_key_reaches_only_the_windows_that_hold_it(ks, D, at, bad):
+    """Two tiles in flight, forward: scores outside a window are left out whatever they hold."""
+    q, k, v, _ = (t.to(DEV) for t in make_inputs((1, 80, 17, 17, D), torch.bfloat16, 3, q_scale=D ** -0.5))
+    clean, clean_lse = na.natten2d_forward(q, k, v, ks)
+    k[:, :, at[0], at[1], D // 2] = bad
+    o, lse = na.natten2d_forward(q, k, v, ks)
+    na.check_kernels(DEV)
+    ws = [orc.window_start(i, 17, ks) for i in range(17)]
+    held = torch.tensor([[a <= at[0] < a + ks and b <= at[1] < b + ks for b in ws] for a in ws], device=DEV)
+    assert torch.equal(o[:, :, ~held], clean[:, :, ~held]) and torch.equal(lse[:, :, ~held], clean_lse[:, :, ~held])
+    if bad != bad:
+        assert o[:, :, held].isnan().all()
