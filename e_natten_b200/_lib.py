@@ -110,7 +110,7 @@ def _load_torch_ext():
         raise ImportError(f"{path} is missing: run `python e_natten_b200/build.py`")
     from . import _na2d_torch
     _na2d_torch.bind_abi(*(C.cast(fn, C.c_void_p).value
-                           for fn in (lib.na2d_forward_ex, lib.na2d_backward_ex, lib.na2d_backward_workspace)))
+                           for fn in (lib.na2d_forward_ex, lib.na2d_backward_ex, lib.na2d_backward_workspace, lib.na2d_poll)))
     return _na2d_torch
 
 

@@ -80,44 +80,69 @@ int check_device(int device) {
     return state[device] == 1 ? NA2D_OK : NA2D_ERR_NO_DEVICE;
 }
 
-// ---- device error word ---------------------------------------------------------------------------
-// Two words per device (a file-scope device variable has one instance per device context).
-// [0]: bits say which kind of bounded wait gave up; kernels get its address as an argument.
-// [1]: the limit of a bounded wait in microseconds, 0 = the built-in 4 s.  Set once per device from
-// the environment variable NA2D_WAIT_LIMIT_US: a profiler pass that instruments every instruction
+// ---- error state ---------------------------------------------------------------------------------
+// What the waits of a device's kernels report to, and their limit; kernels get its address as an argument.  A wait that
+// gives up writes a code for its kind to a pinned host word: na2d_poll looks there, which costs no CUDA call (a copy of a device
+// word and an event per backward took 8 us of a small call, and a slot between its kernels).  The limit, in microseconds, 0 =
+// the built-in 4 s, comes from the environment variable NA2D_WAIT_LIMIT_US: a profiler pass that instruments every instruction
 // can stretch a healthy hand-over past the built-in limit (seen under `ncu --set full`).
-__device__ unsigned int g_error_word[2] = {0u, 0u};
+__device__ na2d_ptx::ErrorState g_errors;
 
-// Device address of g_error_word on `device` (which must be current), looked up once per device.
-int error_word_address(int device, unsigned int** out) {
+struct Errors {
+    const na2d_ptx::ErrorState* device = nullptr;
+    volatile unsigned int* word = nullptr;
+};
+std::atomic<volatile unsigned int*> g_error_words[kMaxDevices];     // null until the device's state is set up
+
+// The error state of `device` (which must be current), set up once per device; that may happen while a stream is being captured,
+// so it stays off the streams of others.
+int error_state(int device, Errors* out) {
     static std::mutex mu;
-    static unsigned int* cache[kMaxDevices];
+    static Errors cache[kMaxDevices];
     if (device < 0 || device >= kMaxDevices) return NA2D_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lock(mu);
-    if (cache[device] == nullptr) {
-        void* p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_error_word);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_error_word)");
-        if (const char* env = getenv("NA2D_WAIT_LIMIT_US")) {
-            const unsigned long long v = strtoull(env, nullptr, 10);
-            if (v > 0 && v <= 0xffffffffull) {
-                const unsigned int limit = (unsigned int)v;
-                e = cudaMemcpy(static_cast<unsigned int*>(p) + 1, &limit, sizeof(limit), cudaMemcpyHostToDevice);
-                if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(wait limit)");
+    if (cache[device].device == nullptr) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        NA2D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const int rc = [&]() -> int {
+            void *state = nullptr, *host = nullptr;
+            cudaStream_t st = nullptr;
+            na2d_ptx::ErrorState init{nullptr, 0u, 0u};
+            if (const char* env = getenv("NA2D_WAIT_LIMIT_US")) {
+                const unsigned long long v = strtoull(env, nullptr, 10);
+                if (v > 0 && v <= 0xffffffffull) init.limit_us = (unsigned int)v;
             }
-        }
-        cache[device] = static_cast<unsigned int*>(p);
+            NA2D_CUDA(cudaGetSymbolAddress(&state, g_errors));
+            NA2D_CUDA(cudaHostAlloc(&host, sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable));
+            *static_cast<unsigned int*>(host) = 0;
+            cudaError_t e = cudaHostGetDevicePointer((void**)&init.word, host, 0);
+            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+            if (e == cudaSuccess) {
+                e = cudaMemcpyAsync(state, &init, sizeof(init), cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                cudaStreamDestroy(st);
+            }
+            if (e != cudaSuccess) {
+                cudaFreeHost(host);
+                return cuda_fail(e, "setting up the error state");
+            }
+            cache[device] = Errors{static_cast<const na2d_ptx::ErrorState*>(state), static_cast<unsigned int*>(host)};
+            g_error_words[device].store(cache[device].word, std::memory_order_release);
+            return NA2D_OK;
+        }();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc != NA2D_OK) return rc;
     }
     *out = cache[device];
     return NA2D_OK;
 }
 
 // The kernel of na2d_selftest_wait_timeout: one thread waits on a barrier nothing completes.
-__global__ void wait_timeout_kernel(unsigned int* err_word, unsigned long long limit_ns) {
+__global__ void wait_timeout_kernel(const na2d_ptx::ErrorState* errors, unsigned long long limit_ns) {
     __shared__ uint64_t bar;
     __shared__ na2d_ptx::WaitState state;
     if (threadIdx.x == 0) {
-        na2d_ptx::wait_state_init(&state, err_word, limit_ns);
+        na2d_ptx::wait_state_init(&state, errors, limit_ns);
         state.limit_us = static_cast<uint32_t>(limit_ns / 1000ull);        // the self-test's own limit, whatever is configured
         na2d_ptx::mbar_init(&bar, 1);
         na2d_ptx::mbar_fence_init();
@@ -321,10 +346,10 @@ int after_tile(int rc, int launches) {
 na2d_tc::TensorArg targ(const Tensor& t) { return na2d_tc::TensorArg{t.ptr, t.st}; }
 
 int launch_ctx(const Problem& p, int* launched, na2d_tc::LaunchCtx* lc) {
-    unsigned int* err = nullptr;
-    int rc = error_word_address(p.device, &err);
+    Errors err;
+    int rc = error_state(p.device, &err);
     if (rc != NA2D_OK) return rc;
-    *lc = na2d_tc::LaunchCtx{p.g, p.dtype, p.B, p.device, p.st, err, launched, p.dkdv_f32, p.sm_margin};
+    *lc = na2d_tc::LaunchCtx{p.g, p.dtype, p.B, p.device, p.st, err.device, launched, p.dkdv_f32, p.sm_margin};
     return NA2D_OK;
 }
 
@@ -610,15 +635,6 @@ int pair_inverse(const PairProblem& p, const void* attn, const void* x, void* ou
     });
 }
 
-// ---- na2d_poll state -----------------------------------------------------------------------------------------
-struct PollState {
-    unsigned int* host = nullptr;     // pinned
-    cudaEvent_t ev = nullptr;
-    bool pending = false;
-};
-std::mutex g_poll_mu;
-PollState g_poll[kMaxDevices];
-
 }  // namespace
 
 extern "C" {
@@ -828,55 +844,27 @@ int na2d_backward_static_scratch(const void* q, const void* k, const void* v, co
 int na2d_check(int device, void* stream) {
     DeviceScope scope(device);
     if (scope.err != cudaSuccess) return cuda_fail(scope.err, "cudaSetDevice");
-    unsigned int* addr = nullptr;
-    int rc = error_word_address(device, &addr);
+    Errors err;
+    int rc = error_state(device, &err);
     if (rc != NA2D_OK) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    unsigned int word = 0;
-    NA2D_CUDA(cudaMemcpyAsync(&word, addr, sizeof(word), cudaMemcpyDeviceToHost, st));
-    NA2D_CUDA(cudaStreamSynchronize(st));
+    NA2D_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    const unsigned int word = *err.word;
     if (word != 0) {
-        NA2D_CUDA(cudaMemsetAsync(addr, 0, sizeof(word), st));
-        NA2D_CUDA(cudaStreamSynchronize(st));
+        *err.word = 0;
         snprintf(t_cuda_err, sizeof(t_cuda_err),
-                 "device error word 0x%x (1: load wait, 2: MMA wait, 4: other wait, 8: shared memory base not 1024-byte aligned)", word);
+                 "error word 0x%x (1: load wait, 2: MMA wait, 4: other wait, 8: shared memory base not 1024-byte aligned)", word);
         return NA2D_ERR_KERNEL_WAIT;
     }
     return NA2D_OK;
 }
 
 int na2d_poll(int device, void* stream) {
+    (void)stream;
     if (device < 0 || device >= kMaxDevices) return NA2D_ERR_BAD_ARG;
-    DeviceScope scope(device);
-    if (scope.err != cudaSuccess) return cuda_fail(scope.err, "cudaSetDevice");
-    unsigned int* addr = nullptr;
-    int rc = error_word_address(device, &addr);
-    if (rc != NA2D_OK) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    std::lock_guard<std::mutex> lock(g_poll_mu);
-    PollState& ps = g_poll[device];
-    if (ps.host == nullptr) {
-        void* h = nullptr;
-        NA2D_CUDA(cudaHostAlloc(&h, sizeof(unsigned int), cudaHostAllocDefault));
-        ps.host = static_cast<unsigned int*>(h);
-        *ps.host = 0;
-        NA2D_CUDA(cudaEventCreateWithFlags(&ps.ev, cudaEventDisableTiming));
-    }
-    int result = NA2D_OK;
-    if (ps.pending) {
-        cudaError_t e = cudaEventQuery(ps.ev);
-        if (e == cudaErrorNotReady) return NA2D_OK;           // the previous copy is still on its way
-        if (e != cudaSuccess) return cuda_fail(e, "cudaEventQuery");
-        ps.pending = false;
-        if (*ps.host != 0) {
-            result = NA2D_ERR_KERNEL_WAIT;
-            NA2D_CUDA(cudaMemsetAsync(addr, 0, sizeof(unsigned int), st));
-        }
-    }
-    NA2D_CUDA(cudaMemcpyAsync(ps.host, addr, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-    NA2D_CUDA(cudaEventRecord(ps.ev, st));
-    ps.pending = true;
-    return result;
+    volatile unsigned int* word = g_error_words[device].load(std::memory_order_acquire);
+    if (word == nullptr || *word == 0) return NA2D_OK;         // null: no kernel that waits has run yet
+    *word = 0;
+    return NA2D_ERR_KERNEL_WAIT;
 }
 
 int na2d_selftest_wait_timeout(int device, void* stream, unsigned int limit_us) {
@@ -885,10 +873,10 @@ int na2d_selftest_wait_timeout(int device, void* stream, unsigned int limit_us) 
     int rc = check_device(device);
     if (rc != NA2D_OK) return rc;
     if (limit_us == 0 || limit_us > 1000000u) return NA2D_ERR_BAD_ARG;       // at most a second
-    unsigned int* addr = nullptr;
-    rc = error_word_address(device, &addr);
+    Errors err;
+    rc = error_state(device, &err);
     if (rc != NA2D_OK) return rc;
-    wait_timeout_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(addr, (unsigned long long)limit_us * 1000ull);
+    wait_timeout_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(err.device, (unsigned long long)limit_us * 1000ull);
     return after_launch();
 }
 

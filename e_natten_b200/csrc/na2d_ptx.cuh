@@ -35,8 +35,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // What a bounded wait needs to report that it gave up, kept in shared memory (one per CTA, set up
 // by one thread before the first wait) so that a waiting thread carries a single pointer: the abort
-// flag (set by the first waiter that gives up, it shortens every later wait of the CTA), the device
-// error word the host reads with na2d_check / na2d_poll, and the time limit of one wait.
+// flag (set by the first waiter that gives up, it shortens every later wait of the CTA), the error
+// word the host reads with na2d_check / na2d_poll, and the time limit of one wait.
 struct WaitState {
     uint32_t abort;
     uint32_t limit_us;       // microseconds a wait may last
@@ -54,12 +54,17 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
 __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.volatile.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void wait_state_init(WaitState* st, unsigned int* err_word, unsigned long long limit_ns) {
+// What a kernel gets of the device's error state: the word that a give-up is written to (pinned host memory, so that the host
+// looks at it without a copy), and the limit of a wait in microseconds where one is configured (else 0).
+struct ErrorState {
+    unsigned int* word;
+    unsigned int limit_us, pad;
+};
+__device__ __forceinline__ void wait_state_init(WaitState* st, const ErrorState* errors, unsigned long long limit_ns) {
     st->abort = 0;
-    // err_word[1], when set, overrides the limit (microseconds)
-    const uint32_t configured = err_word[1];
+    const uint32_t configured = errors->limit_us;
     st->limit_us = configured != 0u ? configured : static_cast<uint32_t>(limit_ns / 1000ull);
-    st->err_word = err_word;
+    st->err_word = errors->word;
 }
 
 // ------------------------------------------------------------------------------------ mbarrier
@@ -127,7 +132,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
         __nanosleep(1000);
     }
     st_shared_u32(st, 1u);
-    atomicOr(wc.st->err_word, err_code);
+    *static_cast<volatile unsigned int*>(wc.st->err_word) = err_code;
     return false;
 }
 

@@ -434,15 +434,15 @@ inline cudaError_t opt_in_smem(K kern, int bytes, int device, std::atomic<unsign
     return e;
 }
 
-// What every launcher gets besides the tensors: geometry, element type, device, stream, the device
-// error word of `device`, and a counter of launched kernels.
+// What every launcher gets besides the tensors: geometry, element type, device, stream, the error
+// state of `device`, and a counter of launched kernels.
 struct LaunchCtx {
     Na2dGeom g;
     int dtype;
     int B;
     int device;
     cudaStream_t st;
-    unsigned int* err_word;
+    const ErrorState* errors;
     int* launched;
     bool dkdv_f32;         // the dK/dV kernel writes fp32 (partial sums of a row band)
     int sm_margin;         // SMs to leave free for a kernel that runs beside this one

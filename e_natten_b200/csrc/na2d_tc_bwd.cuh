@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(384, 1)
 dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
           const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* __restrict__ delta,
-          const int want_dq_arg, unsigned int* __restrict__ err_word,
+          const int want_dq_arg, const ErrorState* __restrict__ errors,
           const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = DqCfg<D, KS, SPLIT>;
@@ -89,7 +89,7 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUte
     const bool want_dq = want_dq_arg != 0;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         mbar_init(q_full, 1);
         mbar_init(q_empty, 1);
         for (int i = 0; i < 2; ++i) {
@@ -471,7 +471,7 @@ int launch_dq(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, d_q.ptr != nullptr, lc.err_word, g,
+    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, d_q.ptr != nullptr, lc.errors, g,
                                         tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;

@@ -100,7 +100,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
             const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
             const float* __restrict__ lse, const float* __restrict__ delta, const int f32_out,
-            unsigned int* __restrict__ err_word, const Na2dGeom g, const int tiles_r, const int tiles_c,
+            const ErrorState* __restrict__ errors, const Na2dGeom g, const int tiles_r, const int tiles_c,
             const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = DkvCfg<D, KS>;
@@ -131,7 +131,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         mbar_init(kv_full, 1);
         mbar_init(kv_empty, 1);
         mbar_init(acc_full, 1);
@@ -640,7 +640,7 @@ int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, con
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 512, C::SMEM, lc.st>>>(tk, tv, tq, tg, tdk, tdv, lse, delta, lc.dkdv_f32 ? 1 : 0, lc.err_word, g,
+    kern<<<grid, 512, C::SMEM, lc.st>>>(tk, tv, tq, tg, tdk, tdv, lse, delta, lc.dkdv_f32 ? 1 : 0, lc.errors, g,
                                         tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;

@@ -41,14 +41,14 @@ __global__ void __launch_bounds__(384, 1)
 dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
            const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
            const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* __restrict__ delta,
-           unsigned int* __restrict__ err_word, const Na2dGeom g, const int tiles_r, const int tiles_c,
+           const ErrorState* __restrict__ errors, const Na2dGeom g, const int tiles_r, const int tiles_c,
            const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = Dq1Cfg<D, KS, SPLIT>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw;
     if (smem_u32(smem_raw) & 1023u) {                 // the swizzled operand layouts need it; never seen
-        if (threadIdx.x == 0) atomicOr(err_word, kErrSmemBase);
+        if (threadIdx.x == 0) *static_cast<volatile unsigned int*>(errors->word) = kErrSmemBase;
         return;
     }
     uint8_t* sQ = smem;
@@ -72,7 +72,7 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         mbar_init(q_full, 1);
         mbar_init(q_empty, 1);
         mbar_init(dq_full, 1);
@@ -495,7 +495,7 @@ int launch_dq1(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, cons
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, lc.err_word, g, tiles_r, tiles_c, (int)tiles);
+    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, lc.errors, g, tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
 }

@@ -67,7 +67,7 @@ template <typename DT, int D, int KS>
 __global__ void __launch_bounds__(512, 1)
 dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
            const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* delta, unsigned int* __restrict__ err_word,
+           const __grid_constant__ CUtensorMap tm_dq, const float* __restrict__ lse, float* delta, const ErrorState* __restrict__ errors,
            const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
     using C = Dq2Cfg<D, KS>;
@@ -101,7 +101,7 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const uint32_t total_units = (uint32_t)n_my * NCH;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         for (int i = 0; i < 4; ++i) {
             mbar_init(k_full + i, 1);
             mbar_init(k_empty + i, 1);
@@ -515,7 +515,7 @@ int launch_dq2(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, cons
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 512, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, lc.err_word, g, tiles_r, tiles_c,
+    kern<<<grid, 512, C::SMEM, lc.st>>>(tq, tg, tk, tv, tdq, lse, delta, lc.errors, g, tiles_r, tiles_c,
                                         (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;

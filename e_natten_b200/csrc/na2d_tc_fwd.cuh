@@ -67,7 +67,7 @@ template <typename DT, int D, int KS>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-           float* __restrict__ lse, unsigned int* __restrict__ err_word,
+           float* __restrict__ lse, const ErrorState* __restrict__ errors,
            const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     using C = FwdCfg<D, KS>;
     constexpr int NSTK = C::NSTK, NSTV = C::NSTV, NQ = C::NQ;
@@ -99,7 +99,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const uint32_t total_units = (uint32_t)n_my * C::NCH;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         for (int i = 0; i < 2; ++i) {
             mbar_init(q_full + i, 1);
             mbar_init(q_empty + i, 1);
@@ -476,6 +476,9 @@ int launch_forward(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, 
     const int tiles_r = (g.Hq + TH - 1) / TH, tiles_c = (g.W + TW - 1) / TW;
     const long long tiles = (long long)g.BN * tiles_r * tiles_c;
     if (tiles > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
+    // From one tile per SM on, two tiles in flight.  Up to there a tile has its SM to itself, and all eight softmax warps on
+    // it end it no later and often sooner (128 tiles, window 7 / 13: head dim 64 10.3 / 12.3 against 10.3 / 14.3 us, 128 10.3 / 14.4
+    // against 12.3 / 15.3); at 256 tiles it is 14.3 / 20.5 against 12.3 / 15.3 and 14.7 / 22.4 against 16.3 / 18.5 us.
     if (tiles > sm_count(lc.device)) return launch_forward2<DT, D, KS>(lc, q, k, v, o, lse, tiles, tiles_r, tiles_c);
     CUtensorMap tq, tk, tv, to;
     int rc = make_map(&tq, q, lc.dtype, lc.B, g.N, g.Hq, g.W, D, TW, TH);
@@ -487,7 +490,7 @@ int launch_forward(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, 
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.err_word, g, tiles_r, tiles_c, (int)tiles);
+    kern<<<grid, 384, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.errors, g, tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
     }

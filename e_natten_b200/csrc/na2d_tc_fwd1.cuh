@@ -37,7 +37,7 @@ template <typename DT, int D, int KS>
 __global__ void __launch_bounds__(512, 1)
 fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-            float* __restrict__ lse, unsigned int* __restrict__ err_word, const Na2dGeom g, const int tiles_r,
+            float* __restrict__ lse, const ErrorState* __restrict__ errors, const Na2dGeom g, const int tiles_r,
             const int tiles_c, const int total_tiles) {
     using C = Fwd1Cfg<D, KS>;
     extern __shared__ uint8_t smem_raw[];
@@ -71,7 +71,7 @@ fwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         mbar_init(q_full, 1);
         mbar_init(q_empty, 1);
         mbar_init(o_full, 1);
@@ -432,7 +432,7 @@ int launch_forward1(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k,
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 512, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.err_word, g, tiles_r, tiles_c, (int)tiles);
+    kern<<<grid, 512, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.errors, g, tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
 }

@@ -58,7 +58,7 @@ template <typename DT, int D, int KS>
 __global__ void __launch_bounds__(512, 1)
 fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
             const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-            float* __restrict__ lse, unsigned int* __restrict__ err_word,
+            float* __restrict__ lse, const ErrorState* __restrict__ errors,
             const Na2dGeom g, const int tiles_r, const int tiles_c, const int total_tiles) {
     using C = Fwd2Cfg<D, KS>;
     constexpr int NSTK = C::NSTK, NSTV = C::NSTV;
@@ -88,7 +88,7 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (tid == 0) {
-        wait_state_init(wctx.st, err_word, kWaitLimitNs);
+        wait_state_init(wctx.st, errors, kWaitLimitNs);
         for (int i = 0; i < 2; ++i) {
             mbar_init(q_full + i, 1);
             mbar_init(q_empty + i, 1);
@@ -479,7 +479,7 @@ int launch_forward2(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k,
     auto kern = fwd2_kernel<DT, D, KS>;
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
-    kern<<<persistent_grid(lc, tiles), 512, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.err_word, g, tiles_r, tiles_c, (int)tiles);
+    kern<<<persistent_grid(lc, tiles), 512, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.errors, g, tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
 }

@@ -202,8 +202,8 @@ def natten2d_backward(q, k, v, o, lse, d_o, kernel_size: int, rows: Optional[_li
 
 def poll_kernels(device) -> None:
     """Raise if a kernel of an earlier call on ``device`` reported that a bounded wait ran out.
-    Never waits for the GPU: it looks at the answer to the question the previous poll asked and
-    asks again (``na2d_poll``), so an error surfaces one call late."""
+    Never waits for the GPU: it looks at a host word that such a kernel writes to (``na2d_poll``), so an
+    error surfaces one call late."""
     dev = torch.device(device)
     _lib.check(_lib.lib.na2d_poll(dev.index or 0, _stream(dev)))
 
@@ -240,7 +240,8 @@ class Natten2d(torch.autograd.Function):
 def natten2d(q, k, v, kernel_size=7, scale=None):
     """Fused 2D neighborhood attention, differentiable; drop-in for ``e_natten.natten2d``.
     ``scale`` (default: none, as in the reference) multiplies the logits inside the kernels."""
-    return Natten2d.apply(q, k, v, kernel_size, scale)[0]
+    o = torch_ext.attention_2d(q, k, v, kernel_size, scale)      # None: not an ordinary call
+    return Natten2d.apply(q, k, v, kernel_size, scale)[0] if o is None else o
 
 
 def natten2d_with_lse(q, k, v, kernel_size=7, scale=None):
@@ -314,7 +315,8 @@ class Natten1d(torch.autograd.Function):
 
 def natten1d(q, k, v, kernel_size=7, scale=None):
     """Fused 1D neighborhood attention, differentiable; drop-in for ``e_natten.natten1d``."""
-    return Natten1d.apply(q, k, v, kernel_size, scale)
+    o = torch_ext.attention_1d(q, k, v, kernel_size, scale)
+    return Natten1d.apply(q, k, v, kernel_size, scale) if o is None else o
 
 
 # ---- the unfused pair (scores, apply) with the call shape of natten.functional --------------------------------

@@ -280,11 +280,10 @@ int na2d_backward_static_scratch(const void* q, const void* k, const void* v, co
  * No reference counterpart. */
 int na2d_check(int device, void* stream);
 
-/* The same check without waiting for the GPU: enqueues a copy of the error word to a pinned host
- * word on `stream` and returns what the previous such copy on this device brought back
- * (NA2D_OK if none has completed yet).  A caller that polls at every entry learns of a tripped
- * wait one call late but never stalls; the host word is allocated at the first poll on a device.
- * Once reported, the error is cleared.  No reference counterpart. */
+/* The same check without waiting for the GPU and without any CUDA call: looks at the host word that a
+ * tripped wait writes to.  A caller that polls at every entry learns of a tripped wait once the write has
+ * arrived, one call late, but never stalls; `stream` is not used.  Once reported, the error is cleared.
+ * No reference counterpart. */
 int na2d_poll(int device, void* stream);
 
 /* Self-test of the bounded waits: launches one small kernel whose only thread waits, with a limit
