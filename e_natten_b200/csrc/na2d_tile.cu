@@ -1,10 +1,13 @@
 // Launchers of the tiled CUDA-core kernels for one element type.
 #include "na2d_tile_entry.h"
 
+#include <initializer_list>
+
 #include "../../include/na2d.h"
 #include "na2d_tile.cuh"
 #include "na2d_tile_bwd.cuh"
 #include "na2d_tile_pair.cuh"
+#include "na2d_line.cuh"
 
 #if NA2D_TILE_DT == 0
 using Elem = float;
@@ -68,6 +71,16 @@ int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream
         return NA2D_ERR_CUDA;
     kernel<<<grid, threads, smem, st>>>(static_cast<P>(args)...);
     return cudaPeekAtLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
+}
+
+// Whether the kernels of na2d_line.cuh take these operands: rows of whole 16-byte pieces that start on 16-byte boundaries and
+// are short enough.
+bool in_line(const Na2dGeom& g, std::initializer_list<const Tensor*> operands) {
+    constexpr long long n = 16 / sizeof(Elem);
+    if (g.C % n != 0 || g.C * (int)sizeof(Elem) > na2d_line::max_row(sizeof(Elem))) return false;
+    for (const Tensor* t : operands)
+        if (reinterpret_cast<uintptr_t>(t->ptr) % 16 != 0 || t->st.b % n != 0 || t->st.n % n != 0 || t->st.w % n != 0) return false;
+    return true;
 }
 
 }  // namespace
@@ -139,6 +152,11 @@ int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, cons
         const auto kernel = g.C > kParkAbove<S> ? fwd_kernel<Elem, S::kKs, S::kOneD, true> : fwd_kernel<Elem, S::kKs, S::kOneD, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
+        if constexpr (S::kOneD) {
+            if (in_line(g, {&q, &k, &v, &o}))
+                return launch(na2d_line::fwd_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(g.C * sizeof(Elem)),
+                              st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(o, g.C), lse, g);
+        }
         return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(o, g.C), lse, g);
     });
@@ -151,6 +169,12 @@ int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, 
         const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
+        if constexpr (S::kOneD) {
+            if (in_line(g, {&q, &k, &v, &d_o, &d_q}))
+                return launch(na2d_line::dq_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(g.C * sizeof(Elem)),
+                              st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta,
+                              row_factor, (float4*)nullptr, (float4*)nullptr, 0, g);
+        }
         return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, row_factor, (float4*)nullptr,
                       (float4*)nullptr, whole_images<S>(g, g.Hq), g);
@@ -168,6 +192,24 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
         for (long long unit0 = 0; unit0 < g.BN; unit0 += turns.units) {
             const int units = (int)(g.BN - unit0 < turns.units ? g.BN - unit0 : turns.units);
             float4 *p = reinterpret_cast<float4*>(workspace), *ds = p + (long long)units * turns.rows * tiles_w * S::kWeights;
+            if constexpr (S::kOneD) {
+                static_assert(S::kTw == na2d_line::kTile && S::kWeights == na2d_line::kStrips * na2d_line::kU<S::kKs>, "one layout of the weights");
+                if (in_line(g, {&q, &k, &v, &d_o, &d_q, &d_k, &d_v})) {
+                    unsigned n = 0;
+                    if (int rc = tiles<S>(g, units, 1, &n)) return rc;
+                    const int row_bytes = g.C * (int)sizeof(Elem);
+                    if (int rc = launch(na2d_line::dq_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(row_bytes), st,
+                                        operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta,
+                                        (float*)nullptr, p, ds, (int)unit0, g))
+                        return rc;
+                    ++*launches;
+                    if (int rc = launch(na2d_line::key_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::key_smem<S::kKs>(row_bytes), st,
+                                        operand(q, g.C), operand(d_o, g.C), operand(d_k, g.C), operand(d_v, g.C), p, ds, (int)unit0, g))
+                        return rc;
+                    ++*launches;
+                    continue;
+                }
+            }
             const KeySum for_dk{ds, operand(q, g.C), operand(d_k, g.C)}, for_dv{p, operand(d_o, g.C), operand(d_v, g.C)};
             // Query tiles as far as the ring has room without losing a row that the next key tiles read, then the
             // key tiles that have all their queries; in one go where the ring holds the whole image.

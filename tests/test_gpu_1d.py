@@ -131,3 +131,33 @@ def test_1d_errors():
         na.natten1d(torch.zeros(1, 1, 8, 8, 32, device=DEV), q, q, 3)
     empty = torch.zeros(0, 1, 8, 32, device=DEV)
     assert na.natten1d(empty, empty, empty, 3).shape == empty.shape
+
+
+# Rows of whole 16-byte pieces: one lane in four with a piece more (48 channels), a tile and its remainders, sequences with both
+# ends within the window of one strip (28 tokens at window 13), the longest rows of either kernel family.
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 4), (torch.float32, 48), (torch.float32, 64), (torch.bfloat16, 8),
+                                     (torch.bfloat16, 48), (torch.float16, 128), (torch.bfloat16, 136)])
+@pytest.mark.parametrize("T,ks", [(128, 3), (129, 7), (140, 13), (268, 13), (28, 13), (13, 13), (391, 5), (127, 11), (260, 9)])
+def test_1d_rows_of_whole_pieces(T, ks, dtype, C):
+    q, k, v, d_o = _inputs((3, 40, T, C), dtype, T, C ** -0.5)
+    qd, kd, vd, gd = (t.to(DEV) for t in (q, k, v, d_o))
+    o, lse = na.natten1d_forward(qd, kd, vd, ks)
+    grads = na.natten1d_backward(qd, kd, vd, o, lse, gd, ks)
+    ro, rlse = orc.natten1d_fwd(q, k, v, ks)
+    for name, got, want in zip(("o", "lse", "dq", "dk", "dv"), (o, lse, *grads), (ro, rlse, *orc.natten1d_bwd(q, k, v, d_o, ks))):
+        assert_close(got, want, torch.float32 if name == "lse" and dtype == torch.float32 else dtype, f"{name} {T} {ks} {C}")
+
+
+def test_1d_infinities_stay_in_their_windows():
+    q, k, v, d_o = (t.to(DEV) for t in _inputs((2, 70, 200, 64), torch.bfloat16, 1, 0.125))
+    o, lse = na.natten1d_forward(q, k, v, 13)
+    clean = na.natten1d_backward(q, k, v, o, lse, d_o, 13)
+    v2, g2 = v.clone(), d_o.clone()
+    v2[:, :, 77] = float("inf")
+    g2[:, :, 120] = float("inf")
+    o2, _ = na.natten1d_forward(q, k, v2, 13)
+    grads = na.natten1d_backward(q, k, v, o, lse, g2, 13)
+    t = torch.arange(200, device=DEV)
+    assert torch.equal((o2 != o).any(-1).any(0).any(0), (t - 77).abs() <= 6) and o2[:, :, 71:84].isinf().all()
+    for got, want, near in zip(grads, clean, (0, 6, 6)):
+        assert torch.equal(got[:, :, (t - 120).abs() > near], want[:, :, (t - 120).abs() > near])
