@@ -14,6 +14,10 @@
 // tile i were), so the next tile's K_A and V_A can be fetched as soon as the score MMAs are done.
 // Twelve warps: 0-7 softmax (warps w and w+4 share 32 queries and split the 16-column blocks),
 // 8 TMA producer, 9 MMA issue, 10-11 idle (register donors).
+//
+// What bounds it: the chain of a tile - score MMAs, two strips of softmax, dS, dQ MMAs - all of tensor memory being in use by one
+// tile.  Arithmetic in packed fp32 pairs took, on one B200: 4 x 4 x 256 x 256 x 128, window 5, bf16 326 -> 306 us;
+// 4 x 4 x 128 x 128 x 64, window 5, bf16 68 -> 58 us; 4 x 4 x 128 x 128 x 32, window 3, fp16 59 -> 43 us.
 #pragma once
 
 namespace na2d_tc {
@@ -348,7 +352,8 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
             uint32_t s[2][NACT][16], dp[2][NACT][16];
             uint32_t vmask[2][NACT];
-            float d0 = 0.f, d1 = 0.f;
+            uint64_t delta2 = 0;                             // this half's part of delta
+            const uint64_t sl2 = pair2(g.sl2, g.sl2), nlse2 = pair2(-lse2, -lse2);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const uint32_t t_s = tmem_lane + (x ? C::TMEM_SB : C::TMEM_SA), t_dp = tmem_lane + (x ? C::TMEM_DPB : C::TMEM_DPA);
@@ -379,16 +384,15 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
                         for (int e = 0; e < 16; e += 2) {
                             const bool ok0 = (vmask[x][a] >> e) & 1u, ok1 = (vmask[x][a] >> (e + 1)) & 1u;
-                            const float p0 = ok0 ? fast_exp2(fmaf(__uint_as_float(s[x][a][e]), g.sl2, -lse2)) : 0.f;
-                            const float p1 = ok1 ? fast_exp2(fmaf(__uint_as_float(s[x][a][e + 1]), g.sl2, -lse2)) : 0.f;
+                            const uint64_t t = fma2(pair2(s[x][a][e], s[x][a][e + 1]), sl2, nlse2);
+                            const float p0 = ok0 ? fast_exp2(lo2(t)) : 0.f, p1 = ok1 ? fast_exp2(hi2(t)) : 0.f;
                             s[x][a][e] = __float_as_uint(p0);
                             s[x][a][e + 1] = __float_as_uint(p1);
                             // masked columns may hold anything: keep them out by selection, never by
                             // multiplying with zero
                             if (!ok0) dp[x][a][e] = 0u;
                             if (!ok1) dp[x][a][e + 1] = 0u;
-                            d0 = fmaf(p0, __uint_as_float(dp[x][a][e]), d0);
-                            d1 = fmaf(p1, __uint_as_float(dp[x][a][e + 1]), d1);
+                            delta2 = fma2(pair2(p0, p1), pair2(dp[x][a][e], dp[x][a][e + 1]), delta2);
                         }
                     }
                 }
@@ -396,14 +400,16 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             // both strips seen: add the partner's part; both halves now hold delta.  The barrier also
             // tells that the partner has read its blocks, so 16-bit operands may go over them.
             if (tid == 0) NA2D_TR(3, 4, i);
-            x_sum[(par * 2 + half) * 128 + row] = d0 + d1;
+            const float part = lo2(delta2) + hi2(delta2);
+            x_sum[(par * 2 + half) * 128 + row] = part;
             bar_sync(1 + quarter, 64);
-            const float dl = (d0 + d1) + x_sum[(par * 2 + (half ^ 1)) * 128 + row];
+            const float dl = part + x_sum[(par * 2 + (half ^ 1)) * 128 + row];
             if (q_valid && half == 0) delta[qi] = dl;
 
             // dS = scale p (dP - delta) as packed 16-bit pairs (head, and residual on the bf16 path); the
             // softmax scale of dQ goes in here, inside a multiply-add that replaces the subtraction
             const float dls = dl * g.scale;
+            const uint64_t scale2 = pair2(g.scale, g.scale), ndls2 = pair2(-dls, -dls);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const uint32_t t_ds = tmem_lane + (x ? C::TMEM_DPB : C::TMEM_DPA);
@@ -415,8 +421,9 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
                         for (int e2 = 0; e2 < 8; ++e2) {
                             // p and dP of masked columns are exact zeros here
-                            const float ds0 = __uint_as_float(s[x][a][2 * e2]) * fmaf(__uint_as_float(dp[x][a][2 * e2]), g.scale, -dls);
-                            const float ds1 = __uint_as_float(s[x][a][2 * e2 + 1]) * fmaf(__uint_as_float(dp[x][a][2 * e2 + 1]), g.scale, -dls);
+                            const uint64_t ds = mul2(pair2(s[x][a][2 * e2], s[x][a][2 * e2 + 1]),
+                                                     fma2(pair2(dp[x][a][2 * e2], dp[x][a][2 * e2 + 1]), scale2, ndls2));
+                            const float ds0 = lo2(ds), ds1 = hi2(ds);
                             wd[e2] = pack2<DT>(ds0, ds1);
                             wr2[e2] = SPLIT ? pack2_residual_bf16(ds0, ds1, wd[e2]) : 0u;
                         }
