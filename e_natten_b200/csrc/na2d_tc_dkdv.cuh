@@ -12,7 +12,7 @@
 // P^T and dS^T are written back over S^T / dP^T as packed 16-bit pairs; on the bf16 path dS^T
 // is written as head + residual (two MMAs), because one bf16 keeps too few bits for dK.
 //
-// Tensor memory holds two chunk stages (S^T, dP^T of NMAX columns each) next to the dV and dK
+// Tensor memory holds two or three chunk stages (S^T, dP^T of NMAX columns each) next to the dV and dK
 // accumulators, so the score MMAs of one chunk run while the softmax warps work on the previous
 // one.  Sixteen warps: 0-7 softmax (warps w and w + 4 own the same 32 keys of a lane quarter and split
 // the 8-column blocks of every chunk between them), 8 producer of the Q / dO chunk ring and of the chunks' lse and
@@ -21,7 +21,7 @@
 // overlaps the next tile.  dK and dV accumulate in tensor memory over all chunks of a tile; no
 // atomics.
 //
-// What bounds it: the chain score MMAs -> softmax warps -> output MMAs -> stage free, of which tensor memory holds two; the
+// What bounds it: the chain score MMAs -> softmax warps -> output MMAs -> stage free, of which tensor memory holds two or three; the
 // softmax part of it was cut by strips, packed fp32 pairs, and lse and delta handed over by the producer.  Measured on one B200
 // against chunks of box rows: 32 x 2 x 56 x 56 x 32, window 7, bf16 104 -> 62 us; 16 x 8 x 28 x 28 x 64, window 13, bf16
 // 135 -> 100 us; 16 x 16 x 14 x 14 x 64, window 13, fp16 39 -> 29 us; 8 heads of 1024 x 1024 x 128, window 13, bf16 7.8 -> 6.6 ms;
@@ -55,6 +55,8 @@ constexpr unsigned long long row_repeat(int hw, int rc) {
 constexpr int dkv_nmax(int d, int ks) { return ks < 7 || d == 128 ? 64 : (512 - 2 * d) / 4 / 16 * 16; }
 // Columns of a chunk from kernel size 7 on: 4 or 2, so that a column pattern repeats every 8 queries.
 constexpr int dkv_strip(int d, int ks) { return (TH + ks - 1) * 4 <= dkv_nmax(d, ks) ? 4 : 2; }
+// Tensor-memory columns of S^T and of dP^T.
+constexpr int dkv_cols(int d, int ks) { return dkv_strip(d, ks) == 4 ? dkv_nmax(d, ks) : 64; }
 
 // (Cfg wants strips that tile the box: it is taken as wide as the next multiple of 8.)
 constexpr int dkv_box_w(int ks) { return (TW + ks - 1 + 7) / 8 * 8; }
@@ -66,8 +68,11 @@ struct DkvCfg : DkvCfgBase<D, KS> {
     using B = DkvCfgBase<D, KS>;
     // names of the base read as "queries per chunk" here: NK = queries in a chunk, NKP padded
     static constexpr bool PATTERN = KS >= 7;                               // masks by pattern (HW divides 8)
-    static constexpr int NMAX = dkv_nmax(D, KS);
+    static constexpr int NMAX = dkv_cols(D, KS);
     static constexpr int TMEM_STAGE = 2 * NMAX;                            // columns per chunk stage
+    // Chunk stages: a third one where it fits (head dims 32 and 64, chunks of up to 64 queries), which takes a chunk's MMAs out of the
+    // softmax warps' way (16 x 8 x 28 x 28 x 64, window 13, bf16: 101 -> 98 us).
+    static constexpr int NSTG = 3 * TMEM_STAGE <= 512 - 2 * D ? 3 : 2;
     static constexpr int TMEM_ST = 0, TMEM_DPT = NMAX, TMEM_DV = 512 - 2 * D, TMEM_DK = TMEM_DV + D;
     static constexpr int TMEM_PT = 0, TMEM_DST = NMAX / 2, TMEM_RES = NMAX;   // 16-bit operands over S^T / dP^T
     static constexpr int STAGE = 2 * B::KV_BYTES;                          // Q chunk then dO chunk
@@ -90,7 +95,7 @@ struct DkvCfg : DkvCfgBase<D, KS> {
     static constexpr uint32_t REP8 = B::HW == 4 ? 0x11u : 0x55u;
     static_assert(SMEM <= kSmemLimit, "dK/dV kernel shared memory");
     static_assert(!PATTERN || B::HW == 2 || B::HW == 4, "strips of 2 or 4 columns");
-    static_assert(B::NKP <= NMAX && 2 * TMEM_STAGE <= TMEM_DV && TMEM_DK + D <= 512 && D % 32 == 0, "tensor memory layout");
+    static_assert(B::NKP <= NMAX && NSTG * TMEM_STAGE <= TMEM_DV && TMEM_DK + D <= 512 && D % 32 == 0, "tensor memory layout");
     static_assert(NMAX % 16 == 0 && NB8 % 2 == 0 && NOWN <= NALL, "blocks in pairs");
 };
 
@@ -117,15 +122,16 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     uint64_t* kv_empty = bars + 1;           //       MMA (commit) -> TMA
     uint64_t* acc_full = bars + 2;           //       MMA (commit) -> epilogue
     uint64_t* acc_free = bars + 3;           //       epilogue -> MMA: dV and dK have been read
-    uint64_t* s_full = bars + 4;             // [2]   MMA (commit) -> softmax group
-    uint64_t* p_full = bars + 6;             // [2]   softmax group -> MMA
-    uint64_t* qd_full = bars + 8;            // [4]   TMA -> MMA
-    uint64_t* qd_empty = bars + 12;          // [4]   MMA (commit) -> TMA
-    uint64_t* st_free = bars + 16;           // [2]   output MMAs (commit) -> score MMAs: the stage is free
-    uint64_t* accv_free = bars + 18;         //       epilogue -> MMA: dV has been read (dK follows)
-    uint64_t* x_full = bars + 19;            // [4]   producer -> score MMAs (and through them softmax): lse and delta
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
-    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 24)};
+    uint64_t* accv_free = bars + 4;          //       epilogue -> MMA: dV has been read (dK follows)
+    uint64_t* s_full = bars + 5;             // [3]   MMA (commit) -> softmax warps, per stage
+    uint64_t* p_full = bars + 8;             // [3]   softmax warps -> MMA
+    uint64_t* st_free = bars + 11;           // [3]   output MMAs (commit) -> score MMAs: the stage is free
+    uint64_t* qd_full = bars + 14;           // [4]   TMA -> MMA
+    uint64_t* qd_empty = bars + 18;          // [4]   MMA (commit) -> TMA
+    uint64_t* x_full = bars + 22;            // [4]   producer -> score MMAs (and through them softmax): lse and delta
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+    const WaitCtx wctx{reinterpret_cast<WaitState*>(bars + 27)};
+    constexpr int NSTG = C::NSTG;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_my = total_tiles > (int)blockIdx.x ? (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -137,7 +143,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         mbar_init(acc_full, 1);
         mbar_init(acc_free, 4);
         mbar_init(accv_free, 4);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < NSTG; ++i) {
             mbar_init(s_full + i, 1);
             mbar_init(p_full + i, 8);
             mbar_init(st_free + i, 1);
@@ -264,8 +270,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     } else if (warp == 9) {
         // ------------------------------------------------------------------ MMA issue: scores
         // Two warps issue MMAs, so that the bookkeeping of one runs under the MMAs of the other:
-        // this one the score MMAs of chunk n into stage n & 1, as soon as the chunk's Q / dO have
-        // landed and the output MMAs of chunk n - 2 (warp 10) have left the stage.  The whole warp
+        // this one the score MMAs of chunk n into stage n % NSTG, as soon as the chunk's Q / dO have
+        // landed and the output MMAs of chunk n - NSTG (warp 10) have left the stage.  The whole warp
         // walks the loop with uniform control flow; one elected lane issues.
         reg_dec<kDkvRegsCtl>();
         constexpr uint32_t idesc_s = umma_idesc(TM, C::NKP, IsBf16<DT>::value, IsBf16<DT>::value, false, false);
@@ -279,14 +285,14 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             for (int ch = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t q_addr = qd_base + (n % NSTQ) * C::STAGE, g_addr = q_addr + C::KV_BYTES;
                 const uint32_t q_lo = smem_desc_lo(q_addr, 16), g_lo = smem_desc_lo(g_addr, 16);
-                const uint32_t tm = tmem_base + (n & 1) * C::TMEM_STAGE;
+                const uint32_t tm = tmem_base + (n % NSTG) * C::TMEM_STAGE;
                 if (lane == 0) NA2D_TR(2, 0, n);
                 if (ch == 0) mbar_wait(kv_full, it & 1, wctx, kErrLoadWait);
                 if (lane == 0) NA2D_TR(2, 1, n);
                 mbar_wait(qd_full + n % NSTQ, (n / NSTQ) & 1, wctx, kErrLoadWait);
                 mbar_wait(x_full + n % NSTQ, (n / NSTQ) & 1, wctx, kErrLoadWait);
                 if (lane == 0) NA2D_TR(2, 3, n);
-                mbar_wait(st_free + (n & 1), ((n >> 1) & 1) ^ 1, wctx, kErrMmaWait);
+                mbar_wait(st_free + n % NSTG, ((n / NSTG) & 1) ^ 1, wctx, kErrMmaWait);
                 if (lane == 0) NA2D_TR(2, 5, n);
                 tc_fence_after();
                 if (elect_one()) {
@@ -300,7 +306,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                         umma_ss(tm + C::TMEM_DPT, desc64(hi, v_lo + ((slab * C::Q_SLAB) >> 4) + 2 * in_slab),
                                 desc64(hi, g_lo + ((slab * C::KV_SLAB) >> 4) + 2 * in_slab), idesc_s, kk > 0);
                     }
-                    umma_commit(s_full + (n & 1));
+                    umma_commit(s_full + n % NSTG);
                     if (ch == t.n_ch - 1) umma_commit(kv_empty);       // K and V are only read by the score MMAs
                     NA2D_TR(2, 2, n);
                 }
@@ -310,7 +316,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         }
     } else if (warp == 10) {
         // ------------------------------------------------------------------ MMA issue: outputs
-        // dV += P^T dO, dK += dS^T Q of chunk n out of stage n & 1, when the chunk's softmax group
+        // dV += P^T dO, dK += dS^T Q of chunk n out of stage n % NSTG, when the chunk's softmax group
         // has written the operands (and, for a tile's first chunk, the epilogue has read the
         // previous tile's accumulators).
         reg_dec<kDkvRegsCtl>();
@@ -324,9 +330,9 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             for (int ch = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t q_addr = qd_base + (n % NSTQ) * C::STAGE, g_addr = q_addr + C::KV_BYTES;
                 const uint32_t qm_lo = smem_desc_lo(q_addr, C::KV_SLAB), gm_lo = smem_desc_lo(g_addr, C::KV_SLAB);
-                const uint32_t tm = tmem_base + (n & 1) * C::TMEM_STAGE;
+                const uint32_t tm = tmem_base + (n % NSTG) * C::TMEM_STAGE;
                 const uint32_t acc = ch == 0 ? 0u : 1u;
-                mbar_wait(p_full + (n & 1), (n >> 1) & 1, wctx, kErrMmaWait);
+                mbar_wait(p_full + n % NSTG, (n / NSTG) & 1, wctx, kErrMmaWait);
                 if (ch == 0) {
                     // A tile's first chunk overwrites the accumulators the epilogue warps are still
                     // reading out for the previous tile.  They read dV first and say so, so its dV
@@ -359,7 +365,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                                     desc64(hi, qm_lo + ((kk * 16 * C::ROWB) >> 4)), idesc_o, 1u);
                     }
                     umma_commit(qd_empty + (n % NSTQ));
-                    umma_commit(st_free + (n & 1));
+                    umma_commit(st_free + n % NSTG);
                     if (ch == t.n_ch - 1) umma_commit(acc_full);
                     NA2D_TR(2, 4, n);
                 }
@@ -510,7 +516,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             row_part(0);
 
             for (int ch = 0, rc = 0, cc = 0; ch < t.n_ch; ++ch, ++n) {
-                const uint32_t stage = n & 1u, k = n >> 1;  // tensor-memory stage and its use counter
+                const uint32_t stage = n % NSTG, k = n / NSTG;  // tensor-memory stage and its use counter
                 const uint32_t t_stage = tmem_lane + stage * C::TMEM_STAGE;
                 const int c_off = cc * C::HW;               // chunk ch = rc * n_cc + cc
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 0, n);
