@@ -275,7 +275,7 @@ int na2d_backward_static_scratch(const void* q, const void* k, const void* v, co
                                  int B, int N, int H, int W, int C, int kernel_size, int dtype,
                                  const na2d_rows* rows, int path, int device, void* stream);
 
-/* Reads and clears the device-side error word that a kernel sets when a bounded wait
+/* Reads and clears the error word that a kernel sets when a bounded wait
  * (mbarrier) ran out.  Synchronises the stream.  Returns NA2D_OK or NA2D_ERR_KERNEL_WAIT.
  * No reference counterpart. */
 int na2d_check(int device, void* stream);
