@@ -151,6 +151,12 @@ struct LoadTracker {
         if (ok) ok = mbar_wait(empty, parity, wc, kErrLoadWait);
         return ok;
     }
+    // The same for a role that a whole warp runs: every lane polls for itself, and one may see the phase complete that another
+    // has just given up on.  They leave together or not at all, or the ones that stay wait for the others at the next __syncwarp.
+    __device__ __forceinline__ bool acquire_warp(uint64_t* empty, uint32_t parity, const WaitCtx& wc) {
+        ok = __all_sync(0xffffffffu, acquire(empty, parity, wc));
+        return ok;
+    }
     __device__ __forceinline__ void arm(uint64_t* full, uint32_t parity, uint32_t bytes) {
         const uint32_t bit = 1u << static_cast<uint32_t>(full - base);
         armed |= bit;

@@ -235,7 +235,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             fetch(t, 0, 0);
             for (int ch = 0, rc = 0, cc = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t st = n % NSTQ;
-                if (!lt.acquire(qd_empty + st, ((n / NSTQ) & 1) ^ 1, wctx)) break;
+                if (!lt.acquire_warp(qd_empty + st, ((n / NSTQ) & 1) ^ 1, wctx)) break;
                 if (lane == 0) {
                     NA2D_TR(2, 7, n);
                     lt.arm(qd_full + st, (n / NSTQ) & 1, 2u * C::NS * C::NK * C::ROWB);
