@@ -82,7 +82,7 @@ int check_device(int device) {
 
 // ---- error state ---------------------------------------------------------------------------------
 // What the waits of a device's kernels report to, and their limit; kernels get its address as an argument.  A wait that
-// gives up writes a code for its kind to a pinned host word: na2d_poll looks there, which costs no CUDA call (a copy of a device
+// gives up marks its kind in a pinned host word, a byte for each: na2d_poll looks there, which costs no CUDA call (a copy of a device
 // word and an event per backward took 8 us of a small call, and a slot between its kernels).  The limit, in microseconds, 0 =
 // the built-in 4 s, comes from the environment variable NA2D_WAIT_LIMIT_US: a profiler pass that instruments every instruction
 // can stretch a healthy hand-over past the built-in limit (seen under `ncu --set full`).
@@ -93,6 +93,16 @@ struct Errors {
     volatile unsigned int* word = nullptr;
 };
 std::atomic<volatile unsigned int*> g_error_words[kMaxDevices];     // null until the device's state is set up
+
+// The kinds in a device's error word, which it clears: bit i for byte i.  Each is seen by one caller, and one that is written
+// meanwhile by the next.
+unsigned int take_errors(volatile unsigned int* word) {
+    if (*word == 0) return 0;
+    const unsigned int bytes = __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL);
+    unsigned int kinds = 0;
+    for (int i = 0; i < 4; ++i) kinds |= ((bytes >> (8 * i)) & 1u) << i;
+    return kinds;
+}
 
 // The error state of `device` (which must be current), set up once per device; that may happen while a stream is being captured,
 // so it stays off the streams of others.
@@ -115,7 +125,7 @@ int error_state(int device, Errors* out) {
             NA2D_CUDA(cudaGetSymbolAddress(&state, g_errors));
             NA2D_CUDA(cudaHostAlloc(&host, sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable));
             *static_cast<unsigned int*>(host) = 0;
-            cudaError_t e = cudaHostGetDevicePointer((void**)&init.word, host, 0);
+            cudaError_t e = cudaHostGetDevicePointer((void**)&init.error_bytes, host, 0);
             if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
             if (e == cudaSuccess) {
                 e = cudaMemcpyAsync(state, &init, sizeof(init), cudaMemcpyHostToDevice, st);
@@ -137,7 +147,8 @@ int error_state(int device, Errors* out) {
     return NA2D_OK;
 }
 
-// The kernel of na2d_selftest_wait_timeout: one thread waits on a barrier nothing completes.
+// The kernel of na2d_selftest_wait_timeout: one thread waits on a barrier nothing completes, once for each kind of wait; the first
+// wait lasts its limit, the others end soon.
 __global__ void wait_timeout_kernel(const na2d_ptx::ErrorState* errors, unsigned long long limit_ns) {
     __shared__ uint64_t bar;
     __shared__ na2d_ptx::WaitState state;
@@ -147,6 +158,8 @@ __global__ void wait_timeout_kernel(const na2d_ptx::ErrorState* errors, unsigned
         na2d_ptx::mbar_init(&bar, 1);
         na2d_ptx::mbar_fence_init();
         const na2d_ptx::WaitCtx wctx{&state};
+        na2d_ptx::mbar_wait(&bar, 0, wctx, na2d_ptx::kErrLoadWait);
+        na2d_ptx::mbar_wait(&bar, 0, wctx, na2d_ptx::kErrMmaWait);
         na2d_ptx::mbar_wait(&bar, 0, wctx, na2d_ptx::kErrOther);
     }
 }
@@ -848,11 +861,10 @@ int na2d_check(int device, void* stream) {
     int rc = error_state(device, &err);
     if (rc != NA2D_OK) return rc;
     NA2D_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    const unsigned int word = *err.word;
-    if (word != 0) {
-        *err.word = 0;
+    const unsigned int kinds = take_errors(err.word);
+    if (kinds != 0) {
         snprintf(t_cuda_err, sizeof(t_cuda_err),
-                 "error word 0x%x (1: load wait, 2: MMA wait, 4: other wait, 8: shared memory base not 1024-byte aligned)", word);
+                 "error kinds 0x%x (1: load wait, 2: MMA wait, 4: other wait, 8: shared memory base not 1024-byte aligned)", kinds);
         return NA2D_ERR_KERNEL_WAIT;
     }
     return NA2D_OK;
@@ -862,9 +874,8 @@ int na2d_poll(int device, void* stream) {
     (void)stream;
     if (device < 0 || device >= kMaxDevices) return NA2D_ERR_BAD_ARG;
     volatile unsigned int* word = g_error_words[device].load(std::memory_order_acquire);
-    if (word == nullptr || *word == 0) return NA2D_OK;         // null: no kernel that waits has run yet
-    *word = 0;
-    return NA2D_ERR_KERNEL_WAIT;
+    if (word == nullptr) return NA2D_OK;         // no kernel that waits has run yet
+    return take_errors(word) == 0 ? NA2D_OK : NA2D_ERR_KERNEL_WAIT;
 }
 
 int na2d_selftest_wait_timeout(int device, void* stream, unsigned int limit_us) {

@@ -1,7 +1,7 @@
 // Thin inline-PTX wrappers for sm_100a: mbarrier, TMA (cp.async.bulk.tensor, no multicast),
 // tcgen05 (TMEM allocation, UMMA issue / commit, TMEM loads) and the descriptor encodings.
 //
-// Every wait is bounded: when the limit runs out the waiter records a code in the device error
+// Every wait is bounded: when the limit runs out the waiter records its kind in the device's error
 // word, raises the CTA-wide abort flag and carries on, so that a kernel can never spin for ever;
 // the host reads the word with na2d_check() or na2d_poll().
 #pragma once
@@ -11,12 +11,18 @@
 
 namespace na2d_ptx {
 
+// Kinds of failure, each the number of its byte in the error word.  After the first wait of a CTA that gives up all its others do
+// too, from other warps and often with another kind: each kind has a byte of its own, so that plain stores keep them all (an atomic
+// operation on host memory would need the bus to support it).
 enum : unsigned int {
-    kErrLoadWait = 1u,      // a TMA load barrier did not complete
-    kErrMmaWait = 2u,       // an MMA commit barrier did not complete
-    kErrOther = 4u,
-    kErrSmemBase = 8u       // the dynamic shared memory did not start on a 1024-byte boundary
+    kErrLoadWait = 0u,      // a TMA load barrier did not complete
+    kErrMmaWait = 1u,       // an MMA commit barrier did not complete
+    kErrOther = 2u,
+    kErrSmemBase = 3u       // the dynamic shared memory did not start on a 1024-byte boundary
 };
+__device__ __forceinline__ void report_error(unsigned char* error_bytes, unsigned int kind) {
+    *static_cast<volatile unsigned char*>(error_bytes + kind) = 1;
+}
 
 // A waiting thread is suspended by the hardware inside mbarrier.try_wait for up to kWaitHintNs
 // (a hint; the hardware may return earlier), so that waiting warps leave the issue slots of their
@@ -40,7 +46,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 struct WaitState {
     uint32_t abort;
     uint32_t limit_us;       // microseconds a wait may last
-    unsigned int* err_word;
+    unsigned char* error_bytes;
 };
 struct WaitCtx {
     WaitState* st;
@@ -54,17 +60,17 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
 __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.volatile.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-// What a kernel gets of the device's error state: the word that a give-up is written to (pinned host memory, so that the host
-// looks at it without a copy), and the limit of a wait in microseconds where one is configured (else 0).
+// What a kernel gets of the device's error state: the bytes of the word that a give-up is written to (pinned host memory, so that the
+// host looks at it without a copy), and the limit of a wait in microseconds where one is configured (else 0).
 struct ErrorState {
-    unsigned int* word;
+    unsigned char* error_bytes;
     unsigned int limit_us, pad;
 };
 __device__ __forceinline__ void wait_state_init(WaitState* st, const ErrorState* errors, unsigned long long limit_ns) {
     st->abort = 0;
     const uint32_t configured = errors->limit_us;
     st->limit_us = configured != 0u ? configured : static_cast<uint32_t>(limit_ns / 1000ull);
-    st->err_word = errors->word;
+    st->error_bytes = errors->error_bytes;
 }
 
 // ------------------------------------------------------------------------------------ mbarrier
@@ -108,7 +114,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-// Bounded wait.  Returns false if the wait gave up (after recording `err_code`).
+// Bounded wait.  Returns false if the wait gave up (after recording its kind).
 //
 // Three stages.  (1) One try_wait, which the hardware may hold for up to kWaitHintNs: most waits
 // end here.  (2) A plain polling loop of kPollRounds rounds.  (3) A wait that is still open after
@@ -120,19 +126,19 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // (a 64-bit start time, say) would be spilled and reloaded around every wait that lasts - which
 // was measured as several per cent of the kernels' time.
 constexpr uint32_t kPollRounds = 1024;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& wc, unsigned int err_code) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& wc, unsigned int kind) {
     if (mbar_try_wait(bar, parity)) return true;              // common case: already complete
 #pragma unroll 1
     for (uint32_t i = 0; i < kPollRounds; ++i)
         if (mbar_try_wait(bar, parity)) return true;
-    const uint32_t st = smem_u32(wc.st);                      // {abort, limit_us, err_word}
+    const uint32_t st = smem_u32(wc.st);                      // {abort, limit_us, error_bytes}
 #pragma unroll 1
     for (uint32_t i = 0; i < ld_shared_u32(st + 4) && ld_shared_u32(st) == 0; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         __nanosleep(1000);
     }
     st_shared_u32(st, 1u);
-    *static_cast<volatile unsigned int*>(wc.st->err_word) = err_code;
+    report_error(wc.st->error_bytes, kind);
     return false;
 }
 

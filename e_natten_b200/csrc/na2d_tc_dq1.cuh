@@ -52,7 +52,7 @@ dq1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw;
     if (smem_u32(smem_raw) & 1023u) {                 // the swizzled operand layouts need it; never seen
-        if (threadIdx.x == 0) *static_cast<volatile unsigned int*>(errors->word) = kErrSmemBase;
+        if (threadIdx.x == 0) report_error(errors->error_bytes, kErrSmemBase);
         return;
     }
     uint8_t* sQ = smem;

@@ -526,14 +526,16 @@ def test_sm_margin_changes_the_grid_not_the_result():
 
 def test_bounded_wait_gives_up_and_is_reported_once():
     """A wait that nothing ever satisfies ends by itself: the self-test kernel waits 2 ms on a
-    barrier nobody completes, records that, and exits normally.  na2d_check reports it once and
-    clears it; the next call is clean and the kernels still compute correctly afterwards."""
+    barrier nobody completes, records that, and exits normally.  na2d_check reports it once, with every
+    kind of wait that gave up, and clears it; the next call is clean and the kernels still compute correctly
+    afterwards."""
     import ctypes as C
     from e_natten_b200 import _lib
     na.check_kernels(DEV)                                       # start clean
     st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
     _lib.check(_lib.lib.na2d_selftest_wait_timeout(0, st, 2000))
     assert _lib.lib.na2d_check(0, st) == _lib.ERR_KERNEL_WAIT
+    assert b"0x7 " in _lib.lib.na2d_last_cuda_error()           # load, MMA and other waits, none lost
     assert _lib.lib.na2d_check(0, st) == 0
     with pytest.raises(ValueError):
         _lib.check(_lib.lib.na2d_selftest_wait_timeout(0, st, 0))
