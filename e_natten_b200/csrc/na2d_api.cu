@@ -874,8 +874,14 @@ int na2d_poll(int device, void* stream) {
     (void)stream;
     if (device < 0 || device >= kMaxDevices) return NA2D_ERR_BAD_ARG;
     volatile unsigned int* word = g_error_words[device].load(std::memory_order_acquire);
-    if (word == nullptr) return NA2D_OK;         // no kernel that waits has run yet
-    return take_errors(word) == 0 ? NA2D_OK : NA2D_ERR_KERNEL_WAIT;
+    if (word != nullptr) return take_errors(word) == 0 ? NA2D_OK : NA2D_ERR_KERNEL_WAIT;
+    // no kernel that waits has run there yet; a device that is none is an error all the same
+    static std::atomic<int> devices{0};
+    if (device < devices.load(std::memory_order_relaxed)) return NA2D_OK;
+    int n = 0;
+    NA2D_CUDA(cudaGetDeviceCount(&n));
+    devices.store(n, std::memory_order_relaxed);
+    return device < n ? NA2D_OK : cuda_fail(cudaErrorInvalidDevice, "na2d_poll");
 }
 
 int na2d_selftest_wait_timeout(int device, void* stream, unsigned int limit_us) {

@@ -280,8 +280,8 @@ int na2d_backward_static_scratch(const void* q, const void* k, const void* v, co
  * No reference counterpart. */
 int na2d_check(int device, void* stream);
 
-/* The same check without waiting for the GPU and without any CUDA call: looks at the host word that a
- * tripped wait writes to.  A caller that polls at every entry learns of a tripped wait once the write has
+/* The same check without waiting for the GPU and, but for the first, without a CUDA call: looks at the host
+ * word that a tripped wait writes to.  A caller that polls at every entry learns of a tripped wait once the write has
  * arrived, one call late, but never stalls; `stream` is not used.  Once reported, the error is cleared.
  * No reference counterpart. */
 int na2d_poll(int device, void* stream);

@@ -73,6 +73,12 @@ def test_forward_refuses_bad_arguments_without_touching_cuda():
     assert _fwd(rows=C.byref(ok)) in (_lib.ERR_CUDA, _lib.ERR_NO_DEVICE)     # past validation: needs a GPU
 
 
+def test_checks_refuse_a_device_that_does_not_exist():
+    for device in (-1, 64):
+        assert _lib.lib.na2d_poll(device, None) == _lib.ERR_BAD_ARG
+    assert _lib.lib.na2d_poll(63, None) == _lib.ERR_CUDA and _lib.lib.na2d_check(63, None) == _lib.ERR_CUDA
+
+
 def _args(**kw):
     a = _lib.Args()
     a.struct_size = C.sizeof(_lib.Args)
