@@ -105,12 +105,17 @@ std::tuple<int, Tensor, Tensor> forward(const Tensor& q_in, const Tensor& k_in, 
     return {status, o, lse};
 }
 
-// Checked operands of whole images -> (status, dQ, dK, dV), None for a half that is not wanted.
+// Operands of whole images, the differentiated ones checked -> (status, dQ, dK, dV), None for a half that is not wanted.
 std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in,
-                                                                const MaybeTensor& o_in, const Tensor& lse,
+                                                                const MaybeTensor& o_in, const Tensor& lse_in,
                                                                 const Tensor& d_o_in, int64_t kernel_size, int path,
                                                                 double scale, bool need_dq, bool need_dkdv) {
-    const Tensor q = in_place_or_copy(q_in), k = in_place_or_copy(k_in), v = in_place_or_copy(v_in);
+    // (saved-tensor hooks may hand back anything for these two as well)
+    TORCH_CHECK_VALUE(!o_in || (o_in->sizes().equals(q_in.sizes()) && o_in->scalar_type() == q_in.scalar_type() && o_in->device() == q_in.device()),
+                      "o must match q in shape, dtype and device");
+    TORCH_CHECK_VALUE(lse_in.sizes().equals(rows_of(q_in)) && lse_in.scalar_type() == at::kFloat && lse_in.device() == q_in.device(),
+                      "lse must hold a float32 for each row of q, on its device");
+    const Tensor lse = lse_in.contiguous(), q = in_place_or_copy(q_in), k = in_place_or_copy(k_in), v = in_place_or_copy(v_in);
     const Tensor d_o = in_place_or_copy(d_o_in);
     MaybeTensor o, d_q, d_k, d_v;
     if (o_in) o = in_place_or_copy(*o_in);
@@ -161,6 +166,16 @@ void check(int status) {
 
 namespace ag = torch::autograd;
 
+// What the operator takes; everything else is for functional.py, to serve or to refuse.
+template <bool ONE_D>
+bool takes(const Tensor& q, const Tensor& k, const Tensor& v, int64_t kernel_size) {
+    const auto dtype = q.scalar_type();
+    return q.is_cuda() && q.dim() == (ONE_D ? 4 : 5) && q.numel() != 0 && k.device() == q.device() && v.device() == q.device() &&
+           k.scalar_type() == dtype && v.scalar_type() == dtype &&
+           (dtype == at::kFloat || dtype == at::kBFloat16 || dtype == at::kHalf) && k.sizes().equals(q.sizes()) &&
+           v.sizes().equals(q.sizes()) && q.size(2) >= kernel_size && (ONE_D || q.size(3) >= kernel_size);
+}
+
 template <bool ONE_D>
 struct Attention : ag::Function<Attention<ONE_D>> {
     static Tensor forward(ag::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, int64_t kernel_size,
@@ -179,14 +194,29 @@ struct Attention : ag::Function<Attention<ONE_D>> {
         // an undefined gradient (a node above returned none) counts as zeros
         const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros(q.sizes(), q.options());
         const bool need_dk = ctx->needs_input_grad(1), need_dv = ctx->needs_input_grad(2);
-        MaybeTensor o;
-        if constexpr (!ONE_D) {
-            // a wait that gave up in an earlier kernel surfaces here, without a sync
-            check(abi.poll(q.device().index(), c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
-            o = saved[3];
+        const int64_t kernel_size = ctx->saved_data["kernel_size"].toInt();
+        const double scale = ctx->saved_data["scale"].toDouble();
+        MaybeTensor o, d_q, d_k, d_v;
+        int status = NA2D_OK;
+        // saved-tensor hooks may hand back other tensors than were saved: what the checks of functional.py say of them
+        if (!takes<ONE_D>(q, k, v, kernel_size) || !d_o.sizes().equals(q.sizes()) || d_o.scalar_type() != q.scalar_type() ||
+            d_o.device() != q.device()) {
+            pybind11::gil_scoped_acquire gil;
+            const auto functional = pybind11::module_::import("e_natten_b200.functional");
+            using namespace pybind11::literals;
+            const auto call = functional.attr(ONE_D ? "natten1d_backward" : "natten2d_backward");
+            std::tie(d_q, d_k, d_v) = call(q, k, v, saved[3], saved[4], d_o, kernel_size, "need_dq"_a = ctx->needs_input_grad(0),
+                                           "need_dkdv"_a = need_dk || need_dv, "scale"_a = scale)
+                                          .template cast<std::tuple<MaybeTensor, MaybeTensor, MaybeTensor>>();
+        } else {
+            if constexpr (!ONE_D) {
+                // a wait that gave up in an earlier kernel surfaces here, without a sync
+                check(abi.poll(q.device().index(), c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
+                o = saved[3];
+            }
+            std::tie(status, d_q, d_k, d_v) = ::backward(q, k, v, o, saved[4], d_o, kernel_size, NA2D_PATH_AUTO, scale,
+                                                         ctx->needs_input_grad(0), need_dk || need_dv);
         }
-        auto [status, d_q, d_k, d_v] = ::backward(q, k, v, o, saved[4], d_o, ctx->saved_data["kernel_size"].toInt(), NA2D_PATH_AUTO,
-                                                  ctx->saved_data["scale"].toDouble(), ctx->needs_input_grad(0), need_dk || need_dv);
         check(status);
         return {d_q.value_or(Tensor()), need_dk ? *d_k : Tensor(), need_dv ? *d_v : Tensor(), Tensor(), Tensor()};
     }
@@ -222,12 +252,7 @@ pybind11::object attention(const pybind11::object& q_in, const pybind11::object&
     if (PyFloat_CheckExact(scale_in.ptr())) scale = PyFloat_AS_DOUBLE(scale_in.ptr());
     else if (!scale_in.is_none()) return pybind11::none();
     const Tensor &q = THPVariable_Unpack(q_in.ptr()), &k = THPVariable_Unpack(k_in.ptr()), &v = THPVariable_Unpack(v_in.ptr());
-    const auto dtype = q.scalar_type();
-    if (looked_into() || !ordinary(q) || !ordinary(k) || !ordinary(v) || q.dim() != (ONE_D ? 4 : 5) || q.numel() == 0 ||
-        k.device() != q.device() || v.device() != q.device() || k.scalar_type() != dtype || v.scalar_type() != dtype ||
-        (dtype != at::kFloat && dtype != at::kBFloat16 && dtype != at::kHalf) || !k.sizes().equals(q.sizes()) ||
-        !v.sizes().equals(q.sizes()) || q.size(2) < kernel_size || (!ONE_D && q.size(3) < kernel_size))
-        return pybind11::none();
+    if (looked_into() || !ordinary(q) || !ordinary(k) || !ordinary(v) || !takes<ONE_D>(q, k, v, kernel_size)) return pybind11::none();
     Tensor o;
     {
         pybind11::gil_scoped_release no_gil;

@@ -46,6 +46,34 @@ def test_saved_tensor_hooks(shape, ks, native, python):
 
 
 @form
+@pytest.mark.parametrize("change,which", [("half", "all"), ("half", "stat"), ("row", "all"), ("row", "stat"), ("cpu", "all"), ("cpu", "stat")])
+def test_saved_tensors_of_another_form_are_refused(shape, ks, native, python, change, which):
+    """Hooks that hand back another type, size or device than was saved: an error in either, and no kernel reads them."""
+    unpack = {"half": lambda t: t.half(), "row": lambda t: t[:1], "cpu": lambda t: t.cpu()}[change]
+    qkv, d_o = inputs(shape)
+    raised = []
+    for f in (native, python):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: unpack(t) if which == "all" or t.dim() < len(shape) else t):
+            o = f(*qkv, ks, None)
+            with pytest.raises(ValueError) as e:
+                torch.autograd.grad(o, qkv, d_o)
+        raised.append(str(e.value).splitlines()[0])
+    assert raised[0] == raised[1] or change == "cpu"      # (there the Python function fails at its poll, one step earlier)
+
+
+@form
+def test_a_batch_of_gradients_is_refused(shape, ks, native, python):
+    qkv, d_o = inputs(shape)
+    raised = []
+    for f in (native, python):
+        o = f(*qkv, ks, None)
+        with pytest.raises(RuntimeError) as e:
+            torch.autograd.grad(o, qkv, torch.stack([d_o, d_o]), is_grads_batched=True)
+        raised.append(type(e.value))
+    assert raised[0] is raised[1]
+
+
+@form
 def test_graph_rules(shape, ks, native, python):
     """A freed graph, an input changed in place and a second derivative are refused; no gradient counts as zeros."""
     for f in (native, python):
