@@ -4,7 +4,9 @@
 // views).  Argument checks with their error texts, and the autograd functions, live in functional.py; an ordinary
 // differentiable call takes the native autograd functions below.
 #include <torch/csrc/utils/pybind.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <ATen/ATen.h>
@@ -222,6 +224,60 @@ struct Attention : ag::Function<Attention<ONE_D>> {
     }
 };
 
+// What the graph node of a call shows in Python: the name and the attributes that the nodes of functional.py have.
+template <bool ONE_D>
+struct AttentionNode {
+    static constexpr const char* kName = ONE_D ? "Natten1dBackward" : "Natten2dBackward";
+    static ag::AutogradContext& context(PyObject* self) {
+        return static_cast<ag::CppNode<Attention<ONE_D>>*>(reinterpret_cast<ag::THPCppFunction*>(self)->cdata.get())->ctx_;
+    }
+    static PyObject* name(PyObject*, PyObject*) { return PyUnicode_FromString(kName); }
+    static PyObject* saved_tensors(PyObject* self, void*) {
+        HANDLE_TH_ERRORS
+        const auto saved = context(self).get_saved_variables();
+        pybind11::tuple tensors(saved.size());
+        for (size_t i = 0; i < saved.size(); ++i) tensors[i] = pybind11::cast(saved[i]);
+        return tensors.release().ptr();
+        END_HANDLE_TH_ERRORS
+    }
+    static PyObject* kernel_size(PyObject* self, void*) {
+        HANDLE_TH_ERRORS
+        return PyLong_FromLongLong(context(self).saved_data["kernel_size"].toInt());
+        END_HANDLE_TH_ERRORS
+    }
+    static PyObject* scale(PyObject* self, void*) {
+        HANDLE_TH_ERRORS
+        return PyFloat_FromDouble(context(self).saved_data["scale"].toDouble());
+        END_HANDLE_TH_ERRORS
+    }
+    static PyObject* set_sequence_nr(PyObject* self, PyObject* number) {
+        HANDLE_TH_ERRORS
+        const auto n = PyLong_AsUnsignedLongLong(number);
+        if (PyErr_Occurred()) return nullptr;
+        reinterpret_cast<ag::THPCppFunction*>(self)->cdata->set_sequence_nr(n);
+        Py_RETURN_NONE;
+        END_HANDLE_TH_ERRORS
+    }
+    static void add() {
+        using namespace torch::autograd;
+        // (those of every node, which PyTorch adds only where a type has none of its own, and the ones above)
+        static PyMethodDef methods[] = {{"_register_hook_dict", THPCppFunction_register_hook_dict, METH_O, nullptr},
+                                        {"register_hook", THPCppFunction_register_hook, METH_O, nullptr},
+                                        {"register_prehook", THPCppFunction_register_prehook, METH_O, nullptr},
+                                        {"_sequence_nr", THPCppFunction_sequence_nr, METH_NOARGS, nullptr},
+                                        {"_set_sequence_nr", set_sequence_nr, METH_O, nullptr},
+                                        {"name", name, METH_NOARGS, nullptr},
+                                        {nullptr}};
+        static PyGetSetDef properties[] = {THP_FUNCTION_DEFAULT_PROPERTIES,
+                                           {"saved_tensors", saved_tensors, nullptr, nullptr, nullptr},
+                                           {"kernel_size", kernel_size, nullptr, nullptr, nullptr},
+                                           {"scale", scale, nullptr, nullptr, nullptr},
+                                           {nullptr}};
+        static PyTypeObject type;
+        ag::registerCppFunction(typeid(ag::CppNode<Attention<ONE_D>>), ag::_initFunctionPyTypeObject(type, kName, properties, methods));
+    }
+};
+
 // Whether anything looks into the call that the functions of functional.py serve and the native ones do not: a functional
 // transform, forward-mode gradients, a trace, a function or dispatch mode.
 bool looked_into() {
@@ -271,6 +327,8 @@ PYBIND11_MODULE(_na2d_torch, m) {
         const na2d_tensor d = describe(t);
         return std::make_tuple(d.stride_b, d.stride_n, d.stride_h, d.stride_w);
     });
+    AttentionNode<false>::add();
+    AttentionNode<true>::add();
     m.def("attention_2d", &attention<false>);
     m.def("attention_1d", &attention<true>);
     m.def("forward", &forward, pybind11::call_guard<pybind11::gil_scoped_release>());

@@ -74,6 +74,22 @@ def test_a_batch_of_gradients_is_refused(shape, ks, native, python):
 
 
 @form
+def test_graph_node(shape, ks, native, python):
+    qkv, d_o = inputs(shape)
+    outputs = [f(*qkv, ks, 0.5) for f in (native, python)]
+    a, b = (o.grad_fn for o in outputs)
+    for node in (a, b):
+        assert node.name() == type(node).__name__ == f"Natten{len(shape) - 3}dBackward"
+        assert node.kernel_size == ks and node.scale == 0.5 and len(node.next_functions) == 3
+    assert len(a.saved_tensors) == len(b.saved_tensors) == 5
+    assert all(torch.equal(x, y) for x, y in zip(a.saved_tensors, b.saved_tensors))
+    o = native(*qkv, ks, None)
+    torch.autograd.grad(o, qkv, d_o)
+    with pytest.raises(RuntimeError, match="freed"):
+        o.grad_fn.saved_tensors
+
+
+@form
 def test_graph_rules(shape, ks, native, python):
     """A freed graph, an input changed in place and a second derivative are refused; no gradient counts as zeros."""
     for f in (native, python):
