@@ -211,19 +211,21 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         // (the K, V tile has a producer of its own, warp 11: a chunk of the next tile can be
         // fetched as soon as a ring slot is free, long before the K, V buffers are)
         // The chunk's lse and delta go with it, as the softmax warps use them: lane l has queries l, l + 32, ...; they are read
-        // one chunk ahead, so that their latency runs under the wait for a ring slot.
+        // one chunk ahead, so that their latency runs under the wait for a ring slot, and first touched when the chunk's loads are on
+        // their way, which a tile's first chunk would wait for otherwise (a call of few tiles, 4 x 4 x 32 x 32 x 128, window 5, bf16:
+        // 12.4 -> 11.8 us).
         reg_dec<kDkvRegsCtl>();
         constexpr int kPer = (C::NKP + 31) / 32;
-        float pre_l2[kPer], pre_dl[kPer];
+        float pre_lse[kPer], pre_delta[kPer];
         auto fetch = [&](const TileGeo& t, int rc, int cc) {
 #pragma unroll
             for (int u = 0; u < kPer; ++u) {
                 const int j = lane + 32 * u, br = rc * C::RC + j / C::HW, qc = t.qb_c0 + cc * C::HW + j % C::HW;
-                pre_l2[u] = pre_dl[u] = 0.f;                     // zero outside the band
+                pre_lse[u] = pre_delta[u] = 0.f;                 // zero outside the band
                 if (j < C::NK && br < t.n_rows && qc < g.W) {
                     const size_t qi = (static_cast<size_t>(t.bn) * g.Hq + (t.q_local_r0 + br)) * g.W + qc;
-                    pre_l2[u] = -(lse[qi] * kLog2e);
-                    pre_dl[u] = -(delta[qi] * g.scale);          // dS^T carries the softmax scale of dK: scale p (dP - delta)
+                    pre_lse[u] = lse[qi];
+                    pre_delta[u] = delta[qi];
                 }
             }
         };
@@ -253,8 +255,8 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                 for (int u = 0; u < kPer; ++u) {
                     const int j = lane + 32 * u;
                     if (j < C::NKP) {
-                        x[j] = pre_l2[u];
-                        x[C::NKP + j] = pre_dl[u];
+                        x[j] = -(pre_lse[u] * kLog2e);
+                        x[C::NKP + j] = -(pre_delta[u] * g.scale);      // dS^T carries the softmax scale of dK: scale p (dP - delta)
                     }
                 }
                 __syncwarp();
