@@ -1,4 +1,5 @@
-// Persistent, warp-specialised tcgen05 forward kernel for the larger windows (kernel sizes >= 7).
+// Persistent, warp-specialised tcgen05 forward kernel for the larger windows (kernel sizes >= 7): calls of up to one tile per
+// SM, and all calls at head dim 128 with windows 7 and 9 (two_tiles_pay below; the others go to na2d_tc_fwd2.cuh).
 // Included by na2d_tc_fwd.cu.
 //
 // One CTA per SM walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...  A tile is TH x TW queries;
@@ -10,8 +11,9 @@
 //              shared memory, and write P back into tensor memory over S as packed 16-bit
 //              pairs, where it is the A operand of the second MMA.  The output accumulates in
 //              tensor memory across the chunks of a tile and is rescaled there only when a row's
-//              maximum grows by more than 2^8 (until then the older maximum keeps being used,
-//              which leaves the result unchanged).  The tile's epilogue (normalise, store o and
+//              maximum grows by more than 2^8 (until then the older maximum keeps being used:
+//              the same quotient, but the largest weight so far, no longer an exact 1, is rounded
+//              to 16 bits like the others).  The tile's epilogue (normalise, store o and
 //              lse) is deferred into the next tile, whose MMAs and loads it overlaps.
 //   warp 8     producer: TMA loads of Q tiles (two buffers), K chunks and V chunks (separate
 //              rings: a K slot is free again as soon as S = Q K^T has been computed);
@@ -464,6 +466,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
 }
 
+// Whether calls of more tiles than SMs take the kernel with two tiles in flight (na2d_tc_fwd2.cuh).  One B200, bf16, images of
+// 48 x 32 (28 x 28 and 14 x 14 alike), this kernel against that one in us, at 1.05, 2, 3, 9 and 60 tiles per SM:
+//   head dim 32, window 7    11.1 8.8   11.4 9.4   15.0 12.2   36 24   223 129      window 13  18.2 12.5  18.4 12.9  25.0 19.0  65 41  408 238
+//   head dim 64, window 7    11.8 9.7   11.9 10.4  15.5 13.5   38 28   230 156      window 11  16.7 13.5  16.8 14.1  22.8 21.0  58 46  361 266
+//   head dim 128, window 7   13.2 13.3  13.5 13.9  17.5 19.4   43 50   252 275      window 9   13.6 13.2  13.9 13.8  18.1 19.4  44 50  276 282
+//   head dim 128, window 11  18.6 16.1  18.9 16.9  25.6 25.1   66 64   431 373      window 13  20.6 16.2  20.8 16.9  28.3 25.1  76 63  517 389
+// At head dim 128 the MMAs are what a tile of a small window lasts, and that kernel's narrower chunks make more of them.
+// Up to one tile per SM a tile has its SM to itself, and all eight softmax warps on it end it sooner at head dim 128 and from
+// window 11 on (0.97 tiles per SM, window 7 / 11: head dim 32 8.4 / 10.7 against 8.2 / 11.4, 64 8.7 / 11.1 against 8.8 / 12.4, 128 10.0 /
+// 12.9 against 11.8 / 14.9).
+constexpr bool two_tiles_pay(int d, int ks) { return d < 128 || ks > 9; }
+
 template <typename DT, int D, int KS>
 int launch_forward(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const TensorArg& o,
                    float* lse) {
@@ -476,10 +490,10 @@ int launch_forward(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, 
     const int tiles_r = (g.Hq + TH - 1) / TH, tiles_c = (g.W + TW - 1) / TW;
     const long long tiles = (long long)g.BN * tiles_r * tiles_c;
     if (tiles > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
-    // From one tile per SM on, two tiles in flight.  Up to there a tile has its SM to itself, and all eight softmax warps on
-    // it end it no later and often sooner (128 tiles, window 7 / 13: head dim 64 10.3 / 12.3 against 10.3 / 14.3 us, 128 10.3 / 14.4
-    // against 12.3 / 15.3); at 256 tiles it is 14.3 / 20.5 against 12.3 / 15.3 and 14.7 / 22.4 against 16.3 / 18.5 us.
-    if (tiles > sm_count(lc.device)) return launch_forward2<DT, D, KS>(lc, q, k, v, o, lse, tiles, tiles_r, tiles_c);
+    if constexpr (two_tiles_pay(D, KS)) {
+        // (by the device's SMs, whatever margin the call leaves: a margin changes no bit of the result)
+        if (tiles > sm_count(lc.device)) return launch_forward2<DT, D, KS>(lc, q, k, v, o, lse, tiles, tiles_r, tiles_c);
+    }
     CUtensorMap tq, tk, tv, to;
     int rc = make_map(&tq, q, lc.dtype, lc.B, g.N, g.Hq, g.W, D, TW, TH);
     if (rc == NA2D_OK) rc = make_map(&to, o, lc.dtype, lc.B, g.N, g.Hq, g.W, D, TW, 32 / TW, OutStage<D / 2>::RW);

@@ -1,5 +1,5 @@
 // Persistent, warp-specialised tcgen05 forward kernel for the larger windows (kernel sizes >= 7), two query tiles in
-// flight.  Included by na2d_tc_fwd.cu.
+// flight, for calls of more tiles than SMs (at head dim 128 from window 11 on; na2d_tc_fwd.cuh).  Included by na2d_tc_fwd.cu.
 //
 // A CTA's tiles alternate between two softmax groups of four warps (warps 0-3 the even ones, 4-7 the odd ones).  Each
 // group has an S / P buffer and an output accumulator of its own in tensor memory, and the tensor pipe takes turns:
