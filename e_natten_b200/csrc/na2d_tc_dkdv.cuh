@@ -3,9 +3,10 @@
 // One CTA per SM walks key tiles (TH x TW keys, row r of every MMA = key r = tensor-memory lane
 // r).  The queries that can see a tile form a box (the union of the keys' inverse
 // neighbourhoods, clipped to the local query band), walked in chunks of RC rows x HW columns
-// (at most NMAX queries).  From kernel size 7 on a chunk is a column strip as tall as the box of an inner tile: a
-// warp's 32 keys (four image rows) are seen from ks + 3 of its rows, the same share of every chunk, while of
-// a group of rows some warps see everything and others nothing, and a chunk lasts as long as its busiest warp.
+// (at most NMAX queries).  Two forms.  STRIPS (from kernel size 7 on, where strips_pay says so): a chunk is a column strip as
+// tall as the box of an inner tile.  A warp's 32 keys (four image rows) are seen from ks + 3 of its rows, the same share of every
+// chunk, while of a group of rows some warps see everything and others nothing, and a chunk lasts as long as its busiest warp.
+// Otherwise (kernel sizes 3 and 5, and images on which strips would mostly hang over the box): groups of box rows.
 //     S^T = K Q_c^T,  dP^T = V dO_c^T                      (tensor memory, fp32)
 //     P^T = exp(S^T - lse),  dS^T = scale P^T (dP^T - delta)   (softmax warps, registers; the scale is dK's)
 //     dV += P^T dO_c,  dK += dS^T Q_c                      (P^T, dS^T read from tensor memory)
@@ -28,6 +29,8 @@
 // 4 x 4 x 256 x 256 x 128, window 5, bf16 (the same chunks as before) 0.39 -> 0.375 ms.
 #pragma once
 
+#include <algorithm>
+
 namespace na2d_tc {
 
 // Chunks of an interior tile's query box when the box is cut into `split` column strips.
@@ -40,7 +43,6 @@ constexpr int dkv_chunks(int ks, int split) {
 // Fewest chunks wins; on a tie the narrower strips, which spread the work evenly over the lane
 // quarters (a key row group sees the same number of queries in every strip).
 constexpr int dkv_w_split(int ks) {
-    if (ks >= 7) return (TW + ks - 1) / 2;
     const int c1 = dkv_chunks(ks, 1), c2 = dkv_chunks(ks, 2), c4 = dkv_chunks(ks, 4);
     return (c4 <= c2 && c4 <= c1) ? 4 : (c2 <= c1 ? 2 : 1);
 }
@@ -51,24 +53,24 @@ constexpr unsigned long long row_repeat(int hw, int rc) {
     return m;
 }
 
-// Queries per chunk at most: 2 x (S^T + dP^T) + dV + dK in 512 columns.  (Kernel sizes 3 and 5 keep chunks of 64.)
-constexpr int dkv_nmax(int d, int ks) { return ks < 7 || d == 128 ? 64 : (512 - 2 * d) / 4 / 16 * 16; }
-// Columns of a chunk from kernel size 7 on: 4 or 2, so that a column pattern repeats every 8 queries.
-constexpr int dkv_strip(int d, int ks) { return (TH + ks - 1) * 4 <= dkv_nmax(d, ks) ? 4 : 2; }
+// Queries per chunk at most: 2 x (S^T + dP^T) + dV + dK in 512 columns.  (Groups of rows are kept to 64.)
+constexpr int dkv_nmax(int d, bool strips) { return !strips || d == 128 ? 64 : (512 - 2 * d) / 4 / 16 * 16; }
+// Columns of a strip: 4 or 2, so that a column pattern repeats every 8 queries.
+constexpr int dkv_strip(int d, int ks) { return (TH + ks - 1) * 4 <= dkv_nmax(d, true) ? 4 : 2; }
 // Tensor-memory columns of S^T and of dP^T.
-constexpr int dkv_cols(int d, int ks) { return dkv_strip(d, ks) == 4 ? dkv_nmax(d, ks) : 64; }
+constexpr int dkv_cols(int d, int ks, bool strips) { return strips && dkv_strip(d, ks) == 4 ? dkv_nmax(d, strips) : 64; }
 
 // (Cfg wants strips that tile the box: it is taken as wide as the next multiple of 8.)
 constexpr int dkv_box_w(int ks) { return (TW + ks - 1 + 7) / 8 * 8; }
-template <int D, int KS>
-using DkvCfgBase = Cfg<D, KS, dkv_nmax(D, KS), KS < 7 ? 0 : dkv_box_w(KS) - (TW + KS - 1), KS < 7 ? dkv_w_split(KS) : dkv_box_w(KS) / dkv_strip(D, KS)>;
+template <int D, int KS, bool STRIPS>
+using DkvCfgBase = Cfg<D, KS, dkv_nmax(D, STRIPS), STRIPS ? dkv_box_w(KS) - (TW + KS - 1) : 0, STRIPS ? dkv_box_w(KS) / dkv_strip(D, KS) : dkv_w_split(KS)>;
 
-template <int D, int KS>
-struct DkvCfg : DkvCfgBase<D, KS> {
-    using B = DkvCfgBase<D, KS>;
+template <int D, int KS, bool STRIPS>
+struct DkvCfg : DkvCfgBase<D, KS, STRIPS> {
+    using B = DkvCfgBase<D, KS, STRIPS>;
     // names of the base read as "queries per chunk" here: NK = queries in a chunk, NKP padded
-    static constexpr bool PATTERN = KS >= 7;                               // masks by pattern (HW divides 8)
-    static constexpr int NMAX = dkv_cols(D, KS);
+    static constexpr bool PATTERN = STRIPS;                                // masks by pattern (HW divides 8)
+    static constexpr int NMAX = dkv_cols(D, KS, STRIPS);
     static constexpr int TMEM_STAGE = 2 * NMAX;                            // columns per chunk stage
     // Chunk stages: a third one where it fits (head dims 32 and 64, chunks of up to 64 queries), which takes a chunk's MMAs out of the
     // softmax warps' way (16 x 8 x 28 x 28 x 64, window 13, bf16: 101 -> 98 us).
@@ -99,7 +101,7 @@ struct DkvCfg : DkvCfgBase<D, KS> {
     static_assert(NMAX % 16 == 0 && NB8 % 2 == 0 && NOWN <= NALL, "blocks in pairs");
 };
 
-template <typename DT, int D, int KS>
+template <typename DT, int D, int KS, bool STRIPS>
 __global__ void __launch_bounds__(512, 1)
 dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
             const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -108,7 +110,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             const ErrorState* __restrict__ errors, const Na2dGeom g, const int tiles_r, const int tiles_c,
             const int total_tiles) {
     constexpr bool SPLIT = IsBf16<DT>::value;
-    using C = DkvCfg<D, KS>;
+    using C = DkvCfg<D, KS, STRIPS>;
     constexpr int NSTQ = C::NSTQ;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -627,10 +629,10 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     }
 }
 
-template <typename DT, int D, int KS>
-int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
-                const TensorArg& d_o, const float* delta, const TensorArg& d_k, const TensorArg& d_v) {
-    using C = DkvCfg<D, KS>;
+template <typename DT, int D, int KS, bool STRIPS>
+int launch_dkdv_as(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
+                   const TensorArg& d_o, const float* delta, const TensorArg& d_k, const TensorArg& d_v) {
+    using C = DkvCfg<D, KS, STRIPS>;
     const Na2dGeom& g = lc.g;
     CUtensorMap tk, tv, tq, tg, tdk, tdv;
     int rc = make_map(&tk, k, lc.dtype, lc.B, g.N, g.Hkv, g.W, D, TW, TH);
@@ -644,7 +646,7 @@ int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, con
     const int tiles_r = (g.Hkv + TH - 1) / TH, tiles_c = (g.W + TW - 1) / TW;
     const long long tiles = (long long)g.BN * tiles_r * tiles_c;
     if (tiles > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
-    auto kern = dkdv_kernel<DT, D, KS>;
+    auto kern = dkdv_kernel<DT, D, KS, STRIPS>;
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
@@ -652,6 +654,47 @@ int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, con
                                         tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
     return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
+}
+
+// What the chunks of one unit cost in one of the forms: each `per_chunk`, and `per_block` for an 8-query block of its busiest warp.
+template <class C>
+long long dkv_cost(const Na2dGeom& g, int per_chunk, int per_block) {
+    long long rows = 0, strips = 0;
+    for (int r0 = 0; r0 < g.Hkv; r0 += TH) {
+        const int first = g.kv_row0 + r0, last = g.kv_row0 + std::min(r0 + TH, g.Hkv) - 1;
+        const int top = std::max(na2d_bws(first, g.ks), g.q_row0), end = std::min(na2d_bwe(last, g.Hg, g.ks), g.q_row0 + g.Hq);
+        for (int at = top; at < end; at += C::RC) {
+            int busiest = C::PATTERN ? (C::kInner * C::HW + 7) / 8 : 0;
+            for (int key = first; key <= last; key += 32 / TW) {
+                const int lo = std::max(na2d_bws(key, g.ks) - at, 0);
+                const int hi = std::min(na2d_bwe(std::min(key + 32 / TW - 1, last), g.Hg, g.ks) - at, C::RC);
+                if (hi > lo) busiest = std::max(busiest, (hi * C::HW + 7) / 8 - lo * C::HW / 8);
+            }
+            rows += per_chunk + per_block * busiest;
+        }
+    }
+    for (int c0 = 0; c0 < g.W; c0 += TW)
+        strips += (na2d_bwe(std::min(c0 + TW, g.W) - 1, g.W, g.ks) - na2d_bws(c0, g.ks) + C::HW - 1) / C::HW;
+    return rows * strips;
+}
+
+// Whether column strips are the faster form.  On a border tile, whose box is smaller, a strip is still a whole inner box tall, and on
+// images of less than two or three windows most tiles are border tiles: 4 x 8 x 18 x 64 x 128, window 11, bf16 33 % slower than with
+// the groups of rows that strips replaced.  The weights are fitted to 216 points (head dims 32, 64, 128, windows 7 to 13, images of
+// 14 x 14 to 128 x 128, one B200): the form chosen takes 1.007 times the better one's time on average, 1.17 times at worst
+// (2 x 8 x 100 x 14 x 128, window 7).
+template <int D, int KS>
+bool strips_pay(const Na2dGeom& g) {
+    return dkv_cost<DkvCfg<D, KS, true>>(g, 3, 6) <= dkv_cost<DkvCfg<D, KS, false>>(g, 12, 4);
+}
+
+template <typename DT, int D, int KS>
+int launch_dkdv(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, const TensorArg& v, const float* lse,
+                const TensorArg& d_o, const float* delta, const TensorArg& d_k, const TensorArg& d_v) {
+    if constexpr (KS >= 7) {
+        if (strips_pay<D, KS>(lc.g)) return launch_dkdv_as<DT, D, KS, true>(lc, q, k, v, lse, d_o, delta, d_k, d_v);
+    }
+    return launch_dkdv_as<DT, D, KS, false>(lc, q, k, v, lse, d_o, delta, d_k, d_v);
 }
 
 }  // namespace na2d_tc

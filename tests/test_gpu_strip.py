@@ -44,6 +44,20 @@ def test_inner_and_border_tiles(ks, D, units):
         assert_close(g, w, torch.bfloat16, f"{name} {shape} ks={ks}")
 
 
+# The key half's two forms of chunks, at images on either side of where they change places (in either direction), and images whose
+# last key tile is seen from more rows than a strip is tall.
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("ks,H,W", [(7, 18, 40), (7, 22, 40), (7, 100, 14), (7, 70, 40), (9, 14, 50), (9, 30, 32), (9, 72, 40), (11, 22, 40),
+                                    (11, 40, 40), (11, 74, 40), (13, 20, 21), (13, 30, 32), (13, 76, 40)])
+def test_both_forms_of_query_chunks(ks, H, W, D):
+    shape = (1, 2, H, W, D)
+    q, k, v, d_o = make_inputs(shape, torch.bfloat16, ks, q_scale=D ** -0.5)
+    got = step(q, k, v, d_o, ks)
+    want = orc.natten2d_fwd_bwd(q, k, v, d_o, ks)
+    for name, g, w in zip(("o", "lse", "dq", "dk", "dv"), got, want):
+        assert_close(g, w, torch.bfloat16, f"{name} {shape} ks={ks}")
+
+
 @pytest.mark.parametrize("bad", [float("inf"), -float("inf"), float("nan")])
 @pytest.mark.parametrize("ks,D,at", [(7, 32, (8, 9)), (13, 128, (0, 15)), (9, 64, (16, 7))])
 def test_a_key_reaches_only_the_windows_that_hold_it(ks, D, at, bad):
