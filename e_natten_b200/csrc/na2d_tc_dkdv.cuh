@@ -97,6 +97,7 @@ struct DkvCfg : DkvCfgBase<D, KS, STRIPS> {
     static constexpr uint32_t REP8 = B::HW == 4 ? 0x11u : 0x55u;
     static_assert(SMEM <= kSmemLimit, "dK/dV kernel shared memory");
     static_assert(!PATTERN || B::HW == 2 || B::HW == 4, "strips of 2 or 4 columns");
+    static_assert(!PATTERN || B::HW <= KS / 2 + 1, "no box is narrower than a strip");
     static_assert(B::NKP <= NMAX && NSTG * TMEM_STAGE <= TMEM_DV && TMEM_DK + D <= 512 && D % 32 == 0, "tensor memory layout");
     static_assert(NMAX % 16 == 0 && NB8 % 2 == 0 && NOWN <= NALL, "blocks in pairs");
 };
@@ -186,7 +187,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
     const uint32_t tmem_base = *tmem_slot;
 
     // Geometry of my i-th tile: key tile origin and the query box it is seen from.
-    struct TileGeo { int bn, hn, hb, kr0, kc0, qb_r0, q_local_r0, n_rows, qb_c0, n_cc, n_ch; };
+    struct TileGeo { int bn, hn, hb, kr0, kc0, qb_r0, q_local_r0, n_rows, qb_c0, n_cols, n_cc, n_ch; };
     // (each role steps through the tiles by itself)
     TileWalk walk((int)blockIdx.x, (int)gridDim.x, tiles_r, tiles_c);
     auto tile_geo = [&](const TileWalk& at) {
@@ -202,11 +203,16 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         t.n_rows = max(qb_r1 - t.qb_r0, 0);
         t.q_local_r0 = t.qb_r0 - g.q_row0;
         t.qb_c0 = na2d_bws(t.kc0, KS);
-        const int n_cols = na2d_bwe(min(t.kc0 + TW, g.W) - 1, g.W, KS) - t.qb_c0;
-        t.n_cc = (n_cols + C::HW - 1) / C::HW;           // strips; more where both borders stretch the box
+        t.n_cols = na2d_bwe(min(t.kc0 + TW, g.W) - 1, g.W, KS) - t.qb_c0;
+        t.n_cc = (t.n_cols + C::HW - 1) / C::HW;         // strips; more where both borders stretch the box
         t.n_ch = ((t.n_rows + C::RC - 1) / C::RC) * t.n_cc;       // (divisions by constants)
         return t;
     };
+
+    // First box column of strip cc.  The last one starts earlier where it would reach past the box, and takes no part of the columns
+    // it shares with the one before: weights of zero meet no query outside the box, whose dO or q need not be finite.  (A box
+    // is at least ks / 2 + 1 columns wide.)
+    auto first_col = [](const TileGeo& t, int cc) { return C::PATTERN ? min(cc * C::HW, t.n_cols - C::HW) : cc * C::HW; };
 
     if (warp == 8) {
         // ------------------------------------------------------------------ producer of the Q / dO chunk ring
@@ -222,7 +228,7 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         auto fetch = [&](const TileGeo& t, int rc, int cc) {
 #pragma unroll
             for (int u = 0; u < kPer; ++u) {
-                const int j = lane + 32 * u, br = rc * C::RC + j / C::HW, qc = t.qb_c0 + cc * C::HW + j % C::HW;
+                const int j = lane + 32 * u, br = rc * C::RC + j / C::HW, qc = t.qb_c0 + first_col(t, cc) + j % C::HW;
                 pre_lse[u] = pre_delta[u] = 0.f;                 // zero outside the band
                 if (j < C::NK && br < t.n_rows && qc < g.W) {
                     const size_t qi = (static_cast<size_t>(t.bn) * g.Hq + (t.q_local_r0 + br)) * g.W + qc;
@@ -244,12 +250,12 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
                     NA2D_TR(2, 7, n);
                     lt.arm(qd_full + st, (n / NSTQ) & 1, 2u * C::NS * C::NK * C::ROWB);
                     uint8_t* dst = sQD + st * C::STAGE;
+                    const int col = t.qb_c0 + first_col(t, cc);
 #pragma unroll
                     for (int s = 0; s < C::NS; ++s) {
-                        tma_load_5d(dst + s * C::KV_SLAB, &tm_q, qd_full + st, s * 64, t.qb_c0 + cc * C::HW,
+                        tma_load_5d(dst + s * C::KV_SLAB, &tm_q, qd_full + st, s * 64, col, t.q_local_r0 + rc * C::RC, t.hn, t.hb);
+                        tma_load_5d(dst + C::KV_BYTES + s * C::KV_SLAB, &tm_do, qd_full + st, s * 64, col,
                                     t.q_local_r0 + rc * C::RC, t.hn, t.hb);
-                        tma_load_5d(dst + C::KV_BYTES + s * C::KV_SLAB, &tm_do, qd_full + st, s * 64,
-                                    t.qb_c0 + cc * C::HW, t.q_local_r0 + rc * C::RC, t.hn, t.hb);
                     }
                 }
                 float* x = s_x + st * 2 * C::NKP;
@@ -522,12 +528,12 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
             for (int ch = 0, rc = 0, cc = 0; ch < t.n_ch; ++ch, ++n) {
                 const uint32_t stage = n % NSTG, k = n / NSTG;  // tensor-memory stage and its use counter
                 const uint32_t t_stage = tmem_lane + stage * C::TMEM_STAGE;
-                const int c_off = cc * C::HW;               // chunk ch = rc * n_cc + cc
+                const int c_off = first_col(t, cc);         // chunk ch = rc * n_cc + cc
                 if (quarter == 0 && lane == 0) NA2D_TR(3 - 2 * group, 0, n);
                 const float* x_lse = s_x + (n % NSTQ) * 2 * C::NKP;
                 const float* x_delta = x_lse + C::NKP;
                 // this thread's column segment inside a chunk row; the chunk's queries that see its key
-                const int cl = max(col_lo - c_off, 0), seg_len = min(col_hi - c_off, C::HW) - cl;
+                const int cl = C::PATTERN ? max(col_lo, cc * C::HW) - c_off : max(col_lo - c_off, 0), seg_len = min(col_hi - c_off, C::HW) - cl;
                 const uint32_t seg = seg_len > 0 ? ((1u << seg_len) - 1u) : 0u;
                 uint32_t cols8 = 0;
                 unsigned long long m64 = 0;

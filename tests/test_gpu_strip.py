@@ -72,3 +72,25 @@ def test_a_key_reaches_only_the_windows_that_hold_it(ks, D, at, bad):
     assert torch.equal(o[:, :, ~held], clean[:, :, ~held]) and torch.equal(lse[:, :, ~held], clean_lse[:, :, ~held])
     if bad != bad:
         assert o[:, :, held].isnan().all()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("ks,D", [(7, 32), (9, 64), (13, 64), (13, 128)])
+def test_a_gradient_reaches_only_the_key_tiles_whose_box_holds_it(ks, D, bad):
+    """Key half on strips, key tiles of 8 columns: a column of d_o beside a tile's box of queries meets none of its keys."""
+    q, k, v, d_o = (t.to(DEV) for t in make_inputs((1, 2, 64, 64, D), torch.bfloat16, 3, q_scale=D ** -0.5))
+    o, lse = na.natten2d_forward(q, k, v, ks)
+    delta, out = torch.empty_like(lse), [torch.empty_like(k) for _ in range(5)]
+    na.functional.backward_dq_into(q, k, v, o, lse, d_o, out[0], delta, ks)
+    na.functional.backward_dkdv_into(q, k, v, lse, d_o, delta, out[1], out[2], ks)
+    for tile in range(8):
+        last = 8 * tile + 7
+        for beside in (8 * tile - ks // 2 - 1 if 8 * tile >= ks else -1, last + ks // 2 + 1 if last < 64 - ks else -1):
+            if beside < 0:
+                continue
+            g = d_o.clone()
+            g[:, :, :, beside] = bad
+            na.functional.backward_dkdv_into(q, k, v, lse, g, delta, out[3], out[4], ks)
+            for a, b in ((out[1], out[3]), (out[2], out[4])):
+                assert torch.equal(a[:, :, :, 8 * tile:last + 1], b[:, :, :, 8 * tile:last + 1]), (tile, beside)
+    na.check_kernels(DEV)
