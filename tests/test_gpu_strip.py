@@ -74,6 +74,39 @@ def test_a_key_reaches_only_the_windows_that_hold_it(ks, D, at, bad):
         assert o[:, :, held].isnan().all()
 
 
+@pytest.mark.parametrize("bad", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("ks,D,at", [(7, 32, (8, 9)), (9, 64, (16, 20)), (13, 64, (20, 15)), (13, 128, (31, 0))])
+def test_a_pixel_reaches_only_the_gradients_of_its_windows(ks, D, at, bad):
+    """Backward on strips: a value of one pixel meets the queries whose window holds it, a query or its gradient the keys of its
+    window, whatever it is.  (The operand that the other gradients multiply with stays finite here: their weights are zero.)"""
+    H = W = 48
+    q, k, v, d_o = (t.to(DEV) for t in make_inputs((1, 2, H, W, D), torch.bfloat16, 3, q_scale=D ** -0.5))
+    o, lse = na.natten2d_forward(q, k, v, ks)
+    ws = [orc.window_start(i, H, ks) for i in range(H)]
+    holds = torch.tensor([[a <= at[0] < a + ks and b <= at[1] < b + ks for b in ws] for a in ws], device=DEV)       # queries
+    held = torch.zeros(H, W, dtype=torch.bool, device=DEV)                                                          # keys
+    held[ws[at[0]]:ws[at[0]] + ks, ws[at[1]]:ws[at[1]] + ks] = True
+
+    def backward(q, v, d_o, delta=None):
+        d_q, d_k, d_v, dl = torch.empty_like(q), torch.empty_like(k), torch.empty_like(k), torch.empty_like(lse)
+        na.functional.backward_dq_into(q, k, v, o, lse, d_o, d_q, dl, ks)
+        na.functional.backward_dkdv_into(q, k, v, lse, d_o, dl if delta is None else delta, d_k, d_v, ks)
+        na.check_kernels(DEV)
+        return d_q, d_k, d_v, dl
+
+    def changed(t):
+        t = t.clone()
+        t[:, :, at[0], at[1], D // 2] = bad
+        return t
+    d_q, d_k, d_v, delta = backward(q, v, d_o)
+    got = backward(q, changed(v), d_o, delta)
+    assert torch.equal(got[0][:, :, ~holds], d_q[:, :, ~holds]) and torch.equal(got[3][:, :, ~holds], delta[:, :, ~holds])
+    got = backward(changed(q), v, d_o, delta)
+    assert torch.equal(got[2][:, :, ~held], d_v[:, :, ~held])
+    got = backward(q, v, changed(d_o), delta)
+    assert torch.equal(got[1][:, :, ~held], d_k[:, :, ~held])
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("ks,D", [(7, 32), (9, 64), (13, 64), (13, 128)])
 def test_a_gradient_reaches_only_the_key_tiles_whose_box_holds_it(ks, D, bad):
