@@ -4,8 +4,8 @@
 // Tiling.  A tile is TH x TW = 16 x 8 = 128 query pixels; query r of the tile is row r of every MMA and lane
 // r of tensor memory.  The keys a tile can see are the union of its pixels' clamped
 // windows: a (TH+ks-1) x (TW+ks-1) "halo box" whose origin is the window origin of the tile's
-// first pixel.  The box is cut into chunks of whole box rows with at most 256 keys each (the
-// UMMA N limit); TMA brings each chunk of K and V into shared memory as [key][channel] rows with
+// first pixel.  The box is cut into chunks of at most 256 keys each (the UMMA N limit), column strips
+// or groups of whole box rows; TMA brings each chunk of K and V into shared memory as [key][channel] rows with
 // the 128-byte (64-byte for head dim 32) swizzle, which is at once the K-major B operand of
 // S = Q K^T and the MN-major B operand of O = P V.  The per-query window mask is applied in
 // registers on the S accumulator read back from tensor memory, followed by an online softmax
@@ -74,12 +74,21 @@ struct TileWalk {
     __device__ __forceinline__ int col() const { return tc * TW; }
 };
 
+// Place in a ring of buffers and the phase of its barriers, carried along: an issuing warp as busy as the pipe has no time to work
+// them out for every chunk.
+struct Ring {
+    uint32_t at = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t n) {
+        if (++at == n) { at = 0; phase ^= 1; }
+    }
+};
+
 // Compile-time geometry of one (head dim, kernel size) instantiation.
 // NMAX caps the keys (forward, dQ) or queries (dK/dV) of one chunk; it is set by how many
 // tensor-memory columns the kernel can spare for the S-shaped accumulators.
-// EXTRA_W widens the box (dK/dV: the inverse neighbourhood of a key tile whose first column is
-// below ks starts at column 0 and is up to ks/2 columns wider than TW + ks - 1).
-// W_SPLIT cuts the box into that many column strips, each walked as a chunk of its own (dK/dV).
+// EXTRA_W rounds the box up to whole strips (dK/dV on column strips: a strip's width divides 8).
+// W_SPLIT cuts the box into that many column strips, each walked as a chunk of its own (dK/dV; a box at the borders
+// can be wider or narrower than this one, which costs strips, not their geometry).
 template <int D, int KS, int NMAX = 256, int EXTRA_W = 0, int W_SPLIT = 1>
 struct Cfg {
     static constexpr int HH = TH + KS - 1;                 // halo box rows

@@ -199,14 +199,7 @@ dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         constexpr uint32_t idesc_s = umma_idesc(TM, C::NKP, IsBf16<DT>::value, IsBf16<DT>::value, false, false);
         constexpr uint32_t idesc_o = umma_idesc(TM, D, IsBf16<DT>::value, IsBf16<DT>::value, false, true);
         constexpr uint32_t hi = smem_desc_hi(C::ATOM, C::SWZ);
-        // The issuing warp is as busy as the pipe (28 MMAs a chunk at head dim 128): ring places and phases are carried along
-        // instead of being worked out for every chunk.
-        struct Ring {
-            uint32_t at = 0, phase = 0;
-            __device__ __forceinline__ void next(uint32_t n) {
-                if (++at == n) { at = 0; phase ^= 1; }
-            }
-        };
+        // (the issuing warp is as busy as the pipe: 28 MMAs a chunk at head dim 128)
         const uint32_t q_lo0 = smem_desc_lo(smem_u32(sQ), 16), g_lo0 = smem_desc_lo(smem_u32(sDO), 16);
         const uint32_t k_lo0 = smem_desc_lo(smem_u32(sK), 16), v_lo0 = smem_desc_lo(smem_u32(sV), 16);
         const uint32_t km_lo0 = smem_desc_lo(smem_u32(sK), C::KV_SLAB);

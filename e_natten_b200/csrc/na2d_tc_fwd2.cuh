@@ -204,13 +204,6 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         constexpr uint32_t idesc_s = umma_idesc(TM, C::NKP, IsBf16<DT>::value, IsBf16<DT>::value, false, false);
         constexpr uint32_t idesc_o = umma_idesc(TM, D, IsBf16<DT>::value, IsBf16<DT>::value, false, true);
         constexpr uint32_t hi = smem_desc_hi(C::ATOM, C::SWZ);
-        // Ring places and phases are carried along instead of being worked out for every chunk.
-        struct Ring {
-            uint32_t at = 0, phase = 0;
-            __device__ __forceinline__ void next(uint32_t n) {
-                if (++at == n) { at = 0; phase ^= 1; }
-            }
-        };
         // the chunks in their order: group x, chunk c and pair of tiles
         struct Place {
             int x = 0, c = 0, pair = 0;

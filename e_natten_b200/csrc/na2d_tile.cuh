@@ -31,9 +31,13 @@
 #include <stdint.h>
 
 #include "na2d_index.cuh"
+#include "na2d_ptx.cuh"
 #include "na2d_softmax.cuh"
 
 namespace na2d_tile {
+
+using na2d_ptx::fma2;
+using na2d_ptx::mul2;
 
 constexpr int kR = 4;             // pixels of a strip
 constexpr int kF = 8;             // float4 per pixel and channel chunk
@@ -253,17 +257,7 @@ __device__ __forceinline__ Strip strip_at(int c0, int W) {
 template <int KS>
 __device__ __forceinline__ bool in_window(const Strip& s, int r, int j) { return (unsigned)(j - s.off[r]) < (unsigned)KS; }
 
-// Two fp32 lanes in one register pair.
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+// Sum of the two fp32 lanes of a register pair.
 __device__ __forceinline__ float sum2(unsigned long long a) {
     return __uint_as_float((unsigned)a) + __uint_as_float((unsigned)(a >> 32));
 }
