@@ -7,11 +7,12 @@
 // which share its channels, 16-byte pieces in turn: a lane keeps its part of the strip's 4 x (KS + 3) scores in registers, a
 // halo piece is read once for four tokens, and a transposing butterfly (3 (KS + 3) shuffles) leaves each lane the whole
 // scores of one token.  Softmax, delta and dS of a token are then one lane's, without a barrier or an exchange; its weights go
-// through shared memory to the strip's other lanes, which all are in the same warp.  The only block barrier is the one behind the
-// copies.
+// through shared memory to the strip's other lanes, which all are in the same warp.  The only block barriers are those behind the
+// copies: two in the forward and the query half, whose halos are waited for one by one, one in the key half.
 //
-// What bounds them: issue slots of the two (query half: three) loops, and the latency of the copies, of which three to four blocks per
-// SM overlap.  The tiled kernels (na2d_tile.cuh) stage 32 channels at a time as fp32 with two barriers each, and repeat a strip's
+// What bounds them: issue slots of the two (query half: three) loops, and the latency of the copies, of which the blocks of an SM
+// overlap: three or four at rows of up to 128 bytes, two at 256 bytes from window 5 on, where shared memory holds no more (the register
+// bounds below are for the shorter rows; 16-bit rows spill up to 130 bytes a thread under them at window 13).  The tiled kernels (na2d_tile.cuh) stage 32 channels at a time as fp32 with two barriers each, and repeat a strip's
 // softmax on all of its lanes.  Measured against those on one B200: 4 x 8 x 4096 x 64, window 13,
 // bf16: forward 70 -> 31 us, both halves of the backward 195 -> 86; 4 x 4 x 32768 x 128, window 7, bf16: 393 -> 158, 859 -> 347;
 // 4 x 8 x 4096 x 32, window 13, fp32: 33 -> 25, 101 -> 66.
@@ -37,7 +38,8 @@ using na2d_tile::Operand;
 constexpr int kTile = 128, kStrips = kTile / kR, kLanes = 4, kThreads = kStrips * kLanes;
 // Bytes of a row at most.  fp32 rows of 256 bytes are no faster here than in the tiled kernels (4 x 8 x 4096 x 64, window 3 / 7:
 // forward 37 / 43 against 33 / 38 us, window 13 50 against 54), of 192 bytes they are (window 7 29 against 35 us, window 13 35
-// against 52); 16-bit rows gain throughout, and above 256 bytes one block would be left on an SM.
+// against 52).  16-bit rows gain throughout, and would beyond this line too: 8 x 16384 tokens, window 7, 272 bytes forward 149 -> 59 and
+// backward 308 -> 128 us, 336 bytes 183 -> 70 and 377 -> 148 (window 13 at 336 bytes 278 -> 82 and 560 -> 262); two blocks fit an SM there.
 constexpr int max_row(int element_bytes) { return element_bytes == 4 ? 192 : 256; }
 
 template <int KS> constexpr int kU = KS + kR - 1;     // halo rows a regular strip reaches

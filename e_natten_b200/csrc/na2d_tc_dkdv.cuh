@@ -24,8 +24,8 @@
 //
 // What bounds it: the chain score MMAs -> softmax warps -> output MMAs -> stage free, of which tensor memory holds two or three; the
 // softmax part of it was cut by strips, packed fp32 pairs, and lse and delta handed over by the producer.  Measured on one B200
-// against chunks of box rows: 32 x 2 x 56 x 56 x 32, window 7, bf16 104 -> 62 us; 16 x 8 x 28 x 28 x 64, window 13, bf16
-// 135 -> 100 us; 16 x 16 x 14 x 14 x 64, window 13, fp16 39 -> 29 us; 8 heads of 1024 x 1024 x 128, window 13, bf16 7.8 -> 6.6 ms;
+// against the chunks of box rows before: 32 x 2 x 56 x 56 x 32, window 7, bf16 104 -> 62 us; 16 x 8 x 28 x 28 x 64, window 13, bf16
+// 135 -> 91 us (groups of rows, without strips); 16 x 16 x 14 x 14 x 64, window 13, fp16 39 -> 29 us; 8 heads of 1024 x 1024 x 128, window 13, bf16 7.8 -> 6.6 ms;
 // 4 x 4 x 256 x 256 x 128, window 5, bf16 (the same chunks as before) 0.39 -> 0.375 ms.
 #pragma once
 
@@ -73,7 +73,7 @@ struct DkvCfg : DkvCfgBase<D, KS, STRIPS> {
     static constexpr int NMAX = dkv_cols(D, KS, STRIPS);
     static constexpr int TMEM_STAGE = 2 * NMAX;                            // columns per chunk stage
     // Chunk stages: a third one where it fits (head dims 32 and 64, chunks of up to 64 queries), which takes a chunk's MMAs out of the
-    // softmax warps' way (16 x 8 x 28 x 28 x 64, window 13, bf16: 101 -> 98 us).
+    // softmax warps' way (16 x 8 x 28 x 28 x 64, window 13, bf16, on strips: 101 -> 98 us).
     static constexpr int NSTG = 3 * TMEM_STAGE <= 512 - 2 * D ? 3 : 2;
     static constexpr int TMEM_ST = 0, TMEM_DPT = NMAX, TMEM_DV = 512 - 2 * D, TMEM_DK = TMEM_DV + D;
     static constexpr int TMEM_PT = 0, TMEM_DST = NMAX / 2, TMEM_RES = NMAX;   // 16-bit operands over S^T / dP^T

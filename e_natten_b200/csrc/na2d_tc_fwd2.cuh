@@ -19,7 +19,7 @@
 //
 // What bounds it: exponentials (8 cycles a warp instruction; a warp's rows see 1.3 to 2.5 times the window) and the chain wait,
 // load, maximum, exp, store of a group, of which two are in flight; at head dim 128 the MMAs are as long.  Measured against
-// na2d_tc_fwd.cuh on one B200: 32 x 2 x 56 x 56 x 32, window 7, bf16 51 -> 32 us; 16 x 8 x 28 x 28 x 64, window 13, bf16 53 -> 39 us;
+// na2d_tc_fwd.cuh on one B200: 32 x 2 x 56 x 56 x 32, window 7, bf16 51 -> 39 us; 16 x 8 x 28 x 28 x 64, window 13, bf16 53 -> 39 us;
 // 2 x 6 x 97 x 131 x 64, window 9, fp16 45 -> 37 us; 8 heads of 1024 x 1024 x 128, window 13, bf16 3.34 -> 2.69 ms.
 #pragma once
 

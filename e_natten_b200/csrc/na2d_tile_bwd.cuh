@@ -146,8 +146,8 @@ struct KeyShape {
     static constexpr int kHalo = max_of(S::kHalo, kMaxCols * (kSpan + 2) * kF);
     static constexpr int kSmem = (kWeights + kHalo) * 16;
     static constexpr int kBlocksSmem = kSmemPerSm / (kSmem + 1024);
-    // With the dense weights of the unfused pair three blocks of 256 threads, 80 registers each, are faster than four with 64, which
-    // spill from window 5 on: 4 x 4 x 64 x 64 x 128, window 5, fp32, both calls' backwards 287 -> 254 us (4 x 8 x 64 x 96 x 48, window 3,
+    // With the dense weights of the unfused pair three blocks of 256 threads, 80 registers each, are faster than four with 64 from window 5
+    // on (both spill: 4 to 48 bytes a thread with 80, 36 to 120 with 64): 4 x 4 x 64 x 64 x 128, window 5, fp32, both calls' backwards 287 -> 254 us (4 x 8 x 64 x 96 x 48, window 3,
     // fp16 237 -> 242).  With tiled ones four are (4 x 4 x 256 x 256 x 128, fp32: 1.0 against 1.1 ms).
     static constexpr int kBlocksTiled = kBlocksSmem * kThreads > 1024 ? 1024 / kThreads : kBlocksSmem;
     static constexpr int kBlocksDense = KS > 3 && kBlocksSmem * kThreads > 768 ? 768 / kThreads : kBlocksTiled;
