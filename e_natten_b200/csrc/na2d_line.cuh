@@ -12,7 +12,8 @@
 //
 // What bounds them: issue slots of the two (query half: three) loops, and the latency of the copies, of which the blocks of an SM
 // overlap: three or four at rows of up to 128 bytes, two at 256 bytes from window 5 on, where shared memory holds no more (the register
-// bounds below are for the shorter rows; 16-bit rows spill up to 130 bytes a thread under them at window 13).  The tiled kernels (na2d_tile.cuh) stage 32 channels at a time as fp32 with two barriers each, and repeat a strip's
+// bounds below are for the shorter rows; 16-bit rows spill up to 130 bytes a thread under them at window 13).
+// The tiled kernels (na2d_tile.cuh) stage 32 channels at a time as fp32 with two barriers each, and repeat a strip's
 // softmax on all of its lanes.  Measured against those on one B200: 4 x 8 x 4096 x 64, window 13,
 // bf16: forward 70 -> 31 us, both halves of the backward 195 -> 86; 4 x 4 x 32768 x 128, window 7, bf16: 393 -> 158, 859 -> 347;
 // 4 x 8 x 4096 x 32, window 13, fp32: 33 -> 25, 101 -> 66.
