@@ -3,8 +3,8 @@
     python e_natten_b200/build.py [--force] [--verbose]
 
 The library is plain CUDA C++ behind a C ABI (include/na2d.h); it needs no framework headers.
-Its kernels are compiled as ten translation units in parallel (the API with the SIMT kernels, the
-tiled CUDA-core kernels once per element type, and each of the three tcgen05 kernel families once per
+Its kernels are compiled as eleven translation units in parallel (the API with the SIMT kernels, the
+tiled CUDA-core kernels once per element type, the fp32 box kernels, and each of the three tcgen05 kernel families once per
 16-bit element type) and linked into one shared object.  The Python package's extension module
 (_na2d_torch.so, host code over PyTorch's C++ API) is compiled beside it with g++; it belongs to one
 PyTorch and one Python version and is compiled again when either changes.
@@ -30,6 +30,7 @@ UNITS = [
     ("na2d_tile.cu", ["-DNA2D_TILE_DT=0"], "na2d_tile_f32.o"),
     ("na2d_tile.cu", ["-DNA2D_TILE_DT=1"], "na2d_tile_bf16.o"),
     ("na2d_tile.cu", ["-DNA2D_TILE_DT=2"], "na2d_tile_f16.o"),
+    ("na2d_box.cu", [], "na2d_box.o"),
     ("na2d_tc_fwd.cu", ["-DNA2D_TC_DT=1"], "na2d_tc_fwd_bf16.o"),
     ("na2d_tc_fwd.cu", ["-DNA2D_TC_DT=2"], "na2d_tc_fwd_f16.o"),
     ("na2d_tc_dq.cu", ["-DNA2D_TC_DT=1"], "na2d_tc_dq_bf16.o"),

@@ -344,6 +344,14 @@ bool query_half_in_tiles(const Na2dGeom& g, int dtype) {
 }
 
 na2d_tile::Tensor tile(const Tensor& t) { return na2d_tile::Tensor{t.ptr, t.st}; }
+// Calls run(place) with where a tiled call's launches run; the fp32 kernels of the 2D operator and the pair get the error state.
+template <typename F>
+int at_place(int device, cudaStream_t st, int dtype, const Na2dGeom& g, F&& run) {
+    Errors err;
+    if (dtype == NA2D_F32 && g.kh > 1)
+        if (int rc = error_state(device, &err)) return rc;
+    return run(na2d_tile::Place{device, st, err.device});
+}
 
 // The launcher of the element type.
 #define NA2D_TILE_PICK(dtype, name) \
@@ -382,7 +390,9 @@ int run_forward(const Problem& p) {
     }
     if (in_tiles(na2d_tile::Work::kForward, g, p.dtype)) {
         const auto run = NA2D_TILE_PICK(p.dtype, forward);
-        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.o), p.lse), 1);
+        return at_place(p.device, p.st, p.dtype, g, [&](const na2d_tile::Place& at) {
+            return after_tile(run(g, at, tile(p.q), tile(p.k), tile(p.v), tile(p.o), p.lse), 1);
+        });
     }
     unsigned grid = 0;
     int rc = grid_for(g.BN, g.Hq, g.W, g.patch, &grid);
@@ -445,7 +455,9 @@ int run_backward_dq(const Problem& p) {
     }
     if (query_half_in_tiles(g, p.dtype)) {
         const auto run = NA2D_TILE_PICK(p.dtype, backward_dq);
-        return after_tile(run(g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), p.lse, p.delta, p.row_factor), 1);
+        return at_place(p.device, p.st, p.dtype, g, [&](const na2d_tile::Place& at) {
+            return after_tile(run(g, at, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), p.lse, p.delta, p.row_factor), 1);
+        });
     }
     unsigned grid = 0;
     int rc = grid_for(g.BN, g.Hq, g.W, g.patch, &grid);
@@ -506,10 +518,12 @@ size_t row_factor_bytes(const Problem& p) { return (size_t)p.g.BN * p.g.Hq * p.g
 int run_backward_shared(const Problem& p, void* workspace, na2d_tile::Turns turns) {
     const auto run = NA2D_TILE_PICK(p.dtype, backward);
     int launches = 0;
-    const int rc = run(p.g, p.st, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), tile(p.d_k), tile(p.d_v), p.lse,
-                       p.delta, (float*)workspace, turns, &launches);
-    g_launches.fetch_add(launches);
-    return after_tile(rc, 0);
+    return at_place(p.device, p.st, p.dtype, p.g, [&](const na2d_tile::Place& at) {
+        const int rc = run(p.g, at, tile(p.q), tile(p.k), tile(p.v), tile(p.d_o), tile(p.d_q), tile(p.d_k), tile(p.d_v), p.lse,
+                           p.delta, (float*)workspace, turns, &launches);
+        g_launches.fetch_add(launches);
+        return after_tile(rc, 0);
+    });
 }
 
 // Validate, select the device, check it; then run `step`.
@@ -572,10 +586,11 @@ struct PairProblem {
     Na2dGeom g;
     int dtype;
     Na2dStride st;          // dense strides of a (B, N, H, W, C) tensor
+    int device;
     cudaStream_t stream;
 };
 
-int make_pair_problem(int B, int N, int H, int W, int C, int ks, int dtype, void* stream, PairProblem* out) {
+int make_pair_problem(int B, int N, int H, int W, int C, int ks, int dtype, int device, void* stream, PairProblem* out) {
     if (B <= 0 || N <= 0 || H <= 0 || W <= 0 || C <= 0) return NA2D_ERR_BAD_ARG;
     if (ks <= 0 || (ks & 1) == 0) return NA2D_ERR_BAD_ARG;
     if (dtype != NA2D_F32 && dtype != NA2D_BF16 && dtype != NA2D_F16) return NA2D_ERR_UNSUPPORTED;
@@ -589,6 +604,7 @@ int make_pair_problem(int B, int N, int H, int W, int C, int ks, int dtype, void
     out->g = g;
     out->dtype = dtype;
     out->st = Na2dStride{(long long)N * H * W * C, (long long)H * W * C, (long long)W * C, C};
+    out->device = device;
     out->stream = (cudaStream_t)stream;
     return NA2D_OK;
 }
@@ -596,7 +612,7 @@ int make_pair_problem(int B, int N, int H, int W, int C, int ks, int dtype, void
 template <typename F>
 int enter_pair(int B, int N, int H, int W, int C, int ks, int dtype, int device, void* stream, F&& step) {
     PairProblem p;
-    int rc = make_pair_problem(B, N, H, W, C, ks, dtype, stream, &p);
+    int rc = make_pair_problem(B, N, H, W, C, ks, dtype, device, stream, &p);
     if (rc != NA2D_OK) return rc;
     DeviceScope scope(device);
     if (scope.err != cudaSuccess) return cuda_fail(scope.err, "cudaSetDevice");
@@ -609,7 +625,10 @@ na2d_tile::Tensor tile_dense(const PairProblem& p, const void* ptr) { return na2
 
 // x . y over the window -> attn
 int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
-    if (in_tiles(na2d_tile::Work::kDot, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_dot)(p.g, p.stream, tile_dense(p, x), tile_dense(p, y), attn), 1);
+    if (in_tiles(na2d_tile::Work::kDot, p.g, p.dtype))
+        return at_place(p.device, p.stream, p.dtype, p.g, [&](const na2d_tile::Place& at) {
+            return after_tile(NA2D_TILE_PICK(p.dtype, pair_dot)(p.g, at, tile_dense(p, x), tile_dense(p, y), attn), 1);
+        });
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -622,7 +641,10 @@ int pair_dot(const PairProblem& p, const void* x, const void* y, void* attn) {
 }
 // sum_j attn_j y_j -> out
 int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out) {
-    if (in_tiles(na2d_tile::Work::kApply, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_apply)(p.g, p.stream, attn, tile_dense(p, y), tile_dense(p, out)), 1);
+    if (in_tiles(na2d_tile::Work::kApply, p.g, p.dtype))
+        return at_place(p.device, p.stream, p.dtype, p.g, [&](const na2d_tile::Place& at) {
+            return after_tile(NA2D_TILE_PICK(p.dtype, pair_apply)(p.g, at, attn, tile_dense(p, y), tile_dense(p, out)), 1);
+        });
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hq, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;
@@ -636,7 +658,10 @@ int pair_apply(const PairProblem& p, const void* attn, const void* y, void* out)
 }
 // key-side sum over the inverse neighbourhood of attn x -> out
 int pair_inverse(const PairProblem& p, const void* attn, const void* x, void* out) {
-    if (in_tiles(na2d_tile::Work::kKeySum, p.g, p.dtype)) return after_tile(NA2D_TILE_PICK(p.dtype, pair_inverse)(p.g, p.stream, attn, tile_dense(p, x), tile_dense(p, out)), 1);
+    if (in_tiles(na2d_tile::Work::kKeySum, p.g, p.dtype))
+        return at_place(p.device, p.stream, p.dtype, p.g, [&](const na2d_tile::Place& at) {
+            return after_tile(NA2D_TILE_PICK(p.dtype, pair_inverse)(p.g, at, attn, tile_dense(p, x), tile_dense(p, out)), 1);
+        });
     unsigned grid = 0;
     int rc = grid_for(p.g.BN, p.g.Hkv, p.g.W, p.g.patch, &grid);
     if (rc != NA2D_OK) return rc;

@@ -8,6 +8,9 @@
 #include "na2d_tile_bwd.cuh"
 #include "na2d_tile_pair.cuh"
 #include "na2d_line.cuh"
+#if NA2D_TILE_DT == 0
+#include "na2d_box_entry.h"
+#endif
 
 #if NA2D_TILE_DT == 0
 using Elem = float;
@@ -83,6 +86,17 @@ bool in_line(const Na2dGeom& g, std::initializer_list<const Tensor*> operands) {
     return true;
 }
 
+#if NA2D_TILE_DT == 0
+// fp32 operands that na2d_box.cuh takes go there: run(call) launches.  True with the status, or false where the tiled kernels are to
+// take the launch.
+template <typename F>
+bool in_boxes(const Na2dGeom& g, const Place& at, std::initializer_list<const Tensor*> operands, int* rc, F&& run) {
+    if (!na2d_box::takes(g, operands)) return false;
+    *rc = run(na2d_box::Call{g, at.device, at.st, at.errors});
+    return *rc != na2d_box::kNoMap;
+}
+#endif
+
 }  // namespace
 
 // ---- how the backward's workspace is shared out -------------------------------------------------------
@@ -145,8 +159,11 @@ Turns workspace_turns(const Na2dGeom& g, long long floats) {
 }
 #endif
 
-int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+int NA2D_NAME(forward)(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,
                        const Tensor& o, float* lse) {
+#if NA2D_TILE_DT == 0
+    if (int rc = 0; in_boxes(g, at, {&q, &k, &v, &o}, &rc, [&](const na2d_box::Call& c) { return na2d_box::forward(c, q, k, v, o, lse); })) return rc;
+#endif
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
         const auto kernel = g.C > kParkAbove<S> ? fwd_kernel<Elem, S::kKs, S::kOneD, true> : fwd_kernel<Elem, S::kKs, S::kOneD, false>;
@@ -155,15 +172,22 @@ int NA2D_NAME(forward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, cons
         if constexpr (S::kOneD) {
             if (in_line(g, {&q, &k, &v, &o}))
                 return launch(na2d_line::fwd_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(g.C * sizeof(Elem)),
-                              st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(o, g.C), lse, g);
+                              at.st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(o, g.C), lse, g);
         }
-        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, at.st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(o, g.C), lse, g);
     });
 }
 
-int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+int NA2D_NAME(backward_dq)(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,
                            const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta, float* row_factor) {
+#if NA2D_TILE_DT == 0
+    if (int rc = 0; in_boxes(g, at, {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
+            const int rows = (g.Hq + 7) / 8;
+            return na2d_box::query_half(c, q, k, v, d_o, d_q, lse, delta, row_factor, nullptr, nullptr, g.BN, na2d_box::Rows{0, 0, rows, rows});
+        }))
+        return rc;
+#endif
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
         const auto kernel = g.C > kParkAbove<S> ? dq_kernel<Elem, S::kKs, S::kOneD, true> : dq_kernel<Elem, S::kKs, S::kOneD, false>;
@@ -172,16 +196,16 @@ int NA2D_NAME(backward_dq)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, 
         if constexpr (S::kOneD) {
             if (in_line(g, {&q, &k, &v, &d_o, &d_q}))
                 return launch(na2d_line::dq_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(g.C * sizeof(Elem)),
-                              st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta,
+                              at.st, operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta,
                               row_factor, (float4*)nullptr, (float4*)nullptr, 0, g);
         }
-        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, at.st, operand(q, g.C), operand(k, g.C),
                       operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta, row_factor, (float4*)nullptr,
                       (float4*)nullptr, whole_images<S>(g, g.Hq), g);
     });
 }
 
-int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,
+int NA2D_NAME(backward)(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,
                         const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v, const float* lse,
                         float* delta, float* workspace, Turns turns, int* launches) {
     return by_window(g, [&](auto shape) -> int {
@@ -198,12 +222,12 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
                     unsigned n = 0;
                     if (int rc = tiles<S>(g, units, 1, &n)) return rc;
                     const int row_bytes = g.C * (int)sizeof(Elem);
-                    if (int rc = launch(na2d_line::dq_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(row_bytes), st,
+                    if (int rc = launch(na2d_line::dq_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::forward_smem<S::kKs>(row_bytes), at.st,
                                         operand(q, g.C), operand(k, g.C), operand(v, g.C), operand(d_o, g.C), operand(d_q, g.C), lse, delta,
                                         (float*)nullptr, p, ds, (int)unit0, g))
                         return rc;
                     ++*launches;
-                    if (int rc = launch(na2d_line::key_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::key_smem<S::kKs>(row_bytes), st,
+                    if (int rc = launch(na2d_line::key_kernel<Elem, S::kKs>, n, na2d_line::kThreads, na2d_line::key_smem<S::kKs>(row_bytes), at.st,
                                         operand(q, g.C), operand(d_o, g.C), operand(d_k, g.C), operand(d_v, g.C), p, ds, (int)unit0, g))
                         return rc;
                     ++*launches;
@@ -221,17 +245,35 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
                 const Band query_band{(int)unit0, queries, query_end - queries, turns.rows};
                 const Band key_band{(int)unit0, keys, key_end - keys, turns.rows};
                 unsigned n = 0;
-                if (query_band.rows > 0) {
-                    if (int rc = tiles<S>(g, units, query_band.rows * S::kTh, &n)) return rc;
-                    if (int rc = launch(kernel, n, S::kThreads, S::kSmem, st, operand(q, g.C), operand(k, g.C), operand(v, g.C),
-                                        operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float*)nullptr, p, ds, query_band, g))
+                const auto query_half = [&]() -> int {
+#if NA2D_TILE_DT == 0
+                    const na2d_box::Rows rows{query_band.unit0, query_band.row0, query_band.rows, query_band.ring};
+                    if (int rc = 0; in_boxes(g, at, {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
+                            return na2d_box::query_half(c, q, k, v, d_o, d_q, lse, delta, nullptr, p, ds, units, rows);
+                        }))
                         return rc;
+#endif
+                    if (int rc = tiles<S>(g, units, query_band.rows * S::kTh, &n)) return rc;
+                    return launch(kernel, n, S::kThreads, S::kSmem, at.st, operand(q, g.C), operand(k, g.C), operand(v, g.C),
+                                  operand(d_o, g.C), operand(d_q, g.C), lse, delta, (float*)nullptr, p, ds, query_band, g);
+                };
+                const auto key_half = [&]() -> int {
+#if NA2D_TILE_DT == 0
+                    const na2d_box::Rows rows{key_band.unit0, key_band.row0, key_band.rows, key_band.ring};
+                    if (int rc = 0; in_boxes(g, at, {&q, &d_o, &d_k, &d_v}, &rc, [&](const na2d_box::Call& c) {
+                            return na2d_box::key_half(c, q, d_o, d_k, d_v, p, ds, units, rows);
+                        }))
+                        return rc;
+#endif
+                    if (int rc = tiles<S>(g, units, key_band.rows * S::kTh, &n)) return rc;
+                    return launch(key_sum_kernel<Elem, float, true, S::kKs, S::kOneD>, dim3(n, 2), K::kThreads, K::kSmem, at.st,
+                                  for_dk, for_dv, key_band, g);
+                };
+                if (query_band.rows > 0) {
+                    if (int rc = query_half()) return rc;
                     ++*launches;
                 }
-                if (int rc = tiles<S>(g, units, key_band.rows * S::kTh, &n)) return rc;
-                if (int rc = launch(key_sum_kernel<Elem, float, true, S::kKs, S::kOneD>, dim3(n, 2), K::kThreads, K::kSmem, st,
-                                    for_dk, for_dv, key_band, g))
-                    return rc;
+                if (int rc = key_half()) return rc;
                 ++*launches;
                 keys = key_end;
                 queries = query_end;
@@ -241,35 +283,44 @@ int NA2D_NAME(backward)(const Na2dGeom& g, cudaStream_t st, const Tensor& q, con
     });
 }
 
-int NA2D_NAME(pair_dot)(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn) {
+int NA2D_NAME(pair_dot)(const Na2dGeom& g, const Place& at, const Tensor& x, const Tensor& y, void* attn) {
+#if NA2D_TILE_DT == 0
+    if (int rc = 0; in_boxes(g, at, {&x, &y}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_dot(c, x, y, (float*)attn); })) return rc;
+#endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
         const auto kernel = g.C > kParkAbove<S> ? window_dot_kernel<Elem, S::kKs, true> : window_dot_kernel<Elem, S::kKs, false>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(kernel, n, S::kThreads, S::kSmem, st, operand(x, g.C),
+        return launch(kernel, n, S::kThreads, S::kSmem, at.st, operand(x, g.C),
                       operand(y, g.C), (Elem*)attn, g);
     });
 }
 
-int NA2D_NAME(pair_apply)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out) {
+int NA2D_NAME(pair_apply)(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& y, const Tensor& out) {
+#if NA2D_TILE_DT == 0
+    if (int rc = 0; in_boxes(g, at, {&y, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_apply(c, (const float*)attn, y, out); })) return rc;
+#endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hq, &n)) return rc;
-        return launch(window_apply_kernel<Elem, S::kKs>, n, S::kThreads, S::kSmem, st, (const Elem*)attn,
+        return launch(window_apply_kernel<Elem, S::kKs>, n, S::kThreads, S::kSmem, at.st, (const Elem*)attn,
                       operand(y, g.C), operand(out, g.C), g);
     });
 }
 
-int NA2D_NAME(pair_inverse)(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out) {
+int NA2D_NAME(pair_inverse)(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& x, const Tensor& out) {
+#if NA2D_TILE_DT == 0
+    if (int rc = 0; in_boxes(g, at, {&x, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_inverse(c, (const float*)attn, x, out); })) return rc;
+#endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
         using K = KeyShape<S>;
         unsigned n = 0;
         if (int rc = tiles<S>(g, g.BN, g.Hkv, &n)) return rc;
         const KeySum sum{attn, operand(x, g.C), operand(out, g.C)};
-        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, false>, n, K::kThreads, K::kSmem, st, sum, sum, whole_images<S>(g, g.Hkv), g);
+        return launch(key_sum_kernel<Elem, Elem, false, S::kKs, false>, n, K::kThreads, K::kSmem, at.st, sum, sum, whole_images<S>(g, g.Hkv), g);
     });
 }
 

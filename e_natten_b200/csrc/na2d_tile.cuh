@@ -1,6 +1,7 @@
 // Tiled CUDA-core kernels for neighborhood attention: fused forward, the query half of the backward
 // (dQ, delta, and the P / dS weights the key half reads), the unfused pair, and the key-side sum over
-// the inverse neighbourhood.  fp32 arithmetic throughout; fp32, bf16 and fp16 tensors.
+// the inverse neighbourhood.  fp32 arithmetic throughout; fp32, bf16 and fp16 tensors.  fp32 calls in 2D whose rows start on 16-byte
+// boundaries go to na2d_box.cuh.
 //
 // A block owns a tile of kTh x (4 * kStrips) pixels of one (batch, head) image.  Channels pass
 // through shared memory 32 at a time (always as fp32): the tile's own rows and the halo of rows its

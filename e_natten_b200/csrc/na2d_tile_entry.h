@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "na2d_index.cuh"
+#include "na2d_ptx.cuh"
 
 namespace na2d_tile {
 
@@ -31,20 +32,27 @@ long long workspace_floats(const Na2dGeom& g, long long limit);
 // The turns a workspace of so many values allows; units is 0 if it is too small for any.
 Turns workspace_turns(const Na2dGeom& g, long long floats);
 
+// Where a launch runs: fp32 kernels fed by TMA report waits that gave up to `errors`.
+struct Place {
+    int device;
+    cudaStream_t st;
+    const na2d_ptx::ErrorState* errors;
+};
+
 // backward_dq: row_factor (or null) takes what the key half multiplies each row's exp(s - lse) by.
 // backward: both halves, for whole images.
 // Status: 0, NA2D_ERR_TOO_LARGE (grid), or NA2D_ERR_CUDA (the launch's error is left for cudaGetLastError).
 #define NA2D_TILE_ENTRIES(suffix)                                                                                     \
-    int forward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,       \
+    int forward_##suffix(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,       \
                          const Tensor& o, float* lse);                                                                \
-    int backward_dq_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,   \
+    int backward_dq_##suffix(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,   \
                              const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta, float* row_factor);                   \
-    int backward_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& q, const Tensor& k, const Tensor& v,      \
+    int backward_##suffix(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,      \
                           const Tensor& d_o, const Tensor& d_q, const Tensor& d_k, const Tensor& d_v,                 \
                           const float* lse, float* delta, float* workspace, Turns turns, int* launches);                \
-    int pair_dot_##suffix(const Na2dGeom& g, cudaStream_t st, const Tensor& x, const Tensor& y, void* attn);          \
-    int pair_apply_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& y, const Tensor& out); \
-    int pair_inverse_##suffix(const Na2dGeom& g, cudaStream_t st, const void* attn, const Tensor& x, const Tensor& out);
+    int pair_dot_##suffix(const Na2dGeom& g, const Place& at, const Tensor& x, const Tensor& y, void* attn);          \
+    int pair_apply_##suffix(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& y, const Tensor& out); \
+    int pair_inverse_##suffix(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& x, const Tensor& out);
 NA2D_TILE_ENTRIES(f32)
 NA2D_TILE_ENTRIES(bf16)
 NA2D_TILE_ENTRIES(f16)
