@@ -57,6 +57,26 @@ int launch(const Call& c, void (*kernel)(P...), dim3 grid, int threads, int smem
 }
 template <int KS, int WHICH, bool FLAG> struct Tag {};
 
+// Channels that a block of the apply and key sum kernels takes, whose blocks need not take all of them.  `blocks` tiles on a GPU with room
+// for `per_sm` blocks an SM: a wave of k blocks an SM lasts about 0.73 + 0.27 k times as long as one block (measured with 1, 2 and 4 an
+// SM), and fetching the weights, which each block does, about as long as a chunk of channels.  4 x 4 x 64 x 64 x 128, window 5, pair: 512 tiles.
+int channels_of_block(const Call& c, long long blocks, int per_sm) {
+    const int sms = na2d_tc::sm_count(c.device), chunks = (c.g.C + kChunk - 1) / kChunk;
+    float best = 0.f;
+    int span = chunks;
+    for (int parts = 1; parts <= chunks; ++parts) {
+        const int per = (chunks + parts - 1) / parts;
+        const long long all = blocks * ((chunks + per - 1) / per), slots = (long long)sms * per_sm, rest = all % slots;
+        const float waves = (float)(all / slots) * (0.73f + 0.27f * per_sm) + (rest ? 0.73f + 0.27f * (float)((rest + sms - 1) / sms) : 0.f);
+        const float time = waves * (float)(1 + per);
+        if (parts == 1 || time < 0.97f * best) {
+            best = time;
+            span = per;
+        }
+    }
+    return span * kChunk;
+}
+
 }  // namespace
 
 int forward(const Call& c, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, float* lse) {
@@ -103,8 +123,9 @@ int key_half(const Call& c, const Tensor& q, const Tensor& d_o, const Tensor& d_
         CUtensorMap xq, wq, xg, wg;
         if (!map_key<S>(&xq, c, q, false) || !map_key<S>(&wq, c, q, true) || !map_key<S>(&xg, c, d_o, false) || !map_key<S>(&wg, c, d_o, true))
             return kNoMap;
-        return launch<Tag<S::kKs, 2, true>>(c, key_sum_kernel<true, S::kKs>, dim3(n, 2), K::kThreads, K::kSmem, xq, wq, xg, wg,
-                                            KeyOut{ds, operand(d_k)}, KeyOut{p, operand(d_v)}, c.errors,
+        const int span = channels_of_block(c, 2ll * n, K::kBlocks);
+        return launch<Tag<S::kKs, 2, true>>(c, key_sum_kernel<true, S::kKs>, dim3(n, 2, (c.g.C + span - 1) / span), K::kThreads, K::kSmem, xq, wq,
+                                            xg, wg, KeyOut{ds, operand(d_k)}, KeyOut{p, operand(d_v)}, span, c.errors,
                                             Band{rows.unit0, rows.row0, rows.rows, rows.ring}, c.g);
     });
 }
@@ -118,7 +139,7 @@ int pair_dot(const Call& c, const Tensor& x, const Tensor& y, float* attn) {
         if (!map_own<S>(&mx, c, x) || !map_dot<S>(&my, c, y)) return kNoMap;
         auto run = [&](auto park) {
             constexpr bool kPark = decltype(park)::value;
-            return launch<Tag<S::kKs, 3, kPark>>(c, window_dot_kernel<S::kKs, kPark>, n, S::kThreads, S::kSmem, mx, my, attn, c.errors, c.g);
+            return launch<Tag<S::kKs, 3, kPark>>(c, window_dot_kernel<S::kKs, kPark>, n, S::kThreads, PairShape<S>::kDotSmem, mx, my, attn, c.errors, c.g);
         };
         return c.g.C > kParkAbove ? run(std::true_type{}) : run(std::false_type{});
     });
@@ -131,7 +152,10 @@ int pair_apply(const Call& c, const float* attn, const Tensor& y, const Tensor& 
         if (int rc = tiles<S>(c.g, c.g.BN, tile_rows<S>(c.g.Hq), &n)) return rc;
         CUtensorMap my;
         if (!map_halo<S>(&my, c, y)) return kNoMap;
-        return launch<Tag<S::kKs, 4, true>>(c, window_apply_kernel<S::kKs>, n, S::kThreads, S::kSmem, attn, my, operand(out), c.errors, c.g);
+        using P = PairShape<S>;
+        const int span = channels_of_block(c, n, P::kApplyBlocks);
+        return launch<Tag<S::kKs, 4, true>>(c, window_apply_kernel<S::kKs>, dim3(n, 1, (c.g.C + span - 1) / span), P::kApplyThreads, P::kApplySmem,
+                                            attn, my, operand(out), span, c.errors, c.g);
     });
 }
 
@@ -145,7 +169,9 @@ int pair_inverse(const Call& c, const float* attn, const Tensor& x, const Tensor
         CUtensorMap mx, mw;
         if (!map_key<S>(&mx, c, x, false) || !map_key<S>(&mw, c, x, true)) return kNoMap;
         const KeyOut sum{attn, operand(out)};
-        return launch<Tag<S::kKs, 5, true>>(c, key_sum_kernel<false, S::kKs>, n, K::kThreads, K::kSmem, mx, mw, mx, mw, sum, sum, c.errors,
+        const int span = channels_of_block(c, n, K::kBlocks);
+        return launch<Tag<S::kKs, 5, true>>(c, key_sum_kernel<false, S::kKs>, dim3(n, 1, (c.g.C + span - 1) / span), K::kThreads, K::kSmem, mx, mw,
+                                            mx, mw, sum, sum, span, c.errors,
                                             Band{0, 0, rows, rows}, c.g);
     });
 }

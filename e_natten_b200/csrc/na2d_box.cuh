@@ -13,9 +13,9 @@
 // block's own threads (cp.async) took a quarter of all instructions and as much of the shared-memory pipe's time; a second buffer
 // for such copies gained nothing.  A TMA box costs one thread one instruction.
 //
-// Measured on one B200 against the tiled kernels (na2d_tile.cuh), fp32: step of 4 x 4 x 256 x 256 x 128, window 5, 3.11 -> 2.53 ms
-// (8 x 128 x 256 x 128: forward 232 -> 176 us, query half 347 -> 270, key half 280 -> 228); forward of 4 x 4 x 117 x 93 x 64, window 7,
-// 151 -> 139 us; step of the unfused pair, 4 x 4 x 64 x 64 x 128, window 5, 395 -> 349 us.
+// Measured on one B200 against the tiled kernels (na2d_tile.cuh): forward / query half of 2 x 4 x 56 x 56 x 128, us: window 3 33 -> 21 / 47 -> 29,
+// 5 45 -> 40 / 66 -> 57, 7 59 -> 57 / 90 -> 84, 9 83 -> 72 / 126 -> 107, 11 100 -> 95 / 159 -> 140, 13 142 -> 138 / 209 -> 216; of 2 x 200 x 260 x 64:
+// 44 -> 28 / 62 -> 39, 56 -> 46 / 79 -> 66, 90 -> 80 / 129 -> 114, 137 -> 127 / 208 -> 180, 178 -> 165 / 269 -> 242, 252 -> 221 / 380 -> 355.
 //
 // Boxes.  Pixel after pixel, 64 or 128 bytes each, in the swizzle that goes with that size, rows an odd number of pixels long: eight
 // rows of a column then lie on different banks, as do the channels of a pixel.
@@ -71,8 +71,11 @@ struct Shape {
     static constexpr int kHaloH = kTh + KS - 1, kHaloW = kTw + KS - 1;
     static constexpr int kOwnW = kTw | 1, kBoxW = kHaloW | 1;            // columns of the boxes
     static constexpr int kItems = kTh * kStrips * KS;     // (row, strip, window row) of the dot loop
-    static constexpr int kRows = KS <= 5 ? 2 : 1;          // image rows of a thread in the apply loop
-    static constexpr int kApply = kTh / kRows * kStrips * kF;
+    // Image rows of a thread in the apply loop, and lanes that share the halo rows that those meet: two rows read a halo pixel once for
+    // both; from window 7 on that leaves threads idle, and two lanes take every other halo row (window 13 would spill with it).
+    // Forward of 2 x 4 x 56 x 56 x 128, window 9, one row / two lanes of two: 77 / 73 us, window 11 104 / 96, window 13 137 / 151.
+    static constexpr int kHalves = KS >= 7 && KS <= 11 ? 2 : 1, kRows = KS <= 11 ? 2 : 1;
+    static constexpr int kApply = kTh / kRows * kHalves * kStrips * kF;
     static constexpr int kThreads = max_of((kItems + 31) / 32 * 32, max_of(kApply, 128));
     // Weights as the key half gets them: a slot of four pixels for each column of a strip's halo band.
     static constexpr int kBand = kTh * kStrips * KS * kU;
@@ -95,7 +98,7 @@ struct Shape {
     static constexpr int kBlocksSmem = na2d_tile::kSmemPerSm / (kSmem + 1024);
     static constexpr int kBlocks = kBlocksSmem < kBlocksReg ? kBlocksSmem : kBlocksReg;
     static_assert(kHaloBuffers == 1 || kExchange * 16 <= kHaloAt, "the exchange is clear of the first halo");
-    static_assert(kBlocks >= 1, "a block fits an SM");
+    static_assert(kBlocks >= 1 && kApply <= kThreads, "a block fits an SM, an apply item a thread");
 };
 
 // Where a pixel of a box lies, its first channels' place in the swizzle included: float4 f of it at (that ^ 16 f).
@@ -207,16 +210,16 @@ __device__ __forceinline__ void set(float& acc, float x) { acc = x; }
 // that every 32; up to 32 not at all.
 constexpr int kParkAbove = 32;
 __device__ __forceinline__ bool park_at(int c, int C) { return c < C && (C <= 64 ? c % 32 != 0 : c % 32 == 0); }
-template <typename S>
-__device__ __forceinline__ void park(Sum<S> (&acc)[kR][S::kKs], float4* parked, bool first) {
+template <typename A, int N>
+__device__ __forceinline__ void park(A (&acc)[kR][N], float4* parked, bool first) {
     float largest = 0.f;
 #pragma unroll
-    for (int i = 0; i < kR * S::kKs; i += kR) {
+    for (int i = 0; i < kR * N; i += kR) {
         const float4 old = first ? make_float4(0.f, 0.f, 0.f, 0.f) : parked[i / kR];
         float sum[kR] = {old.x, old.y, old.z, old.w};
 #pragma unroll
         for (int e = 0; e < kR; ++e) {
-            Sum<S>& own = acc[(i + e) / S::kKs][(i + e) % S::kKs];
+            A& own = acc[(i + e) / N][(i + e) % N];
             const float a = value(own), total = __fadd_rn(sum[e], a);
             set(own, __fsub_rn(a, __fsub_rn(total, sum[e])));
             largest = fmaxf(largest, fabsf(total));
@@ -226,11 +229,11 @@ __device__ __forceinline__ void park(Sum<S> (&acc)[kR][S::kKs], float4* parked, 
     }
     if (largest > FLT_MAX) {                               // an infinite sum stays one
 #pragma unroll
-        for (int i = 0; i < kR * S::kKs; i += kR) {
+        for (int i = 0; i < kR * N; i += kR) {
             const float4 sum = parked[i / kR];
 #pragma unroll
             for (int e = 0; e < kR; ++e)
-                if (fabsf(lane_of(sum, e)) > FLT_MAX) acc[(i + e) / S::kKs][(i + e) % S::kKs] = 0;
+                if (fabsf(lane_of(sum, e)) > FLT_MAX) acc[(i + e) / N][(i + e) % N] = 0;
         }
     }
 }
@@ -260,11 +263,10 @@ __device__ __forceinline__ DotItem score_item(const Tile& t, const Na2dGeom& g, 
     return d;
 }
 
-// acc[r][i] += own pixel r . member i of its window row over a stage, eight channels at a time: even and odd channels
-// in the two lanes of a register pair, four products of a lane summed first and added as one number: five instructions where
-// eight multiply-adds would stand.
-template <typename S, bool REGULAR>
-__device__ __forceinline__ void dot_staged(Sum<S> (&acc)[kR][S::kKs], const uint8_t* stage, const DotItem& d) {
+// acc[r][i] += own pixel r . halo column i of the strip over a stage, or (N = KS) member i of its window row, eight channels at a time: even and odd channels in the two lanes of a register pair, four products of a lane
+// summed first and added as one number: five instructions where eight multiply-adds would stand.
+template <typename S, bool REGULAR, typename A, int N>
+__device__ __forceinline__ void dot_staged(A (&acc)[kR][N], const uint8_t* stage, const DotItem& d) {
     const int own = d.row * S::kOwnW + kR * d.strip, halo = d.hy * S::kBoxW + d.hx;
     const uint8_t* hs = stage + S::kOwn;
 #pragma unroll (REGULAR ? kDotC / 8 : 1)
@@ -275,26 +277,25 @@ __device__ __forceinline__ void dot_staged(Sum<S> (&acc)[kR][S::kKs], const uint
             q0[r] = quad_at(stage, dot_pixel(own + r) ^ 16 * f);
             q1[r] = quad_at(stage, dot_pixel(own + r) ^ 16 * f + 16);
         }
-        auto add = [&](int r, int m, const ulonglong2& x0, const ulonglong2& x1) {
-            add_pair(acc[r][m], fma2(q1[r].y, x1.y, fma2(q1[r].x, x1.x, fma2(q0[r].y, x0.y, mul2(q0[r].x, x0.x)))));
-        };
-        if constexpr (REGULAR) {
-#pragma unroll
-            for (int j = 0; j < S::kU; ++j) {
-                const int at = dot_pixel(halo + j) ^ 16 * f;
-                const ulonglong2 x0 = quad_at(hs, at), x1 = quad_at(hs, at ^ 16);
-#pragma unroll
-                for (int r = 0; r < kR; ++r)
-                    if (j >= r && j - r < S::kKs) add(r, j - r, x0, x1);
-            }
-        } else {
+        if constexpr (!REGULAR && N == S::kKs) {
 #pragma unroll
             for (int r = 0; r < kR; ++r)
 #pragma unroll
-                for (int m = 0; m < S::kKs; ++m) {
+                for (int m = 0; m < N; ++m) {
                     const int at = dot_pixel(halo + d.s.off[r] + m) ^ 16 * f;
-                    add(r, m, quad_at(hs, at), quad_at(hs, at ^ 16));
+                    const ulonglong2 x0 = quad_at(hs, at), x1 = quad_at(hs, at ^ 16);
+                    add_pair(acc[r][m], fma2(q1[r].y, x1.y, fma2(q1[r].x, x1.x, fma2(q0[r].y, x0.y, mul2(q0[r].x, x0.x)))));
                 }
+        } else
+#pragma unroll
+        for (int j = 0; j < S::kU; ++j) {
+            const int at = dot_pixel(halo + j) ^ 16 * f;
+            const ulonglong2 x0 = quad_at(hs, at), x1 = quad_at(hs, at ^ 16);
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                const int i = REGULAR ? j - r : j;
+                if (i >= 0 && i < N) add_pair(acc[r][i], fma2(q1[r].y, x1.y, fma2(q1[r].x, x1.x, fma2(q0[r].y, x0.y, mul2(q0[r].x, x0.x)))));
+            }
         }
     }
 }
@@ -304,15 +305,19 @@ __device__ __forceinline__ int dot_chunks(const Na2dGeom& g) { return (g.C + kDo
 // Scores of the whole tile, all channel chunks; s[r][m] pixel r of the thread's strip and member m of its window row.  `at`: chunks of
 // earlier dot loops of the kernel, `all`: of all of them.  Chunk i of all lies in stage (all - 1 - i) & 1, and the first two are on
 // their way; next(i) starts what comes into the place of chunk i once nobody reads it (one thread).
-template <typename S, bool PARK, typename F>
+// REGULAR: all strips of the tile are; one way for all of them, since warps hold parts of two strips.  In other tiles a strip reads the
+// columns of each pixel's window by themselves up to window 5, and from 7 on gets the scores of all KS + 3 columns it reaches, for each
+// pixel, to keep those of its windows at the end (dQ of 4 x 8 x 28 x 30 x 64, window 7, 55 -> 49 us, window 11 134 -> 103).
+template <typename S, bool PARK, bool REGULAR, typename F>
 __device__ __forceinline__ void tile_dot(float (&s)[kR][S::kKs], const uint8_t* smem, Loads& loads, const DotItem& d, const Na2dGeom& g,
                                          int at, int all, F&& next) {
-    Sum<S> acc[kR][S::kKs];
+    constexpr bool kAll = !REGULAR && S::kKs >= 7;
+    constexpr int N = kAll ? S::kU : S::kKs;
+    using A = std::conditional_t<kAll, float, Sum<S>>;
+    A acc[kR][N];
 #pragma unroll
-    for (int r = 0; r < kR; ++r)
-#pragma unroll
-        for (int m = 0; m < S::kKs; ++m) acc[r][m] = 0;
-    float4 local[PARK ? S::kKs : 1];
+    for (int i = 0; i < kR * N; ++i) acc[i / N][i % N] = 0;
+    float4 local[PARK ? N : 1];
     float4* parked = local;
     if constexpr (PARK) asm volatile("" : "+l"(parked));    // not in registers: those are needed for the loop
     bool first = true;
@@ -322,26 +327,37 @@ __device__ __forceinline__ void tile_dot(float (&s)[kR][S::kKs], const uint8_t* 
         const int stage = (all - 1 - at - i) & 1;
         loads.wait(stage);
         if (d.active) {
-            // (one way for all strips of a tile: warps hold parts of two, and would go both ways)
-            if (d.all_regular) dot_staged<S, true>(acc, smem + stage * S::kStage, d);
-            else dot_staged<S, false>(acc, smem + stage * S::kStage, d);
+            dot_staged<S, REGULAR>(acc, smem + stage * S::kStage, d);
             if (PARK && park_at((i + 1) * kDotC, g.C)) {
-                park<S>(acc, parked, first);
+                park(acc, parked, first);
                 first = false;
             }
         }
         if (loads.last(stage)) next(at + i);
     }
+    float sum[kR][N];
 #pragma unroll
-    for (int i = 0; i < kR * S::kKs; ++i) s[i / S::kKs][i % S::kKs] = value(acc[i / S::kKs][i % S::kKs]);
+    for (int i = 0; i < kR * N; ++i) sum[i / N][i % N] = value(acc[i / N][i % N]);
     if (PARK && !first) {
 #pragma unroll
-        for (int i = 0; i < kR * S::kKs; i += kR) {
-            const float4 sum = parked[i / kR];
+        for (int i = 0; i < kR * N; i += kR) {
+            const float4 old = parked[i / kR];
 #pragma unroll
-            for (int e = 0; e < kR; ++e) s[(i + e) / S::kKs][(i + e) % S::kKs] += lane_of(sum, e);
+            for (int e = 0; e < kR; ++e) sum[(i + e) / N][(i + e) % N] += lane_of(old, e);
         }
     }
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
+#pragma unroll
+        for (int m = 0; m < S::kKs; ++m) {
+            if constexpr (!kAll) {
+                s[r][m] = sum[r][m];
+            } else {                                       // off[r] is at most r
+                s[r][m] = sum[r][m];
+#pragma unroll
+                for (int o = 1; o <= r; ++o) s[r][m] = d.s.off[r] == o ? sum[r][m + o] : s[r][m];
+            }
+        }
 }
 
 // The thread's weight slots: member m of its window row, for the four pixels of its strip, at [m * kTh].
@@ -375,44 +391,71 @@ __device__ __forceinline__ void add(Channels& acc, const Channels& x) {
 }
 __device__ __forceinline__ float4 channels(const Channels& c) { return make_float4(lo2(c.a), hi2(c.a), lo2(c.b), hi2(c.b)); }
 
-// A halo row meets a row of the strip's pixels: acc[r] += sum over its window there, w member m of it at [m * kTh], x(j) column j of
-// those the strip reaches.  Each such row is summed by itself first: many short sums round less than a long one.
-template <typename S, bool REGULAR, typename X>
-__device__ __forceinline__ void apply_row(Channels (&acc)[kR], const float4* w, const Strip& s, X&& x) {
+// A halo row meets a row of the strip's pixels: acc[r] += sum over its window there, w member m of it at [m * kTh], x the KS + 3 columns
+// that the strip reaches.  Each such row is summed by itself first: many short sums round less than a long one.
+template <typename S>
+__device__ __forceinline__ void apply_band(Channels (&acc)[kR], const float4* w, const ulonglong2 (&x)[S::kU]) {
     Channels t[kR];
 #pragma unroll
     for (int m = 0; m < S::kKs; ++m) {
         const float4 wt = w[m * S::kTh];
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
-            const ulonglong2 v = x(REGULAR ? r + m : s.off[r] + m);
-            if (m == 0) t[r] = scaled(lane_of(wt, r), v);
-            else add_scaled(t[r], lane_of(wt, r), v);
+            if (m == 0) t[r] = scaled(lane_of(wt, r), x[r + m]);
+            else add_scaled(t[r], lane_of(wt, r), x[r + m]);
         }
     }
 #pragma unroll
     for (int r = 0; r < kR; ++r) add(acc[r], t[r]);
 }
+// The same where the windows are shifted, for all rows at once (a row that the halo row does not meet gets nothing).
+template <typename S, int N, typename X>
+__device__ __forceinline__ void apply_shifted(Channels (&acc)[N][kR], const float4* const (&w)[N], const bool (&meets)[N], const Strip& s, X&& x) {
+    Channels t[N][kR];
+#pragma unroll
+    for (int m = 0; m < S::kKs; ++m) {
+        float4 wt[N];
+#pragma unroll
+        for (int p = 0; p < N; ++p) wt[p] = w[p][m * S::kTh];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const ulonglong2 v = x(s.off[r] + m);
+#pragma unroll
+            for (int p = 0; p < N; ++p) {
+                if (m == 0) t[p][r] = scaled(lane_of(wt[p], r), v);
+                else add_scaled(t[p][r], lane_of(wt[p], r), v);
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < N; ++p)
+#pragma unroll
+        for (int r = 0; r < kR; ++r)
+            if (meets[p]) add(acc[p][r], t[p][r]);
+}
 
-// What a thread does in the apply loop: four channels of kRows image rows of a strip.
+// What a thread does in the apply loop: four channels of kRows image rows of a strip, and every kHalves-th of the halo rows that they meet.
 template <typename S>
 struct ApplyItem {
-    int f, row, strip;
+    int f, half, row, strip;
     bool active;
     __device__ __forceinline__ explicit ApplyItem(const Tile& t) {
         f = threadIdx.x % kF;
-        row = threadIdx.x / kF % (S::kTh / S::kRows) * S::kRows;
-        strip = threadIdx.x / (kF * (S::kTh / S::kRows));
+        int it = threadIdx.x / kF;
+        half = it % S::kHalves;
+        it /= S::kHalves;
+        row = it % (S::kTh / S::kRows) * S::kRows;
+        strip = it / (S::kTh / S::kRows);
         active = threadIdx.x < S::kApply && row < t.rows && kR * strip < t.cols;
     }
 };
 
-// out = factor * sum over the window of weight * (what load(i) brings to the halo as chunk i), all chunks; as many as there are buffers
-// are on their way.
-template <typename S, typename F>
+// out = factor * sum over the window of weight * (what load(i) brings to the halo as chunk i), the chunks of channels [ch0, ch_end); as many
+// as there are buffers are on their way.
+template <typename S, int BUFFERS, typename F>
 __device__ __forceinline__ void tile_apply(const Operand& out, const uint8_t* smem, Loads& loads, const float4* w, const ApplyItem<S>& a,
-                                           const float4 (&factor)[S::kRows], const Tile& t, const Na2dGeom& g, int ky0, int kx0, F&& load) {
-    static_assert(S::kApply <= S::kThreads, "an item a thread");
+                                           const float4 (&factor)[S::kRows], const Tile& t, const Na2dGeom& g, int ky0, int kx0, int ch0,
+                                           int ch_end, F&& load) {
     const Strip s = strip_at<S::kKs>(t.x0 + kR * a.strip, g.W);
     int off[S::kRows];                                     // first halo row of each pixel row, from the first one's
     const int hy0 = na2d_ws(g.q_row0 + t.y0 + a.row, g.Hg, S::kKh) - g.kv_row0 - ky0;
@@ -424,15 +467,16 @@ __device__ __forceinline__ void tile_apply(const Operand& out, const uint8_t* sm
     const float4* wr = w + a.strip * S::kKh * S::kKs * S::kTh + a.row;
     float* o = unit<float>(out, t) + (t.y0 + a.row) * out.st.h + (t.x0 + kR * a.strip) * out.st.w + 4 * a.f;
 #pragma unroll 1
-    for (int c0 = 0, i = 0; c0 < g.C; c0 += kChunk, ++i) {
-        loads.wait(2 + halo_buffer<S>(i));
-        const uint8_t* halo = smem + halo_at<S>(i);
+    for (int c0 = ch0, i = 0; c0 < ch_end; c0 += kChunk, ++i) {
+        const int buffer = BUFFERS == 2 ? i & 1 : 0;
+        loads.wait(2 + buffer);
+        const uint8_t* halo = smem + (buffer ? 0 : BUFFERS == 2 ? S::kHaloAt : 0);
         if (a.active) {
             Channels acc[S::kRows][kR];
 #pragma unroll
             for (int e = 0; e < S::kRows * kR; ++e) acc[e / kR][e % kR] = Channels{0, 0};
 #pragma unroll 1
-            for (int h = 0; h < n_rows; ++h) {
+            for (int h = a.half; h < n_rows; h += S::kHalves) {
                 const int at = first + h * S::kHaloW;
                 auto column = [&](int j) { return quad_at(halo, pixel(at + j) ^ 16 * a.f); };
                 if (s.regular) {
@@ -441,30 +485,45 @@ __device__ __forceinline__ void tile_apply(const Operand& out, const uint8_t* sm
                     for (int j = 0; j < S::kU; ++j) x[j] = column(j);
 #pragma unroll
                     for (int p = 0; p < S::kRows; ++p)
-                        if ((unsigned)(h - off[p]) < (unsigned)S::kKh)
-                            apply_row<S, true>(acc[p], wr + (h - off[p]) * (S::kKs * S::kTh) + p, s, [&](int j) { return x[j]; });
+                        if ((unsigned)(h - off[p]) < (unsigned)S::kKh) apply_band<S>(acc[p], wr + (h - off[p]) * (S::kKs * S::kTh) + p, x);
                 } else {
+                    const float4* wp[S::kRows];
+                    bool meets[S::kRows];
 #pragma unroll
-                    for (int p = 0; p < S::kRows; ++p)
-                        if ((unsigned)(h - off[p]) < (unsigned)S::kKh)
-                            apply_row<S, false>(acc[p], wr + (h - off[p]) * (S::kKs * S::kTh) + p, s, column);
+                    for (int p = 0; p < S::kRows; ++p) {
+                        meets[p] = (unsigned)(h - off[p]) < (unsigned)S::kKh;
+                        wp[p] = wr + (meets[p] ? h - off[p] : 0) * (S::kKs * S::kTh) + p;
+                    }
+                    apply_shifted<S>(acc, wp, meets, s, column);
+                }
+            }
+            if constexpr (S::kHalves == 2) {               // each half finishes a row and hands the other one on
+                static_assert(S::kRows == 2, "a row each");
+                const unsigned both = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    const Channels keep = a.half ? acc[1][r] : acc[0][r], give = a.half ? acc[0][r] : acc[1][r];
+                    acc[0][r] = keep;
+                    add(acc[0][r], Channels{__shfl_xor_sync(both, give.a, kF), __shfl_xor_sync(both, give.b, kF)});
                 }
             }
             if (c0 + 4 * a.f < g.C) {
 #pragma unroll
-                for (int p = 0; p < S::kRows; ++p) {
-                    if (a.row + p >= t.rows) break;
+                for (int p = 0; p < S::kRows / S::kHalves; ++p) {
+                    const int row = S::kHalves == 2 ? a.half : p;
+                    if (a.row + row >= t.rows) break;
+                    const float4 fac = S::kHalves == 2 && a.half ? factor[S::kRows - 1] : factor[p];
 #pragma unroll
                     for (int r = 0; r < kR; ++r) {
-                        const float m = lane_of(factor[p], r);
+                        const float m = lane_of(fac, r);
                         const float4 x = channels(acc[p][r]);
                         if (t.x0 + kR * a.strip + r < g.W)
-                            *reinterpret_cast<float4*>(o + p * out.st.h + r * out.st.w + c0) = make_float4(x.x * m, x.y * m, x.z * m, x.w * m);
+                            *reinterpret_cast<float4*>(o + row * out.st.h + r * out.st.w + c0) = make_float4(x.x * m, x.y * m, x.z * m, x.w * m);
                     }
                 }
             }
         }
-        if (loads.last(2 + halo_buffer<S>(i)) && c0 + S::kHaloBuffers * kChunk < g.C) load(i + S::kHaloBuffers);
+        if (loads.last(2 + buffer) && c0 + BUFFERS * kChunk < ch_end) load(i + BUFFERS);
     }
 }
 
@@ -505,10 +564,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const DotItem d = score_item<S>(t, g, ky0, kx0);
     __syncthreads();
     float s[kR][KS];
-    tile_dot<S, PARK>(s, smem, loads, d, g, 0, n, [&](int i) {
+    auto next = [&](int i) {
         if (i + 2 < n) load_qk(i + 2);
         else if (S::kHaloBuffers == 2 ? i + 2 == n : i + 1 == n) load_v(0);
-    });
+    };
+    if (d.all_regular) tile_dot<S, PARK, true>(s, smem, loads, d, g, 0, n, next);
+    else tile_dot<S, PARK, false>(s, smem, loads, d, g, 0, n, next);
     __syncthreads();
 
     // Softmax over the kKh threads that share a strip: row maxima and sums go through shared memory.
@@ -565,7 +626,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         inv[p] = make_float4(1.f / l4.x, 1.f / l4.y, 1.f / l4.z, 1.f / l4.w);
     }
     if (S::kHaloBuffers == 2 && g.C > kChunk && loads.last(3)) load_v(1);               // the sums have been read
-    tile_apply<S>(o, smem, loads, w, a, inv, t, g, ky0, kx0, load_v);
+    tile_apply<S, S::kHaloBuffers>(o, smem, loads, w, a, inv, t, g, ky0, kx0, 0, g.C, load_v);
     loads.drain();
 }
 
@@ -631,7 +692,8 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUt
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
         if (pass > 0 && d.active) store_weights<S>(slots, s);
-        tile_dot<S, PARK>(s, smem, loads, d, g, pass * n, all, next);
+        if (d.all_regular) tile_dot<S, PARK, true>(s, smem, loads, d, g, pass * n, all, next);
+        else tile_dot<S, PARK, false>(s, smem, loads, d, g, pass * n, all, next);
     }
     __syncthreads();
     if (d.active) {
@@ -700,7 +762,7 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUt
         float4 one[S::kRows];
 #pragma unroll
         for (int p = 0; p < S::kRows; ++p) one[p] = make_float4(1.f, 1.f, 1.f, 1.f);
-        tile_apply<S>(d_q, smem, loads, w, ApplyItem<S>(t), one, t, g, ky0, kx0, load_k);
+        tile_apply<S, S::kHaloBuffers>(d_q, smem, loads, w, ApplyItem<S>(t), one, t, g, ky0, kx0, 0, g.C, load_k);
     }
     loads.drain();
 }
@@ -712,17 +774,31 @@ __device__ __forceinline__ long long dense_row(const Tile& t, const Na2dGeom& g,
     return (((long long)t.bn * g.Hq + t.y0 + row) * g.W + t.x0) * (KS * KS);
 }
 
+// Each needs a part of the fused kernels' shared memory, which leaves room for more blocks: the stages and, in their place, the tile's
+// scores; a halo and the weights.
+template <typename S>
+struct PairShape {
+    static constexpr int blocks(int smem, int threads, int registers) {
+        return na2d_tile::kSmemPerSm / (smem + 1024) < 65536 / (threads * registers) ? na2d_tile::kSmemPerSm / (smem + 1024) : 65536 / (threads * registers);
+    }
+    static constexpr int kRow = S::kTw * S::kKs * S::kKs + 1;            // floats of an image row's scores: lanes of eight rows write at once
+    static constexpr int kDotBarriersAt = max_of(2 * S::kStage, whole_kb(S::kTh * kRow * 4)), kDotSmem = kDotBarriersAt + S::kBarriers;
+    static constexpr int kDotBlocks = blocks(kDotSmem, S::kThreads, 128);
+    static constexpr int kApplyThreads = S::kApply;
+    static constexpr int kWeightsAt = S::kHalo, kApplyBarriersAt = kWeightsAt + S::kWeights * 16, kApplySmem = kApplyBarriersAt + S::kBarriers;
+    static constexpr int kApplyBlocks = blocks(kApplySmem, kApplyThreads, 128);
+};
+
 // attn[pixel, member] = x[pixel] . y[member of the pixel's window]; tm_x, tm_y: own pixels and halo, 16 channels.
 template <int KS, bool PARK>
-__global__ void __launch_bounds__(Shape<KS>::kThreads, Shape<KS>::kBlocks)
+__global__ void __launch_bounds__(Shape<KS>::kThreads, PairShape<Shape<KS>>::kDotBlocks)
 window_dot_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y, float* __restrict__ attn,
                   const ErrorState* __restrict__ errors, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS>;
-    constexpr int kRow = S::kTw * KS * KS + 1;             // floats of an image row's weights: lanes of eight rows write at once
-    static_assert(S::kTh * kRow * 4 <= S::kBarriersAt, "the weights fit the shared memory");
+    constexpr int kRow = PairShape<S>::kRow;
     extern __shared__ __align__(1024) uint8_t smem[];
     if (!starts_right(smem, errors)) return;
-    Loads loads(smem + S::kBarriersAt, errors);
+    Loads loads(smem + PairShape<S>::kDotBarriersAt, errors);
     const Tile t = tile_of_block<S>(g, g.Hq);
     int ky0, kx0;
     query_halo<S>(t, g, ky0, kx0);
@@ -738,9 +814,11 @@ window_dot_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     const DotItem d = score_item<S>(t, g, ky0, kx0);
     __syncthreads();
     float s[kR][KS];
-    tile_dot<S, PARK>(s, smem, loads, d, g, 0, n, [&](int i) {
+    auto next = [&](int i) {
         if (i + 2 < n) load(i + 2);
-    });
+    };
+    if (d.all_regular) tile_dot<S, PARK, true>(s, smem, loads, d, g, 0, n, next);
+    else tile_dot<S, PARK, false>(s, smem, loads, d, g, 0, n, next);
     loads.drain();
     __syncthreads();
     float* rows = reinterpret_cast<float*>(smem);
@@ -758,29 +836,26 @@ window_dot_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     }
 }
 
-// out[pixel] = sum over the window of attn[pixel, member] * y[member]; tm_y: halo, 32 channels.
+// out[pixel] = sum over the window of attn[pixel, member] * y[member], `span` channels a block; tm_y: halo, 32 channels.
 template <int KS>
-__global__ void __launch_bounds__(Shape<KS>::kThreads, Shape<KS>::kBlocks)
-window_apply_kernel(const float* __restrict__ attn, const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ Operand out,
+__global__ void __launch_bounds__(PairShape<Shape<KS>>::kApplyThreads, PairShape<Shape<KS>>::kApplyBlocks)
+window_apply_kernel(const float* __restrict__ attn, const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ Operand out, const int span,
                     const ErrorState* __restrict__ errors, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS>;
+    using P = PairShape<S>;
     extern __shared__ __align__(1024) uint8_t smem[];
     if (!starts_right(smem, errors)) return;
-    float* w = reinterpret_cast<float*>(smem + S::kWeightsAt);
-    Loads loads(smem + S::kBarriersAt, errors);
+    float* w = reinterpret_cast<float*>(smem + P::kWeightsAt);
+    Loads loads(smem + P::kApplyBarriersAt, errors);
     const Tile t = tile_of_block<S>(g, g.Hq);
     int ky0, kx0;
     query_halo<S>(t, g, ky0, kx0);
-    auto load = [&](int i) {
-        na2d_ptx::tma_load_5d(smem + halo_at<S>(i), &tm_y, loads.expect(2 + halo_buffer<S>(i), kHaloBytes<S>), i * kChunk, kx0, ky0, t.n, t.b);
-    };
-    if (threadIdx.x == 0) {
-        load(0);
-        if (S::kHaloBuffers == 2 && g.C > kChunk) load(1);
-    }
+    const int ch0 = blockIdx.z * span;
+    auto load = [&](int i) { na2d_ptx::tma_load_5d(smem, &tm_y, loads.expect(2, kHaloBytes<S>), ch0 + i * kChunk, kx0, ky0, t.n, t.b); };
+    if (threadIdx.x == 0) load(0);
     for (int row = 0; row < t.rows; ++row) {
         const float* from = attn + dense_row<KS>(t, g, row);
-        for (int i = threadIdx.x; i < t.cols * kTaps<KS>; i += S::kThreads) {
+        for (int i = threadIdx.x; i < t.cols * kTaps<KS>; i += P::kApplyThreads) {
             const int q = i / kTaps<KS>, tap = i - q * kTaps<KS>;
             w[((q / kR * kTaps<KS> + tap) * S::kTh + row) * kR + q % kR] = __ldg(from + i);
         }
@@ -789,7 +864,7 @@ window_apply_kernel(const float* __restrict__ attn, const __grid_constant__ CUte
     float4 one[S::kRows];
 #pragma unroll
     for (int p = 0; p < S::kRows; ++p) one[p] = make_float4(1.f, 1.f, 1.f, 1.f);
-    tile_apply<S>(out, smem, loads, reinterpret_cast<const float4*>(w), ApplyItem<S>(t), one, t, g, ky0, kx0, load);
+    tile_apply<S, 1>(out, smem, loads, reinterpret_cast<const float4*>(w), ApplyItem<S>(t), one, t, g, ky0, kx0, ch0, min(g.C, ch0 + span), load);
     loads.drain();
 }
 

@@ -32,6 +32,12 @@ inline bool takes(const Na2dGeom& g, std::initializer_list<const na2d_tile::Tens
     return true;
 }
 
+// Whether these kernels pay for an image's width.  Where every tile meets a border they do little less than the tiled ones: forward /
+// dQ of 16 x 8 x 14 x 14 x 64, window 11, 70 -> 72 / 104 -> 106 us, window 13 100 -> 116 / 147 -> 175 (4 x 8 x 28 x 30 x 64 102 -> 103 / 152 -> 163; 4 x 33 x 40 x 32
+// 22.5 -> 20.5 / 30 -> 29), key sums at window 7 74 -> 77 (17 columns 49 -> 48).
+inline bool query_side_pays(const Na2dGeom& g) { return g.W >= (g.ks == 13 ? 36 : g.ks == 11 ? 16 : 0); }
+inline bool key_side_pays(const Na2dGeom& g) { return g.ks != 7 || g.W >= 16; }
+
 // Query tiles a launch covers, and where it puts their weights: na2d_tile::Band.
 struct Rows {
     int unit0, row0, rows, ring;

@@ -20,6 +20,10 @@
 //          do its weights take a slot for every pair of a query strip and a key.
 // Measured on one B200, both sums of 32 x 128 x 64 pixels (half of the tiles at a border), 128 channels, edges / strips, us: window 3 165 / 207, 5
 // 248 / 334, 7 462 / 466, 9 832 / 794, 13 2214 / 1713.
+//
+// What bounds it: latencies (eight to sixteen warps an SM issue in half of the cycles) and the FMA pipe.  Against the tiled key sums,
+// both sums, us: 4 x 8 x 28 x 30 x 64, window 5 49 -> 33, 9 105 -> 92, 13 210 -> 187; 2 x 200 x 260 x 64, window 5 82 -> 58, 9 165 -> 139, 13 363 -> 290;
+// with the dense weights of the pair, 4 x 4 x 64 x 64 x 128, window 5, each 74 -> 62.
 #pragma once
 
 #include "na2d_box.cuh"
@@ -43,15 +47,22 @@ struct KeyShape {
     static constexpr int kRowSlots = S::kTh * S::kStrips * S::kU;
     static constexpr int kSlots = kEdges ? KS * (kRowSlots + kRowEdge) : max_of(KS * kRowSlots, S::kTh * S::kStrips * kMaxStrips * kR);
     // Boxes: that of a tile away from the borders, and a wide one for those that meet more columns: edge pairs to the right
-    // of the band, or whole query strips.  As many rows of it as fit the same room, and one more than kSpan at least.
+    // of the band, or whole query strips.  As many rows of that as the room allows that is left beside the blocks an SM holds: with one
+    // or two query rows at a time, each with its loads and its gather, a border tile took up to 17 turns at window 9.
     static constexpr int kMaxCols = (max_of((KS - 1) / S::kTw * S::kTw, kLeft * kR) + S::kTw + KS - 1 + kR - 1) / kR * kR;
     static constexpr int kWideW = (kEdges ? kHalf + S::kTw + KS - 1 : kMaxCols) | 1;
-    static constexpr int kFit = S::kHaloH * S::kBoxW / kWideW, kWideH = max_of(kSpan + 1, kFit < S::kHaloH ? kFit : S::kHaloH);
-    static constexpr int kWeightsAt = whole_kb(max_of(S::kHaloH * S::kBoxW, kWideH * kWideW) * kPixel);
-    static constexpr int kBarriersAt = kWeightsAt + kSlots * 16, kSmem = kBarriersAt + S::kBarriers;
-    static constexpr int kBlocksSmem = na2d_tile::kSmemPerSm / (kSmem + 1024);
-    static constexpr int kBlocks = kBlocksSmem * kThreads > 512 ? 512 / kThreads : kBlocksSmem;
-    static_assert(S::kHaloH > kSpan && kWideH > kSpan && kBlocks >= 1, "a query row of each key row fits");
+    // Tables of the gather: where the group's rows of weights lie, for each key row, and the slots in a row.
+    static constexpr int kMaxSlots = S::kStrips * max_of(S::kU, kEdges ? 0 : kMaxStrips * kR);
+    static constexpr int kBesides = kSlots * 16 + KS * S::kTh * 8 + kMaxSlots * 8 + S::kBarriers + 1024;
+    static constexpr int kBox = S::kHaloH * S::kBoxW * kPixel;
+    static constexpr int kFitting = na2d_tile::kSmemPerSm / (whole_kb(kBox) + kBesides);
+    static constexpr int kBlocks = kFitting * kThreads > 512 ? 512 / kThreads : kFitting;
+    static constexpr int kRoom = (na2d_tile::kSmemPerSm / kBlocks - kBesides) / 1024 * 1024, kFit = kRoom / (kWideW * kPixel);
+    static constexpr int kWideH = kFit < S::kHaloH ? kFit : S::kHaloH;
+    static constexpr int kWeightsAt = whole_kb(max_of(kBox, kWideH * kWideW * kPixel));
+    static constexpr int kRowsAt = kWeightsAt + kSlots * 16, kSlotsAt = kRowsAt + KS * S::kTh * 8;
+    static constexpr int kBarriersAt = kSlotsAt + kMaxSlots * 8, kSmem = kBarriersAt + S::kBarriers;
+    static_assert(S::kHaloH > kSpan && kWideH > kSpan && kBlocks * (kSmem + 1024) <= na2d_tile::kSmemPerSm, "a query row of each key row fits");
     static_assert(!kEdges || S::kTw >= KS, "keys below KS lie in a row's first tile");
 };
 
@@ -77,12 +88,13 @@ struct KeyOut {
     Operand out;
 };
 
-// tm_x0, tm_x1: boxes of the two jobs' x, 32 channels, tm_w0, tm_w1: wide ones.
+// tm_x0, tm_x1: boxes of the two jobs' x, 32 channels, tm_w0, tm_w1: wide ones.  A block sums `span` channels (whole chunks), blockIdx.z
+// the how manieth.
 template <bool TILED, int KS>
 __global__ void __launch_bounds__(KeyShape<Shape<KS>>::kThreads, KeyShape<Shape<KS>>::kBlocks)
 key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_x1,
                const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ KeyOut first, const __grid_constant__ KeyOut second,
-               const ErrorState* __restrict__ errors, const __grid_constant__ Band band, const __grid_constant__ Na2dGeom g) {
+               const int span, const ErrorState* __restrict__ errors, const __grid_constant__ Band band, const __grid_constant__ Na2dGeom g) {
     using S = Shape<KS>;
     using K = KeyShape<S>;
     constexpr int kHalf = KS / 2, kGroups = S::kTh / K::kRows;
@@ -111,7 +123,8 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
             else na2d_ptx::tma_load_5d(smem, &tm_w1, bar, c0, qx0, row, t.n, t.b);
         }
     };
-    if (threadIdx.x == 0) load(0, qy0);
+    const int ch0 = blockIdx.z * span, ch_end = min(g.C, ch0 + span);
+    if (threadIdx.x == 0) load(ch0, qy0);
     const KeyOut& job = blockIdx.y == 0 ? first : second;
     const int row_span = na2d_bws(t.y0 + t.rows - 1, KS) - qy0;          // how far the keys' first query rows lie apart
     int nu = 0, nj = S::kU;                                // query rows of a key row, weight slots of a strip, at most
@@ -124,7 +137,7 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
         for (int x = 0; x < S::kTw; x += kR)
             if (x < t.cols) nj = max(nj, ((na2d_bwe(min(t.x0 + x + kR, W) - 1, W, KS) - 1) / kR - na2d_bws(t.x0 + x, KS) / kR + 1) * kR);
     }
-    const int group = min(nu, min(K::kEdges || inner ? KS : K::kSlots / (S::kTh * S::kStrips * nj), box_h - row_span));
+    const int group = min(nu, min(min(KS, K::kSlots / (S::kTh * S::kStrips * nj)), box_h - row_span));
 
     const int f = threadIdx.x % kF, row0 = threadIdx.x / kF % kGroups * K::kRows, strip = threadIdx.x / (kF * kGroups);
     const bool active = row0 < t.rows && kR * strip < t.cols;
@@ -132,13 +145,15 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
     // (strips) query columns of each key: the first one from the first query strip's, and how many
     const bool regular = K::kEdges || (c0 >= KS && c0 + kR <= W - KS);
     const int strip0 = na2d_bws(min(c0, W - 1), KS) / kR;
-    int lo[kR], n_of[kR], strips = 0;
+    int lo[kR], n_of[kR], strips = 0, lo_all = 0, hi_all = 1 << 20;      // every key meets the queries lo_all to hi_all
     if constexpr (!K::kEdges) {
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
             lo[r] = c0 + r < W ? na2d_bws(c0 + r, KS) - strip0 * kR : 0;
             const int hi = c0 + r < W ? na2d_bwe(c0 + r, W, KS) - strip0 * kR : 0;
             n_of[r] = hi - lo[r];
+            lo_all = max(lo_all, lo[r]);
+            hi_all = min(hi_all, hi);
             strips = max(strips, (hi + kR - 1) / kR);
         }
     }
@@ -177,88 +192,107 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
         if constexpr (TILED) return __ldg(reinterpret_cast<const float*>(slot_at(row, q / kR, key - na2d_ws(q / kR * kR, W, KS))) + q % kR);
         else return __ldg(row + (long long)q * kTaps<KS> + key - na2d_ws(q, W, KS));
     };
-    // The weights of query strip sq for key column `key` of the image, to shared memory; zeros where a query is outside the image.  PAIRS:
-    // nothing is written, and nothing will be read, where none of the strip's windows holds the key.
-    auto fetch = [&](float4* to, const float* row, int sq, int key, bool pairs) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (sq >= 0 && kR * sq < W) {
-            if constexpr (TILED) {
-                const int slot = key - na2d_ws(kR * sq, W, KS);
-                const bool in = (unsigned)slot < (unsigned)S::kU;
-                if (pairs) {
-                    if (in) copy16(to, slot_at(row, sq, slot), true);
-                    return;
-                }
-                if (in) v = __ldg(slot_at(row, sq, slot));
-                if (kR * sq + 1 >= W) v.y = 0.f;           // (not written where the query is outside the image)
-                if (kR * sq + 2 >= W) v.z = 0.f;
-                if (kR * sq + 3 >= W) v.w = 0.f;
-            } else {
-                float e[kR];
-#pragma unroll
-                for (int c = 0; c < kR; ++c) {
-                    const int member = kR * sq + c < W ? key - na2d_ws(kR * sq + c, W, KS) : -1;
-                    e[c] = (unsigned)member < (unsigned)KS ? weight(row, kR * sq + c, key) : 0.f;
-                }
-                v = make_float4(e[0], e[1], e[2], e[3]);
-            }
+    // (dense weights) The slots of the four keys of strip st in query row u, one lane a key and key row: the four keys' weights of a query
+    // lie side by side.  As in fetch, zeros where the band leaves the image, and nothing where a pair has no weight.
+    auto fetch_strip = [&](int st, int u, int gn, const float* row, int ly, int r) {
+        const bool in_band = K::kEdges || inner;
+        const int first = t.x0 + kR * st, key = first + r;
+        if (key >= W) return;
+        const int sq0 = in_band ? first / kR : na2d_bws(first, KS) / kR;               // slots count from this query strip
+        const int q0 = in_band ? first - kHalf : kR * sq0;
+        const int n = in_band ? S::kU : na2d_bwe(min(first + kR, W) - 1, W, KS) - q0;
+        const uint32_t to = na2d_ptx::smem_u32(w + ((st * gn + u) * nj + r) * S::kTh + ly);
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) {
+            const int q = q0 + i, member = key - na2d_ws(q, W, KS);
+            const bool pair = in_band ? (unsigned)(i - r) < (unsigned)KS : (unsigned)member < (unsigned)KS, in = q >= 0 && q < W;
+            const int slot = in_band ? kHalf - kR * ((q >> 2) - sq0) : kR * ((q >> 2) - sq0);
+            const float* from = in ? row + (long long)q * kTaps<KS> + member : row;
+            if (pair)                                      // (a copy of no bytes leaves zeros)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + (slot * (S::kTh * kR) + (q & 3)) * 4), "l"(from), "r"(in ? 4 : 0) : "memory");
         }
-        *to = v;
     };
-    // The group's weights: slots [strip][query row][slot][key row], a thread keeps its slot and key row and goes over the rest (eight key
-    // rows of a slot lie side by side, as their query rows do in a query tile's weights); then edge pairs [query row][border][pair][key row].
+    // The group's weights: slots [strip][query row][slot][key row] (eight key rows of a slot lie side by side, as their query rows do in a
+    // query tile's weights); then edge pairs [query row][border][pair][key row].  Places are worked out once, into tables:
+    // worked out for each copy they took a third of the kernel's instructions at windows 9 to 13.
+    long long* row_table = reinterpret_cast<long long*>(smem + K::kRowsAt);            // [query row][key row]: from attn, -1 for none
+    long long* slot_table = reinterpret_cast<long long*>(smem + K::kSlotsAt);          // [strip][slot]: 8 * (float4 from the row) + its queries in the image
+    const int ly = threadIdx.x % S::kTh, line = threadIdx.x / S::kTh;
+    constexpr int kLines = K::kThreads / S::kTh;
+    auto find_slots = [&] {
+        for (int i = threadIdx.x; TILED && i < S::kStrips * nj; i += K::kThreads) {
+            const int st = i / nj, j = i - st * nj, first = t.x0 + kR * st;
+            int key, sq;
+            if (K::kEdges || inner) {
+                const int d = (j + 4 * KS - kHalf) / kR - KS;            // floor((j - kHalf) / 4): the query strip lies d before the key's
+                key = first + j - kHalf - kR * d;
+                sq = first / kR - d;
+            } else {
+                key = first + j % kR;
+                sq = na2d_bws(min(first, W - 1), KS) / kR + j / kR;
+            }
+            const int slot = key < W && sq >= 0 && kR * sq < W ? key - na2d_ws(kR * sq, W, KS) : -1;
+            slot_table[i] = (unsigned)slot < (unsigned)S::kU ? (slot_at(attn, sq, slot) - reinterpret_cast<const float4*>(attn)) * 8 + min(kR, W - kR * sq) : 0;
+        }
+    };
     auto gather = [&](int g0, int gn) {
-        constexpr int kLines = K::kThreads / S::kTh, kPar = kLines / S::kU;            // query rows at a time
-        static_assert(kPar > 0, "a line a slot");
-        const int ly = threadIdx.x % S::kTh, y = t.y0 + ly, line = threadIdx.x / S::kTh;
-        const int first_row = na2d_bws(min(y, H - 1), KS) + g0;
-        const int rows_here = ly < t.rows ? min(gn, na2d_bwe(y, H, KS) - first_row) : 0;
-        if (K::kEdges || inner) {
-            const int j = line % S::kU, d = (j + 4 * KS - kHalf) / kR - KS;            // floor((j - kHalf) / 4): the query strip lies d before the key's
-            const int key0 = t.x0 + j - kHalf - kR * d, sq0 = t.x0 / kR - d;
-            for (int u = line / S::kU; u < rows_here; u += kPar) {
-                if (line >= kPar * S::kU) break;
-                const float* row = row_at(first_row + u, y);
-#pragma unroll (TILED ? S::kStrips : 1)
-                for (int st = 0; st < S::kStrips; ++st) {
-                    float4* to = w + ((st * gn + u) * S::kU + j) * S::kTh + ly;
-                    if (TILED && inner) copy16(to, slot_at(row, sq0 + st, j), true);
-                    else if (key0 + kR * st < W) fetch(to, row, sq0 + st, key0 + kR * st, false);
+        for (int i = threadIdx.x; i < gn * S::kTh; i += K::kThreads) {
+            const int y = t.y0 + i % S::kTh, qy = na2d_bws(min(y, H - 1), KS) + g0 + i / S::kTh;
+            row_table[i] = y < t.y0 + t.rows && qy < na2d_bwe(y, H, KS) ? row_at(qy, y) - attn : -1;
+        }
+        __syncthreads();
+        if constexpr (TILED) {
+            for (int i = line; i < S::kStrips * nj; i += kLines) {
+                const long long place = slot_table[i];
+                const float* from = attn + (place >> 3) * kR;
+                const int queries = (int)place & 7, st = i / nj;
+                float4* to = w + (st * gn * nj + i - st * nj) * S::kTh + ly;
+                if (!K::kEdges && queries == 0) continue;  // (a pair without weights is not read)
+#pragma unroll 4
+                for (int u = 0; u < gn; ++u) {
+                    const long long row = row_table[u * S::kTh + ly];
+                    if (row < 0) break;
+                    if (!K::kEdges || queries == kR) {
+                        copy16(to + u * nj * S::kTh, from + row, true);
+                    } else {                               // zeros where a query is outside the image: nothing was written there
+                        float4 v = queries > 0 ? __ldg(reinterpret_cast<const float4*>(from + row)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (queries < 2) v.y = 0.f;
+                        if (queries < 3) v.z = 0.f;
+                        v.w = 0.f;
+                        to[u * nj * S::kTh] = v;
+                    }
                 }
             }
         } else {
-            for (int i = line; i < gn * nj; i += kLines) {
-                const int u = i / nj, j = i - u * nj;
-                if (u >= rows_here) break;
-                const float* row = row_at(first_row + u, y);
-#pragma unroll (TILED ? S::kStrips : 1)
-                for (int st = 0; st < S::kStrips; ++st) {
-                    const int key = t.x0 + kR * st + j % kR;
-                    if (key < W) fetch(w + ((st * gn + u) * nj + j) * S::kTh + ly, row, na2d_bws(t.x0 + kR * st, KS) / kR + j / kR, key, true);
-                }
+            constexpr int kPer = kLines / kR;
+            for (int i = line / kR; i < gn * S::kStrips; i += kPer) {
+                const long long row = row_table[i / S::kStrips * S::kTh + ly];
+                if (row >= 0) fetch_strip(i % S::kStrips, i / S::kStrips, gn, attn + row, ly, line % kR);
             }
         }
         if (!K::kEdges || !(left || right)) return;
         float* edge = reinterpret_cast<float*>(w + gn * K::kRowSlots);
-        for (int i = line; i < rows_here * (2 * K::kPairs); i += kLines) {
+        for (int i = line; i < gn * (2 * K::kPairs); i += kLines) {
             const int u = i / (2 * K::kPairs), border = i % (2 * K::kPairs) / K::kPairs, pair = i % K::kPairs;
             int k = 0;
             while ((k + 1) * (k + 2) / 2 <= pair) ++k;
             const int from = kHalf + 1 + k, q = pair - k * (k + 1) / 2, key = border ? W - 1 - from : from;
-            if (key < t.x0 || key >= t.x0 + t.cols) continue;
-            edge[i * S::kTh + ly] = weight(row_at(first_row + u, y), border ? W - 1 - q : q, key);
+            const long long row = row_table[u * S::kTh + ly];
+            if (key < t.x0 || key >= t.x0 + t.cols || row < 0) continue;
+            edge[i * S::kTh + ly] = weight(attn + row, border ? W - 1 - q : q, key);
         }
     };
 
+    find_slots();
     __syncthreads();                                       // the barriers are set up
-    for (int ch = 0; ch < g.C; ch += kChunk) {
+    for (int ch = ch0; ch < ch_end; ch += kChunk) {
         Channels acc[K::kRows][kR];
 #pragma unroll
         for (int i = 0; i < K::kRows * kR; ++i) acc[i / kR][i % kR] = Channels{0, 0};
         for (int g0 = 0; g0 < nu; g0 += group) {
             const int gn = min(group, nu - g0);
-            if (ch == 0 || group < nu) {
-                gather(g0, gn);
+            if (ch == ch0 || group < nu) {
+                gather(g0, gn);                            // (waits for the slots' table, too)
                 copies_done();
                 __syncthreads();
             }
@@ -294,13 +328,18 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
                                 const int u = h - (u0[p] - u0[0]);
                                 if ((unsigned)u >= (unsigned)n[p]) continue;
                                 const float4* wr = ws + (u * nj + kR * m) * S::kTh + p;
+                                auto add = [&](auto all) {
 #pragma unroll
-                                for (int r = 0; r < kR; ++r) {
-                                    const float4 wt = wr[r * S::kTh];
+                                    for (int r = 0; r < kR; ++r) {
+                                        const float4 wt = wr[r * S::kTh];
 #pragma unroll
-                                    for (int c = 0; c < kR; ++c)
-                                        if ((unsigned)(kR * m + c - lo[r]) < (unsigned)n_of[r]) add_scaled(acc[p][r], lane_of(wt, c), x[c]);
-                                }
+                                        for (int c = 0; c < kR; ++c)
+                                            if (decltype(all)::value || (unsigned)(kR * m + c - lo[r]) < (unsigned)n_of[r])
+                                                add_scaled(acc[p][r], lane_of(wt, c), x[c]);
+                                    }
+                                };
+                                if (kR * m >= lo_all && kR * m + kR <= hi_all) add(std::true_type{});
+                                else add(std::false_type{});
                             }
                         }
                     }
@@ -331,7 +370,7 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
                 }
             }
             const bool more = g0 + group < nu;
-            if (more || ch + kChunk < g.C) {
+            if (more || ch + kChunk < ch_end) {
                 __syncthreads();
                 if (threadIdx.x == 0) load(more ? ch : ch + kChunk, more ? qy0 + g0 + group : qy0);
             }
