@@ -366,11 +366,33 @@ int after_tile(int rc, int launches) {
 
 na2d_tc::TensorArg targ(const Tensor& t) { return na2d_tc::TensorArg{t.ptr, t.st}; }
 
+// Whether the kernels of a tensor-core call are launched to overlap the end of the kernel before them.  Blocks that wait hold SMs, so not
+// for calls that leave some to other streams' kernels (a margin, a band of rows beside its exchange).  And up to kOverlapPixels alone, from
+// window 7 on: a launch hides about 2 us, but kernels of some rounds of tiles last up to 4 us longer when their blocks start as SMs fall
+// free (their places on the chip change, so L2's far half is the likely reason).  A step, one B200, bf16, cold L2, us without and with:
+//   pixels            8 K - 64 K    125 K - 131 K   200 K         262 K - 280 K   520 K
+//   28 x 28 x 64, 13  166.9 157.7   287.7 276.5     398.3 385.0   525.2 510.1     986.1 976.9
+//   100^2 x 64, 9     109.6 102.3   152.6 145.4     224.3 221.2   298.0 294.9     513.0 511.9
+//   56 x 56 x 32, 7   74.8 67.6     117.5 110.5     164.9 161.8   203.6 196.7     369.7 366.7
+//   48 x 48 x 128, 13 171.0 165.9   281.6 278.5     414.9 414.7   510.9 506.0     951.4 950.2
+// Replayed from a graph launches lie closer, and the line is at half: 100^2 x 64, window 9, L2 warm 92.4 90.4, 132.1 131.8, 202.9 209.1.
+// Window 5 as a graph loses from 64 K pixels on (64 x 64 x 128: 72.2 82.5, 122.3 136.8), and 1024^2 x 128, window 13, 17.3 17.6 ms.
+constexpr long long kOverlapPixels = 1 << 18;
+bool overlaps(const Problem& p) {
+    const Na2dGeom& g = p.g;
+    if (g.ks < 7 || p.sm_margin != 0 || g.Hq != g.Hg || g.Hkv != g.Hg) return false;
+    const long long pixels = (long long)g.BN * g.Hg * g.W;
+    if (pixels > kOverlapPixels) return false;
+    if (pixels <= kOverlapPixels / 2) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(p.st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+}
+
 int launch_ctx(const Problem& p, int* launched, na2d_tc::LaunchCtx* lc) {
     Errors err;
     int rc = error_state(p.device, &err);
     if (rc != NA2D_OK) return rc;
-    *lc = na2d_tc::LaunchCtx{p.g, p.dtype, p.B, p.device, p.st, err.device, launched, p.dkdv_f32, p.sm_margin};
+    *lc = na2d_tc::LaunchCtx{p.g, p.dtype, p.B, p.device, p.st, err.device, launched, p.dkdv_f32, p.sm_margin, overlaps(p)};
     return NA2D_OK;
 }
 
@@ -410,22 +432,23 @@ int run_forward(const Problem& p) {
 // The dO . o estimate of the row deltas, into p.delta (tensor path: head dim 32, 64 or 128, rows on
 // 16-byte boundaries).
 template <typename T, int LPP>
-int launch_delta_as(const Problem& p) {
+int launch_delta_as(const Problem& p, bool overlap) {
     const Na2dGeom& g = p.g;
     const long long hw = (long long)g.Hq * g.W;
     const long long per_image = (hw + na2d_delta::pixels_per_block<LPP>() - 1) / na2d_delta::pixels_per_block<LPP>();
     if (hw > 0x7fffffffLL || per_image * g.BN > 0x7fffffffLL) return NA2D_ERR_TOO_LARGE;
-    na2d_delta::delta_kernel<T, LPP><<<(unsigned)(per_image * g.BN), na2d_delta::kThreads, 0, p.st>>>(
-        (const T*)p.d_o.ptr, (const T*)p.o.ptr, p.delta, p.d_o.st, p.o.st, g, (unsigned)per_image);
-    return after_launch();
+    NA2D_CUDA(na2d_launch::launch(overlap, na2d_delta::delta_kernel<T, LPP>, (unsigned)(per_image * g.BN), na2d_delta::kThreads, 0, p.st,
+                                  (const T*)p.d_o.ptr, (const T*)p.o.ptr, p.delta, p.d_o.st, p.o.st, g, (unsigned)per_image));
+    g_launches.fetch_add(1);
+    return NA2D_OK;
 }
 
-int launch_delta(const Problem& p) {
+int launch_delta(const Problem& p, bool overlap) {
     const bool bf = p.dtype == NA2D_BF16;
     switch (p.g.C) {
-        case 32: return bf ? launch_delta_as<__nv_bfloat16, 4>(p) : launch_delta_as<__half, 4>(p);
-        case 64: return bf ? launch_delta_as<__nv_bfloat16, 8>(p) : launch_delta_as<__half, 8>(p);
-        case 128: return bf ? launch_delta_as<__nv_bfloat16, 16>(p) : launch_delta_as<__half, 16>(p);
+        case 32: return bf ? launch_delta_as<__nv_bfloat16, 4>(p, overlap) : launch_delta_as<__half, 4>(p, overlap);
+        case 64: return bf ? launch_delta_as<__nv_bfloat16, 8>(p, overlap) : launch_delta_as<__half, 8>(p, overlap);
+        case 128: return bf ? launch_delta_as<__nv_bfloat16, 16>(p, overlap) : launch_delta_as<__half, 16>(p, overlap);
         default: return NA2D_ERR_UNSUPPORTED;
     }
 }
@@ -442,7 +465,7 @@ int run_backward_dq(const Problem& p) {
         // exact deltas.
         bool have_estimate = false;
         if (g.ks >= 7 && p.o.ptr && p.d_q.ptr) {
-            rc = launch_delta(p);
+            rc = launch_delta(p, lc.overlap);
             if (rc != NA2D_OK) return rc;
             have_estimate = true;
         }

@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 
 #include "na2d_index.cuh"
+#include "na2d_ptx.cuh"
 
 namespace na2d_delta {
 
@@ -50,6 +51,8 @@ template <typename T, int LPP>
 __global__ void __launch_bounds__(kThreads)
 delta_kernel(const T* __restrict__ d_o, const T* __restrict__ o, float* __restrict__ delta, const Na2dStride s_do,
              const Na2dStride s_o, const Na2dGeom g, const unsigned blocks_per_image) {
+    na2d_ptx::after_previous_grid();
+    na2d_ptx::next_grid_may_start();
     const unsigned hw = (unsigned)g.Hq * (unsigned)g.W;
     const unsigned bn = blockIdx.x / blocks_per_image;
     const unsigned pix = (blockIdx.x - bn * blocks_per_image) * pixels_per_block<LPP>() + threadIdx.x / LPP;

@@ -73,6 +73,13 @@ __device__ __forceinline__ void wait_state_init(WaitState* st, const ErrorState*
     st->error_bytes = errors->error_bytes;
 }
 
+// For kernels launched with na2d_launch::launch.  after_previous_grid: waits until the kernel before this one in the stream has ended and
+// its writes are visible; before the first access to global memory and before TMEM is taken, which that kernel's blocks may still have to
+// take.  next_grid_may_start: lets the blocks of the kernel behind start once every block of this one has come here; after TMEM is taken,
+// since those blocks may take it before they wait.
+__device__ __forceinline__ void after_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

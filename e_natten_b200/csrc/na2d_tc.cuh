@@ -28,6 +28,7 @@
 
 #include "../../include/na2d.h"
 #include "na2d_index.cuh"
+#include "na2d_launch.h"
 #include "na2d_ptx.cuh"
 
 namespace na2d_tc {
@@ -455,6 +456,7 @@ struct LaunchCtx {
     int* launched;
     bool dkdv_f32;         // the dK/dV kernel writes fp32 (partial sums of a row band)
     int sm_margin;         // SMs to leave free for a kernel that runs beside this one
+    bool overlap;          // blocks may start before the kernel before this one has ended
 };
 
 // CTAs of a persistent launch over `tiles` tiles.

@@ -164,11 +164,6 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         tma_prefetch_desc(&tm_dk);
         tma_prefetch_desc(&tm_dv);
     }
-    if (warp == 0) {
-        __syncwarp();
-        tmem_alloc(tmem_slot, 512);
-        tmem_relinquish();
-    }
     // Rows [NK, NKP) of every query / dO chunk buffer are contraction rows of the output MMAs that
     // TMA never writes: zero them once.
     if constexpr (C::NKP > C::NK) {
@@ -181,9 +176,16 @@ dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CU
         }
         fence_proxy_async();
     }
+    after_previous_grid();
+    if (warp == 0) {
+        __syncwarp();
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    next_grid_may_start();
     const uint32_t tmem_base = *tmem_slot;
 
     // Geometry of my i-th tile: key tile origin and the query box it is seen from.
@@ -656,10 +658,11 @@ int launch_dkdv_as(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k, 
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
     const int grid = persistent_grid(lc, tiles);
-    kern<<<grid, 512, C::SMEM, lc.st>>>(tk, tv, tq, tg, tdk, tdv, lse, delta, lc.dkdv_f32 ? 1 : 0, lc.errors, g,
-                                        tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
-    return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
+    return na2d_launch::launch(lc.overlap, kern, grid, 512, C::SMEM, lc.st,
+                               tk, tv, tq, tg, tdk, tdv, lse, delta, lc.dkdv_f32 ? 1 : 0, lc.errors, g, tiles_r, tiles_c, (int)tiles) == cudaSuccess
+               ? NA2D_OK
+               : NA2D_ERR_CUDA;
 }
 
 // What the chunks of one unit cost in one of the forms: each `per_chunk`, and `per_block` for an 8-query block of its busiest warp.

@@ -109,11 +109,6 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         tma_prefetch_desc(&tm_v);
         tma_prefetch_desc(&tm_o);
     }
-    if (warp == 0) {
-        __syncwarp();
-        tmem_alloc(tmem_slot, 512);
-        tmem_relinquish();
-    }
     // V rows [NK, NKP) of every stage are contraction rows of P V that TMA never writes.
     if constexpr (C::NKP > C::NK) {
         constexpr int pad16 = (C::NKP - C::NK) * C::ROWB / 16;
@@ -124,9 +119,16 @@ fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         }
         fence_proxy_async();
     }
+    after_previous_grid();
+    if (warp == 0) {
+        __syncwarp();
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    next_grid_may_start();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 8 || warp == 10) {
@@ -478,9 +480,11 @@ int launch_forward2(const LaunchCtx& lc, const TensorArg& q, const TensorArg& k,
     auto kern = fwd2_kernel<DT, D, KS>;
     static std::atomic<unsigned long long> opted{0};
     if (opt_in_smem(kern, C::SMEM, lc.device, opted) != cudaSuccess) return NA2D_ERR_CUDA;
-    kern<<<persistent_grid(lc, tiles), 512, C::SMEM, lc.st>>>(tq, tk, tv, to, lse, lc.errors, g, tiles_r, tiles_c, (int)tiles);
     *lc.launched += 1;
-    return cudaGetLastError() == cudaSuccess ? NA2D_OK : NA2D_ERR_CUDA;
+    return na2d_launch::launch(lc.overlap, kern, persistent_grid(lc, tiles), 512, C::SMEM, lc.st,
+                               tq, tk, tv, to, lse, lc.errors, g, tiles_r, tiles_c, (int)tiles) == cudaSuccess
+               ? NA2D_OK
+               : NA2D_ERR_CUDA;
 }
 
 }  // namespace na2d_tc
