@@ -15,8 +15,8 @@
 // bounds below are for the shorter rows; 16-bit rows spill up to 130 bytes a thread under them at window 13).
 // The tiled kernels (na2d_tile.cuh) stage 32 channels at a time as fp32 with two barriers each, and repeat a strip's
 // softmax on all of its lanes.  Measured against those on one B200: 4 x 8 x 4096 x 64, window 13,
-// bf16: forward 70 -> 31 us, both halves of the backward 195 -> 86; 4 x 4 x 32768 x 128, window 7, bf16: 393 -> 158, 859 -> 347;
-// 4 x 8 x 4096 x 32, window 13, fp32: 33 -> 25, 101 -> 66.
+// bf16: forward 70 -> 29 us, both halves of the backward 195 -> 84; 4 x 4 x 32768 x 128, window 7, bf16: 393 -> 153, 859 -> 337;
+// 4 x 8 x 4096 x 32, window 13, fp32: 33 -> 23, 101 -> 64.
 //
 // Windows are clamped at the borders; a strip away from them ("regular") takes loops whose band is known at compile time, any other
 // takes loops that test each pair.  Pairs outside a window never enter a sum.
@@ -111,13 +111,30 @@ __device__ __forceinline__ T* sequence(const Operand& o, const Place& p) {
     return static_cast<T*>(o.ptr) + p.b * o.st.b + p.n * o.st.n;
 }
 
-// Copies rows [first, first + rows) of a sequence, all of them inside it, to shared memory.
-template <typename T>
-__device__ __forceinline__ void copy_rows(uint4* dst, const T* src, const Na2dStride& st, int first, int rows, int pieces, int pitch) {
+// Copies rows [first, first + rows) of N sequences, all of them inside, to shared memory.  A thread's next piece lies kThreads pieces on; it
+// steps there by rows and pieces, so that it divides once: with a division for each piece copying was a tenth of the forward at window 3
+// (4 x 8 x 4096 x 64, bf16, window 3 / 13: forward 16.4 / 30.8 -> 15.1 / 28.9 us, dQ alone 21.8 / 45.4 -> 20.5 / 43.3).
+template <typename T, int N>
+__device__ __forceinline__ void copy_rows(uint4* const (&dst)[N], const T* const (&src)[N], const Na2dStride* const (&st)[N], int first, int rows,
+                                          int pieces, int pitch) {
     constexpr int kN = 16 / sizeof(T);
-    for (int i = threadIdx.x; i < rows * pieces; i += kThreads) {
-        const int row = i / pieces, piece = i - row * pieces;
-        na2d_tile::copy16(reinterpret_cast<float4*>(dst) + row * pitch + piece, src + (long long)(first + row) * st.w + piece * kN, true);
+    const int down = kThreads / pieces, across = kThreads - down * pieces;
+    int row = (int)threadIdx.x / pieces, piece = (int)threadIdx.x - row * pieces, to = row * pitch + piece;
+    const T* from[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) from[i] = src[i] + (long long)(first + row) * st[i]->w + piece * kN;
+    while (row < rows) {
+        row += down;
+        piece += across;
+        const bool wrap = piece >= pieces;
+        if (wrap) piece -= pieces, ++row;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            na2d_tile::copy16(reinterpret_cast<float4*>(dst[i]) + to, from[i], true);
+            from[i] += (long long)down * st[i]->w + across * kN;
+            if (wrap) from[i] += st[i]->w - pieces * kN;
+        }
+        to += down * pitch + across + (wrap ? pitch - pieces : 0);
     }
 }
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -225,9 +242,9 @@ fwd_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k,
     float* weights = reinterpret_cast<float*>(sv + kRows<KS> * pitch);
     const Place p = place_of_block(g, 0);
     const int h0 = na2d_ws(p.x0, g.W, KS), rows = na2d_ws(min(p.x0 + kTile, g.W) - 1, g.W, KS) + KS - h0;
-    copy_rows<T>(sk, sequence<T>(k, p), k.st, h0, rows, pieces, pitch);
+    copy_rows<T, 1>({sk}, {sequence<T>(k, p)}, {&k.st}, h0, rows, pieces, pitch);
     commit();
-    copy_rows<T>(sv, sequence<T>(v, p), v.st, h0, rows, pieces, pitch);
+    copy_rows<T, 1>({sv}, {sequence<T>(v, p)}, {&v.st}, h0, rows, pieces, pitch);
     commit();
     const na2d_tile::Strip w = na2d_tile::strip_at<KS>(p.t0, g.W);
     const int hx = w.start - h0;
@@ -278,9 +295,9 @@ dq_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand k, 
     float* weights = reinterpret_cast<float*>(sv + kRows<KS> * pitch);
     const Place p = place_of_block(g, unit0);
     const int h0 = na2d_ws(p.x0, g.W, KS), rows = na2d_ws(min(p.x0 + kTile, g.W) - 1, g.W, KS) + KS - h0;
-    copy_rows<T>(sv, sequence<T>(v, p), v.st, h0, rows, pieces, pitch);
+    copy_rows<T, 1>({sv}, {sequence<T>(v, p)}, {&v.st}, h0, rows, pieces, pitch);
     commit();
-    copy_rows<T>(sk, sequence<T>(k, p), k.st, h0, rows, pieces, pitch);
+    copy_rows<T, 1>({sk}, {sequence<T>(k, p)}, {&k.st}, h0, rows, pieces, pitch);
     commit();
     const na2d_tile::Strip w = na2d_tile::strip_at<KS>(p.t0, g.W);
     const int hx = w.start - h0;
@@ -413,8 +430,7 @@ key_kernel(const __grid_constant__ Operand q, const __grid_constant__ Operand d_
     float *weights_ds = reinterpret_cast<float*>(sg + kKeyRows<KS> * pitch), *weights_p = weights_ds + kStrips * kStrip;
     const Place p = place_of_block(g, unit0);
     const int h0 = na2d_bws(p.x0, KS), rows = na2d_bwe(min(p.x0 + kTile, g.W) - 1, g.W, KS) - h0;
-    copy_rows<T>(sq, sequence<T>(q, p), q.st, h0, rows, pieces, pitch);
-    copy_rows<T>(sg, sequence<T>(d_o, p), d_o.st, h0, rows, pieces, pitch);
+    copy_rows<T, 2>({sq, sg}, {sequence<T>(q, p), sequence<T>(d_o, p)}, {&q.st, &d_o.st}, h0, rows, pieces, pitch);
     commit();
     // This lane's key t: its weights from the strips of queries that see it, a float4 (four queries) each.
     const Met m = met_by<KS>(p.t0, g.W);

@@ -161,3 +161,18 @@ def test_1d_infinities_stay_in_their_windows():
     assert torch.equal((o2 != o).any(-1).any(0).any(0), (t - 77).abs() <= 6) and o2[:, :, 71:84].isinf().all()
     for got, want, near in zip(grads, clean, (0, 6, 6)):
         assert torch.equal(got[:, :, (t - 120).abs() > near], want[:, :, (t - 120).abs() > near])
+
+
+@pytest.mark.parametrize("dtype,pieces", [(torch.bfloat16, n) for n in (2, 3, 5, 7, 9, 11, 13, 14, 15, 16)] + [(torch.float32, n) for n in (3, 7, 11)])
+def test_1d_rows_of_every_number_of_pieces(dtype, pieces):
+    """Rows of 16-byte pieces whose number the threads of a block are no multiple of, in packed and in spaced sequences."""
+    C = pieces * 16 // dtype.itemsize
+    q, k, v, d_o = _inputs((2, 24, 261, C), dtype, pieces, C ** -0.5)
+    ro, rlse = orc.natten1d_fwd(q, k, v, 5)
+    want = (ro, rlse, *orc.natten1d_bwd(q, k, v, d_o, 5))
+    spaced = torch.stack([q, k, v], 3).to(DEV).unbind(3)
+    for qd, kd, vd in ([t.to(DEV) for t in (q, k, v)], spaced):
+        o, lse = na.natten1d_forward(qd, kd, vd, 5)
+        got = (o, lse, *na.natten1d_backward(qd, kd, vd, o, lse, d_o.to(DEV), 5))
+        for name, a, b in zip(("o", "lse", "dq", "dk", "dv"), got, want):
+            assert_close(a, b, torch.float32 if name == "lse" and dtype == torch.float32 else dtype, f"{name} {pieces}")
