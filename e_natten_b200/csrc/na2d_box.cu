@@ -59,7 +59,9 @@ template <int KS, int WHICH, bool FLAG> struct Tag {};
 
 // Channels that a block of the apply and key sum kernels takes, whose blocks need not take all of them.  `blocks` tiles on a GPU with room
 // for `per_sm` blocks an SM: a wave of k blocks an SM lasts about 0.73 + 0.27 k times as long as one block (measured with 1, 2 and 4 an
-// SM), and fetching the weights, which each block does, about as long as a chunk of channels.  4 x 4 x 64 x 64 x 128, window 5, pair: 512 tiles.
+// SM), and fetching the weights, which each block does, about as long as a chunk of channels.
+// One B200, all channels in a block against this split: backward of 1 x 4 x 33 x 40 x 48, window 5, 49 -> 37 us; the pair's apply of 4 x 4 x
+// 48 x 48 x 96, window 9, 49 -> 39 us.
 int channels_of_block(const Call& c, long long blocks, int per_sm) {
     const int sms = na2d_tc::sm_count(c.device), chunks = (c.g.C + kChunk - 1) / kChunk;
     float best = 0.f;

@@ -5,6 +5,7 @@
 // issue slots in the key sums.  Keeping P and dS (2 ks * (ks + 3) floats per pixel) costs less than the two score loops
 // that would form them again.  Measured on one B200 against the warp-per-pixel kernels, 4 x 4 x 256 x 256 x 128,
 // window 5, fp32: both halves 27.6 -> 2.24 ms; 4 x 8 x 4096 x 64, window 13, bf16, 1D: step 1.72 -> 0.29 ms.
+// (fp32 in 2D goes to na2d_box.cuh and 1D rows to na2d_line.cuh where rows start on 16-byte boundaries; these kernels keep the rest.)
 #pragma once
 
 #include "na2d_tile.cuh"

@@ -12,9 +12,10 @@
 // 13 (240 to 700 points each).  There the kernel chosen takes 1.00 (unfused pair 1.01) times the better one's time on
 // average, 1.2 times (pair 1.6) at worst; tiles alone took up to 3.0 (pair 6.3) times in fp32 and 7.5 times in 16 bits.
 //
-// The 1D constants are those of the tiled kernels also for the rows that na2d_line.cuh takes, where "tiles" means a kernel twice as
-// fast: such calls cross over later than they could.  The same goes for the fp32 2D calls that na2d_box.cuh takes.  One sequence of 64 channels, window 7, bf16, per pixel / na2d_line, us: forward 2048 tokens
-// 6.2 / 8.2, 4096 10.9 / 8.3, 8192 16.5 / 8.1; backward 1024 tokens 19.1 / 17.8, 4096 38.5 / 18.0.
+// The constants are those of the tiled kernels also for the 1D rows that na2d_line.cuh takes, where "tiles" means a kernel twice as fast,
+// and for the fp32 2D calls that na2d_box.cuh takes: such calls cross over later than they could.  One sequence of 64 channels, window 7,
+// bf16, per pixel / na2d_line, us: forward 2048 tokens 6.2 / 8.2, 4096 10.9 / 8.3, 8192 16.5 / 8.1; backward 1024 tokens 19.1 / 17.8,
+// 4096 38.5 / 18.0.
 #pragma once
 
 namespace na2d_tile {
