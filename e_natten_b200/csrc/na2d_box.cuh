@@ -625,7 +625,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const float4 l4 = sum_rows<S>(sum + a.strip * S::kKh * S::kTh + a.row + p);
         inv[p] = make_float4(1.f / l4.x, 1.f / l4.y, 1.f / l4.z, 1.f / l4.w);
     }
-    if (S::kHaloBuffers == 2 && g.C > kChunk && loads.last(3)) load_v(1);               // the sums have been read
+    // The exchange has been read, and the second halo comes in its place.  It was written with ordinary stores: each thread's fence puts
+    // those before the copy that the last warp asks for.
+    if (S::kHaloBuffers == 2 && g.C > kChunk) {
+        na2d_ptx::fence_proxy_async();
+        if (loads.last(3)) load_v(1);
+    }
     tile_apply<S, S::kHaloBuffers>(o, smem, loads, w, a, inv, t, g, ky0, kx0, 0, g.C, load_v);
     loads.drain();
 }
@@ -757,7 +762,10 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUt
         if (ds_out) store_band<S>(ds_out + place, d, s, slots);
     }
     if (d_q.ptr) {
-        if (S::kHaloBuffers == 2 && g.C > kChunk && loads.last(3)) load_k(1);           // the sums have been read
+        if (S::kHaloBuffers == 2 && g.C > kChunk) {                                     // the sums have been read (fwd_kernel says why the fence)
+            na2d_ptx::fence_proxy_async();
+            if (loads.last(3)) load_k(1);
+        }
         __syncthreads();
         float4 one[S::kRows];
 #pragma unroll

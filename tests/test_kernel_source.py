@@ -30,3 +30,13 @@ def test_a_wait_that_decides_a_branch_decides_it_for_its_warp(path):
     for call, heads in scopes_of(open(path).read(), r"\blt\.acquire(_warp)?\("):
         one_lane = any(re.search(r"\bif \(lane == 0\)\s*$", head) for head in heads)
         assert one_lane == (call == "lt.acquire(")
+
+
+def test_box_loads_over_ordinary_stores_come_behind_a_fence():
+    """The second halo of the box kernels lands where their row maxima and sums were written with ordinary stores; only a proxy fence
+    of the threads that wrote them orders those before the copy (the count of the warps does not)."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "na2d_box.cuh")).read())
+    places = [m.start() for m in re.finditer(r"\bloads\.last\(3\)", text)]
+    assert len(places) == 2                                       # fwd_kernel, dq_kernel
+    for at in places:
+        assert re.search(r"fence_proxy_async\(\);\s*if \($", text[:at])
