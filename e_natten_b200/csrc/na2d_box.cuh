@@ -114,11 +114,12 @@ struct Loads {
     uint64_t* bars;
     unsigned* done;
     WaitCtx wc;
-    uint32_t phases;              // parity of each barrier's next phase
+    uint32_t state;               // bits 0-3: parity of each barrier's next phase; 4-7: this thread started a load and has not seen it land,
+                                  // 8-11: which completes a phase of this parity
     bool gave_up;
     __device__ __forceinline__ explicit Loads(uint8_t* at, const ErrorState* errors)
         : bars(reinterpret_cast<uint64_t*>(at)), done(reinterpret_cast<unsigned*>(at + 32)), wc{reinterpret_cast<WaitState*>(at + 48)},
-          phases(0), gave_up(false) {
+          state(0), gave_up(false) {
         if (threadIdx.x == 0) {
             na2d_ptx::wait_state_init(wc.st, errors, na2d_ptx::kWaitLimitNs);
             for (int i = 0; i < kBuffers; ++i) {
@@ -128,13 +129,19 @@ struct Loads {
             na2d_ptx::mbar_fence_init();
         }
     }
-    __device__ __forceinline__ uint64_t* expect(int b, int bytes) const {
+    // The barrier for the buffer's next load, which expects so many bytes; null, and no load may start, once a wait of the block has given
+    // up: the barrier's phase may still be open then, and a second arrival in it would be an error of its own.  (A wait that gives up says
+    // so in the abort flag before its warp counts itself off the buffer, so that whoever loads next has seen it.)
+    __device__ __forceinline__ uint64_t* expect(int b, int bytes) {
+        if (na2d_ptx::ld_shared_u32(na2d_ptx::smem_u32(wc.st)) != 0) return nullptr;
+        state = (state & ~(256u << b)) | 16u << b | (state >> b & 1) << (8 + b);
         na2d_ptx::mbar_expect_tx(bars + b, bytes);
         return bars + b;
     }
     __device__ __forceinline__ void wait(int b) {
-        if (!na2d_ptx::mbar_wait(bars + b, phases >> b & 1, wc, na2d_ptx::kErrLoadWait)) gave_up = true;
-        phases ^= 1u << b;
+        if (!na2d_ptx::mbar_wait(bars + b, state >> b & 1, wc, na2d_ptx::kErrLoadWait)) gave_up = true;
+        if (!gave_up) state &= ~(16u << b);                // (afterwards parities say nothing: no load starts any more)
+        state ^= 1u << b;
     }
     // The warp has read the buffer; true in one thread of the last warp to say so.
     __device__ __forceinline__ bool last(int b) const {
@@ -145,12 +152,12 @@ struct Loads {
                      : "=r"(before) : "r"(na2d_ptx::smem_u32(done + b)), "r"(blockDim.x / 32 - 1) : "memory");
         return before == blockDim.x / 32 - 1;
     }
-    // After a wait that gave up: no load may land in shared memory that is another block's by then.  (Of the two phases of a barrier
-    // one is complete.)
+    // After a wait that gave up: waits once more, for about a millisecond at most, for the loads that this thread has started and not seen
+    // land, before its shared memory becomes another block's.  A load that another thread started is that one's to wait for.
     __device__ __forceinline__ void drain() const {
         if (!gave_up) return;
         for (int b = 0; b < kBuffers; ++b)
-            for (uint32_t parity = 0; parity < 2; ++parity) na2d_ptx::mbar_wait(bars + b, parity, wc, na2d_ptx::kErrLoadWait);
+            if (state >> b & 16u) na2d_ptx::mbar_wait(bars + b, state >> (8 + b) & 1, wc, na2d_ptx::kErrLoadWait);
     }
 };
 
@@ -550,11 +557,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     query_halo<S>(t, g, ky0, kx0);
     const int n = dot_chunks(g);
     auto load_v = [&](int i) {
-        na2d_ptx::tma_load_5d(smem + halo_at<S>(i), &tm_v, loads.expect(2 + halo_buffer<S>(i), kHaloBytes<S>), i * kChunk, kx0, ky0, t.n, t.b);
+        if (uint64_t* bar = loads.expect(2 + halo_buffer<S>(i), kHaloBytes<S>))
+            na2d_ptx::tma_load_5d(smem + halo_at<S>(i), &tm_v, bar, i * kChunk, kx0, ky0, t.n, t.b);
     };
     auto load_qk = [&](int i) {
         const int stage = (n - 1 - i) & 1;
-        load_dot<S>(&tm_q, &tm_k, smem + stage * S::kStage, loads.expect(stage, kDotBytes<S>), i, t, ky0, kx0);
+        if (uint64_t* bar = loads.expect(stage, kDotBytes<S>)) load_dot<S>(&tm_q, &tm_k, smem + stage * S::kStage, bar, i, t, ky0, kx0);
     };
     if (threadIdx.x == 0) {
         load_qk(0);
@@ -672,12 +680,15 @@ dq_kernel(const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUt
     query_halo<S>(t, g, ky0, kx0);
     const int n = dot_chunks(g), all = 2 * n;
     auto load_k = [&](int i) {
-        na2d_ptx::tma_load_5d(smem + halo_at<S>(i), &tm_k32, loads.expect(2 + halo_buffer<S>(i), kHaloBytes<S>), i * kChunk, kx0, ky0, t.n, t.b);
+        if (uint64_t* bar = loads.expect(2 + halo_buffer<S>(i), kHaloBytes<S>))
+            na2d_ptx::tma_load_5d(smem + halo_at<S>(i), &tm_k32, bar, i * kChunk, kx0, ky0, t.n, t.b);
     };
     auto load_pair = [&](int i) {
         const int stage = (all - 1 - i) & 1;
-        if (i < n) load_dot<S>(&tm_do, &tm_v, smem + stage * S::kStage, loads.expect(stage, kDotBytes<S>), i, t, ky0, kx0);
-        else load_dot<S>(&tm_q, &tm_k, smem + stage * S::kStage, loads.expect(stage, kDotBytes<S>), i - n, t, ky0, kx0);
+        if (uint64_t* bar = loads.expect(stage, kDotBytes<S>)) {
+            if (i < n) load_dot<S>(&tm_do, &tm_v, smem + stage * S::kStage, bar, i, t, ky0, kx0);
+            else load_dot<S>(&tm_q, &tm_k, smem + stage * S::kStage, bar, i - n, t, ky0, kx0);
+        }
     };
     auto next = [&](int i) {
         if (i + 2 < all) load_pair(i + 2);
@@ -813,7 +824,7 @@ window_dot_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     const int n = dot_chunks(g);
     auto load = [&](int i) {
         const int stage = (n - 1 - i) & 1;
-        load_dot<S>(&tm_x, &tm_y, smem + stage * S::kStage, loads.expect(stage, kDotBytes<S>), i, t, ky0, kx0);
+        if (uint64_t* bar = loads.expect(stage, kDotBytes<S>)) load_dot<S>(&tm_x, &tm_y, smem + stage * S::kStage, bar, i, t, ky0, kx0);
     };
     if (threadIdx.x == 0) {
         load(0);
@@ -859,7 +870,9 @@ window_apply_kernel(const float* __restrict__ attn, const __grid_constant__ CUte
     int ky0, kx0;
     query_halo<S>(t, g, ky0, kx0);
     const int ch0 = blockIdx.z * span;
-    auto load = [&](int i) { na2d_ptx::tma_load_5d(smem, &tm_y, loads.expect(2, kHaloBytes<S>), ch0 + i * kChunk, kx0, ky0, t.n, t.b); };
+    auto load = [&](int i) {
+        if (uint64_t* bar = loads.expect(2, kHaloBytes<S>)) na2d_ptx::tma_load_5d(smem, &tm_y, bar, ch0 + i * kChunk, kx0, ky0, t.n, t.b);
+    };
     if (threadIdx.x == 0) load(0);
     for (int row = 0; row < t.rows; ++row) {
         const float* from = attn + dense_row<KS>(t, g, row);

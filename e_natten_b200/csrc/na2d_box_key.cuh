@@ -114,6 +114,7 @@ key_sum_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant_
     const int box_w = wide ? K::kWideW : S::kBoxW, box_h = wide ? K::kWideH : S::kHaloH;
     auto load = [&](int c0, int row) {
         uint64_t* bar = loads.expect(0, box_w * box_h * kPixel);
+        if (!bar) return;
         // (each map by its name: one chosen through a pointer may be copied to where TMA cannot read it)
         if (blockIdx.y == 0) {
             if (!wide) na2d_ptx::tma_load_5d(smem, &tm_x0, bar, c0, qx0, row, t.n, t.b);
