@@ -114,12 +114,11 @@ struct Loads {
     uint64_t* bars;
     unsigned* done;
     WaitCtx wc;
-    uint32_t state;               // bits 0-3: parity of each barrier's next phase; 4-7: this thread started a load and has not seen it land,
-                                  // 8-11: which completes a phase of this parity
-    bool gave_up;
+    uint32_t phases;              // parity of each barrier's next phase
+    bool gave_up;                 // a wait of this thread
     __device__ __forceinline__ explicit Loads(uint8_t* at, const ErrorState* errors)
         : bars(reinterpret_cast<uint64_t*>(at)), done(reinterpret_cast<unsigned*>(at + 32)), wc{reinterpret_cast<WaitState*>(at + 48)},
-          state(0), gave_up(false) {
+          phases(0), gave_up(false) {
         if (threadIdx.x == 0) {
             na2d_ptx::wait_state_init(wc.st, errors, na2d_ptx::kWaitLimitNs);
             for (int i = 0; i < kBuffers; ++i) {
@@ -129,19 +128,18 @@ struct Loads {
             na2d_ptx::mbar_fence_init();
         }
     }
-    // The barrier for the buffer's next load, which expects so many bytes; null, and no load may start, once a wait of the block has given
-    // up: the barrier's phase may still be open then, and a second arrival in it would be an error of its own.  (A wait that gives up says
-    // so in the abort flag before its warp counts itself off the buffer, so that whoever loads next has seen it.)
-    __device__ __forceinline__ uint64_t* expect(int b, int bytes) {
-        if (na2d_ptx::ld_shared_u32(na2d_ptx::smem_u32(wc.st)) != 0) return nullptr;
-        state = (state & ~(256u << b)) | 16u << b | (state >> b & 1) << (8 + b);
+    // The barrier for the buffer's next load, which expects so many bytes; null, and no load may start, once a wait of this thread has given
+    // up: the phase that it waited for may still be open, and a second arrival in it would be an error of its own.  A phase that this thread
+    // has seen complete is over for all, also where others have given up on it.  (The block's abort flag says less, and reading it
+    // here, between a buffer's last reader and its next load, took 4 to 10 % of the kernels' time.)
+    __device__ __forceinline__ uint64_t* expect(int b, int bytes) const {
+        if (gave_up) return nullptr;
         na2d_ptx::mbar_expect_tx(bars + b, bytes);
         return bars + b;
     }
     __device__ __forceinline__ void wait(int b) {
-        if (!na2d_ptx::mbar_wait(bars + b, state >> b & 1, wc, na2d_ptx::kErrLoadWait)) gave_up = true;
-        if (!gave_up) state &= ~(16u << b);                // (afterwards parities say nothing: no load starts any more)
-        state ^= 1u << b;
+        if (!na2d_ptx::mbar_wait(bars + b, phases >> b & 1, wc, na2d_ptx::kErrLoadWait)) gave_up = true;
+        phases ^= 1u << b;
     }
     // The warp has read the buffer; true in one thread of the last warp to say so.
     __device__ __forceinline__ bool last(int b) const {
@@ -152,12 +150,13 @@ struct Loads {
                      : "=r"(before) : "r"(na2d_ptx::smem_u32(done + b)), "r"(blockDim.x / 32 - 1) : "memory");
         return before == blockDim.x / 32 - 1;
     }
-    // After a wait that gave up: waits once more, for about a millisecond at most, for the loads that this thread has started and not seen
-    // land, before its shared memory becomes another block's.  A load that another thread started is that one's to wait for.
+    // After a wait that gave up: waits once more, about a millisecond for each barrier at most, before the block's shared memory becomes
+    // another one's.  A load that this thread has started and not seen land is in its barrier's open phase, since none follows it; of the two
+    // parities the other one's phase is over.  A load that another thread started is that one's to wait for.
     __device__ __forceinline__ void drain() const {
         if (!gave_up) return;
         for (int b = 0; b < kBuffers; ++b)
-            if (state >> b & 16u) na2d_ptx::mbar_wait(bars + b, state >> (8 + b) & 1, wc, na2d_ptx::kErrLoadWait);
+            for (uint32_t parity = 0; parity < 2; ++parity) na2d_ptx::mbar_wait(bars + b, parity, wc, na2d_ptx::kErrLoadWait);
     }
 };
 

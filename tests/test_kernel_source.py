@@ -44,8 +44,8 @@ def test_box_loads_over_ordinary_stores_come_behind_a_fence():
 
 @pytest.mark.parametrize("name", ["na2d_box.cuh", "na2d_box_key.cuh"])
 def test_box_loads_stop_when_a_wait_has_given_up(name):
-    """Loads::expect says whether a load may still start (no wait of the block has given up, and so the barrier's last phase is over); no
-    barrier is armed and no load issued without asking it."""
+    """Loads::expect says whether a load may still start (no wait of the thread that asks has given up, and so the barrier's last phase is
+    over); no barrier is armed and no load issued without asking it."""
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
     asked = re.findall(r"(if \()?uint64_t\* bar = loads\.expect\([^;{]*?\)(\)|;\s*if \(!bar\) return;)", text)
     assert len(asked) == len(re.findall(r"\bexpect\(", text)) - text.count("uint64_t* expect(") > 0
@@ -53,4 +53,4 @@ def test_box_loads_stop_when_a_wait_has_given_up(name):
     assert all("bar" in call.split(",")[2] for call in re.findall(r"tma_load_5d\(([^;]*)\);", text))
     for call, heads in scopes_of(text, r"mbar_expect_tx\("):
         assert "uint64_t* expect(" in heads[-1]
-        assert re.search(r"if \(na2d_ptx::ld_shared_u32\(na2d_ptx::smem_u32\(wc\.st\)\) != 0\) return nullptr;", text)
+        assert re.search(r"if \(gave_up\) return nullptr;\s*na2d_ptx::$", text[:text.index(call)])
