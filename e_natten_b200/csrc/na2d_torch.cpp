@@ -180,8 +180,13 @@ bool takes(const Tensor& q, const Tensor& k, const Tensor& v, int64_t kernel_siz
 
 template <bool ONE_D>
 struct Attention : ag::Function<Attention<ONE_D>> {
+    // A wait that gave up in a kernel of an earlier call surfaces here, without a sync.
+    static void poll(const Tensor& q) {
+        if constexpr (!ONE_D) check(abi.poll(q.device().index(), nullptr));
+    }
     static Tensor forward(ag::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, int64_t kernel_size,
                           double scale) {
+        poll(q);
         auto [status, o, lse] = ::forward(q, k, v, kernel_size, NA2D_PATH_AUTO, scale);
         check(status);
         ctx->save_for_backward({q, k, v, o, lse});
@@ -211,11 +216,8 @@ struct Attention : ag::Function<Attention<ONE_D>> {
                                            "need_dkdv"_a = need_dk || need_dv, "scale"_a = scale)
                                           .template cast<std::tuple<MaybeTensor, MaybeTensor, MaybeTensor>>();
         } else {
-            if constexpr (!ONE_D) {
-                // a wait that gave up in an earlier kernel surfaces here, without a sync
-                check(abi.poll(q.device().index(), c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
-                o = saved[3];
-            }
+            poll(q);
+            if constexpr (!ONE_D) o = saved[3];
             std::tie(status, d_q, d_k, d_v) = ::backward(q, k, v, o, saved[4], d_o, kernel_size, NA2D_PATH_AUTO, scale,
                                                          ctx->needs_input_grad(0), need_dk || need_dv);
         }

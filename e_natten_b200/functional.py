@@ -205,7 +205,7 @@ def poll_kernels(device) -> None:
     Never waits for the GPU: it looks at a host word that such a kernel writes to (``na2d_poll``), so an
     error surfaces one call late."""
     dev = torch.device(device)
-    _lib.check(_lib.lib.na2d_poll(dev.index or 0, _stream(dev)))
+    _lib.check(_lib.lib.na2d_poll(dev.index or 0, None))
 
 
 class Natten2d(torch.autograd.Function):
@@ -216,6 +216,7 @@ class Natten2d(torch.autograd.Function):
     def forward(ctx, q, k, v, kernel_size=7, scale=None):
         scale = 1.0 if scale is None else float(scale)
         o, lse = natten2d_forward(q, k, v, kernel_size, scale=scale)
+        poll_kernels(o.device)            # a wait that gave up in an earlier kernel surfaces here, without a sync
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.kernel_size, ctx.scale = kernel_size, scale
         ctx.mark_non_differentiable(lse)
@@ -227,7 +228,7 @@ class Natten2d(torch.autograd.Function):
         q, k, v, o, lse = ctx.saved_tensors
         if grad_output is None:               # an undefined gradient (a node above returned None) counts as zeros
             grad_output = torch.zeros_like(q, memory_format=torch.contiguous_format)
-        poll_kernels(q.device)            # a wait that gave up in an earlier kernel surfaces here, without a sync
+        poll_kernels(q.device)
         need_dq = ctx.needs_input_grad[0]
         need_dkdv = ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
         d_q, d_k, d_v = natten2d_backward(q, k, v, o, lse, grad_output, ctx.kernel_size,
@@ -338,6 +339,7 @@ class _Natten2dQK(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, kernel_size, dilation):
         _check_pair(q, k, kernel_size, dilation)
+        poll_kernels(q.device)            # as in Natten2d: the pair's fp32 kernels have waits, too
         q, k = q.contiguous(), k.contiguous()
         B, N, H, W, _ = q.shape
         attn = torch.empty((B, N, H, W, kernel_size * kernel_size), dtype=q.dtype, device=q.device)
@@ -349,6 +351,7 @@ class _Natten2dQK(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_attn):
         q, k = ctx.saved_tensors
+        poll_kernels(q.device)
         d_attn = d_attn.contiguous()
         d_q, d_k = torch.empty_like(q), torch.empty_like(k)
         _lib.check(_lib.lib.na2d_qk_backward(_ptr(q), _ptr(k), _ptr(d_attn), _ptr(d_q), _ptr(d_k),
@@ -360,6 +363,7 @@ class _Natten2dAV(torch.autograd.Function):
     @staticmethod
     def forward(ctx, attn, v, kernel_size, dilation):
         _check_pair(attn, v, kernel_size, dilation)
+        poll_kernels(v.device)
         attn, v = attn.contiguous(), v.contiguous()
         if attn.shape[:4] != v.shape[:4] or attn.shape[4] != kernel_size * kernel_size:
             raise ValueError("attn must be (B, heads, H, W, kernel_size**2) for v of (B, heads, H, W, C)")
@@ -372,6 +376,7 @@ class _Natten2dAV(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out):
         attn, v = ctx.saved_tensors
+        poll_kernels(v.device)
         d_out = d_out.contiguous()
         d_attn, d_v = torch.empty_like(attn), torch.empty_like(v)
         _lib.check(_lib.lib.na2d_av_backward(_ptr(attn), _ptr(v), _ptr(d_out), _ptr(d_attn), _ptr(d_v),

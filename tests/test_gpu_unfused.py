@@ -71,3 +71,32 @@ def test_unfused_errors():
         na.natten2dqk(q, q, 4, 1)
     with pytest.raises(ValueError):
         na.natten2dav(torch.zeros(1, 1, 8, 8, 9, device=DEV), q, 5, 1)     # attn of another kernel size
+
+
+def test_a_wait_that_gave_up_is_raised_by_the_next_call():
+    """The pair's fp32 kernels have waits, and so has every inference call of the fused operator: an error that an earlier kernel reported
+    is raised by the next of these calls, whichever it is, once."""
+    import ctypes as C
+    from e_natten_b200 import _lib
+    na.check_kernels(DEV)
+    q, k, v = (t.to(DEV).requires_grad_() for t in make_inputs((1, 2, 12, 12, 32), torch.float32, 2)[:3])
+    attn = na.natten2dqk(q, k, 5)
+    out = na.natten2dav(attn, v, 5)
+
+    def inference(dtype, scale=None):
+        with torch.no_grad():
+            return na.natten2d(q.to(dtype), k.to(dtype), v.to(dtype), 5, scale)
+
+    calls = [lambda: na.natten2dqk(q, k, 5), lambda: na.natten2dav(attn, v, 5),
+             lambda: torch.autograd.grad(attn, (q, k), torch.ones_like(attn), retain_graph=True),
+             lambda: torch.autograd.grad(out, v, torch.ones_like(out), retain_graph=True),
+             lambda: inference(torch.float32), lambda: inference(torch.bfloat16),
+             lambda: inference(torch.float32, 1)]                 # (an int: through the Python function)
+    for i, call in enumerate(calls):
+        _lib.check(_lib.lib.na2d_selftest_wait_timeout(0, C.c_void_p(torch.cuda.current_stream().cuda_stream), 1000))
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            call()
+            pytest.fail(f"call {i} did not look")
+        call()
+    na.check_kernels(DEV)
