@@ -37,7 +37,7 @@ Operand operand(const Tensor& t) { return Operand{t.ptr, t.st, 1}; }
 
 // Map of boxes of channels x w x h pixels of a tensor of `rows` image rows; false where there is none.
 bool map(CUtensorMap* m, const Call& c, const Tensor& t, int rows, int w, int h, int channels) {
-    return na2d_tc::make_map(m, na2d_tc::TensorArg{t.ptr, t.st}, NA2D_F32, c.g.BN / c.g.N, c.g.N, rows, c.g.W, c.g.C, w, h, channels, true) == NA2D_OK;
+    return na2d_tc::try_map(m, na2d_tc::TensorArg{t.ptr, t.st}, NA2D_F32, c.g.BN / c.g.N, c.g.N, rows, c.g.W, c.g.C, w, h, channels, true);
 }
 template <typename S> bool map_own(CUtensorMap* m, const Call& c, const Tensor& t) { return map(m, c, t, c.g.Hq, S::kOwnW, S::kTh, kDotC); }
 template <typename S> bool map_dot(CUtensorMap* m, const Call& c, const Tensor& t) { return map(m, c, t, c.g.Hkv, S::kBoxW, S::kHaloH, kDotC); }

@@ -433,6 +433,15 @@ inline int make_map(CUtensorMap* map, const TensorArg& t, int dtype, int B, int 
     return NA2D_OK;
 }
 
+// make_map for a launcher whose call other kernels can take: false where there is no map, and then no driver result is left that the
+// report of a later failure would take for its own.
+template <typename... A>
+inline bool try_map(CUtensorMap* map, A... args) {
+    if (make_map(map, args...) == NA2D_OK) return true;
+    last_driver_result() = 0;
+    return false;
+}
+
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per kernel and device instead of on every
 // launch.  `done` is a per-kernel bit set (one bit per device ordinal).
 template <typename K>
