@@ -36,6 +36,7 @@ int main() {
     EXPECT(na2d_tc::try_map(&map, a, NA2D_F32, 1, 2, 32, 128, 64, 17, 8, 16, true) && map.opaque[0] == 4096);
     EXPECT(na2d_tc::try_map(&map, b, NA2D_F32, 1, 2, 32, 128, 64, 17, 8, 16, true) && map.opaque[0] == 8192);
     EXPECT(na2d_tc::make_map(&map, a, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16) == NA2D_OK && map.opaque[0] == 4096);
+    EXPECT(na2d_tc::make_map(&map, a, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16) == NA2D_OK && calls == 6);     // nothing is kept by address
     return 0;
 }
 """
