@@ -162,7 +162,7 @@ Turns workspace_turns(const Na2dGeom& g, long long floats) {
 int NA2D_NAME(forward)(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,
                        const Tensor& o, float* lse) {
 #if NA2D_TILE_DT == 0
-    if (int rc = 0; in_boxes(g, at, na2d_box::query_side_pays(g), {&q, &k, &v, &o}, &rc, [&](const na2d_box::Call& c) { return na2d_box::forward(c, q, k, v, o, lse); })) return rc;
+    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kForward, g), {&q, &k, &v, &o}, &rc, [&](const na2d_box::Call& c) { return na2d_box::forward(c, q, k, v, o, lse); })) return rc;
 #endif
     return by_window(g, [&](auto shape) -> int {
         using S = decltype(shape);
@@ -182,7 +182,7 @@ int NA2D_NAME(forward)(const Na2dGeom& g, const Place& at, const Tensor& q, cons
 int NA2D_NAME(backward_dq)(const Na2dGeom& g, const Place& at, const Tensor& q, const Tensor& k, const Tensor& v,
                            const Tensor& d_o, const Tensor& d_q, const float* lse, float* delta, float* row_factor) {
 #if NA2D_TILE_DT == 0
-    if (int rc = 0; in_boxes(g, at, na2d_box::query_side_pays(g), {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
+    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kQueryHalf, g), {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
             const int rows = (g.Hq + 7) / 8;
             return na2d_box::query_half(c, q, k, v, d_o, d_q, lse, delta, row_factor, nullptr, nullptr, g.BN, na2d_box::Rows{0, 0, rows, rows});
         }))
@@ -248,7 +248,7 @@ int NA2D_NAME(backward)(const Na2dGeom& g, const Place& at, const Tensor& q, con
                 const auto query_half = [&]() -> int {
 #if NA2D_TILE_DT == 0
                     const na2d_box::Rows rows{query_band.unit0, query_band.row0, query_band.rows, query_band.ring};
-                    if (int rc = 0; in_boxes(g, at, na2d_box::query_side_pays(g), {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
+                    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kQueryHalf, g), {&q, &k, &v, &d_o, &d_q}, &rc, [&](const na2d_box::Call& c) {
                             return na2d_box::query_half(c, q, k, v, d_o, d_q, lse, delta, nullptr, p, ds, units, rows);
                         }))
                         return rc;
@@ -260,7 +260,7 @@ int NA2D_NAME(backward)(const Na2dGeom& g, const Place& at, const Tensor& q, con
                 const auto key_half = [&]() -> int {
 #if NA2D_TILE_DT == 0
                     const na2d_box::Rows rows{key_band.unit0, key_band.row0, key_band.rows, key_band.ring};
-                    if (int rc = 0; in_boxes(g, at, na2d_box::key_side_pays(g), {&q, &d_o, &d_k, &d_v}, &rc, [&](const na2d_box::Call& c) {
+                    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kKeySum, g), {&q, &d_o, &d_k, &d_v}, &rc, [&](const na2d_box::Call& c) {
                             return na2d_box::key_half(c, q, d_o, d_k, d_v, p, ds, units, rows);
                         }))
                         return rc;
@@ -285,7 +285,7 @@ int NA2D_NAME(backward)(const Na2dGeom& g, const Place& at, const Tensor& q, con
 
 int NA2D_NAME(pair_dot)(const Na2dGeom& g, const Place& at, const Tensor& x, const Tensor& y, void* attn) {
 #if NA2D_TILE_DT == 0
-    if (int rc = 0; in_boxes(g, at, na2d_box::query_side_pays(g), {&x, &y}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_dot(c, x, y, (float*)attn); })) return rc;
+    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kDot, g), {&x, &y}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_dot(c, x, y, (float*)attn); })) return rc;
 #endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
@@ -299,7 +299,7 @@ int NA2D_NAME(pair_dot)(const Na2dGeom& g, const Place& at, const Tensor& x, con
 
 int NA2D_NAME(pair_apply)(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& y, const Tensor& out) {
 #if NA2D_TILE_DT == 0
-    if (int rc = 0; in_boxes(g, at, na2d_box::query_side_pays(g), {&y, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_apply(c, (const float*)attn, y, out); })) return rc;
+    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kApply, g), {&y, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_apply(c, (const float*)attn, y, out); })) return rc;
 #endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
@@ -312,7 +312,7 @@ int NA2D_NAME(pair_apply)(const Na2dGeom& g, const Place& at, const void* attn, 
 
 int NA2D_NAME(pair_inverse)(const Na2dGeom& g, const Place& at, const void* attn, const Tensor& x, const Tensor& out) {
 #if NA2D_TILE_DT == 0
-    if (int rc = 0; in_boxes(g, at, na2d_box::key_side_pays(g), {&x, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_inverse(c, (const float*)attn, x, out); })) return rc;
+    if (int rc = 0; in_boxes(g, at, na2d_box::pays(na2d_box::Work::kKeySum, g), {&x, &out}, &rc, [&](const na2d_box::Call& c) { return na2d_box::pair_inverse(c, (const float*)attn, x, out); })) return rc;
 #endif
     return by_size<false>(g, [&](auto shape) -> int {
         using S = decltype(shape);
