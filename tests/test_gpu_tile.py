@@ -83,11 +83,20 @@ def test_packed_views_equal_dense(ks, H, W, Cd):
         assert torch.equal(a, b)
 
 
+def _off_boundary(t):
+    """The same tensor, its rows starting 4 bytes past a 16-byte boundary: fp32 operands that stay with these kernels in 2D."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    return flat[1:].view(t.shape).copy_(t)
+
+
 @pytest.mark.parametrize("ks,H,W", [(5, 20, 21), (9, 12, 33)])
-def test_workspace_of_any_size(ks, H, W):
+@pytest.mark.parametrize("off", [False, True])
+def test_workspace_of_any_size(ks, H, W, off):
     """All units at once, one unit at a time, and no workspace (the key half forms the weights again)."""
     B, N, Cd = 1, _units(H, W, ks, torch.float32), 64
     q, k, v, d_o = _device(*make_inputs((B, N, H, W, Cd), torch.float32, 77))
+    if off:
+        q, k, v, d_o = (_off_boundary(t) for t in (q, k, v, d_o))
     o, lse = na.natten2d_forward(q, k, v, ks, scale=0.125)
     want = orc.natten2d_bwd(q.cpu(), k.cpu(), v.cpu(), d_o.cpu(), ks, scale=0.125)
     delta = torch.empty_like(lse)
@@ -128,13 +137,17 @@ def _backward(q, k, v, o, lse, d_o, ks, scale, bytes_of, path="auto"):
     return grads, na.launch_count() - before
 
 
-@pytest.mark.parametrize("ks,H,W,dtype", [(3, 41, 9, torch.float32), (5, 67, 18, torch.bfloat16), (9, 50, 19, torch.float32),
-                                          (13, 75, 14, torch.float32)])
-def test_workspace_of_some_rows(ks, H, W, dtype):
+@pytest.mark.parametrize("ks,H,W,dtype,off", [(3, 41, 9, torch.float32, False), (5, 67, 18, torch.bfloat16, False),
+                                              (9, 50, 19, torch.float32, False), (13, 75, 14, torch.float32, False),
+                                              (3, 41, 9, torch.float32, True), (5, 67, 18, torch.float32, True),
+                                              (9, 50, 19, torch.float32, True), (13, 75, 14, torch.float32, True)])
+def test_workspace_of_some_rows(ks, H, W, dtype, off):
     """A workspace below one image: rows of tiles are used again as the key half is done with them."""
     Cd, scale = 40, 0.2
     N = _units(H, W, ks, dtype)
     q, k, v, d_o = _device(*make_inputs((1, N, H, W, Cd), dtype, 78))
+    if off:
+        q, k, v, d_o = (_off_boundary(t) for t in (q, k, v, d_o))
     o, lse = na.natten2d_forward(q, k, v, ks, path="simt", scale=scale)
     run = lambda bytes_of: _backward(q, k, v, o, lse, d_o, ks, scale, bytes_of, path="simt")
     whole, launches = run(lambda n: n)
@@ -187,11 +200,16 @@ def test_short_memory():
 
 @pytest.mark.parametrize("ks", [3, 5, 9])
 @pytest.mark.parametrize("at", [(0, 0), (7, 7), (8, 16), (23, 30)])
-def test_infinities_stay_in_their_windows(ks, at):
+@pytest.mark.parametrize("off", [False, True])
+def test_infinities_stay_in_their_windows(ks, at, off):
     """An infinite value (and an infinite gradient) reaches the pixels whose windows hold it and no others."""
     H, W = 24, 31
     q, k, v, d_o = _device(*make_inputs((1, _units(H, W, ks, torch.float32), H, W, 32), torch.float32, 5, q_scale=0.2))
-    v2, g2 = v.clone(), d_o.clone()
+    clone = torch.clone
+    if off:
+        q, k, v, d_o = (_off_boundary(t) for t in (q, k, v, d_o))
+        clone = _off_boundary
+    v2, g2 = clone(v), clone(d_o)
     v2[0, 0, at[0], at[1]] = float("inf")
     g2[0, 0, at[0], at[1]] = float("inf")
     o, lse = na.natten2d_forward(q, k, v, ks)

@@ -63,6 +63,20 @@ def test_scores_and_apply_against_oracle(shape, ks, dtype):
     assert_close(vd.grad, vr.grad, dtype, "apply dv")
 
 
+@pytest.mark.parametrize("ks,H,W,Cd", [(3, 21, 18, 30), (5, 17, 23, 66), (9, 19, 26, 30), (13, 27, 14, 66)])
+def test_pair_of_many_pixels_and_ragged_rows(ks, H, W, Cd):
+    """fp32 rows that are no whole 16-byte pieces, of one channel chunk and of several: the tiled kernels."""
+    units = -(-20000 // (H * W))
+    q, k, v, d_o = make_inputs((1, units, H, W, Cd), torch.float32, ks + Cd, q_scale=Cd ** -0.5)
+    qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
+    attn = na.natten2dqk(qd, kd, ks, 1)
+    out = na.natten2dav(torch.softmax(attn, -1), vd, ks, 1)
+    got = (attn.detach(), out.detach(), *torch.autograd.grad(out, (qd, kd, vd), d_o.to(DEV)))
+    want = (orc.natten2d_qk(q.double(), k.double(), ks), orc.natten2d_fwd(q, k, v, ks, scale=1.0)[0], *orc.natten2d_bwd(q, k, v, d_o, ks, scale=1.0))
+    for a, c, what in zip(got, want, ("scores", "o", "dq", "dk", "dv")):
+        assert_close(a, c, torch.float32, f"{what} ks={ks} {H}x{W}x{Cd}")
+
+
 def test_unfused_errors():
     q = torch.zeros(1, 1, 8, 8, 32, device=DEV)
     with pytest.raises(ValueError):
