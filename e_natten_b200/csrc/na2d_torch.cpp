@@ -40,6 +40,9 @@ void bind_abi(uintptr_t forward, uintptr_t backward, uintptr_t backward_workspac
     abi.poll = reinterpret_cast<int (*)(int, void*)>(poll);
 }
 
+int poll_device(int device) { return abi.poll(device, nullptr); }
+uintptr_t current_stream(int device) { return reinterpret_cast<uintptr_t>(c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()); }
+
 // Whether the kernels can read t in place: contiguous channels, no broadcast dimension, and for 16-bit types (the
 // tensor-core path's TMA tensor maps) a base and strides on 16-byte boundaries.
 bool kernel_ready(const Tensor& t) {
@@ -182,7 +185,7 @@ template <bool ONE_D>
 struct Attention : ag::Function<Attention<ONE_D>> {
     // A wait that gave up in a kernel of an earlier call surfaces here, without a sync.
     static void poll(const Tensor& q) {
-        if constexpr (!ONE_D) check(abi.poll(q.device().index(), nullptr));
+        if constexpr (!ONE_D) check(poll_device(q.device().index()));
     }
     static Tensor forward(ag::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, int64_t kernel_size,
                           double scale) {
@@ -324,6 +327,8 @@ pybind11::object attention(const pybind11::object& q_in, const pybind11::object&
 PYBIND11_MODULE(_na2d_torch, m) {
     m.attr("built_for") = NA2D_EXT_TAG;         // looked for in the file by build.py
     m.def("bind_abi", &bind_abi);
+    m.def("poll", &poll_device);
+    m.def("stream", &current_stream);
     m.def("kernel_ready", &kernel_ready);
     m.def("strides", [](const Tensor& t) {      // (batch, heads, row, column), as they go into na2d_tensor
         const na2d_tensor d = describe(t);

@@ -205,7 +205,13 @@ def poll_kernels(device) -> None:
     Never waits for the GPU: it looks at a host word that such a kernel writes to (``na2d_poll``), so an
     error surfaces one call late."""
     dev = torch.device(device)
-    _lib.check(_lib.lib.na2d_poll(dev.index or 0, None))
+    _poll(dev.index or 0)
+
+
+def _poll(index: int) -> None:
+    status = torch_ext.poll(index)        # (through ctypes, with a torch.device made for it, 2 us more per call)
+    if status:
+        _lib.check(status)
 
 
 class Natten2d(torch.autograd.Function):
@@ -323,7 +329,8 @@ def natten1d(q, k, v, kernel_size=7, scale=None):
 # ---- the unfused pair (scores, apply) with the call shape of natten.functional --------------------------------
 def _pair_args(t, kernel_size):
     B, N, H, W, Cd = t.shape
-    return (B, N, H, W, Cd, kernel_size, _DTYPES[t.dtype], t.device.index, _stream(t.device))
+    device = t.device.index               # (torch.cuda.current_stream takes 2 us longer to name the stream)
+    return (B, N, H, W, Cd, kernel_size, _DTYPES[t.dtype], device, torch_ext.stream(device))
 
 
 def _check_pair(x, y, kernel_size, dilation):
@@ -339,7 +346,7 @@ class _Natten2dQK(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, kernel_size, dilation):
         _check_pair(q, k, kernel_size, dilation)
-        poll_kernels(q.device)            # as in Natten2d: the pair's fp32 kernels have waits, too
+        _poll(q.device.index)             # as in Natten2d: the pair's fp32 kernels have waits, too
         q, k = q.contiguous(), k.contiguous()
         B, N, H, W, _ = q.shape
         attn = torch.empty((B, N, H, W, kernel_size * kernel_size), dtype=q.dtype, device=q.device)
@@ -351,7 +358,7 @@ class _Natten2dQK(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_attn):
         q, k = ctx.saved_tensors
-        poll_kernels(q.device)
+        _poll(q.device.index)
         d_attn = d_attn.contiguous()
         d_q, d_k = torch.empty_like(q), torch.empty_like(k)
         _lib.check(_lib.lib.na2d_qk_backward(_ptr(q), _ptr(k), _ptr(d_attn), _ptr(d_q), _ptr(d_k),
@@ -363,7 +370,7 @@ class _Natten2dAV(torch.autograd.Function):
     @staticmethod
     def forward(ctx, attn, v, kernel_size, dilation):
         _check_pair(attn, v, kernel_size, dilation)
-        poll_kernels(v.device)
+        _poll(v.device.index)
         attn, v = attn.contiguous(), v.contiguous()
         if attn.shape[:4] != v.shape[:4] or attn.shape[4] != kernel_size * kernel_size:
             raise ValueError("attn must be (B, heads, H, W, kernel_size**2) for v of (B, heads, H, W, C)")
@@ -376,7 +383,7 @@ class _Natten2dAV(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out):
         attn, v = ctx.saved_tensors
-        poll_kernels(v.device)
+        _poll(v.device.index)
         d_out = d_out.contiguous()
         d_attn, d_v = torch.empty_like(attn), torch.empty_like(v)
         _lib.check(_lib.lib.na2d_av_backward(_ptr(attn), _ptr(v), _ptr(d_out), _ptr(d_attn), _ptr(d_v),
