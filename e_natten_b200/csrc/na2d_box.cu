@@ -58,19 +58,28 @@ int launch(const Call& c, void (*kernel)(P...), dim3 grid, int threads, int smem
 template <int KS, int WHICH, bool FLAG> struct Tag {};
 
 // Channels that a block of the apply and key sum kernels takes, whose blocks need not take all of them.  `blocks` tiles on a GPU with room
-// for `per_sm` blocks an SM: a wave of k blocks an SM lasts about 0.73 + 0.27 k times as long as one block (measured with 1, 2 and 4 an
-// SM), and fetching the weights, which each block does, about as long as a chunk of channels.
-// One B200, all channels in a block against this split: backward of 1 x 4 x 33 x 40 x 48, window 5, 49 -> 37 us; the pair's apply of 4 x 4 x
-// 48 x 48 x 96, window 9, 49 -> 39 us.
-int channels_of_block(const Call& c, long long blocks, int per_sm) {
+// for `per_sm` blocks an SM.  A wave of k blocks an SM lasts 0.73 + 0.27 k times as long as one block, or k * alone times where that is more: the
+// part of an SM's throughput that a block uses which has it to itself.  Fetching the weights, which each block does, takes as long as `fetch` chunks
+// of channels.  Fitted to times of all splits of 2 to 4 chunks, 20 to 1536 tiles, windows 3 to 13, one B200: on average the split taken is within
+// 1 % of the best one's time for the apply, 2 to 7 % for the pair's key sums and 1 to 3 % for the backward's.  One chunk's time for
+// fetching, and no `alone`, gave 0 to 2, 9 to 18 and 4 to 7 %, and calls slower than the tiled kernels: apply of 6 x 50 x 52 x 64,
+// window 9, 18.5 -> 22.5 us, now 18.5; apply and key sums of 6 x 64 x 64 x 128, window 7, 100 -> 106, now 82.  Left: apply of 150 tiles, two more than
+// SMs, at 0.77 (window 11) and 0.86 (9) of the tiled kernels' speed.
+struct Split {
+    float fetch, alone;
+};
+template <typename S> constexpr Split kApplySplit{0.75f, S::kKs <= 5 ? 0.4f : S::kKs == 9 ? 0.55f : 0.8f};
+template <typename S> constexpr Split kKeySplit{0.1f, S::kKs <= 5 ? 0.3f : S::kKs == 9 ? 0.5f : 0.85f};
+int channels_of_block(const Call& c, const Split& split, long long blocks, int per_sm) {
     const int sms = na2d_tc::sm_count(c.device), chunks = (c.g.C + kChunk - 1) / kChunk;
+    const auto wave = [&](long long k) { return fmaxf(0.73f + 0.27f * (float)k, split.alone * (float)k); };
     float best = 0.f;
     int span = chunks;
     for (int parts = 1; parts <= chunks; ++parts) {
-        const int per = (chunks + parts - 1) / parts;
-        const long long all = blocks * ((chunks + per - 1) / per), slots = (long long)sms * per_sm, rest = all % slots;
-        const float waves = (float)(all / slots) * (0.73f + 0.27f * per_sm) + (rest ? 0.73f + 0.27f * (float)((rest + sms - 1) / sms) : 0.f);
-        const float time = waves * (float)(1 + per);
+        const int per = (chunks + parts - 1) / parts, used = (chunks + per - 1) / per;
+        const long long all = blocks * used, slots = (long long)sms * per_sm, rest = all % slots;
+        const float waves = (float)(all / slots) * wave(per_sm) + (rest ? wave((rest + sms - 1) / sms) : 0.f);
+        const float time = waves * (split.fetch + (float)chunks / (float)used);
         if (parts == 1 || time < 0.97f * best) {
             best = time;
             span = per;
@@ -125,7 +134,7 @@ int key_half(const Call& c, const Tensor& q, const Tensor& d_o, const Tensor& d_
         CUtensorMap xq, wq, xg, wg;
         if (!map_key<S>(&xq, c, q, false) || !map_key<S>(&wq, c, q, true) || !map_key<S>(&xg, c, d_o, false) || !map_key<S>(&wg, c, d_o, true))
             return kNoMap;
-        const int span = channels_of_block(c, 2ll * n, K::kBlocks);
+        const int span = channels_of_block(c, kKeySplit<S>, 2ll * n, K::kBlocks);
         return launch<Tag<S::kKs, 2, true>>(c, key_sum_kernel<true, S::kKs>, dim3(n, 2, (c.g.C + span - 1) / span), K::kThreads, K::kSmem, xq, wq,
                                             xg, wg, KeyOut{ds, operand(d_k)}, KeyOut{p, operand(d_v)}, span, c.errors,
                                             Band{rows.unit0, rows.row0, rows.rows, rows.ring}, c.g);
@@ -155,7 +164,7 @@ int pair_apply(const Call& c, const float* attn, const Tensor& y, const Tensor& 
         CUtensorMap my;
         if (!map_halo<S>(&my, c, y)) return kNoMap;
         using P = PairShape<S>;
-        const int span = channels_of_block(c, n, P::kApplyBlocks);
+        const int span = channels_of_block(c, kApplySplit<S>, n, P::kApplyBlocks);
         return launch<Tag<S::kKs, 4, true>>(c, window_apply_kernel<S::kKs>, dim3(n, 1, (c.g.C + span - 1) / span), P::kApplyThreads, P::kApplySmem,
                                             attn, my, operand(out), span, c.errors, c.g);
     });
@@ -171,7 +180,7 @@ int pair_inverse(const Call& c, const float* attn, const Tensor& x, const Tensor
         CUtensorMap mx, mw;
         if (!map_key<S>(&mx, c, x, false) || !map_key<S>(&mw, c, x, true)) return kNoMap;
         const KeyOut sum{attn, operand(out)};
-        const int span = channels_of_block(c, n, K::kBlocks);
+        const int span = channels_of_block(c, kKeySplit<S>, n, K::kBlocks);
         return launch<Tag<S::kKs, 5, true>>(c, key_sum_kernel<false, S::kKs>, dim3(n, 1, (c.g.C + span - 1) / span), K::kThreads, K::kSmem, mx, mw,
                                             mx, mw, sum, sum, span, c.errors,
                                             Band{0, 0, rows, rows}, c.g);
