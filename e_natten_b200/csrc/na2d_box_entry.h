@@ -46,13 +46,13 @@ inline bool takes(const Na2dGeom& g, std::initializer_list<const na2d_tile::Tens
 //   query half, others        0.83 - 1.07    0.87 - 1.06    0.95 - 1.10    1.05 - 1.14
 // (others: 28 x 40, 39 x 45, 50 x 52, 100 x 90, 200 x 260; 64 and 128 channels.)  The pair's scores 1.00 to 1.34 everywhere; its apply 1.00 to 2.2 up
 // to 98 tiles, whose channels are split over blocks, from 120 on 0.82 to 1.03 (147 tiles of 50 x 52 1.07 and 1.18).  At window 11 the forward
-// is at 0.96 to 1.00 from 192 to 256 tiles, two blocks for some SMs and no second wave, and at 1.01 or more elsewhere.
+// is at 0.96 to 1.00 where 192 to 256 tiles, two blocks for some SMs and no second wave, are all whole, and at 1.01 to 1.2 elsewhere.
 using na2d_tile::Work;
 inline bool pays(Work work, const Na2dGeom& g) {
     if (work == Work::kKeySum) return g.ks != 7 || g.W >= 16;
     if (g.ks < 11) return true;
     const long long tiles = (long long)g.BN * ((g.Hg + 7) / 8) * ((g.W + 7) / 8);
-    if (g.ks == 11) return g.W >= 16 && (work != Work::kForward || tiles <= 148 || tiles > 296);
+    if (g.ks == 11) return g.W >= 16 && (work != Work::kForward || g.Hg % 8 != 0 || g.W % 8 != 0 || tiles <= 148 || tiles > 296);
     if (g.W < 36) return false;
     return work == Work::kForward ? tiles >= 5 * 148 : work == Work::kQueryHalf ? tiles >= 12 * 148 : work != Work::kApply || tiles <= 100;
 }
