@@ -36,7 +36,33 @@ int main() {
     EXPECT(na2d_tc::try_map(&map, a, NA2D_F32, 1, 2, 32, 128, 64, 17, 8, 16, true) && map.opaque[0] == 4096);
     EXPECT(na2d_tc::try_map(&map, b, NA2D_F32, 1, 2, 32, 128, 64, 17, 8, 16, true) && map.opaque[0] == 8192);
     EXPECT(na2d_tc::make_map(&map, a, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16) == NA2D_OK && map.opaque[0] == 4096);
-    EXPECT(na2d_tc::make_map(&map, a, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16) == NA2D_OK && calls == 6);     // nothing is kept by address
+    EXPECT(na2d_tc::make_map(&map, a, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16) == NA2D_OK && map.opaque[0] == 4096 && calls == 5);   // kept
+    // a model of ten layers, three steps on the same buffers: nearly all of its maps are still there
+    calls = 0;
+    for (int step = 0; step < 3; ++step)
+        for (int layer = 0; layer < 10; ++layer)
+            for (int operand = 0; operand < 12; ++operand) {
+                const size_t at = (size_t)(1 + layer * 12 + operand) << 21;
+                const na2d_tc::TensorArg x{(void*)at, {1 << 20, 1 << 18, 1 << 13, 64}};
+                EXPECT(na2d_tc::make_map(&map, x, NA2D_BF16, 1, 2, 32, 128, 64, 8, 16 + operand % 3) == NA2D_OK && map.opaque[0] == at);
+            }
+    EXPECT(calls >= 120 && calls < 180);
+    // whatever differs in a description makes another map of it
+    calls = 0;
+    const Na2dStride st{1 << 24, 1 << 20, 1 << 14, 128};
+    const na2d_tc::TensorArg y{(void*)(1 << 20), st};
+    const int base[9] = {NA2D_BF16, 2, 3, 40, 50, 64, 8, 16, 32};
+    for (int i = -1; i < 15; ++i) {
+        int n[9];
+        for (int j = 0; j < 9; ++j) n[j] = base[j] + (i == j ? (j == 0 ? NA2D_F16 - NA2D_BF16 : 8) : 0);
+        na2d_tc::TensorArg x = y;
+        if (i == 9) x.ptr = (void*)((1 << 20) + 16);
+        if (i == 10) x.st.b += 8;
+        if (i == 11) x.st.n += 8;
+        if (i == 12) x.st.h += 8;
+        if (i == 13) x.st.w += 8;
+        EXPECT(na2d_tc::make_map(&map, x, n[0], n[1], n[2], n[3], n[4], n[5], n[6], n[7], n[8], i == 14) == NA2D_OK && calls == i + 2);
+    }
     return 0;
 }
 """
