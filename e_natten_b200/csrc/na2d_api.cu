@@ -368,15 +368,18 @@ na2d_tc::TensorArg targ(const Tensor& t) { return na2d_tc::TensorArg{t.ptr, t.st
 
 // Whether the kernels of a tensor-core call are launched to overlap the end of the kernel before them.  Blocks that wait hold SMs, so not
 // for calls that leave some to other streams' kernels (a margin, a band of rows beside its exchange).  And up to kOverlapPixels alone, from
-// window 7 on: a launch hides about 2 us, but kernels of some rounds of tiles last up to 4 us longer when their blocks start as SMs fall
-// free (their places on the chip change, so L2's far half is the likely reason).  A step, one B200, bf16, cold L2, us without and with:
+// window 7 on: a launch hides about 2 us, a quarter of the smallest calls' time, 1 to 3 % at the line and at most 1 % at twice as many
+// pixels, but kernels of some rounds of tiles last up to 4 us longer when their blocks start as SMs fall free (their places on the
+// chip change, so L2's far half is the likely reason).  A step, one B200, bf16, cold L2, us without and with:
 //   pixels            8 K - 64 K    125 K - 131 K   200 K         262 K - 280 K   520 K
 //   28 x 28 x 64, 13  166.9 157.7   287.7 276.5     398.3 385.0   525.2 510.1     986.1 976.9
 //   100^2 x 64, 9     109.6 102.3   152.6 145.4     224.3 221.2   298.0 294.9     513.0 511.9
 //   56 x 56 x 32, 7   74.8 67.6     117.5 110.5     164.9 161.8   203.6 196.7     369.7 366.7
 //   48 x 48 x 128, 13 171.0 165.9   281.6 278.5     414.9 414.7   510.9 506.0     951.4 950.2
 // Replayed from a graph launches lie closer, and the line is at half: 100^2 x 64, window 9, L2 warm 92.4 90.4, 132.1 131.8, 202.9 209.1.
-// Window 5 as a graph loses from 64 K pixels on (64 x 64 x 128: 72.2 82.5, 122.3 136.8), and 1024^2 x 128, window 13, 17.3 17.6 ms.
+// Windows 3 and 5 in a stream, cold L2, 1.00 to 1.04 times as fast, but 5 as a graph loses from 64 K pixels on (64 x 64 x 128: 72.2 82.5,
+// 122.3 136.8), and 1024^2 x 128, window 13, 17.3 17.6 ms.  What it costs: four streams at once, each with steps of its own of 100 K to 175 K
+// pixels, are 1 to 2 % slower in all (236.1 241.6, 334.5 339.7 us a step), since a block that waits takes the place of another stream's.
 constexpr long long kOverlapPixels = 1 << 18;
 bool overlaps(const Problem& p) {
     const Na2dGeom& g = p.g;

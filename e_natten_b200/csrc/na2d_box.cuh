@@ -269,8 +269,9 @@ __device__ __forceinline__ DotItem score_item(const Tile& t, const Na2dGeom& g, 
     return d;
 }
 
-// acc[r][i] += own pixel r . halo column i of the strip over a stage, or (N = KS) member i of its window row, eight channels at a time: even and odd channels in the two lanes of a register pair, four products of a lane
-// summed first and added as one number: five instructions where eight multiply-adds would stand.
+// acc[r][i] += own pixel r . halo column i of the strip over a stage, or (N = KS) member i of its window row, eight channels at a time:
+// even and odd channels in the two lanes of a register pair, four products of a lane summed first and added as one number: five
+// instructions where eight multiply-adds would stand.
 template <typename S, bool REGULAR, typename A, int N>
 __device__ __forceinline__ void dot_staged(A (&acc)[kR][N], const uint8_t* stage, const DotItem& d) {
     const int own = d.row * S::kOwnW + kR * d.strip, halo = d.hy * S::kBoxW + d.hx;

@@ -5,7 +5,7 @@
 
 namespace na2d_launch {
 
-// Launches a kernel that calls na2d_ptx::after_previous_grid() before it touches global memory.  `overlap`: its blocks may start once the
+// Launches a kernel that calls na2d_ptx::after_previous_grid() before it touches what kernels write.  `overlap`: its blocks may start once the
 // kernel before it in the stream lets them (na2d_ptx::next_grid_may_start; any other kernel does by ending), and set themselves up while
 // the last blocks of that one run.
 template <typename... P, typename... A>

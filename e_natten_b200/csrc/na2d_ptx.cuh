@@ -74,8 +74,8 @@ __device__ __forceinline__ void wait_state_init(WaitState* st, const ErrorState*
 }
 
 // For kernels launched with na2d_launch::launch.  after_previous_grid: waits until the kernel before this one in the stream has ended and
-// its writes are visible; before the first access to global memory and before TMEM is taken, which that kernel's blocks may still have to
-// take.  next_grid_may_start: lets the blocks of the kernel behind start once every block of this one has come here; after TMEM is taken,
+// its writes are visible; before the first access to global memory but the error state, which is written once, ahead of any launch, and
+// before TMEM is taken, which that kernel's blocks may still have to take.  next_grid_may_start: lets the blocks of the kernel behind start once every block of this one has come here; after TMEM is taken,
 // since those blocks may take it before they wait.
 __device__ __forceinline__ void after_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

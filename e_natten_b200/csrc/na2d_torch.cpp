@@ -158,7 +158,7 @@ std::tuple<int, MaybeTensor, MaybeTensor, MaybeTensor> backward(const Tensor& q_
 
 // ---- native autograd functions -----------------------------------------------------------------------------------
 // Natten2d.apply(...)[0] and Natten1d.apply(...) of functional.py without the interpreter between autograd and the calls above:
-// a step of 1 x 2 x 16 x 16 x 32, window 5, fp32, whose kernels take 43 us, takes 85 us instead of 114 (the poll without a copy is
+// a step of 1 x 2 x 16 x 16 x 32, window 5, fp32, whose kernels took 43 us (39 now), took 85 us instead of 114 (the poll without a copy is
 // part of that), one of 4 x 4 x 32 x 32 x 128, bf16, 81 instead of 113.  They save the same tensors in the same order and
 // return the same gradients.
 
