@@ -22,8 +22,8 @@
 // 248 / 334, 7 462 / 466, 9 832 / 794, 13 2214 / 1713.
 //
 // What bounds it: latencies (eight to sixteen warps an SM issue in half of the cycles) and the FMA pipe.  Against the tiled key sums,
-// both sums, us: 4 x 8 x 28 x 30 x 64, window 5 49 -> 33, 9 105 -> 92, 13 210 -> 187; 2 x 200 x 260 x 64, window 5 82 -> 58, 9 165 -> 139, 13 363 -> 290;
-// with the dense weights of the pair, 4 x 4 x 64 x 64 x 128, window 5, each 74 -> 62.
+// both sums, us: 4 x 8 x 28 x 30 x 64, window 5 49 -> 32, 9 107 -> 87, 13 211 -> 186; 2 x 200 x 260 x 64, window 5 82 -> 59, 9 164 -> 140, 13 363 -> 290;
+// with the dense weights of the pair, 4 x 4 x 64 x 64 x 128, window 5, each 72 -> 55.
 #pragma once
 
 #include "na2d_box.cuh"

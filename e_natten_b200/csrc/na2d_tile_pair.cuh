@@ -1,6 +1,6 @@
 // Tiled CUDA-core kernels of the unfused pair (scores, apply); its key-side gradients are key sums.
 // Measured on one B200 against the warp-per-pixel kernels: step of 4 x 4 x 64 x 64 x 128, window 5, fp32
-// 0.80 -> 0.43 ms, the softmax between the two calls included.  (fp32 rows that start on 16-byte boundaries go to na2d_box.cuh: 0.29 ms.)
+// 0.80 -> 0.43 ms, the softmax between the two calls included.  (fp32 rows that start on 16-byte boundaries go to na2d_box.cuh: 0.28 ms.)
 #pragma once
 
 #include "na2d_tile.cuh"

@@ -48,11 +48,11 @@ def test_step_against_oracle_and_tiles(ks, H, W, Cd):
     na.check_kernels()
 
 
-@pytest.mark.parametrize("Cd", [20, 68])
-def test_window_13_of_many_tiles(Cd):
+@pytest.mark.parametrize("H,W,Cd,tiles", [(17, 37, 68, 740), (15, 36, 96, 296), (14, 40, 20, 296)])
+def test_window_13_of_many_tiles(H, W, Cd, tiles):
     """So many tiles that the query side of the largest window goes to the boxes, too."""
-    ks, H, W = 13, 17, 37
-    units, few = -(-1776 // (3 * 5)), 5
+    ks, few = 13, 5
+    units = tiles // (-(-H // 8) * 5) + 1
     q, k, v, d_o = (t.to(DEV) for t in make_inputs((1, units, H, W, Cd), torch.float32, Cd))
     got = _step(q, k, v, d_o, ks, Cd ** -0.5)
     tiles = _step(*(_off_boundary(t) for t in (q, k, v, d_o)), ks, Cd ** -0.5)
