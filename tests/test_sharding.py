@@ -112,6 +112,8 @@ def _lonely_worker(rank, world, port, result):
         result.put("no error")
     except Exception as exc:                          # noqa: BLE001 - any error from the transport is the point
         result.put("error: " + type(exc).__name__)
+    result.close()                                    # the queue's thread has written the answer before the process ends
+    result.join_thread()
     os._exit(0)
 
 
